@@ -6,6 +6,7 @@
 #include "conv_dw_halo.cuh"
 #include "conv_tapstack.cuh"
 #include "winograd.cuh"
+#include "gemm_f32.cuh"
 #include "host_common.h"
 
 #include <nvtx3/nvToolsExt.h>   // header-only: resolves a profiler's injection library at run time, no link dependency
@@ -1555,6 +1556,55 @@ static int launch_dx_col2im(DeviceCtx* c, const AlphaConvShape* s, const float* 
     return check_launch("col2im_gather_kernel");
 }
 
+// ---- deltaX in fp32: every stride, filter and channel count -------------------------------------------
+//
+// What the tensor-core paths leave (OC % 8 != 0 at stride 1, OC % 32 != 0 under a stride) and ALPHA_ALGO_SIMT.  A launch of
+// fewer CTAs than SMs whose reduction is long (a classifier's 2762 x 53 layer: eight row tiles) is cut into up to 16 parts
+// that are added in order; without scratch for them (stream capture, a caller's small workspace) it runs unsplit.
+// 50 x 35 x 29, 100 -> 36 channels, 3x3: 1.21 ms with one thread per element, 0.18 ms here; 13 x 15 x 15, 636 -> 648, 1x1: 0.96
+// and 0.12 ms; 944 x 2764 x 56: 0.50 and 0.11 ms.
+static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream)
+{
+    const long long rows = (long long)s->N * ((s->IH + s->sh - 1) / s->sh) * ((s->IW + s->sw - 1) / s->sw);
+    const int nsh = s->sh < s->IH ? s->sh : s->IH, nsw = s->sw < s->IW ? s->sw : s->IW;   // phases that own a pixel
+    const long long phases = (long long)nsh * nsw;
+    const int sms = sm_budget(c);
+    const GemmTile t = pick_gemm_tile(rows, s->IC, phases, sms);
+    const long long gx = (rows + t.bm - 1) / t.bm, gy = (s->IC + t.bn - 1) / t.bn, ctas = gx * gy * phases;
+    DxGemm g{};
+    g.dY = dY; g.W = W; g.out = dX;
+    g.N = s->N; g.IH = s->IH; g.IW = s->IW; g.IC = s->IC; g.FH = s->FH; g.FW = s->FW; g.OH = s->OH; g.OW = s->OW; g.OC = s->OC;
+    g.sh = s->sh; g.sw = s->sw; g.ph = s->ph; g.pw = s->pw; g.nsw = nsw;
+    g.kt = (s->OC + kGemmBK - 1) / kGemmBK;
+    g.by_kt = fast_div(g.kt);
+    g.size = (size_t)s->N * s->IH * s->IW * s->IC;
+    g.ksplit = 1;
+    const long long its = (long long)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * g.kt;
+    if (ctas < sms && its >= 8) {
+        long long ks = 2LL * sms / ctas;
+        if (ks > its / 4) ks = its / 4;
+        if (ks > 16) ks = 16;
+        float* ws = nullptr;
+        if (ks > 1 && get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws) == ALPHA_OK) { g.ksplit = (int)ks; g.out = ws; }
+    }
+    const long long nz = phases * g.ksplit;
+    for (long long z0 = 0; z0 < nz; z0 += 65535) {
+        g.z0 = (int)z0;
+        const unsigned z = (unsigned)(nz - z0 < 65535 ? nz - z0 : 65535);
+        if (!t_dry) launch_gemm_f32(g, t, dim3((unsigned)gx, (unsigned)gy, z), stream);
+        note_launch("simt");
+    }
+    int rc = check_launch("gemm_f32_kernel");
+    if (rc || g.ksplit == 1) return rc;
+    const size_t n4 = g.size / 4;
+    size_t blocks = (n4 + 255) / 256;
+    if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
+    if (!t_dry) splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(g.out), n4, g.ksplit, nullptr, 1, 0, 0.f,
+                                                               reinterpret_cast<float4*>(dX));
+    note_launch("simt");
+    return check_launch("splitk_reduce_kernel");
+}
+
 // ---- deltaW, halo-tile kernel (strides 1 and 2): plan and launch -----------------------------------
 
 template <int FW_T, int R_T, int CW_T, bool STR_T = false>
@@ -2420,10 +2470,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
         rc = launch_dx_phases(c, s, deltaY, W, deltaX, cur_mode3x(), stream);
         if (rc != 1) return rc;
     }
-    const size_t total = (size_t)s->N * s->IH * s->IW * s->IC;
-    if (!t_dry) conv_dx_simt<<<simt_grid(total, c->sm_count), 256, 0, stream>>>(deltaY, W, deltaX, to_dev_shape(s));
-    note_launch("simt");
-    return check_launch("conv_dx_simt");
+    return launch_dx_f32(c, s, deltaY, W, deltaX, stream);
 }
 
 int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* deltaY, float* deltaW,

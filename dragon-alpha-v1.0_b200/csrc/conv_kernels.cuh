@@ -978,39 +978,6 @@ __global__ void conv_fwd_simt(const float* __restrict__ X, const float* __restri
     }
 }
 
-// One thread per (n, ih, iw, ic); gathers the taps whose stride phase matches, no atomics.
-__global__ void conv_dx_simt(const float* __restrict__ dY, const float* __restrict__ W,
-                             float* __restrict__ dX, ConvShape s)
-{
-    const size_t total = static_cast<size_t>(s.N) * s.IH * s.IW * s.IC;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const int ic = static_cast<int>(i % s.IC);
-        size_t t = i / s.IC;
-        const int iw = static_cast<int>(t % s.IW); t /= s.IW;
-        const int ih = static_cast<int>(t % s.IH);
-        const int n = static_cast<int>(t / s.IH);
-        float v = 0.f;
-        for (int fh = 0; fh < s.FH; ++fh) {
-            const int a = ih + s.ph - fh;
-            if (a < 0 || a % s.sh != 0) continue;
-            const int oh = a / s.sh;
-            if (oh >= s.OH) continue;
-            for (int fw = 0; fw < s.FW; ++fw) {
-                const int b = iw + s.pw - fw;
-                if (b < 0 || b % s.sw != 0) continue;
-                const int ow = b / s.sw;
-                if (ow >= s.OW) continue;
-                const float* dy = dY + ((static_cast<size_t>(n) * s.OH + oh) * s.OW + ow) * s.OC;
-                const float* w = W + (static_cast<size_t>(fh) * s.FW + fw) * s.IC + ic;
-                const size_t wstride = static_cast<size_t>(s.FH) * s.FW * s.IC;
-                for (int oc = 0; oc < s.OC; ++oc) v = fmaf(dy[oc], w[oc * wstride], v);
-            }
-        }
-        dX[i] = v;
-    }
-}
-
 // One block per deltaW element (oc, fh, fw, ic): 128 threads stride over the pixels, then a
 // fixed-shape tree sum in shared memory (deterministic).
 __global__ void __launch_bounds__(128)

@@ -9,6 +9,7 @@
 // pitches) run a plain fp32 kernel.
 #include "../../include/alpha_conv_b200.h"
 #include "host_common.h"
+#include "gemm_f32.cuh"
 
 namespace alpha {
 int launch_buf_summary(cudaStream_t stream, const float* buf, float* deltaW, int part, size_t sizeW);
@@ -107,6 +108,24 @@ int launch_bmm_simt(const float* A, const float* B, float* C, int Batch, int N, 
     return ALPHA_OK;
 }
 
+// The three forms on the register-tiled fp32 kernel: pitches that are multiples of 4 and 16-byte aligned matrices (what the
+// engine's tensors have); other layouts stay on bmm_simt_kernel.
+template <bool A_KC, bool B_KC>
+int launch_bmm_f32(const float* A, const float* B, float* C, int Batch, int N, int M, int K, int lda, int ldb, int ldc, size_t strA,
+                   size_t strB, size_t strC, alpha_stream_t stream)
+{
+    const GemmTile t = pick_gemm_tile(N, M, Batch, 148);
+    for (int b0 = 0; b0 < Batch; b0 += 65535) {   // gridDim.z limit
+        const int nb = Batch - b0 < 65535 ? Batch - b0 : 65535;
+        const BatchGemm<A_KC, B_KC> g{A + b0 * strA, B + b0 * strB, C + b0 * strC, N, M, K, lda, ldb, ldc, strA, strB, strC};
+        launch_gemm_f32(g, t, dim3((M + t.bn - 1) / t.bn, (N + t.bm - 1) / t.bm, nb), static_cast<cudaStream_t>(stream));
+    }
+    note_launch("bmm_simt");
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "gemm_f32_kernel launch failed: %s", cudaGetErrorString(e));
+    return ALPHA_OK;
+}
+
 int check_batch(const char* what, const void* A, const void* B, const void* C, int Batch, int d0, int d1, int d2, int d3)
 {
     if (!A || !B || !C) return fail(ALPHA_E_ARG, "%s: null matrix pointer", what);
@@ -115,6 +134,10 @@ int check_batch(const char* what, const void* A, const void* B, const void* C, i
     return ALPHA_OK;
 }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+inline bool vec_ok(const void* A, const void* B, const void* C, int lda, int ldb, int ldc, int rows)
+{
+    return aligned16(A) && aligned16(B) && aligned16(C) && ((lda | ldb | ldc) & 3) == 0 && rows <= 65535 * 64;   // gridDim.y limit
+}
 
 int check_dims(const char* what, const void* A, const void* B, const void* C, int N, int M, int K)
 {
@@ -182,6 +205,8 @@ int alpha_batchMatMul(const float* A, const float* B, float* C, int Batch, int N
         rc = launch_bmm_tensor(0, A, B, C, Batch, N, M, BK, static_cast<cudaStream_t>(stream));
         if (rc != 1) return rc;
     }
+    if (vec_ok(A, B, C, AK, M, M, N))
+        return launch_bmm_f32<true, false>(A, B, C, Batch, N, M, BK, AK, M, M, (size_t)N * AK, (size_t)BK * M, (size_t)N * M, stream);
     const BmmStrides st{(long long)N * AK, (long long)BK * M, (long long)N * M, AK, 1, M, 1, M};
     return launch_bmm_simt(A, B, C, Batch, N, M, BK, st, stream);
 }
@@ -196,6 +221,8 @@ int alpha_batchMatMulT1(const float* A, const float* B, float* C, int Batch, int
         rc = launch_bmm_tensor(1, A, B, C, Batch, CN, M, K, static_cast<cudaStream_t>(stream));
         if (rc != 1) return rc;
     }
+    if (vec_ok(A, B, C, AN, M, M, CN))
+        return launch_bmm_f32<false, false>(A, B, C, Batch, CN, M, K, AN, M, M, (size_t)K * AN, (size_t)K * M, (size_t)CN * M, stream);
     const BmmStrides st{(long long)K * AN, (long long)K * M, (long long)CN * M, 1, AN, M, 1, M};
     return launch_bmm_simt(A, B, C, Batch, CN, M, K, st, stream);
 }
@@ -210,6 +237,8 @@ int alpha_batchMatMulT2(const float* A, const float* B, float* C, int Batch, int
         rc = launch_bmm_tensor(2, A, B, C, Batch, N, BM, K, static_cast<cudaStream_t>(stream));
         if (rc != 1) return rc;
     }
+    if (vec_ok(A, B, C, K, K, CM, N))
+        return launch_bmm_f32<true, true>(A, B, C, Batch, N, BM, K, K, K, CM, (size_t)N * K, (size_t)BM * K, (size_t)N * CM, stream);
     const BmmStrides st{(long long)N * K, (long long)BM * K, (long long)N * CM, K, 1, 1, K, CM};
     return launch_bmm_simt(A, B, C, Batch, N, BM, K, st, stream);
 }

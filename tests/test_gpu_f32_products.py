@@ -1,0 +1,82 @@
+"""The register-tiled fp32 kernel: deltaX of channel counts the tensor-core paths do not take and batched products of ragged
+sizes, within the bound of an fp32 sum of K products in any order, K * 2^-24 * sum |product|."""
+import numpy as np
+import pytest
+
+from helpers import gen, out_hw
+
+pytestmark = pytest.mark.gpu
+
+# N, IH, IW, IC, OC, F, s, p: column tiles of 32, 64 and 128, row remainders, phases without a tap, split reductions
+SHAPES = [
+    (2, 35, 29, 36, 100, 3, 1, 1), (1, 9, 9, 4, 12, 3, 1, 1), (3, 16, 16, 132, 20, 3, 2, 1), (2, 15, 17, 64, 68, 1, 2, 0), (2, 9, 11, 40, 44, 2, 3, 0),
+    (1, 6, 6, 260, 36, 4, 2, 1), (5, 1, 4, 52, 2764, 1, 1, 0), (1, 7, 5, 8, 4, 7, 2, 3), (2, 20, 20, 128, 36, 5, 1, 2), (40, 30, 30, 128, 44, 3, 2, 1),
+]
+
+
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+def test_fp32_deltaX(pkg, oracle_mod, shape, mode):
+    import torch
+    engine = pkg.submodule("engine")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+    N, IH, IW, IC, OC, F, s, p = shape
+    OH, OW = out_hw(IH, IW, F, F, s, s, p, p)
+    IH, IW = (OH - 1) * s + F - 2 * p, (OW - 1) * s + F - 2 * p
+    rng = np.random.default_rng(IC * 1000 + OC)
+    W, dY = gen((OC, F, F, IC), "u11", rng), gen((N, OH, OW, OC), "n01", rng)
+    got = eng.dconv3D_deltaX(torch.from_numpy(dY).cuda(), torch.from_numpy(W).cuda(), IH, IW, s, s, p, p).cpu().numpy()
+    ref, mag = oracle_mod.deconv3D_deltaX_f64(dY, W, IH, IW, s, s, p, p, threads=8)
+    if OC % 32 and (s > 1 or OC % 8):
+        assert pkg.submodule("lib").last_algo() == "simt"
+        assert (np.abs(got - ref) <= F * F * OC * 2.0 ** -24 * mag).all()
+
+
+@pytest.mark.parametrize("dims", [(2, 1, 1, 1), (3, 20, 20, 20), (2, 65, 33, 17), (2, 130, 129, 50), (1, 264, 425, 220), (5, 88, 79, 24), (2, 64, 128, 36)], ids=str)
+def test_fp32_batched_products(pkg, dims):
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math="tf32"))
+    Bt, N, M, K = dims
+    g = torch.Generator().manual_seed(Bt + N + M + K)
+    A, B = torch.randn((Bt, N, K), generator=g), torch.randn((Bt, K, M), generator=g)
+    ref, mag = A.double() @ B.double(), A.double().abs() @ B.double().abs()
+    for op, a, b in (("batchMatMul", A, B), ("batchMatMulT1", A.transpose(1, 2).contiguous(), B), ("batchMatMulT2", A, B.transpose(1, 2).contiguous())):
+        y = getattr(eng, op)(a.cuda(), b.cuda()).cpu().double()
+        assert lib.last_algo() == "bmm_simt"
+        assert bool(((y - ref).abs() <= K * 2.0 ** -24 * mag).all()), op
+
+
+def test_padding_columns_and_neighbours_do_not_leak(pkg):
+    """Row padding of A full of NaN, batch entries beside each other: only the first K columns count, only N x M is written."""
+    import ctypes as C
+    import torch
+    lib = pkg.submodule("lib")
+    L = lib.load()
+    Bt, N, M, K, AK = 3, 21, 36, 18, 20
+    A = torch.full((Bt, N, AK), float("nan"), device="cuda")
+    A[..., :K] = torch.randn((Bt, N, K), device="cuda")
+    B = torch.randn((Bt, K, M), device="cuda")
+    out = torch.full((Bt * N * M + 64,), 7.0, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    lib.check(L.alpha_engine_batchMatMul(p(out), p(A), p(B), Bt, N, M, K, AK, C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    got = out[:Bt * N * M].view(Bt, N, M).double()
+    want = A[..., :K].double() @ B.double()
+    assert bool(((got - want).abs() <= K * 2.0 ** -24 * (A[..., :K].double().abs() @ B.double().abs())).all())
+    assert bool((out[Bt * N * M:] == 7.0).all())
+
+
+def test_reduction_split_needs_no_scratch(pkg):
+    """A call that never needed scratch still runs in a stream capture, which may not allocate any."""
+    import torch
+    eng = pkg.submodule("engine").Engine()
+    dY, W = torch.randn((8, 1, 1, 2764), device="cuda"), torch.randn((2764, 1, 1, 52), device="cuda")
+    want = eng.dconv3D_deltaX(dY, W, 1, 1, 1, 1, 0, 0)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        got = eng.dconv3D_deltaX(dY, W, 1, 1, 1, 1, 0, 0)
+    graph.replay()
+    torch.cuda.synchronize()
+    mag = dY.double().abs().reshape(8, -1) @ W.double().abs().reshape(2764, 52)
+    assert bool(((got.double() - want.double()).abs().reshape(8, 52) <= 2 * 2764 * 2.0 ** -24 * mag).all())

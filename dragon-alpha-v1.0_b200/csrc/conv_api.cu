@@ -64,6 +64,7 @@ enum Opt {
     OPT_SKINNY, OPT_HALO_DEEP, OPT_HALO_SPLITB, OPT_NVTX, OPT_DW_LANES, OPT_HALO_TAPSTACK, OPT_HALO_FLAT32,
     OPT_DW_STRIDED,     // 0 = strided deltaW on the split-K im2col kernel only
     OPT_DW_TAPGROUPS,   // 0 = a CTA always owns a whole filter row, 2 = rows of more than three taps always split
+    OPT_HALO_PAD,       // channels that are no multiple of 32 on the halo kernels: 0 never, 1 by cost, 2 wherever possible
     OPT_COUNT
 };
 struct OptDef { const char* name; int dflt; };
@@ -73,7 +74,7 @@ static const OptDef kOptDefs[OPT_COUNT] = {
     {"HALO_NARROW", 1}, {"HALO_DUAL", 1}, {"PATCH_MATRIX", 1}, {"DX_PHASES", 1}, {"DX_COL2IM", 1}, {"DX_TRANSPOSE", 1},
     {"DW_STACKED", -1}, {"DW_DIAG", 1}, {"DW_CW", 0}, {"DW_R", 0}, {"DW_STATIC", 1}, {"CONV_PROF", 0}, {"SM_BUDGET", 0},
     {"SKINNY", 1}, {"HALO_DEEP", 1}, {"HALO_SPLITB", 0}, {"NVTX", 1}, {"DW_LANES", 0}, {"HALO_TAPSTACK", 1}, {"HALO_FLAT32", 1},
-    {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1},
+    {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_PAD", 1},
 };
 static std::atomic<int> g_opt[OPT_COUNT];
 static std::once_flag g_opt_once;
@@ -622,11 +623,33 @@ struct IgemmPlan {
     int oSH = 1, oSW = 1, oNH = 0, oNW = 0;
     bool force = false;              // take the halo kernel even when few tile pixels are real
     int w_img_rows = 0;              // > 0: image n uses rows [n * w_img_rows, ...) of W (batched matrix products)
+    bool pad = false;                // kdim may be any multiple of 4: the TMA fills the last 32-channel chunk of both operands with zeros
 };
+
+static inline int chunks32(int channels) { return (channels + 31) / 32; }
+static inline bool whole_chunks(const IgemmPlan& pl) { return pl.kdim % 32 == 0 || pl.pad; }
+
+// Reduction channels K that are no multiple of 32 (odd layers, K % 4 == 0): run the convolution kernels on chunks whose
+// tail the TMA zero-fills - taps * ceil32(K) reduction steps, nothing else - or write the patch matrix, whose rows pad
+// only once (ceil32(taps * K) steps) but pass through memory twice?  Per pixel and reduction step an MMA over nc columns
+// costs nc * 2 FLOPs at the rate these kernels sustain (190 TFLOP/s in 3xTF32, 450 in plain TF32) and the patch matrix
+// 8 bytes at 5 TB/s, as much as 150 (3xTF32) or 360 columns; blocks of fewer than 64 columns cost as much as 64.
+// Both sides measured, patch matrix or 8-channel im2col tiles first: 50 x 35 x 29, 36 -> 100 channels 3x3 82 / 66 us;
+// 9 x 47 x 47, 280 -> 192 3x3 267 / 165 us; 512 x 1000 times 1000 x 4096 84 / 46 us.
+static bool pad_beats_patch(int K, int taps, int ncols, int mode3x)
+{
+    const int force = opt(OPT_HALO_PAD);
+    if (force != 1) return force == 2;
+    const double nc = ncols < 64 ? 64 : ncols, mem = mode3x ? 150 : 360;
+    return (double)taps * chunks32(K) * nc <= (double)chunks32(taps * K) * (nc + mem);
+}
+// A route that needs scratch may not take away what a route without any could do: under stream capture, or in a
+// caller-owned workspace, the call then goes on to the older route.
+static inline bool scratch_refused(int rc) { return rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH; }
 
 static int launch_igemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStream_t stream)
 {
-    const int KC = pick_kc(pl.kdim);
+    const int KC = pl.pad ? 32 : pick_kc(pl.kdim);
     IgemmParams p{};
     p.out = pl.out; p.bias = pl.bias; p.act_on = pl.act_on; p.act_k = pl.act_k; p.status = c->status;
     p.M_total = pl.aN * pl.oH * pl.oW;
@@ -634,7 +657,7 @@ static int launch_igemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStrea
     p.OHo = pl.oH; p.OWo = pl.oW;
     p.sh = pl.sh; p.sw = pl.sw; p.ph = pl.pad_h; p.pw = pl.pad_w;
     p.FH = pl.FH; p.FW = pl.FW;
-    p.KC = KC; p.kchunks = pl.kdim / KC;
+    p.KC = KC; p.kchunks = (pl.kdim + KC - 1) / KC;
     p.mode3x = mode3x; p.b_mn = pl.b_mn; p.flip = pl.flip;
     const int gran = pl.b_mn ? 32 : 16;
     int BN = ((pl.ncols + gran - 1) / gran) * gran;
@@ -749,7 +772,7 @@ static int halo_ksplit(const IgemmPlan& pl, long long tiles, int kchunks, int sm
 static HaloChoice plan_halo(const IgemmPlan& pl, int BN, int mode3x, int b_mn, int sm_count)
 {
     HaloChoice best;
-    const int taps = pl.FH * pl.FW, kchunks = pl.kdim / 32;
+    const int taps = pl.FH * pl.FW, kchunks = chunks32(pl.kdim);
     const int planes = mode3x ? 2 : 1;
     const uint32_t b_tx = b_mn ? (BN / 32) * 4096 : BN * 128;
     const uint32_t b_tile = ((b_tx + 1023) & ~1023u) * planes;
@@ -902,7 +925,7 @@ static void halo_pair_launch_one(const HaloLaunch& L)
 // One 16 x 8 pixel accumulator per CTA, two CTAs per MMA.  Returns 1 when the shape does not fit.
 static int launch_halo_pair(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStream_t stream)
 {
-    if (pl.FW != 3 || pl.sh != 1 || pl.sw != 1 || pl.kdim % 32 != 0 || pl.b_mn) return 1;
+    if (pl.FW != 3 || pl.sh != 1 || pl.sw != 1 || !whole_chunks(pl) || pl.b_mn) return 1;
     int BN = ((pl.ncols + 15) / 16) * 16;
     // wide 3xTF32 needs 2 * BN <= 256 columns per MMA; ALPHA_HALO_PAIR=2 takes three MMAs of BN <= 256 instead
     const int pair_env = opt(OPT_HALO_PAIR);
@@ -927,7 +950,7 @@ static int launch_halo_pair(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaS
     p.N = pl.aN; p.OH = pl.oH; p.OW = pl.oW;
     p.Ncols = pl.ncols; p.ldo = pl.ncols;
     p.FH = pl.FH; p.FW = pl.FW; p.pad_h = pl.pad_h; p.pad_w = pl.pad_w;
-    p.kchunks = pl.kdim / 32;
+    p.kchunks = chunks32(pl.kdim);
     p.BN = BN; p.n_tiles = (pl.ncols + BN - 1) / BN;
     p.JH = 1; p.JW = 1; p.NI = NI; p.SG = SG;
     p.PH = NI > 1 ? NI * SG : 16 + pl.FH - 1; p.PW = 8 + pl.FW - 1;
@@ -1031,12 +1054,12 @@ static TapStackPlan plan_tapstack(const IgemmPlan& pl, int mode3x, int sm_count)
 {
     TapStackPlan ts;
     const int mode = opt(OPT_HALO_TAPSTACK);
-    if (!mode || mode3x || pl.b_mn || pl.sh != 1 || pl.sw != 1 || pl.kdim % 32 != 0) return ts;
+    if (!mode || mode3x || pl.b_mn || pl.sh != 1 || pl.sw != 1 || !whole_chunks(pl)) return ts;
     if (pl.oSH != 1 || pl.oSW != 1 || pl.oNH != 0 || pl.oNW != 0) return ts;
     if (pl.FW < 2 || pl.FW > 8 || pl.ncols % 4 != 0) return ts;
     const int BN = (pl.ncols + 15) / 16 * 16;
     if (pl.FW * BN > 256) return ts;
-    const int kchunks = pl.kdim / 32;
+    const int kchunks = chunks32(pl.kdim);
     const int PH = 4 + pl.FH - 1;
     if (PH > 256) return ts;
     ts.BN = BN;
@@ -1077,7 +1100,7 @@ static int launch_tapstack(DeviceCtx* c, const IgemmPlan& pl, const TapStackPlan
     p.out = pl.out; p.bias = pl.bias; p.act_on = pl.act_on; p.act_k = pl.act_k; p.status = c->status; p.prof = c->prof;
     p.N = pl.aN; p.OH = pl.oH; p.OW = pl.oW; p.Ncols = pl.ncols; p.ldo = pl.ncols;
     p.FH = pl.FH; p.FW = pl.FW; p.pad_h = pl.pad_h; p.pad_w = pl.pad_w;
-    p.kchunks = pl.kdim / 32; p.BN = ts.BN; p.CB = ts.CB;
+    p.kchunks = chunks32(pl.kdim); p.BN = ts.BN; p.CB = ts.CB;
     p.row_blocks = ts.row_blocks; p.col_blocks = ts.col_blocks;
     p.total_tiles = (int)((long long)pl.aN * ts.row_blocks * ts.col_blocks);
     p.npb = ts.npb; p.patch_bytes = ts.patch_bytes; p.w_tile = ts.w_tile; p.w_bytes = ts.w_bytes;
@@ -1123,7 +1146,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const int tile_mode = env_tile_mode();
     if (tile_mode == 1) return 1;
     IgemmPlan pl = pl_in;
-    if (pl.sh != 1 || pl.sw != 1 || pl.kdim % 32 != 0) return 1;
+    if (pl.sh != 1 || pl.sw != 1 || !whole_chunks(pl)) return 1;
     // CTA pairs: the single-CTA forms are bound by shared-memory bandwidth once an MMA covers 128 or
     // more columns (operand reads alone take 128 B/clk at N = 128), and a pair halves the W-tile part
     // of it.  Measured faster in plain TF32 where one MMA covers 256 output channels (OC % 256 == 0:
@@ -1141,7 +1164,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         const int ni = (sg <= 16 && opt(OPT_HALO_STACK)) ? 1 + (16 - pl.oH) / sg : 1;
         const long long tiles128 = (long long)((pl.aN + ni - 1) / ni) * (ni > 1 ? 1 : (pl.oH + 15) / 16) * ((pl.oW + 7) / 8) *
                                    ((pl.ncols + 127) / 128);
-        skinny = 2 * tiles128 <= sm_budget(c) && (long long)(pl.kdim / 32) * pl.FH * pl.FW >= 32;
+        skinny = 2 * tiles128 <= sm_budget(c) && (long long)chunks32(pl.kdim) * pl.FH * pl.FW >= 32;
     }
     // per-image weights: only the single-CTA kernel knows them (its W-tile loads add the image's first row)
     const bool try_pair = !pl.w_img_rows && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
@@ -1188,7 +1211,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     p.N = pl.aN; p.OH = pl.oH; p.OW = pl.oW;
     p.Ncols = pl.ncols; p.ldo = pl.ncols;
     p.FH = pl.FH; p.FW = pl.FW; p.pad_h = pl.pad_h; p.pad_w = pl.pad_w;
-    p.kchunks = pl.kdim / 32;
+    p.kchunks = chunks32(pl.kdim);
     p.BN = BN; p.n_tiles = (pl.ncols + BN - 1) / BN;
     p.JH = ch.JH; p.JW = ch.JW;
     p.NI = ch.NI; p.SG = pl.oH + pl.FH - 1;
@@ -1361,7 +1384,7 @@ static int launch_patch_gemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cuda
     IgemmPlan g = pl;
     g.act = A; g.aH = pl.oH; g.aW = pl.oW; g.aC = Kp;
     g.FH = 1; g.FW = 1; g.sh = 1; g.sw = 1; g.pad_h = 0; g.pad_w = 0;
-    g.wIC = K; g.kdim = Kp; g.b_mn = false; g.flip = false; g.force = true;
+    g.wIC = K; g.kdim = Kp; g.b_mn = false; g.flip = false; g.force = true; g.pad = false;
     rc = launch_halo(c, g, mode3x, stream);
     if (rc != 1) return rc;
     if (g.W_lo) return 1;   // the per-tap kernel splits W itself and cannot take pre-split planes
@@ -1614,6 +1637,68 @@ static void dw_halo_set_attr()
 }
 static inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
+struct DwForm { int G, NT; bool stacked, diag; long long cost; };   // cost: clocks of a filter row's MMAs per 8 pixels; < 0: none fits
+
+static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image, int mode3x)
+{
+    // Input channels per CTA: the accumulators of a CTA's G taps, NT columns each, must fit the 512 tensor-memory
+    // columns.  A CTA owns a whole filter row (G = FW) unless rows of more than three taps do better split over
+    // several CTAs of three taps (5x5, 7x7: three accumulators of 128 columns instead of five or seven of 64; an MMA of
+    // N columns costs max(N / 2, 59) clocks whatever its height, and a last group with fewer taps idles its spare slots).
+    auto mma_clk = [](int n) { return n / 2 > 59 ? n / 2 : 59; };
+    // Channel blocks: the multiple of 32 columns whose MMAs (cols_per columns for each channel of the block) take the fewest
+    // clocks over all blocks - 96 channels are one block of 96, 192 under three taps two of 96, where blocks of a power of
+    // two would need three of 32 and three of 64.  Fewer blocks on a tie.  Channels past IC arrive as zeros and are not stored.
+    // 88 x 56 x 56, 80 -> 64 channels 3x3 in plain TF32: 473 us over a patch matrix in blocks of 32, 177 us as one block of 96.
+    auto tiles = [&](int nt) { return (long long)((s->IC + nt - 1) / nt); };
+    auto nt_for = [&](int slots_cols, int top, int cols_per) {
+        int best = 0;
+        long long best_clk = 0;
+        for (int nt = 32; nt <= top && slots_cols * nt <= 512; nt += 32) {
+            const long long clk = tiles(nt) * mma_clk(cols_per * nt);
+            if (!best || clk < best_clk || (clk == best_clk && tiles(nt) < tiles(best))) { best = nt; best_clk = clk; }
+        }
+        return best;
+    };
+    auto pick = [&](int G) {
+        DwForm f{G, nt_for(G, 256, 1), false, false, 0};
+        if (!f.NT) { f.cost = -1; return f; }
+        const long long slots = (long long)((s->FW + G - 1) / G) * G;   // MMAs per 8 pixels and channel tile
+        f.cost = slots * (mode3x ? 3 : 1) * mma_clk(f.NT) * ((s->OC + 127) / 128) * tiles(f.NT);
+        // 3xTF32: three MMAs of (128 x NT), or one MMA on stacked hi/lo planes (64 + 64) x (NTq + NTq): the
+        // stacked form wins where 128 output channels or 64 input channels would be half empty
+        if (mode3x && !per_image) {   // the stacked form leaves two partial planes to add
+            const int NTq = nt_for(2 * G, 128, 2);
+            if (NTq) {
+                const long long stk_cost = slots * mma_clk(2 * NTq) * ((s->OC + 63) / 64) * tiles(NTq);
+                bool stacked = stk_cost < f.cost;
+                const int force = opt(OPT_DW_STACKED);
+                if (force >= 0) stacked = force != 0;
+                if (stacked) { f.stacked = true; f.NT = NTq; f.cost = stk_cost; }
+            }
+        }
+        // plain TF32 with at most 64 output channels: two half tiles side by side ("diagonal" form), half an MMA of
+        // 2 * NTd columns per 8 pixels
+        if (!mode3x && !per_image && s->OC <= 64 && s->OH >= 2 && opt(OPT_DW_DIAG)) {
+            const int NTd = nt_for(2 * G, 128, 2);
+            if (NTd) {
+                const long long dg2 = slots * mma_clk(2 * NTd) * tiles(NTd);
+                if (dg2 < 2 * f.cost) { f.diag = true; f.stacked = true; f.NT = NTd; f.cost = (dg2 + 1) / 2; }
+            }
+        }
+        return f;
+    };
+    DwForm form = pick(s->FW);
+    if (s->FW > 3 && !strided && !per_image && opt(OPT_DW_TAPGROUPS)) {
+        // groups of three run the kernel whose MMAs are straight-line code; a whole row of four or more taps runs the
+        // looped form, whose issuing thread needs about twice as long per MMA (5x5, 64 -> 128 channels at 112 x 112
+        // in plain TF32: 3.06 ms as one row of five, 1.50 ms as 3 + 2 although that issues six MMAs for five taps)
+        const DwForm g3 = pick(3);
+        if (g3.cost >= 0 && (form.cost < 0 || 10 * g3.cost <= 16 * form.cost || opt(OPT_DW_TAPGROUPS) == 2)) form = g3;
+    }
+    return form;
+}
+
 // Returns 1 when the shape is left to the split-K im2col kernel, 0 on launch, < 0 on error.
 // deltaB != nullptr: the kernel also sums the columns of deltaY (bias gradient); *bias_fused tells whether it did.
 // per_image: dW receives N separate results, dW[n] = the sum over the pixels of image n only (batched matrix
@@ -1634,7 +1719,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
         flat.N = 1; flat.OW = flat.IW = 16; flat.OH = flat.IH = (int)(flat_m / 16);
         s = &flat;
     }
-    if (s->sh < 1 || s->sh > 2 || s->sw < 1 || s->sw > 2 || s->IC % 32 != 0) return 1;
+    if (s->sh < 1 || s->sh > 2 || s->sw < 1 || s->sw > 2 || s->IC % 4 != 0) return 1;
     const bool strided = s->sh != 1 || s->sw != 1;
     if (strided && (per_image || !opt(OPT_DW_STRIDED))) return 1;
     if (s->FW > 8 || s->ph >= s->FH || s->pw >= s->FW) return 1;
@@ -1652,53 +1737,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     for (int k = 0; k < nph; ++k)
         if (ph_psi[k] >= s->IW) return 1;                 // a lattice without a column
     if (s->sh > s->IH) return 1;
-    // Input channels per CTA: the accumulators of a CTA's G taps, NT columns each, must fit the 512 tensor-memory
-    // columns.  A CTA owns a whole filter row (G = FW) unless rows of more than three taps do better split over
-    // several CTAs of three taps (5x5, 7x7: three accumulators of 128 columns instead of five or seven of 64; an MMA of
-    // N columns costs max(N / 2, 59) clocks whatever its height, and a last group with fewer taps idles its spare slots).
-    struct DwForm { int G, NT; bool stacked, diag; long long cost; };
-    auto mma_clk = [](int n) { return n / 2 > 59 ? n / 2 : 59; };
-    auto nt_for = [&](int slots_cols, int top) {
-        for (int cand = top; cand >= 32; cand >>= 1)
-            if (s->IC % cand == 0 && slots_cols * cand <= 512) return cand;
-        return 0;
-    };
-    auto pick = [&](int G) {
-        DwForm f{G, nt_for(G, 256), false, false, 0};
-        if (!f.NT) { f.cost = -1; return f; }
-        const long long slots = (long long)((s->FW + G - 1) / G) * G;   // MMAs per 8 pixels and channel tile
-        f.cost = slots * (mode3x ? 3 : 1) * mma_clk(f.NT) * ((s->OC + 127) / 128) * (s->IC / f.NT);
-        // 3xTF32: three MMAs of (128 x NT), or one MMA on stacked hi/lo planes (64 + 64) x (NTq + NTq): the
-        // stacked form wins where 128 output channels or 64 input channels would be half empty
-        if (mode3x && !per_image) {   // the stacked form leaves two partial planes to add
-            const int NTq = nt_for(2 * G, 128);
-            if (NTq) {
-                const long long stk_cost = slots * mma_clk(2 * NTq) * ((s->OC + 63) / 64) * (s->IC / NTq);
-                bool stacked = stk_cost < f.cost;
-                const int force = opt(OPT_DW_STACKED);
-                if (force >= 0) stacked = force != 0;
-                if (stacked) { f.stacked = true; f.NT = NTq; f.cost = stk_cost; }
-            }
-        }
-        // plain TF32 with at most 64 output channels: two half tiles side by side ("diagonal" form), half an MMA of
-        // 2 * NTd columns per 8 pixels
-        if (!mode3x && !per_image && s->OC <= 64 && s->OH >= 2 && opt(OPT_DW_DIAG)) {
-            const int NTd = nt_for(2 * G, 128);
-            if (NTd) {
-                const long long dg2 = slots * mma_clk(2 * NTd) * (s->IC / NTd);
-                if (dg2 < 2 * f.cost) { f.diag = true; f.stacked = true; f.NT = NTd; f.cost = (dg2 + 1) / 2; }
-            }
-        }
-        return f;
-    };
-    DwForm form = pick(s->FW);
-    if (s->FW > 3 && !strided && !per_image && opt(OPT_DW_TAPGROUPS)) {
-        // groups of three run the kernel whose MMAs are straight-line code; a whole row of four or more taps runs the
-        // looped form, whose issuing thread needs about twice as long per MMA (5x5, 64 -> 128 channels at 112 x 112
-        // in plain TF32: 3.06 ms as one row of five, 1.50 ms as 3 + 2 although that issues six MMAs for five taps)
-        const DwForm g3 = pick(3);
-        if (g3.cost >= 0 && (form.cost < 0 || 10 * g3.cost <= 16 * form.cost || opt(OPT_DW_TAPGROUPS) == 2)) form = g3;
-    }
+    const DwForm form = plan_dw_form(s, strided, per_image, mode3x);
     if (form.cost < 0) return 1;
     const int G = form.G, tgroups = (s->FW + G - 1) / G;
     int NT = form.NT;
@@ -1708,7 +1747,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     p.status = c->status; p.prof = c->prof;
     p.N = s->N; p.OH = s->OH; p.OW = s->OW;
     p.IC = s->IC; p.OC = s->OC; p.FH = s->FH; p.FW = s->FW; p.ph = s->ph; p.pw = s->pw;
-    p.NT = NT; p.ic_tiles = s->IC / NT; p.oc_tiles = (s->OC + oc_tile - 1) / oc_tile;
+    p.NT = NT; p.ic_tiles = (s->IC + NT - 1) / NT; p.oc_tiles = (s->OC + oc_tile - 1) / oc_tile;
     const int groups = tgroups * s->FH * p.ic_tiles * p.oc_tiles;
     if (groups > 65535) return 1;
     p.G = G; p.tgroups = tgroups;
@@ -1897,6 +1936,24 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
         if (bias_fused) *bias_fused = true;
     }
     return rc;
+}
+
+// deltaW of a layer whose input channels are no multiple of 32 (IC % 4 == 0): straight from X, with channel blocks whose
+// tail the TMA zero-fills, or over the patch matrix (a 1x1 deltaW with FH * FW * IC channels)?  Both sides in clocks of one
+// SM per 8 pixels: the MMAs of each form, and for the patch matrix 8 bytes per element at 5 TB/s (3.4 clocks per column
+// and 8 pixels over 148 SMs at 1.8 GHz).  50 x 35 x 29, 36 -> 100 channels 3x3: 192 us over the patch matrix, 62 us straight.
+static bool dw_pad_beats_patch(const AlphaConvShape* s, int mode3x)
+{
+    const int force = opt(OPT_HALO_PAD);
+    if (force != 1) return force == 2;
+    const bool strided = s->sh != 1 || s->sw != 1;
+    const DwForm own = plan_dw_form(s, strided, false, mode3x);
+    if (own.cost < 0) return false;
+    AlphaConvShape t = *s;
+    t.IC = chunks32(s->FH * s->FW * s->IC) * 32; t.FH = t.FW = 1; t.sh = t.sw = 1; t.ph = t.pw = 0;
+    t.IH = s->OH; t.IW = s->OW;
+    const DwForm patch = plan_dw_form(&t, false, false, mode3x);
+    return patch.cost < 0 || (double)own.cost * s->FH <= (double)patch.cost + 3.4 * t.IC;
 }
 
 // Batched matrix products (the reference's Cuda_batchMatMul) on the convolution kernels: entry b of the batch is
@@ -2382,9 +2439,22 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
             rc = launch_patch_gemm(c, pl, mode3x, stream);
             if (rc != 1) return rc;
         }
+        pl.pad = s->IC % 32 != 0 && env_tile_mode() != 1 && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x);
         rc = launch_halo(c, pl, mode3x, stream);
-        if (rc != 1) return rc;
+        if (rc != 1 && !(pl.pad && scratch_refused(rc))) return rc;
         return launch_igemm(c, pl, mode3x, stream);
+    }
+    if (algo != ALPHA_ALGO_SIMT && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
+        !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x())) {
+        IgemmPlan pl{};
+        pl.act = X; pl.aN = s->N; pl.aH = s->IH; pl.aW = s->IW; pl.aC = s->IC;
+        pl.FH = s->FH; pl.FW = s->FW; pl.sh = s->sh; pl.sw = s->sw; pl.pad_h = s->ph; pl.pad_w = s->pw;
+        pl.out = Y; pl.oH = s->OH; pl.oW = s->OW; pl.ncols = s->OC;
+        pl.W = W; pl.wOC = s->OC; pl.wIC = s->IC; pl.bias = bias; pl.act_on = act_on; pl.act_k = act_k;
+        pl.b_mn = false; pl.flip = false; pl.kdim = s->IC; pl.pad = true;
+        rc = launch_halo(c, pl, cur_mode3x(), stream);
+        if (rc != 1 && !scratch_refused(rc)) return rc;
+        return launch_igemm(c, pl, cur_mode3x(), stream);
     }
     if (algo != ALPHA_ALGO_SIMT && patch_path_ok(s)) {
         IgemmPlan pl{};
@@ -2429,7 +2499,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
         pl.W = W; pl.wOC = s->OC; pl.wIC = s->IC; pl.bias = nullptr;
         pl.b_mn = true; pl.flip = true; pl.kdim = s->OC;
         const int mode3x = cur_mode3x();
-        if (env_tile_mode() != 1 && s->OC % 32 == 0 && taps_fit64(s) && opt(OPT_DX_TRANSPOSE)) {
+        if (env_tile_mode() != 1 && (s->OC % 32 == 0 || opt(OPT_HALO_PAD)) && taps_fit64(s) && opt(OPT_DX_TRANSPOSE)) {
             // deltaX as a forward conv over deltaY with Wt[ic][rotated tap][oc], built once per call
             const int taps = s->FH * s->FW;
             const size_t nW = (size_t)s->OC * taps * s->IC;
@@ -2437,6 +2507,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
             bool fresh = true;
             const DeviceCtx::WeightKey wkey{W, WK_DX_S1, s->OC, s->IC, s->FH * 256 + s->FW, 0, mode3x};
             rc = weight_planes(c, stream, wkey, (mode3x ? 2 : 1) * nW * sizeof(float), &ws, &fresh);
+            if (s->OC % 32 != 0 && scratch_refused(rc)) goto in_place;
             if (rc) return rc;
             IgemmPlan pt = pl;
             pt.W = ws; pt.W_lo = mode3x ? ws + nW : nullptr;
@@ -2453,13 +2524,16 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
                 weight_planes_ready(c, stream, wkey);
             }
             if (!mode3x) pt.W_lo = nullptr;
-            if (tiny_image(s->IH, s->IW) && (s->FH > 1 || s->FW > 1) && (long long)taps * s->OC <= 16384) {
+            pt.pad = s->OC % 32 != 0;
+            if ((tiny_image(s->IH, s->IW) || (pt.pad && !pad_beats_patch(s->OC, taps, s->IC, mode3x))) && (s->FH > 1 || s->FW > 1) &&
+                (long long)taps * s->OC <= 16384 && (!pt.pad || opt(OPT_PATCH_MATRIX))) {
                 rc = launch_patch_gemm(c, pt, mode3x, stream);
-                if (rc != 1) return rc;
+                if (rc != 1 && !(pt.pad && scratch_refused(rc))) return rc;
             }
             rc = launch_halo(c, pt, mode3x, stream);
-            if (rc != 1) return rc;
+            if (rc != 1 && !(pt.pad && scratch_refused(rc))) return rc;
         }
+in_place:
         rc = launch_halo(c, pl, mode3x, stream);
         if (rc != 1) return rc;
         return launch_igemm(c, pl, cur_mode3x(), stream);
@@ -2488,6 +2562,10 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     const bool tensor_ok = (s->IC % 32 == 0) && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256;
     if (algo == ALPHA_ALGO_TENSOR && !tensor_ok)
         return fail(ALPHA_E_ARG, "tensor deltaW path needs IC %% 32 == 0 (IC=%d)", s->IC);
+    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1 && dw_pad_beats_patch(s, cur_mode3x())) {
+        rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream);
+        if (rc != 1 && !scratch_refused(rc)) return rc;
+    }
     if (algo != ALPHA_ALGO_SIMT && patch_path_ok(s) && env_tile_mode() != 1 &&
         (!tensor_ok || (s->OH * s->OW <= 9 && (s->FH > 1 || s->FW > 1)))) {
         // deltaW[oc][k] = sum over pixels of deltaY[pixel][oc] * A[pixel][k]: a 1x1 deltaW over the patch matrix

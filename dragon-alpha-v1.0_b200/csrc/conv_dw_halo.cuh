@@ -62,7 +62,7 @@ struct DwHaloParams {
     int N, OH, OW;         // deltaY geometry
     int IC, OC, FH, FW, ph, pw;
     int NT;                // input channels per CTA (multiple of 32, <= 256)
-    int ic_tiles, oc_tiles;  // IC / NT, ceil(OC / 128)
+    int ic_tiles, oc_tiles;  // ceil(IC / NT), ceil(OC / 128)
     int R, CW;             // pixel tile: rows x columns (CW multiple of 8)
     int PW;                // X tile columns = CW + FW - 1
     int row_blocks, col_blocks, tiles_per_img;
@@ -409,6 +409,7 @@ __global__ void __launch_bounds__(kDwHaloThreads, 1)
                         float* dst = obase + (static_cast<size_t>(oc) * taps + tap) * p.IC + ic0 + c;
 #pragma unroll
                         for (int q = 0; q < 32; q += 4) {
+                            if (ic0 + c + q >= p.IC) break;   // the last block's zero-filled channels
                             float4 o = has_tiles ? make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]),
                                                                __uint_as_float(v[q + 2]), __uint_as_float(v[q + 3]))
                                                  : make_float4(0.f, 0.f, 0.f, 0.f);

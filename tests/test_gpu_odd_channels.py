@@ -1,0 +1,45 @@
+"""Channel counts that are no multiple of 32: zero-filled last chunks in the halo kernels and channel blocks of any multiple of
+32 columns in deltaW, against the fp64 oracle, with the route chosen by cost (HALO_PAD = 1) and forced (2)."""
+import numpy as np
+import pytest
+
+from helpers import gen, metrics, out_hw
+
+pytestmark = pytest.mark.gpu
+TOL = {"3xtf32": dict(norm=1e-4, comp=1e-5), "tf32": dict(norm=5e-3, comp=2e-3)}   # the bounds of the other shape tests
+
+# N, IH, IW, IC, OC, FH, FW, s, p: remainders 4 ... 28 of a chunk, one chunk and several, blocks of 96 and 160 columns, tails in
+# every kernel form (pair, single CTA, tap-stacked, split reduction, strided deltaW, tap groups)
+SHAPES = [
+    (3, 35, 29, 36, 100, 3, 3, 1, 1), (2, 18, 18, 40, 64, 3, 3, 1, 1), (4, 20, 20, 16, 32, 3, 3, 1, 1), (2, 16, 16, 8, 128, 3, 3, 1, 1),
+    (4, 28, 28, 60, 128, 3, 3, 1, 1), (2, 14, 14, 132, 256, 3, 3, 1, 1), (2, 13, 11, 92, 48, 5, 5, 1, 2), (3, 17, 15, 100, 72, 1, 1, 1, 0),
+    (2, 24, 24, 96, 96, 3, 3, 1, 1), (2, 16, 16, 192, 40, 3, 3, 1, 1), (2, 12, 12, 320, 64, 3, 3, 1, 1), (2, 33, 31, 44, 20, 3, 3, 2, 1),
+    (2, 17, 17, 72, 36, 3, 3, 2, 1), (1, 5, 5, 420, 24, 3, 3, 1, 1), (2, 16, 16, 68, 68, 4, 4, 2, 1), (1, 8, 8, 1028, 8, 1, 1, 1, 0),
+]
+
+
+@pytest.mark.parametrize("pad", [1, 2])
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+def test_zero_filled_chunks(pkg, oracle_mod, shape, mode, pad):
+    import torch
+    lib, engine = pkg.submodule("lib"), pkg.submodule("engine")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+    N, IH, IW, IC, OC, FH, FW, s, p = shape
+    OH, OW = out_hw(IH, IW, FH, FW, s, s, p, p)
+    rng = np.random.default_rng(IC * 1000 + OC)
+    X, W, dY = gen((N, IH, IW, IC), "relu", rng), gen((OC, FH, FW, IC), "u11", rng), gen((N, OH, OW, OC), "n01", rng)
+    tX, tW, tdY = (torch.from_numpy(a).cuda() for a in (X, W, dY))
+    lib.set_option("HALO_PAD", pad)
+    try:
+        got = {"fwd": eng.conv3D(tX, tW, s, s, p, p), "dw": eng.dconv3D_deltaW(tX, tdY, FH, FW, s, s, p, p)}
+        ref = {"fwd": oracle_mod.conv3D_f64(X, W, s, s, p, p, threads=8), "dw": oracle_mod.deconv3D_deltaW_f64(X, dY, FH, FW, s, s, p, p, threads=8)}
+        if (IH + 2 * p - FH) % s == 0 and (IW + 2 * p - FW) % s == 0:
+            got["dx"] = eng.dconv3D_deltaX(tdY, tW, IH, IW, s, s, p, p)
+            ref["dx"] = oracle_mod.deconv3D_deltaX_f64(dY, W, IH, IW, s, s, p, p, threads=8)
+    finally:
+        lib.set_option("HALO_PAD", 1)
+    assert lib.device_status() == 0
+    for op, y in got.items():
+        m = metrics(y.cpu().numpy(), *ref[op])
+        assert m["finite"] and m["norm"] <= TOL[mode]["norm"] and m["comp"] <= TOL[mode]["comp"], (op, m)

@@ -38,7 +38,7 @@ int fail(int code, const char* fmt, ...)
     return code;
 }
 
-static thread_local char g_plan[128] = "";
+static thread_local char g_plan[192] = "";
 // The calling thread is sizing a call (alpha_conv_workspace_bytes): scratch requests are added up
 // and answered with a placeholder address; nothing is allocated, launched or copied.
 static thread_local bool t_dry = false;
@@ -64,6 +64,7 @@ enum Opt {
     OPT_SKINNY, OPT_HALO_DEEP, OPT_HALO_SPLITB, OPT_NVTX, OPT_DW_LANES, OPT_HALO_TAPSTACK, OPT_HALO_FLAT32,
     OPT_DW_STRIDED,     // 0 = strided deltaW on the split-K im2col kernel only
     OPT_DW_TAPGROUPS,   // 0 = a CTA always owns a whole filter row, 2 = rows of more than three taps always split
+    OPT_HALO_LATTICE,   // strided forward on the halo kernel: 0 never, 1 by cost, 2 wherever possible
     OPT_HALO_PAD,       // channels that are no multiple of 32 on the halo kernels: 0 never, 1 by cost, 2 wherever possible
     OPT_COUNT
 };
@@ -74,7 +75,7 @@ static const OptDef kOptDefs[OPT_COUNT] = {
     {"HALO_NARROW", 1}, {"HALO_DUAL", 1}, {"PATCH_MATRIX", 1}, {"DX_PHASES", 1}, {"DX_COL2IM", 1}, {"DX_TRANSPOSE", 1},
     {"DW_STACKED", -1}, {"DW_DIAG", 1}, {"DW_CW", 0}, {"DW_R", 0}, {"DW_STATIC", 1}, {"CONV_PROF", 0}, {"SM_BUDGET", 0},
     {"SKINNY", 1}, {"HALO_DEEP", 1}, {"HALO_SPLITB", 0}, {"NVTX", 1}, {"DW_LANES", 0}, {"HALO_TAPSTACK", 1}, {"HALO_FLAT32", 1},
-    {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_PAD", 1},
+    {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_LATTICE", 1}, {"HALO_PAD", 1},
 };
 static std::atomic<int> g_opt[OPT_COUNT];
 static std::once_flag g_opt_once;
@@ -623,7 +624,17 @@ struct IgemmPlan {
     int oSH = 1, oSW = 1, oNH = 0, oNW = 0;
     bool force = false;              // take the halo kernel even when few tile pixels are real
     int w_img_rows = 0;              // > 0: image n uses rows [n * w_img_rows, ...) of W (batched matrix products)
+    const struct LatticePlan* lat = nullptr;   // strided forward on the halo kernel: the phases; FH, FW, kdim then describe the
+                                     // lattice convolution (most taps of a phase, channels of all phases together)
     bool pad = false;                // kdim may be any multiple of 4: the TMA fills the last 32-channel chunk of both operands with zeros
+};
+
+// Phases of a strided forward convolution (HaloParams::lat_*): input rows phi, phi + sh, ... and columns psi, psi + sw, ...
+struct LatticePlan {
+    int n = 0, U = 0, V = 0, taps = 0;         // phases, most taps along a column / row, taps of all phases
+    int FH, FW, sh, sw, aH, aW, aC;            // the layer's own filter, strides and input
+    double im2col_cost = 0;                    // clocks of the busiest SM on the im2col kernel
+    int phi[4], psi[4], u[4], v[4], tap0[4], h0[4], w0[4];
 };
 
 static inline int chunks32(int channels) { return (channels + 31) / 32; }
@@ -646,6 +657,19 @@ static bool pad_beats_patch(int K, int taps, int ncols, int mode3x)
 // A route that needs scratch may not take away what a route without any could do: under stream capture, or in a
 // caller-owned workspace, the call then goes on to the older route.
 static inline bool scratch_refused(int rc) { return rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH; }
+
+// Clocks of the busiest SM of conv_igemm_kernel (32-channel tiles), measured: a step of 8 channels takes 1.6 times the time
+// its bytes need at 128 B/clk of shared memory - both operands written by the TMA and read by each MMA, and in 3xTF32 read
+// and written once more by the split - and a tile 65 clocks per column for its epilogue and the fill of its ring.
+static double igemm_cost(const IgemmPlan& pl, int mode3x, int sms)
+{
+    int BN = (pl.ncols + 15) / 16 * 16;
+    if (BN > 256) BN = (pl.ncols % 256 == 0 || pl.ncols > 512) ? 256 : 128;
+    const double tiles = (double)((long long)pl.aN * pl.oH * pl.oW + kBM - 1) / kBM * ((pl.ncols + BN - 1) / BN);
+    const double steps = 4.0 * pl.FH * pl.FW * ((pl.kdim + 31) / 32);
+    const double step = 1.6 * (mode3x ? 6 : 2) * (4096.0 + 32.0 * BN) / 128.0;
+    return (tiles > sms ? tiles / sms : 1.0) * (steps * (step > 100 ? step : 100) + 65.0 * BN);
+}
 
 static int launch_igemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStream_t stream)
 {
@@ -726,19 +750,28 @@ struct HaloLaunch {
     int grid;
     size_t smem;
     cudaStream_t stream;
-    const CUtensorMap *tmA, *tmB, *tmBlo, *tmO;
+    const HaloAMaps* tmA;          // (the pair kernel takes entry 0)
+    const CUtensorMap *tmB, *tmBlo, *tmO;
     const HaloParams* p;
 };
 
-template <int FW_T, int JH_T, int JW_T, bool ROW_T, bool FLAT_T = false>
+template <int FW_T, int JH_T, int JW_T, bool ROW_T, bool FLAT_T = false, bool LAT_T = false>
 static void halo_launch_one(const HaloLaunch& L)
 {
     static bool attr_done = false;  // per instantiation; the attribute is per function, any device
     if (!attr_done) {
-        cudaFuncSetAttribute(conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_done = true;
     }
-    if (!t_dry) conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T><<<L.grid, kHaloThreads2, L.smem, L.stream>>>(*L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+    if (!t_dry) conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T><<<L.grid, kHaloThreads2, L.smem, L.stream>>>(*L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+}
+
+template <int FW_T>
+static void halo_launch_lat(const HaloLaunch& L, int JH, int JW)
+{
+    if (JH == 2) halo_launch_one<FW_T, 2, 1, false, false, true>(L);
+    else if (JW == 2) halo_launch_one<FW_T, 1, 2, false, false, true>(L);
+    else halo_launch_one<FW_T, 1, 1, false, false, true>(L);
 }
 
 template <int FW_T>
@@ -802,8 +835,9 @@ static HaloChoice plan_halo(const IgemmPlan& pl, int BN, int mode3x, int b_mn, i
             const int PH = NI > 1 ? NI * SG : 16 * JH + pl.FH - 1, PW = 8 * JW + pl.FW - 1;
             if (PH > 256 || PW > 256) continue;
             const uint32_t patch_stride = (((uint32_t)PH * PW * 128 + 1023) & ~1023u) * planes;
+            if (pl.lat && JH * JW > 2) continue;
             const bool stat = allow_row && !b_mn && halo_has_row_kernel(pl.FW, JH, JW);  // a static specialisation exists (K-major W only)
-            bool row = stat;
+            bool row = stat && !pl.lat;
             uint32_t b_stride = b_tile * (row ? pl.FW : 1);
             if (row && (size_t)patch_stride + 2 * (size_t)b_stride + 32768 + 1536 > smem_cap) { row = false; b_stride = b_tile; }
             const int max_sb = row ? pl.FH * 2 : 8;
@@ -827,18 +861,20 @@ static HaloChoice plan_halo(const IgemmPlan& pl, int BN, int mode3x, int b_mn, i
             // cycles per macro tile: one tcgen05.mma of this shape takes max(N/2, 59) clocks
             auto clk = [](double n) { return n / 2.0 > 59.0 ? n / 2.0 : 59.0; };
             const double step_clk = wide ? clk(2.0 * BN) + clk(BN) : (mode3x ? 3 : 1) * clk(BN);
-            const double t_mma = (double)taps * kchunks * 4 * J * step_clk;
+            // W tiles of the whole reduction (phases of a strided layer have different numbers of taps)
+            const double w_tiles = pl.lat ? (double)pl.lat->taps * kchunks / pl.lat->n : (double)taps * kchunks;
+            const double t_mma = w_tiles * 4 * J * step_clk;
             // shared-memory traffic per macro tile at 128 B/clk: the operands every MMA reads (4 KB of A,
             // 32 B per column of B), what the TMA writes, the lo planes the split warps read and write,
             // and the epilogue's staging.  A tcgen05.mma of 128 columns saturates this by itself.
             const double step_bytes = wide ? (4096.0 + 64.0 * BN) + (4096.0 + 32.0 * BN)
                                            : (mode3x ? 3 : 1) * (4096.0 + 32.0 * BN);
-            const double tma_bytes = (double)kchunks * ((double)PH * PW * 128 + (double)taps * b_tx * planes);
-            const double smem_bytes = (double)taps * kchunks * 4 * J * step_bytes + tma_bytes +
+            const double tma_bytes = (double)kchunks * PH * PW * 128 + w_tiles * b_tx * planes;
+            const double smem_bytes = w_tiles * 4 * J * step_bytes + tma_bytes +
                                       (mode3x ? 2.0 * kchunks * PH * PW * 128 : 0.0) + 2.0 * 128 * J * BN * 4;
             const double t_smem = smem_bytes / 128.0;
             // W tiles are read by every CTA at about the same time and cost about half of private bytes
-            const double bytes = (double)kchunks * ((double)PH * PW * 128 + 0.5 * taps * b_tx * planes) + 128.0 * J * BN * 4;
+            const double bytes = (double)kchunks * PH * PW * 128 + 0.5 * w_tiles * b_tx * planes + 128.0 * J * BN * 4;
             const double t_l2 = bytes / 28.0;  // ~28 B/clk/SM between L2 and an SM when all SMs pull
             double t = t_mma + 1500.0;         // fixed per-tile overhead of the issue loop
             if (t_smem + 500.0 > t) t = t_smem + 500.0;
@@ -861,7 +897,7 @@ static HaloChoice plan_halo(const IgemmPlan& pl, int BN, int mode3x, int b_mn, i
     // Flat tiles (images at most 30 pixels wide, 3x3 filters, K-major W): two accumulators of 4 rows x 32 patch
     // columns per W tile, each with its own patch, taken from the list of all four-row blocks of the batch - a
     // 28 x 28 image is seven of them, which 16 x 8 tiles cover with 0.77 of their lanes and these with 0.875.
-    if (opt(OPT_HALO_FLAT32) && allow_row && !b_mn && pl.FW == 3 && pl.oW + pl.FW - 1 <= 32 && !pl.w_img_rows &&
+    if (opt(OPT_HALO_FLAT32) && allow_row && !b_mn && !pl.lat && pl.FW == 3 && pl.oW + pl.FW - 1 <= 32 && !pl.w_img_rows &&
         pl.oSH == 1 && pl.oSW == 1 && pl.oNH == 0 && pl.oNW == 0 && 2 * 2 * BN <= 512 && !force_jh && !force_jw) {
         const int J = 2, wide = (mode3x && BN <= 128 && wide_env != 0) ? 1 : 0;
         const int accw = wide ? 2 * BN : BN;
@@ -919,7 +955,7 @@ static void halo_pair_launch_one(const HaloLaunch& L)
         cudaFuncSetAttribute(conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_done = true;
     }
-    if (!t_dry) conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T><<<L.grid, kHaloThreads, L.smem, L.stream>>>(*L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+    if (!t_dry) conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T><<<L.grid, kHaloThreads, L.smem, L.stream>>>(L.tmA->m[0], *L.tmB, *L.tmBlo, *L.tmO, *L.p);
 }
 
 // One 16 x 8 pixel accumulator per CTA, two CTAs per MMA.  Returns 1 when the shape does not fit.
@@ -1000,11 +1036,12 @@ static int launch_halo_pair(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaS
     p.sb = sb;
     const size_t smem = need(row, sb);
 
-    CUtensorMap tmA, tmB, tmBlo, tmO;
+    HaloAMaps tmA;
+    CUtensorMap tmB, tmBlo, tmO;
     cuuint64_t ad[4] = {(cuuint64_t)pl.aC, (cuuint64_t)pl.aW, (cuuint64_t)pl.aH, (cuuint64_t)pl.aN};
     cuuint64_t as[3] = {(cuuint64_t)pl.aC * 4, (cuuint64_t)pl.aW * pl.aC * 4, (cuuint64_t)pl.aH * pl.aW * pl.aC * 4};
     cuuint32_t abox[4] = {32, (cuuint32_t)p.PW, (cuuint32_t)(NI > 1 ? p.SG : p.PH), (cuuint32_t)NI};
-    int rc = make_tiled_map(&tmA, pl.act, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
+    int rc = make_tiled_map(&tmA.m[0], pl.act, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     const float* w_hi = pl.W;
     const float* w_lo = pl.W_lo ? pl.W_lo : pl.W;
@@ -1167,7 +1204,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         skinny = 2 * tiles128 <= sm_budget(c) && (long long)chunks32(pl.kdim) * pl.FH * pl.FW >= 32;
     }
     // per-image weights: only the single-CTA kernel knows them (its W-tile loads add the image's first row)
-    const bool try_pair = !pl.w_img_rows && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
+    const bool try_pair = !pl.w_img_rows && !pl.lat && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
     if (try_pair && !skinny) {
         const int rc2 = launch_halo_pair(c, pl, mode3x, stream);
         if (rc2 != 1) return rc2;
@@ -1177,7 +1214,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const long long flat_m = (long long)pl.aN * pl.aH * pl.aW;
     if (pl.FH == 1 && pl.FW == 1 && pl.pad_h == 0 && pl.pad_w == 0 && pl.oSH == 1 && pl.oSW == 1 && pl.oNH == 0 &&
         pl.oNW == 0 && pl.oH == pl.aH && pl.oW == pl.aW && flat_m % 8 == 0 && flat_m / 8 <= 2147483647LL &&
-        opt(OPT_HALO_FLAT) && !pl.w_img_rows) {
+        opt(OPT_HALO_FLAT) && !pl.w_img_rows && !pl.lat) {
         pl.aN = 1; pl.aW = 8; pl.aH = (int)(flat_m / 8);
         pl.oH = pl.aH; pl.oW = 8;
     }
@@ -1194,10 +1231,10 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     }
     {
         // plain TF32 with few output channels: one MMA per filter row where the model says it is faster
-        const TapStackPlan ts = pl.w_img_rows ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
+        const TapStackPlan ts = (pl.w_img_rows || pl.lat) ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
         if (ts.valid && (opt(OPT_HALO_TAPSTACK) == 2 || !ch.valid || ts.cost < 0.8 * ch.cost)) return launch_tapstack(c, pl, ts, stream);
     }
-    if (!ch.valid || (tile_mode == 0 && ch.eff < 0.6 && !pl.force)) {
+    if (!ch.valid || (tile_mode == 0 && ch.eff < 0.6 && !pl.force && !pl.lat)) {
         // a skinny shape whose tiles the single-CTA kernel would leave mostly empty: the pair kernel after all
         if (try_pair && skinny) {
             const int rc2 = launch_halo_pair(c, pl_in, mode3x, stream);
@@ -1232,6 +1269,14 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const long long total = (long long)p.n_tiles * p.n_blocks * p.row_blocks * p.col_blocks;
     if (total > 2147483647LL) return 1;
     p.total_tiles = (int)total;
+    if (pl.lat && !pl.force) {
+        // Against the im2col kernel.  One tap per W-tile stage and patches that change with every phase run at 1.4 times the
+        // plan's clocks (2.2 times with column tiles under 64, whose MMAs are all issue); the lo plane of W and the sum of
+        // split reductions are a launch each, 15000 clocks.  128 x 112 x 112, 128 -> 64 channels 3x3 s2: 735 us im2col, 521 us
+        // here; 16 x 14 x 14, 256 -> 512: 118 and 38 us; 512 x 16 x 16, 64 -> 128, whose 8 x 8 images half fill a tile: 50 and 70.
+        const double extra = (mode3x ? 15000.0 : 0.0) + (halo_ksplit(pl, total, p.kchunks, sm_budget(c)) > 1 ? 15000.0 : 0.0);
+        if (ch.cost * (BN < 64 ? 2.2 : 1.42) + extra > 0.9 * pl.lat->im2col_cost) return 1;
+    }
     p.npb = ch.npb; p.sb = ch.sb; p.acc_bufs = ch.acc_bufs;
     p.mode3x = ch.wide ? 2 : mode3x; p.b_mn = pl.b_mn; p.flip = pl.flip;
     p.w_img_rows = pl.w_img_rows;
@@ -1253,12 +1298,28 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const size_t smem = (size_t)p.npb * p.patch_bytes * planes + (size_t)p.sb * p.b_bytes * planes * tps + 32768 +
                         (3 * p.npb + 3 * p.sb + 8) * 8 + 1024;
 
-    CUtensorMap tmA, tmB;
-    cuuint64_t ad[4] = {(cuuint64_t)pl.aC, (cuuint64_t)pl.aW, (cuuint64_t)pl.aH, (cuuint64_t)pl.aN};
-    cuuint64_t as[3] = {(cuuint64_t)pl.aC * 4, (cuuint64_t)pl.aW * pl.aC * 4, (cuuint64_t)pl.aH * pl.aW * pl.aC * 4};
+    HaloAMaps tmA;
+    CUtensorMap tmB;
     cuuint32_t abox[4] = {32, (cuuint32_t)p.PW, (cuuint32_t)(ch.NI > 1 ? p.SG : p.PH), (cuuint32_t)ch.NI};
-    int rc = make_tiled_map(&tmA, pl.act, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
+    int rc = 0;
+    if (pl.lat) {
+        const LatticePlan& l = *pl.lat;
+        p.lat_n = l.n; p.lat_du = l.sh * l.FW; p.lat_dv = l.sw;
+        for (int k = 0; k < l.n && !rc; ++k) {
+            p.lat_U[k] = l.u[k]; p.lat_V[k] = l.v[k]; p.lat_tap0[k] = l.tap0[k]; p.lat_h0[k] = l.h0[k]; p.lat_w0[k] = l.w0[k];
+            cuuint64_t ad[4] = {(cuuint64_t)l.aC, (cuuint64_t)((l.aW - l.psi[k] + l.sw - 1) / l.sw), (cuuint64_t)((l.aH - l.phi[k] + l.sh - 1) / l.sh), (cuuint64_t)pl.aN};
+            cuuint64_t as[3] = {(cuuint64_t)l.sw * l.aC * 4, (cuuint64_t)l.sh * l.aW * l.aC * 4, (cuuint64_t)l.aH * l.aW * l.aC * 4};
+            rc = make_tiled_map(&tmA.m[k], pl.act + ((size_t)l.phi[k] * l.aW + l.psi[k]) * l.aC, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
+        }
+        for (int k = l.n; k < 4; ++k) tmA.m[k] = tmA.m[0];
+    } else {
+        cuuint64_t ad[4] = {(cuuint64_t)pl.aC, (cuuint64_t)pl.aW, (cuuint64_t)pl.aH, (cuuint64_t)pl.aN};
+        cuuint64_t as[3] = {(cuuint64_t)pl.aC * 4, (cuuint64_t)pl.aW * pl.aC * 4, (cuuint64_t)pl.aH * pl.aW * pl.aC * 4};
+        rc = make_tiled_map(&tmA.m[0], pl.act, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
+        tmA.m[1] = tmA.m[2] = tmA.m[3] = tmA.m[0];
+    }
     if (rc) return rc;
+    const int w_taps = pl.lat ? pl.lat->FH * pl.lat->FW : pl.FH * pl.FW;
     // 3xTF32: split W into hi/lo planes once per call (scratch of this stream), load both by TMA
     const float* w_hi = pl.W;
     const float* w_lo = pl.W_lo ? pl.W_lo : pl.W;
@@ -1267,15 +1328,15 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     // Measured: no gain on the L2-bound tiny-image layers (3.84 against 3.82 ms for the ResNet-18 stack) and a
     // loss on large products (8192^3 C = A * B^T: 187 against 212 TFLOP/s), where the extra shared-memory
     // traffic of the split competes with the operand reads of the MMAs.
-    p.split_b = (mode3x && !pl.W_lo && !pl.b_mn && pl.FH * pl.FW == 1 && opt(OPT_HALO_SPLITB) &&
+    p.split_b = (mode3x && !pl.lat && !pl.W_lo && !pl.b_mn && pl.FH * pl.FW == 1 && opt(OPT_HALO_SPLITB) &&
                  !(t_prepared_lo.W == pl.W && t_prepared_lo.lo)) ? 1 : 0;
     if (mode3x && !pl.W_lo && !p.split_b) {
-        rc = forward_lo_plane(c, stream, pl.W, (size_t)pl.wOC * pl.FH * pl.FW * pl.wIC, &w_lo);
+        rc = forward_lo_plane(c, stream, pl.W, (size_t)pl.wOC * w_taps * pl.wIC, &w_lo);
         if (rc) return rc;
     }
     CUtensorMap tmBlo, tmO;
-    cuuint64_t wd[3] = {(cuuint64_t)pl.wIC, (cuuint64_t)pl.FH * pl.FW, (cuuint64_t)pl.wOC};
-    cuuint64_t wst[2] = {(cuuint64_t)pl.wIC * 4, (cuuint64_t)pl.FH * pl.FW * pl.wIC * 4};
+    cuuint64_t wd[3] = {(cuuint64_t)pl.wIC, (cuuint64_t)w_taps, (cuuint64_t)pl.wOC};
+    cuuint64_t wst[2] = {(cuuint64_t)pl.wIC * 4, (cuuint64_t)w_taps * pl.wIC * 4};
     if (!pl.b_mn) {
         cuuint32_t box[3] = {32, 1, (cuuint32_t)BN};
         rc = make_tiled_map(&tmB, w_hi, 3, wd, wst, box, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -1313,15 +1374,20 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const long long vtiles = (long long)p.total_tiles * ksplit;
     int grid = sm_budget(c) < vtiles ? sm_budget(c) : (int)vtiles;
     HaloLaunch L{grid, smem, stream, &tmA, &tmB, &tmBlo, &tmO, &p};
-    if (ch.flat) { if (ch.row) halo_launch_one<3, 2, 1, true, true>(L); else halo_launch_one<3, 2, 1, false, true>(L); }
+    if (pl.lat) {
+        if (pl.FW == 1) halo_launch_lat<1>(L, ch.JH, ch.JW);
+        else if (pl.FW == 2) halo_launch_lat<2>(L, ch.JH, ch.JW);
+        else halo_launch_lat<3>(L, ch.JH, ch.JW);
+    }
+    else if (ch.flat) { if (ch.row) halo_launch_one<3, 2, 1, true, true>(L); else halo_launch_one<3, 2, 1, false, true>(L); }
     else if (!ch.stat) halo_launch_one<0, 0, 0, false>(L);
     else if (pl.FW == 1) halo_launch_fw<1>(L, ch.JH, ch.JW, ch.row);
     else if (pl.FW == 2) halo_launch_fw<2>(L, ch.JH, ch.JW, ch.row);
     else if (pl.FW == 3) halo_launch_fw<3>(L, ch.JH, ch.JW, ch.row);
     else halo_launch_fw<5>(L, ch.JH, ch.JW, ch.row);
-    note_launch(ch.row ? "halo_row" : (ch.stat ? "halo_tap" : "halo"));
-    snprintf(g_plan, sizeof(g_plan), "halo%s%s%s%s JH=%d JW=%d NI=%d BN=%d npb=%d sb=%d acc=%d eff=%.2f ksplit=%d", ch.row ? "_row" : (ch.stat ? "_tap" : ""),
-             ch.wide ? " wide" : "", p.dual ? " dual" : "", ch.flat ? " flat32" : "", ch.JH, ch.JW, ch.NI, BN, ch.npb, p.sb, ch.acc_bufs, ch.eff, ksplit);
+    note_launch(pl.lat ? "halo_lat" : (ch.row ? "halo_row" : (ch.stat ? "halo_tap" : "halo")));
+    snprintf(g_plan, sizeof(g_plan), "halo%s%s%s%s JH=%d JW=%d NI=%d BN=%d npb=%d sb=%d acc=%d eff=%.2f ksplit=%d cost=%.0f/%.0f", pl.lat ? "_lat" : (ch.row ? "_row" : (ch.stat ? "_tap" : "")),
+             ch.wide ? " wide" : "", p.dual ? " dual" : "", ch.flat ? " flat32" : "", ch.JH, ch.JW, ch.NI, BN, ch.npb, p.sb, ch.acc_bufs, ch.eff, ksplit, ch.cost, pl.lat ? pl.lat->im2col_cost : 0.0);
     rc = check_launch("conv_halo_kernel");
     if (rc || ksplit == 1) return rc;
     const size_t n4 = out_floats / 4;
@@ -1329,8 +1395,51 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
     if (!t_dry) splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(out_ptr), n4, ksplit, pl.bias, pl.ncols / 4,
                                                                pl.act_on, pl.act_k, reinterpret_cast<float4*>(pl.out));
-    note_launch(ch.row ? "halo_row" : (ch.stat ? "halo_tap" : "halo"));
+    note_launch(pl.lat ? "halo_lat" : (ch.row ? "halo_row" : (ch.stat ? "halo_tap" : "halo")));
     return check_launch("splitk_reduce_kernel");
+}
+
+// ---- strided forward: the phases of the stride lattice on the halo kernel ---------------------------
+//
+// The im2col kernel fetches and splits every input pixel once per tap that meets it (9/4 times for 3x3 stride 2) and its
+// three MMAs per step share shared memory with that; here a pixel is fetched and split once, and the wide form of the MMAs
+// applies.  Returns 1 when the shape is left to the im2col kernel.
+static int launch_halo_lattice(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStream_t stream)
+{
+    if (!opt(OPT_HALO_LATTICE) || env_tile_mode() == 1 || pl.b_mn || pl.sh > 2 || pl.sw > 2 || !whole_chunks(pl)) return 1;
+    LatticePlan l;
+    l.FH = pl.FH; l.FW = pl.FW; l.sh = pl.sh; l.sw = pl.sw; l.aH = pl.aH; l.aW = pl.aW; l.aC = pl.aC;
+    // along one axis: taps f with (f - pad) mod s == phase, the first of them at lattice offset floor((f - pad) / s)
+    struct Axis { int taps, first, q; };
+    auto axis = [](int F, int pad, int s, int phase) {
+        Axis a{0, 0, 0};
+        for (int f = 0; f < F; ++f) {
+            const int q = (f - pad) >= 0 ? (f - pad) / s : -((pad - f + s - 1) / s);
+            if (f - pad - q * s != phase) continue;
+            if (!a.taps) { a.first = f; a.q = q; }
+            ++a.taps;
+        }
+        return a;
+    };
+    for (int phi = 0; phi < pl.sh; ++phi)
+        for (int psi = 0; psi < pl.sw; ++psi) {
+            const Axis r = axis(pl.FH, pl.pad_h, pl.sh, phi), q = axis(pl.FW, pl.pad_w, pl.sw, psi);
+            if (!r.taps || !q.taps || phi >= pl.aH || psi >= pl.aW) continue;   // no tap, or a lattice without a pixel: adds nothing
+            l.phi[l.n] = phi; l.psi[l.n] = psi; l.u[l.n] = r.taps; l.v[l.n] = q.taps;
+            l.tap0[l.n] = r.first * pl.FW + q.first; l.h0[l.n] = r.q; l.w0[l.n] = q.q;
+            l.taps += r.taps * q.taps;
+            if (r.taps > l.U) l.U = r.taps;
+            if (q.taps > l.V) l.V = q.taps;
+            ++l.n;
+        }
+    if (!l.n || l.V > 3) return 1;   // (kernels exist for up to three taps of a phase along a row)
+    IgemmPlan g = pl;
+    g.lat = &l;
+    g.FH = l.U; g.FW = l.V; g.sh = g.sw = 1; g.pad_h = g.pad_w = 0;
+    g.kdim = l.n * chunks32(pl.kdim) * 32;
+    g.force = opt(OPT_HALO_LATTICE) == 2;
+    l.im2col_cost = igemm_cost(pl, mode3x, sm_budget(c));
+    return launch_halo(c, g, mode3x, stream);
 }
 
 // ---- channel counts the tensor kernels cannot stage: patch matrix + 1x1 convolution ---------------
@@ -2440,8 +2549,9 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
             if (rc != 1) return rc;
         }
         pl.pad = s->IC % 32 != 0 && env_tile_mode() != 1 && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x);
-        rc = launch_halo(c, pl, mode3x, stream);
-        if (rc != 1 && !(pl.pad && scratch_refused(rc))) return rc;
+        const bool strided = s->sh != 1 || s->sw != 1;
+        rc = strided ? launch_halo_lattice(c, pl, mode3x, stream) : launch_halo(c, pl, mode3x, stream);
+        if (rc != 1 && !((pl.pad || strided) && scratch_refused(rc))) return rc;
         return launch_igemm(c, pl, mode3x, stream);
     }
     if (algo != ALPHA_ALGO_SIMT && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
@@ -2452,7 +2562,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         pl.out = Y; pl.oH = s->OH; pl.oW = s->OW; pl.ncols = s->OC;
         pl.W = W; pl.wOC = s->OC; pl.wIC = s->IC; pl.bias = bias; pl.act_on = act_on; pl.act_k = act_k;
         pl.b_mn = false; pl.flip = false; pl.kdim = s->IC; pl.pad = true;
-        rc = launch_halo(c, pl, cur_mode3x(), stream);
+        rc = (s->sh != 1 || s->sw != 1) ? launch_halo_lattice(c, pl, cur_mode3x(), stream) : launch_halo(c, pl, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
         return launch_igemm(c, pl, cur_mode3x(), stream);
     }

@@ -78,6 +78,13 @@ struct HaloParams {
                               // t * J ... of the flat_total = N * flat_rb4 four-row blocks of the batch (flat_rb4 per image)
     int w_img_rows;           // > 0: every image has its own W (batched matrix products); rows of W per image, added to the
                               // row coordinate of every W tile (stacked images and split-K are then off)
+    // Strided forward (LAT_T): the input pixels one tap meets lie sh rows and sw columns apart, so X is read through one map
+    // per phase of that lattice, whose tiles are dense, and the reduction runs over channel chunks and, innermost, their
+    // lat_n phases (so that phases of few taps, bound by their patch load, lie between phases of many) with a phase's
+    // lat_U x lat_V taps: tap (u, v) is filter tap lat_tap0 + u * lat_du + v * lat_dv and reads lattice row
+    // lat_h0 + u + (output row).  The patch holds the rows and columns of the phase with the most taps.
+    int lat_n, lat_du, lat_dv;
+    int lat_U[4], lat_V[4], lat_tap0[4], lat_h0[4], lat_w0[4];
     int ksplit, cps;          // split-K: every tile is computed as ksplit partial sums over cps reduction chunks each;
                               // partial sp of image n is stored as image sp * N + n of the output map
     uint32_t idesc, idesc_wide, tmem_cols;   // idesc_wide: N = 2 * BN
@@ -85,6 +92,11 @@ struct HaloParams {
     uint32_t patch_tx;     // bytes one patch load delivers
     uint32_t b_bytes;      // one plane of one B stage, multiple of 1024
     uint32_t b_tx;
+};
+
+// Activation tensor maps: entry 0, or (strided forward) one per lattice phase.
+struct HaloAMaps {
+    CUtensorMap m[4];
 };
 
 // Bounded wait that also charges the waited cycles to a counter when profiling is on.
@@ -208,9 +220,11 @@ __device__ __forceinline__ void issue_row(uint32_t d0, uint32_t a_row, uint32_t 
 // straight-line code with immediate descriptor offsets; with ROW_T one B stage holds the FW taps of
 // one filter row, otherwise one tap.  FW_T == 0 is the generic form: any filter, one tap per stage.
 // FLAT_T (static forms only): the JH_T * JW_T accumulators are flat tiles of 4 rows x 32 patch columns, see HaloParams::flat.
-template <int FW_T, int JH_T, int JW_T, bool ROW_T, bool FLAT_T = false>
+// LAT_T (static forms, one tap per stage): strided forward over lattice phases, FW_T = most taps a phase has along a row; a
+// phase with fewer leaves out whole stages, never a single MMA of one.
+template <int FW_T, int JH_T, int JW_T, bool ROW_T, bool FLAT_T = false, bool LAT_T = false>
 __global__ void __launch_bounds__(kHaloThreads2, 1)
-    conv_halo_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+    conv_halo_kernel(const __grid_constant__ HaloAMaps tmAs, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmBlo, const __grid_constant__ CUtensorMap tmO,
                      const HaloParams p)
 {
@@ -258,7 +272,7 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
             mbar_init(&tile_started[i], 1);
         }
         fence_barrier_init();
-        prefetch_tmap(&tmA);
+        prefetch_tmap(&tmAs.m[0]);
         prefetch_tmap(&tmB);
         prefetch_tmap(&tmBlo);
         prefetch_tmap(&tmO);
@@ -313,13 +327,31 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
                             int a = rb * J + j;
                             if (a >= p.flat_total) a = p.flat_total - 1;
                             const int an = a / p.flat_rb4, arb = a - an * p.flat_rb4;
-                            tma_load_4d_a(patches_a + pp.idx * patch_stride + j * sub, &tmA, pfull_a + 8 * pp.idx, c * 32, -p.pad_w,
+                            tma_load_4d_a(patches_a + pp.idx * patch_stride + j * sub, &tmAs.m[0], pfull_a + 8 * pp.idx, c * 32, -p.pad_w,
                                           arb * 4 - p.pad_h, an);
                         }
+                    } else if (LAT_T) {
+                        const int cc = c / p.lat_n, ph = c - cc * p.lat_n;
+                        tma_load_4d_a(patches_a + pp.idx * patch_stride, &tmAs.m[ph], pfull_a + 8 * pp.idx, cc * 32,
+                                      cb * 8 * p.JW + p.lat_w0[ph], rb * 16 * p.JH + p.lat_h0[ph], n);
                     } else {
-                        tma_load_4d_a(patches_a + pp.idx * patch_stride, &tmA, pfull_a + 8 * pp.idx, c * 32, w0, h0, n);
+                        tma_load_4d_a(patches_a + pp.idx * patch_stride, &tmAs.m[0], pfull_a + 8 * pp.idx, c * 32, w0, h0, n);
                     }
                     pp.advance(p.npb);
+                    if constexpr (LAT_T) {
+                        const int cc = c / p.lat_n, ph = c - cc * p.lat_n, V = p.lat_V[ph];
+                        for (int u = 0; u < p.lat_U[ph] && ok; ++u)
+                            for (int v = 0; v < V; ++v) {
+                                if (!wait_prof(bempty_a + 8 * bp.idx, bp.phase ^ 1, prof_on, w_b)) { report(p.status, kStatusProducerTimeout); ok = false; break; }
+                                const uint32_t bar = bfull_a + 8 * bp.idx, b_dst = bring_a + bp.idx * b_stride;
+                                const int tap = p.lat_tap0[ph] + u * p.lat_du + v * p.lat_dv;
+                                mbar_arrive_expect_tx_a(bar, p.b_tx * planes);
+                                tma_load_3d_a(b_dst, &tmB, bar, cc * 32, tap, oc0);
+                                if (p.mode3x) tma_load_3d_a(b_dst + p.b_bytes, &tmBlo, bar, cc * 32, tap, oc0);
+                                bp.advance(p.sb);
+                            }
+                        continue;
+                    }
                     for (int st = 0; st < stages_per_chunk; ++st) {
                         if (!wait_prof(bempty_a + 8 * bp.idx, bp.phase ^ 1, prof_on, w_b)) { report(p.status, kStatusProducerTimeout); ok = false; break; }
                         const uint32_t bar = bfull_a + 8 * bp.idx;
@@ -408,11 +440,14 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
                         }
                     } else if constexpr (kStatic) {
                         constexpr uint32_t kPW8 = FLAT_T ? 256u : (8 * JW_T + FW_T - 1) * 8;
-                        for (int fh = 0; fh < p.FH && ok; ++fh, a_row += kPW8) {
+                        const int ph = LAT_T ? c % p.lat_n : 0;
+                        const int rows = LAT_T ? p.lat_U[ph] : p.FH;
+                        const uint32_t cols = LAT_T ? static_cast<uint32_t>(p.lat_V[ph]) : static_cast<uint32_t>(FW_T);
+                        for (int fh = 0; fh < rows && ok; ++fh, a_row += kPW8) {
                             const uint32_t a_row_lo = a_row + a_lo_off;
                             static_for<0, FW_T>([&](auto fw_) {
                                 constexpr uint32_t fw = decltype(fw_)::value;
-                                if (!ok) return;
+                                if (!ok || (LAT_T && fw >= cols)) return;
                                 const bool take = !dual || ((sg++) & 1u) == which;
                                 if (take) {
                                     if (must_wait) {

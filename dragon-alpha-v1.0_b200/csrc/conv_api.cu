@@ -65,6 +65,7 @@ enum Opt {
     OPT_DW_STRIDED,     // 0 = strided deltaW on the split-K im2col kernel only
     OPT_DW_TAPGROUPS,   // 0 = a CTA always owns a whole filter row, 2 = rows of more than three taps always split
     OPT_HALO_LATTICE,   // strided forward on the halo kernel: 0 never, 1 by cost, 2 wherever possible
+    OPT_HALO_WINDOW,    // layers of few channels as convolutions over windows of a filter row: 0 never, 1 by cost, 2 wherever possible
     OPT_HALO_PAD,       // channels that are no multiple of 32 on the halo kernels: 0 never, 1 by cost, 2 wherever possible
     OPT_COUNT
 };
@@ -75,7 +76,7 @@ static const OptDef kOptDefs[OPT_COUNT] = {
     {"HALO_NARROW", 1}, {"HALO_DUAL", 1}, {"PATCH_MATRIX", 1}, {"DX_PHASES", 1}, {"DX_COL2IM", 1}, {"DX_TRANSPOSE", 1},
     {"DW_STACKED", -1}, {"DW_DIAG", 1}, {"DW_CW", 0}, {"DW_R", 0}, {"DW_STATIC", 1}, {"CONV_PROF", 0}, {"SM_BUDGET", 0},
     {"SKINNY", 1}, {"HALO_DEEP", 1}, {"HALO_SPLITB", 0}, {"NVTX", 1}, {"DW_LANES", 0}, {"HALO_TAPSTACK", 1}, {"HALO_FLAT32", 1},
-    {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_LATTICE", 1}, {"HALO_PAD", 1},
+    {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_LATTICE", 1}, {"HALO_WINDOW", 1}, {"HALO_PAD", 1},
 };
 static std::atomic<int> g_opt[OPT_COUNT];
 static std::once_flag g_opt_once;
@@ -381,7 +382,7 @@ static int check_launch(const char* what);
 // (alpha_conv_weight_cache) a transform is computed once and kept in library-owned memory until
 // alpha_conv_weights_updated() names its source tensor; with the cache off it is recomputed by
 // every call into that call's scratch.
-enum { WK_FWD_LO = 1, WK_DX_S1 = 2, WK_DX_PHASES = 3, WK_DX_COL2IM = 4 };
+enum { WK_FWD_LO = 1, WK_DX_S1 = 2, WK_DX_PHASES = 3, WK_DX_COL2IM = 4, WK_FWD_WINDOW = 5 };
 static std::atomic<int> g_weight_cache{0};
 
 // A forward native that was handed the caller's CW block finds the lo plane kernel_remode left there.
@@ -624,6 +625,7 @@ struct IgemmPlan {
     int oSH = 1, oSW = 1, oNH = 0, oNW = 0;
     bool force = false;              // take the halo kernel even when few tile pixels are real
     int w_img_rows = 0;              // > 0: image n uses rows [n * w_img_rows, ...) of W (batched matrix products)
+    size_t aPix = 0, aRow = 0, aImg = 0;   // floats between pixels, rows and images of the activation (0: dense)
     const struct LatticePlan* lat = nullptr;   // strided forward on the halo kernel: the phases; FH, FW, kdim then describe the
                                      // lattice convolution (most taps of a phase, channels of all phases together)
     bool pad = false;                // kdim may be any multiple of 4: the TMA fills the last 32-channel chunk of both operands with zeros
@@ -647,12 +649,12 @@ static inline bool whole_chunks(const IgemmPlan& pl) { return pl.kdim % 32 == 0 
 // 8 bytes at 5 TB/s, as much as 150 (3xTF32) or 360 columns; blocks of fewer than 64 columns cost as much as 64.
 // Both sides measured, patch matrix or 8-channel im2col tiles first: 50 x 35 x 29, 36 -> 100 channels 3x3 82 / 66 us;
 // 9 x 47 x 47, 280 -> 192 3x3 267 / 165 us; 512 x 1000 times 1000 x 4096 84 / 46 us.
-static bool pad_beats_patch(int K, int taps, int ncols, int mode3x)
+static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, bool strided = false)
 {
     const int force = opt(OPT_HALO_PAD);
     if (force != 1) return force == 2;
     const double nc = ncols < 64 ? 64 : ncols, mem = mode3x ? 150 : 360;
-    return (double)taps * chunks32(K) * nc <= (double)chunks32(taps * K) * (nc + mem);
+    return (double)taps * chunks32(K) * nc * (strided ? 1.4 : 1.0) <= (double)chunks32(taps * K) * (nc + mem);
 }
 // A route that needs scratch may not take away what a route without any could do: under stream capture, or in a
 // caller-owned workspace, the call then goes on to the older route.
@@ -1204,7 +1206,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         skinny = 2 * tiles128 <= sm_budget(c) && (long long)chunks32(pl.kdim) * pl.FH * pl.FW >= 32;
     }
     // per-image weights: only the single-CTA kernel knows them (its W-tile loads add the image's first row)
-    const bool try_pair = !pl.w_img_rows && !pl.lat && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
+    const bool try_pair = !pl.w_img_rows && !pl.lat && !pl.aPix && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
     if (try_pair && !skinny) {
         const int rc2 = launch_halo_pair(c, pl, mode3x, stream);
         if (rc2 != 1) return rc2;
@@ -1214,7 +1216,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const long long flat_m = (long long)pl.aN * pl.aH * pl.aW;
     if (pl.FH == 1 && pl.FW == 1 && pl.pad_h == 0 && pl.pad_w == 0 && pl.oSH == 1 && pl.oSW == 1 && pl.oNH == 0 &&
         pl.oNW == 0 && pl.oH == pl.aH && pl.oW == pl.aW && flat_m % 8 == 0 && flat_m / 8 <= 2147483647LL &&
-        opt(OPT_HALO_FLAT) && !pl.w_img_rows && !pl.lat) {
+        opt(OPT_HALO_FLAT) && !pl.w_img_rows && !pl.lat && !pl.aPix) {
         pl.aN = 1; pl.aW = 8; pl.aH = (int)(flat_m / 8);
         pl.oH = pl.aH; pl.oW = 8;
     }
@@ -1231,7 +1233,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     }
     {
         // plain TF32 with few output channels: one MMA per filter row where the model says it is faster
-        const TapStackPlan ts = (pl.w_img_rows || pl.lat) ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
+        const TapStackPlan ts = (pl.w_img_rows || pl.lat || pl.aPix) ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
         if (ts.valid && (opt(OPT_HALO_TAPSTACK) == 2 || !ch.valid || ts.cost < 0.8 * ch.cost)) return launch_tapstack(c, pl, ts, stream);
     }
     if (!ch.valid || (tile_mode == 0 && ch.eff < 0.6 && !pl.force && !pl.lat)) {
@@ -1315,6 +1317,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     } else {
         cuuint64_t ad[4] = {(cuuint64_t)pl.aC, (cuuint64_t)pl.aW, (cuuint64_t)pl.aH, (cuuint64_t)pl.aN};
         cuuint64_t as[3] = {(cuuint64_t)pl.aC * 4, (cuuint64_t)pl.aW * pl.aC * 4, (cuuint64_t)pl.aH * pl.aW * pl.aC * 4};
+        if (pl.aPix) { as[0] = pl.aPix * 4; as[1] = pl.aRow * 4; as[2] = pl.aImg * 4; }
         rc = make_tiled_map(&tmA.m[0], pl.act, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
         tmA.m[1] = tmA.m[2] = tmA.m[3] = tmA.m[0];
     }
@@ -1498,6 +1501,87 @@ static int launch_patch_gemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cuda
     if (rc != 1) return rc;
     if (g.W_lo) return 1;   // the per-tap kernel splits W itself and cannot take pre-split planes
     return launch_igemm(c, g, mode3x, stream);
+}
+
+// ---- few input channels: windows of a filter row -----------------------------------------------------
+//
+// See window_pack_kernel.  K = FW * sh * IC floats per window, U = ceil(FH / sh) windows (rows) per output pixel.
+struct WindowPlan {
+    int K, U, Hq, Wp;
+    size_t row, elems;      // floats of a row of Xp and of Xp
+    double per_pixel;       // floats of Xp per output pixel
+};
+static WindowPlan window_plan(const AlphaConvShape* s)
+{
+    WindowPlan w;
+    w.K = s->FW * s->sh * s->IC; w.U = (s->FH + s->sh - 1) / s->sh;
+    w.Hq = s->OH + w.U - 1; w.Wp = (s->OW - 1) * s->sw + s->FW;
+    w.row = (size_t)w.Wp * s->sh * s->IC;
+    w.elems = (size_t)s->N * w.Hq * w.row;
+    w.per_pixel = (double)w.Hq * w.row / ((double)s->OH * s->OW);
+    return w;
+}
+static bool window_fits(const AlphaConvShape* s, const WindowPlan& w)
+{
+    return opt(OPT_HALO_WINDOW) && env_tile_mode() != 1 && s->FW > 1 && s->IC % 32 != 0 && w.K <= 512 && w.U <= 64 && w.elems <= 2147483647ull;
+}
+// Forward: windows against zero-filled chunks and the patch matrix, in the units of pad_beats_patch (columns per reduction
+// chunk of 32 and output pixel; a strided layer on zero-filled chunks runs the im2col or lattice kernel, 1.4 times as long).
+// 32 x 224 x 224, 4 -> 64 channels 7x7 s2 (K = 56, U = 4): patch matrix 75 us + 135 us for the product that reads its 360 MB, 116 us
+// here; 64 x 56 x 56, 20 -> 128 3x3: 119 / 102 / 84 us over the patch matrix / zero-filled chunks / windows.  In plain TF32 chunks
+// of a stride-1 layer, whose filter row is one stage, win from 8 channels on (62 against 71 us for 128 x 56 x 56, 8 -> 64).
+static bool window_beats_rest(const AlphaConvShape* s, const WindowPlan& w, int mode3x, int sms)
+{
+    if (!window_fits(s, w)) return false;
+    if (opt(OPT_HALO_WINDOW) == 2) return true;
+    if ((long long)s->N * s->OH * s->OW < 128LL * sms) return false;   // under one tile per SM all forms are launch latency
+    const int taps = s->FH * s->FW;
+    const double nc = s->OC < 64 ? 64 : s->OC, mem = mode3x ? 150 : 360;
+    const bool strided = s->sh != 1 || s->sw != 1;
+    if (!mode3x && !strided && s->IC >= 8) return false;
+    const double own = (double)w.U * chunks32(w.K) * nc + w.per_pixel / 32.0 * mem;
+    const double pad = (double)taps * chunks32(s->IC) * nc * (strided ? 1.4 : 1.0), patch = (double)chunks32(taps * s->IC) * (nc + mem);
+    // (an IC of whole 8-channel tiles has no patch matrix to compare with: it would go to the im2col kernel)
+    return own < 0.9 * (pad < patch || s->IC % 8 == 0 ? pad : patch);
+}
+static int launch_window_pack(DeviceCtx* c, const AlphaConvShape* s, const WindowPlan& w, const float* X, cudaStream_t stream, float** Xp)
+{
+    int rc = get_workspace(c, stream, w.elems * sizeof(float), Xp);
+    if (rc) return rc;
+    const WindowShape ws{s->N, s->IH, s->IW, s->IC, s->sh, s->ph, s->pw, w.Hq, w.Wp};
+    const WindowDivs dv{fast_div(s->IC / 4), fast_div(s->sh), fast_div(w.Wp), fast_div(w.Hq)};
+    size_t blocks = (w.elems / 4 + 255) / 256;
+    if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
+    if (!t_dry) window_pack_kernel<<<(unsigned)blocks, 256, 0, stream>>>(X, reinterpret_cast<float4*>(*Xp), ws, dv);
+    note_launch("window");
+    return check_launch("window_pack_kernel");
+}
+// Returns 1 when no kernel takes the window convolution.
+static int launch_window_forward(DeviceCtx* c, const AlphaConvShape* s, const IgemmPlan& pl_in, const WindowPlan& w, int mode3x, cudaStream_t stream)
+{
+    const size_t nW = (size_t)s->OC * w.U * w.K;
+    float *Ww = nullptr, *Xp = nullptr;
+    bool fresh = true;
+    const DeviceCtx::WeightKey wkey{pl_in.W, WK_FWD_WINDOW, s->OC, s->IC, s->FH * 256 + s->FW, s->sh, mode3x};
+    int rc = weight_planes(c, stream, wkey, (mode3x ? 2 : 1) * nW * sizeof(float), &Ww, &fresh);
+    if (rc) return rc;
+    if (fresh) {
+        size_t blocks = (nW + 255) / 256;
+        if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
+        if (transforms_run()) window_weights_kernel<<<(unsigned)blocks, 256, 0, stream>>>(pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
+        note_launch("window_w");
+        rc = check_launch("window_weights_kernel");
+        if (rc) return rc;
+        weight_planes_ready(c, stream, wkey);
+    }
+    rc = launch_window_pack(c, s, w, pl_in.act, stream, &Xp);
+    if (rc) return rc;
+    IgemmPlan pl = pl_in;
+    pl.act = Xp; pl.aH = w.Hq; pl.aW = s->OW; pl.aC = w.K;
+    pl.aPix = (size_t)s->sw * s->sh * s->IC; pl.aRow = w.row; pl.aImg = w.row * w.Hq;
+    pl.FH = w.U; pl.FW = 1; pl.sh = pl.sw = 1; pl.pad_h = pl.pad_w = 0;
+    pl.W = Ww; pl.W_lo = mode3x ? Ww + nW : nullptr; pl.wIC = w.K; pl.kdim = w.K; pl.pad = true; pl.force = true;
+    return launch_halo(c, pl, mode3x, stream);
 }
 
 // Images so small that the 16 x 8 pixel tiles of the halo kernel stay mostly empty
@@ -1812,9 +1896,10 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
 // deltaB != nullptr: the kernel also sums the columns of deltaY (bias gradient); *bias_fused tells whether it did.
 // per_image: dW receives N separate results, dW[n] = the sum over the pixels of image n only (batched matrix
 // products C[n] = A[n]^T * B[n]); every CTA column of the grid then owns one image and writes its result in place.
+// x_pitch: floats between pixels, rows and images of X where it is not dense (stride 1 only).
 static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float* X, const float* dY, float* dW,
                           int mode3x, cudaStream_t stream, float* deltaB = nullptr, bool* bias_fused = nullptr,
-                          bool per_image = false)
+                          bool per_image = false, const size_t* x_pitch = nullptr)
 {
     if (bias_fused) *bias_fused = false;
     if (opt(OPT_CONV_DW) == 1 && !per_image) return 1;
@@ -1824,7 +1909,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     const long long flat_m = (long long)s_in->N * s_in->OH * s_in->OW;
     if (s_in->FH == 1 && s_in->FW == 1 && s_in->ph == 0 && s_in->pw == 0 && s_in->sh == 1 && s_in->sw == 1 &&
         s_in->IH == s_in->OH && s_in->IW == s_in->OW && flat_m % 16 == 0 && flat_m / 16 <= 2147483647LL &&
-        opt(OPT_HALO_FLAT) && !per_image) {
+        opt(OPT_HALO_FLAT) && !per_image && !x_pitch) {
         flat.N = 1; flat.OW = flat.IW = 16; flat.OH = flat.IH = (int)(flat_m / 16);
         s = &flat;
     }
@@ -1962,6 +2047,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
             cuuint64_t xd[4] = {(cuuint64_t)s->IC, (cuuint64_t)((s->IW - psi + s->sw - 1) / s->sw),
                                 (cuuint64_t)((s->IH - phi + s->sh - 1) / s->sh), (cuuint64_t)s->N};
             cuuint64_t xs[3] = {(cuuint64_t)s->sw * s->IC * 4, (cuuint64_t)s->sh * s->IW * s->IC * 4, (cuuint64_t)s->IH * s->IW * s->IC * 4};
+            if (x_pitch) { xs[0] = x_pitch[0] * 4; xs[1] = x_pitch[1] * 4; xs[2] = x_pitch[2] * 4; }
             cuuint32_t xbox[4] = {32, (cuuint32_t)PW, (cuuint32_t)R, 1};
             rc = make_tiled_map(&tmXs.m[phi * nph + k], X + ((size_t)phi * s->IW + psi) * s->IC, 4, xd, xs, xbox, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
             if (rc) return rc;
@@ -1981,6 +2067,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
         dw_halo_set_attr<3, 2, 8>(); dw_halo_set_attr<3, 4, 8>(); dw_halo_set_attr<3, 8, 8>();
         dw_halo_set_attr<3, 7, 16>(); dw_halo_set_attr<3, 7, 8>();
         dw_halo_set_attr<1, 2, 16>(); dw_halo_set_attr<1, 4, 16>(); dw_halo_set_attr<1, 8, 16>();
+        dw_halo_set_attr<1, 7, 16>(); dw_halo_set_attr<1, 1, 16>(); dw_halo_set_attr<1, 2, 8>(); dw_halo_set_attr<1, 4, 8>(); dw_halo_set_attr<1, 7, 8>(); dw_halo_set_attr<1, 8, 8>();
         dw_halo_set_attr<3, 2, 16, true>(); dw_halo_set_attr<3, 4, 16, true>(); dw_halo_set_attr<3, 8, 16, true>(); dw_halo_set_attr<3, 7, 16, true>();
         dw_halo_set_attr<3, 4, 8, true>(); dw_halo_set_attr<3, 8, 8, true>(); dw_halo_set_attr<3, 7, 8, true>();
         dw_halo_set_attr<4, 2, 16, true>(); dw_halo_set_attr<4, 4, 16, true>(); dw_halo_set_attr<4, 8, 16, true>();
@@ -1991,7 +2078,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
 #define DWH_LAUNCH(FW_, R_, CW_) do { if (!t_dry) conv_dw_halo_kernel<FW_, R_, CW_><<<grid, kDwHaloThreads, smem, stream>>>(tmXs, tmDY, p); } while (0)
 #define DWH_LAUNCH_S(FW_, R_, CW_) do { if (!t_dry) conv_dw_halo_kernel<FW_, R_, CW_, true><<<grid, kDwHaloThreads, smem, stream>>>(tmXs, tmDY, p); } while (0)
     const bool st = G == 3 && !strided && opt(OPT_DW_STATIC) != 0;
-    const bool st1 = s->FW == 1 && CW == 16 && opt(OPT_DW_STATIC) != 0;   // 1x1 (flat 16-column view; with a stride: one phase, start 0)
+    const bool st1 = s->FW == 1 && opt(OPT_DW_STATIC) != 0;   // one tap per row (with a stride: one phase, start 0)
     const bool ss3 = s->FW == 3 && strided && opt(OPT_DW_STATIC) != 0, ss4 = s->FW == 4 && strided && opt(OPT_DW_STATIC) != 0;
     if (ss3 && R == 2 && CW == 16) DWH_LAUNCH_S(3, 2, 16);
     else if (ss3 && R == 4 && CW == 16) DWH_LAUNCH_S(3, 4, 16);
@@ -2018,9 +2105,15 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     else if (st && R == 8 && CW == 8) DWH_LAUNCH(3, 8, 8);
     else if (st && R == 7 && CW == 16) DWH_LAUNCH(3, 7, 16);
     else if (st && R == 7 && CW == 8) DWH_LAUNCH(3, 7, 8);
-    else if (st1 && R == 2) DWH_LAUNCH(1, 2, 16);
-    else if (st1 && R == 4) DWH_LAUNCH(1, 4, 16);
-    else if (st1 && R == 8) DWH_LAUNCH(1, 8, 16);
+    else if (st1 && R == 1 && CW == 16) DWH_LAUNCH(1, 1, 16);
+    else if (st1 && R == 2 && CW == 16) DWH_LAUNCH(1, 2, 16);
+    else if (st1 && R == 4 && CW == 16) DWH_LAUNCH(1, 4, 16);
+    else if (st1 && R == 7 && CW == 16) DWH_LAUNCH(1, 7, 16);
+    else if (st1 && R == 8 && CW == 16) DWH_LAUNCH(1, 8, 16);
+    else if (st1 && R == 2 && CW == 8) DWH_LAUNCH(1, 2, 8);
+    else if (st1 && R == 4 && CW == 8) DWH_LAUNCH(1, 4, 8);
+    else if (st1 && R == 7 && CW == 8) DWH_LAUNCH(1, 7, 8);
+    else if (st1 && R == 8 && CW == 8) DWH_LAUNCH(1, 8, 8);
     else DWH_LAUNCH(0, 0, 0);
 #undef DWH_LAUNCH
 #undef DWH_LAUNCH_S
@@ -2047,22 +2140,62 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     return rc;
 }
 
-// deltaW of a layer whose input channels are no multiple of 32 (IC % 4 == 0): straight from X, with channel blocks whose
-// tail the TMA zero-fills, or over the patch matrix (a 1x1 deltaW with FH * FW * IC channels)?  Both sides in clocks of one
-// SM per 8 pixels: the MMAs of each form, and for the patch matrix 8 bytes per element at 5 TB/s (3.4 clocks per column
-// and 8 pixels over 148 SMs at 1.8 GHz).  50 x 35 x 29, 36 -> 100 channels 3x3: 192 us over the patch matrix, 62 us straight.
-static bool dw_pad_beats_patch(const AlphaConvShape* s, int mode3x)
+// deltaW of a layer whose input channels are no multiple of 32 (IC % 4 == 0): straight from X with channel blocks whose tail
+// the TMA zero-fills, over windows of a filter row (see window_pack_kernel), or over the patch matrix (a 1x1 deltaW with
+// FH * FW * IC channels)?  In clocks of one SM per 8 pixels: the MMAs of each form, and 3.4 clocks per float and pixel that
+// passes through memory on the way (8 bytes at 5 TB/s over 148 SMs at 1.8 GHz).  50 x 35 x 29, 36 -> 100 channels 3x3: 192 us
+// over the patch matrix, 62 us straight; 512 x 32 x 32, 4 -> 64 channels 7x7 s2: 98 us over the patch matrix.
+enum class DwRoute { Patch, Straight, Window };
+static AlphaConvShape window_shape(const AlphaConvShape* s, const WindowPlan& w)
 {
-    const int force = opt(OPT_HALO_PAD);
-    if (force != 1) return force == 2;
-    const bool strided = s->sh != 1 || s->sw != 1;
-    const DwForm own = plan_dw_form(s, strided, false, mode3x);
-    if (own.cost < 0) return false;
+    AlphaConvShape t = *s;
+    t.IH = w.Hq; t.IW = s->OW; t.IC = w.K; t.FH = w.U; t.FW = 1; t.sh = t.sw = 1; t.ph = t.pw = 0;
+    return t;
+}
+static DwRoute pick_dw_route(const AlphaConvShape* s, const WindowPlan& w, int mode3x)
+{
+    const int fpad = opt(OPT_HALO_PAD);
+    if (opt(OPT_HALO_WINDOW) == 2 && window_fits(s, w)) return DwRoute::Window;
+    if (fpad == 2) return DwRoute::Straight;
+    DwRoute best = DwRoute::Patch;
     AlphaConvShape t = *s;
     t.IC = chunks32(s->FH * s->FW * s->IC) * 32; t.FH = t.FW = 1; t.sh = t.sw = 1; t.ph = t.pw = 0;
     t.IH = s->OH; t.IW = s->OW;
     const DwForm patch = plan_dw_form(&t, false, false, mode3x);
-    return patch.cost < 0 || (double)own.cost * s->FH <= (double)patch.cost + 3.4 * t.IC;
+    double cost = patch.cost < 0 ? 1e30 : (double)patch.cost + 3.4 * t.IC;
+    // (windows of more channels read X so often, every window its whole row, that the straight form wins: 36 -> 100 channels in
+    // plain TF32 34 us straight, 57 over windows; 80 -> 64 in 3xTF32 251 and 310)
+    if (window_fits(s, w) && s->IC <= (mode3x ? 32 : 4)) {
+        const AlphaConvShape ws = window_shape(s, w);
+        const DwForm f = plan_dw_form(&ws, false, false, mode3x);
+        const double cw = (double)f.cost * w.U + 3.4 * w.per_pixel;
+        if (f.cost >= 0 && cw < 0.95 * cost) { best = DwRoute::Window; cost = cw; }
+    }
+    if (fpad) {
+        const DwForm own = plan_dw_form(s, s->sh != 1 || s->sw != 1, false, mode3x);
+        if (own.cost >= 0 && (double)own.cost * s->FH <= cost) best = DwRoute::Straight;
+    }
+    return best;
+}
+// Returns 1 when the deltaW kernel does not take the window convolution.
+static int launch_dw_window(DeviceCtx* c, const AlphaConvShape* s, const WindowPlan& w, const float* X, const float* dY, float* dW, int mode3x,
+                            cudaStream_t stream)
+{
+    const AlphaConvShape t = window_shape(s, w);
+    float *Xp = nullptr, *tmp = nullptr;
+    int rc = get_workspace(c, stream, (size_t)s->OC * w.U * w.K * sizeof(float), &tmp);
+    if (rc) return rc;
+    rc = launch_window_pack(c, s, w, X, stream, &Xp);
+    if (rc) return rc;
+    const size_t pitch[3] = {(size_t)s->sw * s->sh * s->IC, w.row, w.row * w.Hq};
+    rc = launch_dw_halo(c, &t, Xp, dY, tmp, mode3x, stream, nullptr, nullptr, false, pitch);
+    if (rc) return rc;
+    const size_t n = (size_t)s->OC * s->FH * s->FW * s->IC;
+    size_t blocks = (n + 255) / 256;
+    if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
+    if (!t_dry) window_unpack_kernel<<<(unsigned)blocks, 256, 0, stream>>>(tmp, dW, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
+    note_launch("dw_window");
+    return check_launch("window_unpack_kernel");
 }
 
 // Batched matrix products (the reference's Cuda_batchMatMul) on the convolution kernels: entry b of the batch is
@@ -2548,14 +2681,31 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
             rc = launch_patch_gemm(c, pl, mode3x, stream);
             if (rc != 1) return rc;
         }
-        pl.pad = s->IC % 32 != 0 && env_tile_mode() != 1 && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x);
+        const WindowPlan win = window_plan(s);
         const bool strided = s->sh != 1 || s->sw != 1;
+        // A layer of few tiles and steps is launch latency: the im2col kernel splits W itself and is one launch (3xTF32)
+        const bool small = mode3x && s->IC % 32 != 0 && igemm_cost(pl, mode3x, sm_budget(c)) < 20000.0;
+        if (window_beats_rest(s, win, mode3x, sm_budget(c))) {
+            rc = launch_window_forward(c, s, pl, win, mode3x, stream);
+            if (rc != 1 && !scratch_refused(rc)) return rc;
+        }
+        pl.pad = s->IC % 32 != 0 && env_tile_mode() != 1 && (!small || opt(OPT_HALO_PAD) == 2) &&
+                 pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x, strided && s->IC % 8 != 0);
         rc = strided ? launch_halo_lattice(c, pl, mode3x, stream) : launch_halo(c, pl, mode3x, stream);
         if (rc != 1 && !((pl.pad || strided) && scratch_refused(rc))) return rc;
         return launch_igemm(c, pl, mode3x, stream);
     }
+    const WindowPlan win = window_plan(s);
+    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && !(tiny_image(s->OH, s->OW) && patch_path_ok(s)) && window_beats_rest(s, win, cur_mode3x(), sm_budget(c))) {
+        IgemmPlan pl{};
+        pl.act = X; pl.aN = s->N;
+        pl.out = Y; pl.oH = s->OH; pl.oW = s->OW; pl.ncols = s->OC;
+        pl.W = W; pl.wOC = s->OC; pl.bias = bias; pl.act_on = act_on; pl.act_k = act_k;
+        rc = launch_window_forward(c, s, pl, win, cur_mode3x(), stream);
+        if (rc != 1 && !scratch_refused(rc)) return rc;
+    }
     if (algo != ALPHA_ALGO_SIMT && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
-        !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x())) {
+        !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x(), s->sh != 1 || s->sw != 1)) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N; pl.aH = s->IH; pl.aW = s->IW; pl.aC = s->IC;
         pl.FH = s->FH; pl.FW = s->FW; pl.sh = s->sh; pl.sw = s->sw; pl.pad_h = s->ph; pl.pad_w = s->pw;
@@ -2672,8 +2822,12 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     const bool tensor_ok = (s->IC % 32 == 0) && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256;
     if (algo == ALPHA_ALGO_TENSOR && !tensor_ok)
         return fail(ALPHA_E_ARG, "tensor deltaW path needs IC %% 32 == 0 (IC=%d)", s->IC);
-    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1 && dw_pad_beats_patch(s, cur_mode3x())) {
-        rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream);
+    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
+        const WindowPlan win = window_plan(s);
+        const DwRoute route = pick_dw_route(s, win, cur_mode3x());
+        rc = 1;
+        if (route == DwRoute::Straight) rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream);
+        else if (route == DwRoute::Window) rc = launch_dw_window(c, s, win, X, deltaY, deltaW, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
     }
     if (algo != ALPHA_ALGO_SIMT && patch_path_ok(s) && env_tile_mode() != 1 &&

@@ -1331,8 +1331,10 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     // Measured: no gain on the L2-bound tiny-image layers (3.84 against 3.82 ms for the ResNet-18 stack) and a
     // loss on large products (8192^3 C = A * B^T: 187 against 212 TFLOP/s), where the extra shared-memory
     // traffic of the split competes with the operand reads of the MMAs.
-    p.split_b = (mode3x && !pl.lat && !pl.W_lo && !pl.b_mn && pl.FH * pl.FW == 1 && opt(OPT_HALO_SPLITB) &&
-                 !(t_prepared_lo.W == pl.W && t_prepared_lo.lo)) ? 1 : 0;
+    // A batched product always does: every entry's W meets only a few row tiles, so a pass over all of them (and a second
+    // read) costs more than the split (256 x 128 x 128 x 256: 12.5 us of 41 us per product).
+    p.split_b = (mode3x && !pl.lat && !pl.W_lo && (pl.w_img_rows || (!pl.b_mn && pl.FH * pl.FW == 1 && opt(OPT_HALO_SPLITB) &&
+                 !(t_prepared_lo.W == pl.W && t_prepared_lo.lo)))) ? 1 : 0;
     if (mode3x && !pl.W_lo && !p.split_b) {
         rc = forward_lo_plane(c, stream, pl.W, (size_t)pl.wOC * w_taps * pl.wIC, &w_lo);
         if (rc) return rc;

@@ -72,7 +72,7 @@ struct HaloParams {
     int mode3x, b_mn, flip;   // mode3x: 0 plain TF32, 1 three MMAs, 2 wide B
     int dual;                 // 1: two MMA-issuing threads take alternate W-tile stages (sb is even)
     int split_b;              // 3xTF32: 1 = only the hi plane of every W tile is loaded and the split warps form its lo
-                              // plane in shared memory (1x1 products, whose W traffic from L2 is what binds them)
+                              // plane in shared memory (batched products; option HALO_SPLITB for other 1x1 products)
     int flat, flat_rb4, flat_total;   // flat = 1: accumulators of 4 output rows x 32 patch columns, each with its own patch of
                               // FH + 3 rows x 32 pixels (images at most 30 pixels wide); macro tile t holds the accumulators
                               // t * J ... of the flat_total = N * flat_rb4 four-row blocks of the batch (flat_rb4 per image)
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
                                 const int tapw = p.flip ? (taps - 1 - tap) : tap;
                                 for (int j = 0; j < p.BN / 32; ++j) {
                                     tma_load_3d_a(b_dst + j * 4096, &tmB, bar, oc0 + j * 32, tapw, c * 32 + wrow0);
-                                    if (p.mode3x) tma_load_3d_a(b_dst + p.b_bytes + j * 4096, &tmBlo, bar, oc0 + j * 32, tapw, c * 32 + wrow0);
+                                    if (p.mode3x && !p.split_b) tma_load_3d_a(b_dst + p.b_bytes + j * 4096, &tmBlo, bar, oc0 + j * 32, tapw, c * 32 + wrow0);
                                 }
                             }
                         }

@@ -481,7 +481,8 @@ class Engine:
         if Bt != Bt2 or K != K2:
             raise ValueError("batchMatMul: A %s against B %s" % (tuple(A.shape), tuple(B.shape)))
         Ap, Bp = _pad_last(A, _pad4(K)), _pad_last(B, _pad4(M))
-        C = torch.zeros((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
+        # the kernels write the M columns; only padding columns need zeros
+        C = (torch.empty if M % 4 == 0 else torch.zeros)((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
         self.base.batchMatMul(C, Ap, Bp, Bt, N, _pad4(M), K, _pad4(K))
         return C[..., :M]
 
@@ -491,7 +492,8 @@ class Engine:
         if Bt != Bt2 or K != K2:
             raise ValueError("batchMatMulT1: A %s against B %s" % (tuple(A.shape), tuple(B.shape)))
         Ap, Bp = _pad_last(A, _pad4(N)), _pad_last(B, _pad4(M))
-        C = torch.zeros((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
+        # the kernels write the M columns; only padding columns need zeros
+        C = (torch.empty if M % 4 == 0 else torch.zeros)((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
         self.base.batchMatMulT1(C, Ap, Bp, Bt, N, _pad4(N), _pad4(M), K)
         return C[..., :M]
 
@@ -501,7 +503,8 @@ class Engine:
         if Bt != Bt2 or K != K2:
             raise ValueError("batchMatMulT2: A %s against B %s" % (tuple(A.shape), tuple(B.shape)))
         Ap, Bp = _pad_last(A, _pad4(K)), _pad_last(B, _pad4(K))
-        C = torch.zeros((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
+        # the kernels write the M columns; only padding columns need zeros
+        C = (torch.empty if M % 4 == 0 else torch.zeros)((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
         self.base.batchMatMulT2(C, Ap, Bp, Bt, N, _pad4(M), M, _pad4(K))
         return C[..., :M]
 

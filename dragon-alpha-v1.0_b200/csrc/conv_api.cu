@@ -1061,7 +1061,7 @@ static int launch_halo_pair(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaS
     cuuint64_t od[4] = {(cuuint64_t)pl.ncols, (cuuint64_t)pl.oW, (cuuint64_t)pl.oH, (cuuint64_t)pl.aN};
     cuuint64_t ost[3] = {(cuuint64_t)pl.oSW * pl.ncols * 4, (cuuint64_t)pl.oSH * oNW * pl.ncols * 4,
                          (cuuint64_t)oNH * oNW * pl.ncols * 4};
-    cuuint32_t obox[4] = {32, (cuuint32_t)(flat32 ? 32 : 8), (cuuint32_t)(flat32 ? 4 : (NI > 1 ? pl.oH : 16)), 1};
+    cuuint32_t obox[4] = {32, (cuuint32_t)(flat32 ? 32 : 8), (cuuint32_t)(flat32 || NI > 1 ? 1 : 4), 1};   // a warp's quarter of a slab
     rc = make_tiled_map(&tmO, pl.out, 4, od, ost, obox, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     int pairs = sm_budget(c) / 2;
@@ -1368,12 +1368,12 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         if (rc) return rc;
         p.bias = nullptr; p.act_on = 0;
     }
-    // output [N][OH][OW][ldo] for the epilogue's TMA stores: one slab = 32 channels x 8 columns x 16 rows
+    // output [N][OH][OW][ldo] for the epilogue's TMA stores of 32 channels at a time
     const int oNH = pl.oNH ? pl.oNH : pl.oH, oNW = pl.oNW ? pl.oNW : pl.oW;
     cuuint64_t od[4] = {(cuuint64_t)pl.ncols, (cuuint64_t)pl.oW, (cuuint64_t)pl.oH, (cuuint64_t)pl.aN * ksplit};
     cuuint64_t ost[3] = {(cuuint64_t)pl.oSW * pl.ncols * 4, (cuuint64_t)pl.oSH * oNW * pl.ncols * 4,
                          (cuuint64_t)oNH * oNW * pl.ncols * 4};
-    cuuint32_t obox[4] = {32, (cuuint32_t)(ch.flat ? 32 : 8), (cuuint32_t)(ch.flat ? 4 : (ch.NI > 1 ? pl.oH : 16)), 1};
+    cuuint32_t obox[4] = {32, (cuuint32_t)(ch.flat ? 32 : 8), (cuuint32_t)(ch.flat || ch.NI > 1 ? 1 : 4), 1};   // a warp's quarter of a slab
     rc = make_tiled_map(&tmO, out_ptr, 4, od, ost, obox, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     const long long vtiles = (long long)p.total_tiles * ksplit;

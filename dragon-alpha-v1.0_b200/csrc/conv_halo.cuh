@@ -124,6 +124,26 @@ __device__ __forceinline__ TilePart tile_part(const HaloParams& p, int v)
     return r;
 }
 
+// Stores the 32 accumulator rows x 32 columns that one epilogue warp has staged (4 KB, 128-byte swizzle): 4 output rows x 8
+// pixels, one row of 32 pixels (flat tiles), or of stacked images those of its four 8-pixel rows that belong to an image (image i
+// starts SG rows further down the accumulator).  Every warp stores its own quarter: a slab of all four warps took a barrier
+// before and after it and, with two slabs in flight, 1900 clocks - more than the MMAs of a layer with a short reduction.
+template <bool FLAT_T>
+__device__ __forceinline__ void store_quarter(const CUtensorMap* tmO, uint32_t src, int quad, int col0, int ow0, int oh0, int n, int n_off,
+                                              const HaloParams& p)
+{
+    if (FLAT_T || p.NI == 1) {
+        const int oh = oh0 + (FLAT_T ? quad : 4 * quad);
+        if (oh < p.OH) tma_store_4d_a(tmO, src, col0, ow0, oh, n + n_off);
+    } else {
+        for (int i = 0; i < 4; ++i) {
+            const int g = quad * 4 + i, img = g / p.SG, r = g - img * p.SG;
+            if (img < p.NI && r < p.OH && n + img < p.N) tma_store_4d_a(tmO, src + i * 1024, col0, ow0, r, n + img + n_off);
+        }
+    }
+    tma_store_commit();
+}
+
 // The four K=8 steps of one 32-channel chunk into one accumulator.  MODE 0: 4 MMAs; 1: 12 MMAs
 // (three per step); 2: 8 MMAs (hi x [hi | lo] over 2*BN columns, then lo x hi over BN columns).
 template <int MODE>
@@ -548,16 +568,14 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
                     for (int c = 0; c < p.BN; c += 32) {
                         const int col0 = n0 + c;
                         if (col0 >= p.Ncols) break;
-                        // slab `sbuf` was last read by the store issued two slabs ago
-                        if (threadIdx.x == 64) tma_store_wait_read<1>();
-                        named_barrier_sync(1, 128);
-                        uint32_t v[32];
+                        uint32_t v[32], w[32];
                         tmem_ld_32x32(tcol + c, v);
+                        if (wide) tmem_ld_32x32(tcol + p.BN + c, w);
+                        // this warp's quarter of slab `sbuf` was last read by the store it issued two slabs ago
+                        if (lane == 0) tma_store_wait_read<1>();
                         tmem_ld_wait();
+                        __syncwarp();
                         if (wide) {
-                            uint32_t w[32];
-                            tmem_ld_32x32(tcol + p.BN + c, w);
-                            tmem_ld_wait();
 #pragma unroll
                             for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(w[q]));
                         }
@@ -575,18 +593,8 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
                             st_shared_v4(srow + ((q ^ (row & 7)) << 4), o);
                         }
                         fence_proxy_async_smem();
-                        named_barrier_sync(1, 128);
-                        if (threadIdx.x == 64) {
-                            if (p.NI == 1) {
-                                tma_store_4d_a(&tmO, stage_a + sbuf * 16384, col0, ow0, oh0, n_img + tp.sp * p.N);
-                            } else {
-                                // stacked images: image i starts SG groups (of 8 rows) further down the slab
-                                for (int img = 0; img < p.NI; ++img)
-                                    if (n + img < p.N)
-                                        tma_store_4d_a(&tmO, stage_a + sbuf * 16384 + img * p.SG * 1024, col0, ow0, 0, n + img + tp.sp * p.N);
-                            }
-                            tma_store_commit();
-                        }
+                        __syncwarp();
+                        if (lane == 0) store_quarter<FLAT_T>(&tmO, stage_a + sbuf * 16384 + quad * 4096, quad, col0, ow0, oh0, n_img, tp.sp * p.N, p);
                         sbuf ^= 1u;
                     }
                 }
@@ -594,7 +602,7 @@ __global__ void __launch_bounds__(kHaloThreads2, 1)
             mbar_arrive_a(aempty_a + 8 * ap.idx);
             ap.advance(p.acc_bufs);
         }
-        if (threadIdx.x == 64) tma_store_wait_all();  // the slabs must outlive their stores
+        if (lane == 0) tma_store_wait_all();  // the slabs must outlive their stores
         if (prof_on && threadIdx.x == 64) {
             p.prof[kProfEpiWait] = w_acc;
             p.prof[kProfEpiWork] = static_cast<unsigned long long>(clock64() - t_begin) - w_acc;

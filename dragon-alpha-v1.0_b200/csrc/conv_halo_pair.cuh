@@ -327,15 +327,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHaloThreads, 1)
             for (int c = 0; c < p.BN; c += 32) {
                 const int col0 = n0 + c;
                 if (col0 >= p.Ncols) break;
-                if (threadIdx.x == 64) tma_store_wait_read<1>();
-                named_barrier_sync(1, 128);
-                uint32_t v[32];
+                uint32_t v[32], w[32];
                 tmem_ld_32x32(tcol + c, v);
+                if (side) tmem_ld_32x32(tcol + p.BN + c, w);
+                if (lane == 0) tma_store_wait_read<1>();
                 tmem_ld_wait();
+                __syncwarp();
                 if (side) {
-                    uint32_t w[32];
-                    tmem_ld_32x32(tcol + p.BN + c, w);
-                    tmem_ld_wait();
 #pragma unroll
                     for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(w[q]));
                 }
@@ -352,24 +350,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHaloThreads, 1)
                     st_shared_v4(srow + ((q ^ (row & 7)) << 4), o);
                 }
                 fence_proxy_async_smem();
-                named_barrier_sync(1, 128);
-                if (threadIdx.x == 64) {
-                    if (p.NI == 1) {
-                        tma_store_4d_a(&tmO, stage_a + sbuf * 16384, col0, ow0, oh0, n);
-                    } else {
-                        for (int img = 0; img < p.NI; ++img)
-                            if (n + img < p.N)
-                                tma_store_4d_a(&tmO, stage_a + sbuf * 16384 + img * p.SG * 1024, col0, ow0, 0, n + img);
-                    }
-                    tma_store_commit();
-                }
+                __syncwarp();
+                if (lane == 0) store_quarter<FLAT_T>(&tmO, stage_a + sbuf * 16384 + quad * 4096, quad, col0, ow0, oh0, n, 0, p);
                 sbuf ^= 1u;
             }
             tc_fence_before_sync();
             mbar_arrive_cluster(aempty_L + 8 * ap.idx);
             ap.advance(p.acc_bufs);
         }
-        if (threadIdx.x == 64) tma_store_wait_all();
+        if (lane == 0) tma_store_wait_all();
     } else {
         // ---- operand split (3xTF32, both CTAs): warps 6..9 ----
         if (p.mode3x) {

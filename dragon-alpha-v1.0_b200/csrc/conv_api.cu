@@ -1236,8 +1236,9 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         const TapStackPlan ts = (pl.w_img_rows || pl.lat || pl.aPix) ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
         if (ts.valid && (opt(OPT_HALO_TAPSTACK) == 2 || !ch.valid || ts.cost < 0.8 * ch.cost)) return launch_tapstack(c, pl, ts, stream);
     }
-    if (!ch.valid || (tile_mode == 0 && ch.eff < 0.6 && !pl.force && !pl.lat)) {
-        // a skinny shape whose tiles the single-CTA kernel would leave mostly empty: the pair kernel after all
+    // (A skinny shape runs half-empty tiles all the same: with its reduction split over the idle SMs, or 64-column tiles on all
+    // of them, they beat the CTA pairs, which would fill half of the SMs with tiles as empty - 64 x 8 x 8, 128 -> 128 channels.)
+    if (!ch.valid || (tile_mode == 0 && ch.eff < 0.6 && !pl.force && !pl.lat && !(try_pair && skinny && ch.eff >= 0.4))) {
         if (try_pair && skinny) {
             const int rc2 = launch_halo_pair(c, pl_in, mode3x, stream);
             if (rc2 != 1) return rc2;
@@ -1985,6 +1986,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     }
     int stages = (int)((220 * 1024) / stage_bytes(R));
     if (stages > 4) stages = 4;
+    if ((size_t)stages * stage_bytes(R) < 16384) return 1;   // the epilogue stages its rows in the ring (24 KB at the least)
     p.R = R; p.CW = CW; p.PW = PW;
     const int tile_rows = diag ? 2 * R : R;   // R = rows per half tile in the diagonal form
     p.row_blocks = (s->OH + tile_rows - 1) / tile_rows; p.col_blocks = (s->OW + CW - 1) / CW;

@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(kDwHaloThreads, 1)
                 const int oc = oc0 + b * 32 + q * 4;
                 if (oc < p.OC) *reinterpret_cast<float4*>(p.bias_out + static_cast<size_t>(blockIdx.x) * p.OC + oc) = a;
             }
+            named_barrier_sync(2, kDwSplitThreads);   // the epilogue stages its rows where the sums lay
         }
         if (warp >= 6) ok = false;   // the extra split warps take no part in the epilogue
         if (ok && !mbar_wait(accum, 0)) { report(p.status, kStatusEpilogueTimeout); ok = false; }
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kDwHaloThreads, 1)
         if (ok) {
             const int quad = warp & 3;
             // stacked: tensor-memory lanes 0-63 are the hi rows, 64-127 the lo rows of the same channels
-            const int oc = oc0 + (stacked ? (quad & 1) * 32 : quad * 32) + lane;
+            const int oc_w = oc0 + (stacked ? (quad & 1) * 32 : quad * 32);   // output channel of this warp's first row
             const int sub = stacked ? (quad >> 1) : 0;
             const int nsub = stacked ? 2 : 1;
             const int taps = p.FH * p.FW;
@@ -405,16 +406,27 @@ __global__ void __launch_bounds__(kDwHaloThreads, 1)
 #pragma unroll
                         for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(w[q]));
                     }
-                    if (oc < p.OC) {
-                        float* dst = obase + (static_cast<size_t>(oc) * taps + tap) * p.IC + ic0 + c;
+                    // A lane holds 32 input channels of one output channel, and rows of deltaW lie taps * IC floats apart: written
+                    // from the registers, a store instruction would touch 32 lines for 16 bytes each.  The warp's 32 x 32 block
+                    // goes through 4 KB of the idle operand ring (16-byte pieces exchanged by row, as the 128-byte swizzle does)
+                    // and leaves as whole 128-byte rows, four per instruction.
+                    const uint32_t blk = smem_a + static_cast<uint32_t>(quad) * 4096u;
+                    __syncwarp();
 #pragma unroll
-                        for (int q = 0; q < 32; q += 4) {
-                            if (ic0 + c + q >= p.IC) break;   // the last block's zero-filled channels
-                            float4 o = has_tiles ? make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]),
-                                                               __uint_as_float(v[q + 2]), __uint_as_float(v[q + 3]))
-                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
-                            *reinterpret_cast<float4*>(dst + q) = o;
-                        }
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 o = has_tiles ? make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
+                                                                 __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]))
+                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+                        st_shared_v4(blk + lane * 128 + ((q ^ (lane & 7)) << 4), o);
+                    }
+                    __syncwarp();
+                    const int piece = lane & 7, ic = ic0 + c + piece * 4;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int row = k * 4 + (lane >> 3), oc = oc_w + row;
+                        const float4 o = ld_shared_v4(blk + row * 128 + ((piece ^ (row & 7)) << 4));
+                        if (oc < p.OC && ic < p.IC)     // (channels past IC are the last block's zeros)
+                            *reinterpret_cast<float4*>(obase + (static_cast<size_t>(oc) * taps + tap) * p.IC + ic) = o;
                     }
                 }
             }

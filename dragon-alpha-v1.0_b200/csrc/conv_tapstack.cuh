@@ -72,13 +72,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         : "memory");
 }
 
-__device__ __forceinline__ float4 ld_shared_v4(uint32_t addr)
-{
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 // 32 channels of one tile row: Y[c] = sum over fw of D[lane + fw][fw * BN + channel], the partial sums of the
 // FW taps gathered from the next lanes.  FW_T = 2 or 3 issues all loads before one wait; FW_T = 0 is any FW.
 template <int FW_T>

@@ -382,6 +382,13 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, float4 v)
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
+__device__ __forceinline__ float4 ld_shared_v4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
 // ---- tensor memory --------------------------------------------------------------------------
 
 // Whole-warp call.  Writes the base address of `ncols` (power of two, >= 32) columns to *dst.

@@ -33,6 +33,28 @@ __global__ void add_bias_rows_kernel(float4* __restrict__ C, const float* __rest
     }
 }
 
+// dst[rows4][cols4] = src[rows][cols] with zeros around it: the engine's pad-to-4 memory rule in one pass.  One thread per four
+// destination floats; the source row pitch is no multiple of 4, so its words are loaded singly (a warp covers 512 consecutive
+// bytes either way).
+__global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, float4* __restrict__ dst, unsigned rows, unsigned cols,
+                                                       unsigned total, FastDiv by_c4)
+{
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        unsigned r, q;
+        by_c4.divmod(i, r, q);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        const unsigned c = q * 4;
+        if (r < rows && c < cols) {
+            const float* p = src + static_cast<size_t>(r) * cols + c;
+            v.x = __ldg(p);
+            if (c + 1 < cols) v.y = __ldg(p + 1);
+            if (c + 2 < cols) v.z = __ldg(p + 2);
+            if (c + 3 < cols) v.w = __ldg(p + 3);
+        }
+        dst[i] = v;
+    }
+}
+
 // `rows` matrix rows as the pixels of a 1x1 convolution: images of 1 x 4 pixels when the row count
 // allows it (the engine pads every dimension to a multiple of 4), single pixels otherwise.  The
 // kernels flatten 1x1 problems over all pixels anyway; the image shape only matters to their fallbacks.
@@ -194,6 +216,24 @@ int alpha_matMulT2(const float* A, const float* B, const float* bias, float* C, 
 }
 
 // ---- batched products (src/cu32_src/Cuda_batch_matMul/Cuda_batchMatMul/test.cuh:95-140 states the three forms) ----
+
+int alpha_pad_rows(const float* src, long long rows, int cols, float* dst, long long rows4, int cols4, alpha_stream_t stream)
+{
+    if (!src || !dst) return fail(ALPHA_E_ARG, "pad_rows: null pointer");
+    if (rows <= 0 || cols <= 0 || rows4 < rows || cols4 < cols || cols4 % 4 != 0)
+        return fail(ALPHA_E_ARG, "pad_rows: bad shape (%lld x %d into %lld x %d)", rows, cols, rows4, cols4);
+    if (reinterpret_cast<uintptr_t>(dst) & 15) return fail(ALPHA_E_ARG, "pad_rows: the destination must be 16-byte aligned");
+    const long long total = rows4 * (cols4 / 4);
+    if (total > 2000000000LL) return fail(ALPHA_E_ARG, "pad_rows: more than 8e9 elements");   // 31-bit indices with a grid stride
+    long long blocks = (total + 255) / 256;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    pad_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        src, reinterpret_cast<float4*>(dst), static_cast<unsigned>(rows), static_cast<unsigned>(cols), static_cast<unsigned>(total), fast_div(cols4 / 4));
+    note_launch("pad_rows");
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "pad_rows_kernel launch failed: %s", cudaGetErrorString(e));
+    return ALPHA_OK;
+}
 
 // C[b][N][M] = A[b][N][AK] (first BK columns) * B[b][BK][M]
 int alpha_batchMatMul(const float* A, const float* B, float* C, int Batch, int N, int M, int BK, int AK, alpha_stream_t stream)

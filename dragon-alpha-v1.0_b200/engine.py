@@ -9,20 +9,29 @@ and the pad-to-4 memory rule of src/alpha_src/z/dragon/engine/Tensor.java:208-22
 PyTorch only provides device memory and streams here; every contraction runs in
 libalpha_conv_b200.so.  There is no CPU or PyTorch fallback: a missing library raises ImportError.
 """
+import contextlib
 import ctypes as C
+import functools
 
 import torch
 
 from . import lib as _l
 
 
-def _ptr(t):
-    return C.c_void_p(t.data_ptr())
-
-
 def _stream(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    """The raw handle of `stream`, or of the current device's current stream."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+# Shapes as the C structures the library reads (it never writes them): a program calls a few layers over and over.
+_conv_shape = functools.lru_cache(maxsize=512)(_l.AlphaConvShape)
+_pool_shape = functools.lru_cache(maxsize=512)(_l.AlphaPoolShape)
+
+
+def _new(like, shape, dtype=torch.float32):
+    return like.new_empty(shape, dtype=dtype)
 
 
 class CudaFloat32EngineBase:
@@ -125,13 +134,13 @@ class CudaFloat32EngineBase:
 
     @staticmethod
     def _addr(a):
-        return C.c_void_p(a.data_ptr()) if isinstance(a, torch.Tensor) else C.c_void_p(int(a))
+        return a.data_ptr() if isinstance(a, torch.Tensor) else int(a)
 
     def conv3D(self, Y_address, OH, OW, X_address, IH, IW, W_address, FH, FW, N, IC, OC, sh, sw, ph, pw):
         """CudaFloat32EngineBase.conv3D (:1355-1474)."""
         a = self._addr
         if self._own_settings():
-            shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+            shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
             return _l.check(self._lib.alpha_conv3d_forward_ex(C.byref(shp), a(X_address), a(W_address), None, a(Y_address),
                                                               self._math, self._algo, _stream(self._stream)))
         _l.check(self._lib.alpha_engine_conv3D(a(Y_address), OH, OW, a(X_address), IH, IW, a(W_address),
@@ -142,7 +151,7 @@ class CudaFloat32EngineBase:
         """CudaFloat32EngineBase.conv3D_biased (:1478-1627); the bias add is fused in the epilogue."""
         a = self._addr
         if self._own_settings():
-            shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+            shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
             return _l.check(self._lib.alpha_conv3d_forward_ex(C.byref(shp), a(X_address), a(W_address), a(Bias_address),
                                                               a(Y_address), self._math, self._algo, _stream(self._stream)))
         _l.check(self._lib.alpha_engine_conv3D_biased(a(Y_address), OH, OW, a(X_address), IH, IW,
@@ -154,7 +163,7 @@ class CudaFloat32EngineBase:
         """CudaFloat32EngineBase.dconv3D_deltaW (:1666-1762)."""
         a = self._addr
         if self._own_settings():
-            shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+            shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
             return _l.check(self._lib.alpha_conv3d_deltaW_ex(C.byref(shp), a(X_address), a(deltaY_address), a(deltaW_address),
                                                              self._math, self._algo, _stream(self._stream)))
         _l.check(self._lib.alpha_engine_dconv3D_deltaW(a(deltaW_address), FH, FW, a(X_address), IH, IW,
@@ -166,7 +175,7 @@ class CudaFloat32EngineBase:
         """CudaFloat32EngineBase.dconv3D_deltaX (:1796-2005)."""
         a = self._addr
         if self._own_settings():
-            shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+            shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
             return _l.check(self._lib.alpha_conv3d_deltaX_ex(C.byref(shp), a(deltaY_address), a(W_address), a(deltaX_address),
                                                              self._math, self._algo, _stream(self._stream)))
         _l.check(self._lib.alpha_engine_dconv3D_deltaX(a(deltaX_address), IH, IW, a(deltaY_address), OH,
@@ -180,7 +189,7 @@ class CudaFloat32EngineBase:
         the block (a torch uint8 tensor, or None when the operator needs none).  A training loop runs these for
         all layers on a side stream after the optimizer step; conv3D / dconv3D_deltaX then take the block through
         their `prepared` argument.  The caller orders prepare before use."""
-        shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+        shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
         nbytes = _l.prepared_weights_bytes(shp, op)
         if nbytes == 0:
             return None
@@ -190,13 +199,13 @@ class CudaFloat32EngineBase:
         return block
 
     def prepare_weights_into(self, block, op, W_address, FH, FW, N, IH, IW, OH, OW, IC, OC, sh, sw, ph, pw, stream=None):
-        shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+        shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
         _l.check(self._lib.alpha_conv_prepare_weights(C.byref(shp), _l.OPS[op], self._addr(W_address), self._addr(block),
                                                       block.numel(), _stream(stream if stream is not None else self._stream)))
 
     def conv3D_prepared(self, Y_address, OH, OW, X_address, IH, IW, W_address, FH, FW, N, IC, OC, sh, sw, ph, pw, prepared):
         a = self._addr
-        shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+        shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
         _l.check(self._lib.alpha_conv3d_forward_prepared(C.byref(shp), a(X_address), a(W_address),
                                                          a(prepared) if prepared is not None else None,
                                                          prepared.numel() if prepared is not None else 0, None, a(Y_address),
@@ -205,7 +214,7 @@ class CudaFloat32EngineBase:
     def dconv3D_deltaX_prepared(self, deltaX_address, IH, IW, deltaY_address, OH, OW, W_address, FH, FW, N, IC, OC, sh, sw, ph, pw,
                                 prepared):
         a = self._addr
-        shp = _l.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+        shp = _conv_shape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
         _l.check(self._lib.alpha_conv3d_deltaX_prepared(C.byref(shp), a(deltaY_address), a(W_address),
                                                         a(prepared) if prepared is not None else None,
                                                         prepared.numel() if prepared is not None else 0, a(deltaX_address),
@@ -213,8 +222,8 @@ class CudaFloat32EngineBase:
 
     # ---- matrix products (CudaFloat32EngineBase.java:1129-1245) ---------------------------------------
     def _mm(self, fn, *args):
-        if self._math >= 0:
-            old = self._lib.alpha_conv_get_math_mode()
+        old = self._lib.alpha_conv_get_math_mode() if self._math >= 0 else self._math
+        if self._math != old:
             _l.check(self._lib.alpha_conv_set_math_mode(self._math))
             try:
                 _l.check(fn(*args))
@@ -264,7 +273,7 @@ class CudaFloat32EngineBase:
 
     # ---- pooling, Java argument order (CudaFloat32EngineBase.java:2012-2215) ----
     def _pool(self, fn, N, IH, IW, IC, FH, FW, OH, OW, sh, sw, ph, pw, *ptrs_and_flags):
-        s = _l.AlphaPoolShape(N, IH, IW, IC, FH, FW, OH, OW, sh, sw, ph, pw)
+        s = _pool_shape(N, IH, IW, IC, FH, FW, OH, OW, sh, sw, ph, pw)
         _l.check(fn(C.byref(s), *ptrs_and_flags, _stream(self._stream)))
 
     def pool2D_max(self, Y_address, OH, OW, X_address, IH, IW, FH, FW, N, IC, sh, sw, ph, pw):
@@ -309,18 +318,25 @@ def _pad4(n):
 
 def _pad_last(t, c4):
     """Copy of t whose last dimension is zero-padded to c4 (Tensor.java:208-221 memory rule)."""
-    if t.shape[-1] == c4:
-        return t.contiguous()
-    out = torch.zeros(t.shape[:-1] + (c4,), dtype=t.dtype, device=t.device)
-    out[..., : t.shape[-1]] = t
-    return out
+    if t.dim() == 1:
+        return _pad_both(t.reshape(1, -1), 1, c4).reshape(-1)
+    return _pad_both(t, t.shape[0], c4)
 
 
-def _pad_first(t, n4):
-    if t.shape[0] == n4:
+def _pad_both(t, n4, c4):
+    """t with its first dimension zero-padded to n4 and its last to c4 (contiguous; t itself where nothing is to pad)."""
+    t = t.contiguous()
+    shape = tuple(t.shape)
+    if shape[-1] == c4 and shape[0] == n4:
         return t
-    out = torch.zeros((n4,) + t.shape[1:], dtype=t.dtype, device=t.device)
-    out[: t.shape[0]] = t
+    if t.dtype != torch.float32 or not t.is_cuda or t.numel() == 0:
+        out = torch.zeros((n4,) + shape[1:-1] + (c4,), dtype=t.dtype, device=t.device)
+        out[: shape[0], ..., : shape[-1]] = t
+        return out
+    out = t.new_empty((n4,) + shape[1:-1] + (c4,))
+    rows = t.numel() // shape[-1]
+    with torch.cuda.device(t.device) if t.device.index != torch.cuda.current_device() else contextlib.nullcontext():
+        _l.check(_l.load().alpha_pad_rows(t.data_ptr(), rows, shape[-1], out.data_ptr(), rows // shape[0] * n4, c4, _stream()))
     return out
 
 
@@ -346,8 +362,8 @@ class Engine:
         OH, OW = self.out_size(IH, IW, FH, FW, sh, sw, ph, pw)
         ic4, oc4 = _pad4(IC), _pad4(OC)
         Xp = _pad_last(X, ic4)
-        Wp = _pad_first(_pad_last(W, ic4), oc4)
-        Y = torch.empty((N, OH, OW, oc4), dtype=torch.float32, device=X.device)
+        Wp = _pad_both(W, oc4, ic4)
+        Y = _new(X, (N, OH, OW, oc4))
         if Bias is None:
             self.base.conv3D(Y, OH, OW, Xp, IH, IW, Wp, FH, FW, N, ic4, oc4, sh, sw, ph, pw)
         else:
@@ -369,10 +385,10 @@ class Engine:
         OH, OW = self.out_size(IH, IW, FH, FW, sh, sw, ph, pw)
         ic4, oc4 = _pad4(IC), _pad4(OC)
         Xp = _pad_last(X, ic4)
-        Wp = _pad_first(_pad_last(W, ic4), oc4)
+        Wp = _pad_both(W, oc4, ic4)
         Bp = None if Bias is None else _pad_last(Bias.reshape(1, -1), oc4).reshape(-1)
-        Y = torch.empty((N, OH, OW, oc4), dtype=torch.float32, device=X.device)
-        shape = _l.AlphaConvShape(N, IH, IW, ic4, oc4, FH, FW, OH, OW, sh, sw, ph, pw)
+        Y = _new(X, (N, OH, OW, oc4))
+        shape = _conv_shape(N, IH, IW, ic4, oc4, FH, FW, OH, OW, sh, sw, ph, pw)
         a = self.base._addr
         _l.check(self.base._lib.alpha_conv3d_forward_leakyRelu(C.byref(shape), a(Xp), a(Wp), a(Bp) if Bp is not None else None,
                                                                float(k), a(Y), _stream(self.base._stream)))
@@ -387,7 +403,7 @@ class Engine:
             raise ValueError("field_sum: row_length must be the last dimension")
         oc4 = _pad4(row_length)
         Xp = _pad_last(X, oc4).contiguous()
-        out = torch.empty((oc4,), dtype=torch.float32, device=X.device)
+        out = _new(X, (oc4,))
         rows = Xp.numel() // oc4
         _l.check(self.base._lib.alpha_conv_bias_grad(self.base._addr(Xp), rows, oc4, self.base._addr(out),
                                                      _stream(self.base._stream)))
@@ -398,7 +414,7 @@ class Engine:
         _, OH, OW, OC = deltaY.shape
         ic4, oc4 = _pad4(IC), _pad4(OC)
         Xp, dYp = _pad_last(X, ic4), _pad_last(deltaY, oc4)
-        dW = torch.empty((oc4, FH, FW, ic4), dtype=torch.float32, device=X.device)
+        dW = _new(X, (oc4, FH, FW, ic4))
         self.base.dconv3D_deltaW(dW, FH, FW, Xp, IH, IW, dYp, OH, OW, N, ic4, oc4, sh, sw, ph, pw)
         return dW if (ic4 == IC and oc4 == OC) else dW[:OC, :, :, :IC]
 
@@ -410,9 +426,9 @@ class Engine:
         _, OH, OW, OC = deltaY.shape
         ic4, oc4 = _pad4(IC), _pad4(OC)
         Xp, dYp = _pad_last(X, ic4), _pad_last(deltaY, oc4)
-        dW = torch.empty((oc4, FH, FW, ic4), dtype=torch.float32, device=X.device)
-        dB = torch.empty((oc4,), dtype=torch.float32, device=X.device)
-        shape = _l.AlphaConvShape(N, IH, IW, ic4, oc4, FH, FW, OH, OW, sh, sw, ph, pw)
+        dW = _new(X, (oc4, FH, FW, ic4))
+        dB = _new(X, (oc4,))
+        shape = _conv_shape(N, IH, IW, ic4, oc4, FH, FW, OH, OW, sh, sw, ph, pw)
         a = self.base._addr
         _l.check(self.base._lib.alpha_conv3d_deltaW_bias(C.byref(shape), a(Xp), a(dYp), a(dW), a(dB), _stream(self.base._stream)))
         return (dW if (ic4 == IC and oc4 == OC) else dW[:OC, :, :, :IC]), (dB if oc4 == OC else dB[:OC])
@@ -422,20 +438,15 @@ class Engine:
         _, FH, FW, IC = W.shape
         ic4, oc4 = _pad4(IC), _pad4(OC)
         dYp = _pad_last(deltaY, oc4)
-        Wp = _pad_first(_pad_last(W, ic4), oc4)
-        dX = torch.empty((N, IH, IW, ic4), dtype=torch.float32, device=deltaY.device)
+        Wp = _pad_both(W, oc4, ic4)
+        dX = _new(deltaY, (N, IH, IW, ic4))
         self.base.dconv3D_deltaX(dX, IH, IW, dYp, OH, OW, Wp, FH, FW, N, ic4, oc4, sh, sw, ph, pw)
         return dX if ic4 == IC else dX[..., :IC]
 
     # ---- matrix products (Engine.matMul / matMulT1 / matMulT2, Engine.java) -------------------------------
     @staticmethod
     def _pad2(t):
-        r4, c4 = _pad4(t.shape[0]), _pad4(t.shape[1])
-        if (r4, c4) == tuple(t.shape):
-            return t.contiguous()
-        out = torch.zeros((r4, c4), dtype=t.dtype, device=t.device)
-        out[: t.shape[0], : t.shape[1]] = t
-        return out
+        return _pad_both(t, _pad4(t.shape[0]), _pad4(t.shape[1]))
 
     def matMul(self, A, B, Bias=None):
         """C[N,M] = A[N,K] * B[K,M] (+ Bias[M] per row); dimensions are zero-padded to multiples of 4 as the
@@ -444,7 +455,7 @@ class Engine:
         if K != K2:
             raise ValueError("A.width=%d != B.height=%d" % (K, K2))
         Ap, Bp = self._pad2(A), self._pad2(B)
-        C = torch.empty((Ap.shape[0], Bp.shape[1]), dtype=torch.float32, device=A.device)
+        C = _new(A, (Ap.shape[0], Bp.shape[1]))
         if Bias is None:
             self.base.matMul(C, Ap, Bp, Ap.shape[0], Bp.shape[1], Ap.shape[1])
         else:
@@ -458,7 +469,7 @@ class Engine:
         if K != K2:
             raise ValueError("A.height=%d != B.height=%d" % (K, K2))
         Ap, Bp = self._pad2(A), self._pad2(B)
-        C = torch.empty((Ap.shape[1], Bp.shape[1]), dtype=torch.float32, device=A.device)
+        C = _new(A, (Ap.shape[1], Bp.shape[1]))
         self.base.matMulT1(C, Ap, Bp, Ap.shape[1], Bp.shape[1], Ap.shape[0])
         return C[:N, :M]
 
@@ -468,7 +479,7 @@ class Engine:
         if K != K2:
             raise ValueError("A.width=%d != B.width=%d" % (K, K2))
         Ap, Bp = self._pad2(A), self._pad2(B)
-        C = torch.empty((Ap.shape[0], Bp.shape[0]), dtype=torch.float32, device=A.device)
+        C = _new(A, (Ap.shape[0], Bp.shape[0]))
         self.base.matMulT2(C, Ap, Bp, Ap.shape[0], Bp.shape[0], Ap.shape[1])
         return C[:N, :M]
 
@@ -512,16 +523,16 @@ class Engine:
     def _pool_shape(self, X, FH, FW, sh, sw, ph, pw):
         N, IH, IW, IC = X.shape
         OH, OW = (IH + 2 * ph - FH) // sh + 1, (IW + 2 * pw - FW) // sw + 1
-        return _l.AlphaPoolShape(N, IH, IW, _pad4(IC), FH, FW, OH, OW, sh, sw, ph, pw), OH, OW
+        return _pool_shape(N, IH, IW, _pad4(IC), FH, FW, OH, OW, sh, sw, ph, pw), OH, OW
 
     def pool2D_max(self, X, FH, FW, sh, sw, ph, pw, indexed=False):
         """Y (and, with indexed=True, the int32 index tensor the indexed gradient reads)."""
         s, OH, OW = self._pool_shape(X, FH, FW, sh, sw, ph, pw)
         IC = X.shape[3]
         Xp = _pad_last(X, s.IC)
-        Y = torch.empty((s.N, OH, OW, s.IC), dtype=torch.float32, device=X.device)
+        Y = _new(X, (s.N, OH, OW, s.IC))
         if indexed:
-            Index = torch.empty((s.N, OH, OW, s.IC), dtype=torch.int32, device=X.device)
+            Index = _new(X, (s.N, OH, OW, s.IC), torch.int32)
             self.base.pool2D_max_indexed(Y, Index, OH, OW, Xp, s.IH, s.IW, FH, FW, s.N, s.IC, sh, sw, ph, pw)
             return (Y if s.IC == IC else Y[..., :IC]), Index
         self.base.pool2D_max(Y, OH, OW, Xp, s.IH, s.IW, FH, FW, s.N, s.IC, sh, sw, ph, pw)
@@ -531,7 +542,7 @@ class Engine:
         s, OH, OW = self._pool_shape(X, FH, FW, sh, sw, ph, pw)
         IC = X.shape[3]
         Xp = _pad_last(X, s.IC)
-        Y = torch.empty((s.N, OH, OW, s.IC), dtype=torch.float32, device=X.device)
+        Y = _new(X, (s.N, OH, OW, s.IC))
         a = self.base._addr
         _l.check(self.base._lib.alpha_pool2D_avg(C.byref(s), a(Xp), a(Y), int(bool(ignore_padding)), _stream(self.base._stream)))
         return Y if s.IC == IC else Y[..., :IC]
@@ -550,9 +561,9 @@ class Engine:
         """deltaX of pool2D_max from the index tensor of the forward pass (its channel count is the padded one)."""
         N, OH, OW, IC = deltaY.shape
         ic4 = Index.shape[3]
-        s = _l.AlphaPoolShape(N, IH, IW, ic4, FH, FW, OH, OW, sh, sw, ph, pw)
+        s = _pool_shape(N, IH, IW, ic4, FH, FW, OH, OW, sh, sw, ph, pw)
         dYp = _pad_last(deltaY, ic4)
-        dX = torch.empty((N, IH, IW, ic4), dtype=torch.float32, device=deltaY.device)
+        dX = _new(deltaY, (N, IH, IW, ic4))
         a = self.base._addr
         _l.check(self.base._lib.alpha_upool2D_max_indexed(C.byref(s), a(dYp), a(Index), a(dX), _stream(self.base._stream)))
         return dX if ic4 == IC else dX[..., :IC]
@@ -560,9 +571,9 @@ class Engine:
     def upool2D_avg(self, deltaY, IH, IW, FH, FW, sh, sw, ph, pw, ignore_padding=False):
         N, OH, OW, IC = deltaY.shape
         ic4 = _pad4(IC)
-        s = _l.AlphaPoolShape(N, IH, IW, ic4, FH, FW, OH, OW, sh, sw, ph, pw)
+        s = _pool_shape(N, IH, IW, ic4, FH, FW, OH, OW, sh, sw, ph, pw)
         dYp = _pad_last(deltaY, ic4)
-        dX = torch.empty((N, IH, IW, ic4), dtype=torch.float32, device=deltaY.device)
+        dX = _new(deltaY, (N, IH, IW, ic4))
         a = self.base._addr
         _l.check(self.base._lib.alpha_upool2D_avg(C.byref(s), a(dYp), a(dX), int(bool(ignore_padding)), _stream(self.base._stream)))
         return dX if ic4 == IC else dX[..., :IC]

@@ -400,6 +400,9 @@ int alpha_engine_matMul_biased(float* C, const float* A, const float* B, int N, 
 int alpha_engine_matMulT1(float* C, const float* A, const float* B, int N, int M, int K, alpha_stream_t stream);
 int alpha_engine_matMulT2(float* C, const float* A, const float* B, int N, int M, int K, alpha_stream_t stream);
 
+/* dst[rows4][cols4] = src[rows][cols] (dense), zeros where src has no element; cols4 % 4 == 0, dst 16-byte aligned. */
+int alpha_pad_rows(const float* src, long long rows, int cols, float* dst, long long rows4, int cols4, alpha_stream_t stream);
+
 /* ---- batched matrix products (FullConnect / attention-style operators) ----------------------------------
  * Replace the SIMT kernels behind src/cu32_src/Cuda_batch_matMul/Cuda_batchMatMul/batchMatMul.cuh,
  * batchMatMulT1.cuh, batchMatMulT2.cuh (the three forms are stated as CPU loops in its test.cuh:95-140).

@@ -472,7 +472,7 @@ static int forward_lo_plane(DeviceCtx* c, cudaStream_t stream, const float* W, s
         const size_t n4 = nW / 4;
         size_t blocks = (n4 + 255) / 256;
         if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-        if (transforms_run()) split_lo_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(W), reinterpret_cast<float4*>(ws), n4);
+        if (transforms_run()) launch_after(split_lo_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(W), reinterpret_cast<float4*>(ws), n4);
         note_launch("split_w");
         rc = check_launch("split_lo_kernel");
         if (rc) return rc;
@@ -490,7 +490,7 @@ int launch_split_lo(cudaStream_t stream, const float* W, float* lo, size_t n)
     size_t blocks = (n4 + 255) / 256;
     if (blocks > (size_t)sms * 8) blocks = (size_t)sms * 8;
     if (blocks < 1) blocks = 1;
-    split_lo_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(W), reinterpret_cast<float4*>(lo), n4);
+    launch_after(split_lo_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(W), reinterpret_cast<float4*>(lo), n4);
     note_launch("split_w");
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "split_lo_kernel launch failed: %s", cudaGetErrorString(e));
@@ -721,7 +721,7 @@ static int launch_igemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStrea
     if (rc) return rc;
 
     dim3 grid((p.M_total + kBM - 1) / kBM, (pl.ncols + BN - 1) / BN, 1);
-    if (!t_dry) conv_igemm_kernel<<<grid, kIgemmThreads, smem, stream>>>(tmA, tmB, p);
+    if (!t_dry) launch_after(conv_igemm_kernel, grid, kIgemmThreads, smem, stream, tmA, tmB, p);
     note_launch("igemm");
     return check_launch("conv_igemm_kernel");
 }
@@ -765,7 +765,7 @@ static void halo_launch_one(const HaloLaunch& L)
         cudaFuncSetAttribute(conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_done = true;
     }
-    if (!t_dry) conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T><<<L.grid, kHaloThreads2, L.smem, L.stream>>>(*L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+    if (!t_dry) launch_after(conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T>, L.grid, kHaloThreads2, L.smem, L.stream, *L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
 }
 
 template <int FW_T>
@@ -957,7 +957,7 @@ static void halo_pair_launch_one(const HaloLaunch& L)
         cudaFuncSetAttribute(conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr_done = true;
     }
-    if (!t_dry) conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T><<<L.grid, kHaloThreads, L.smem, L.stream>>>(L.tmA->m[0], *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+    if (!t_dry) launch_after(conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T>, L.grid, kHaloThreads, L.smem, L.stream, L.tmA->m[0], *L.tmB, *L.tmBlo, *L.tmO, *L.p);
 }
 
 // One 16 x 8 pixel accumulator per CTA, two CTAs per MMA.  Returns 1 when the shape does not fit.
@@ -1399,7 +1399,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const size_t n4 = out_floats / 4;
     size_t blocks = (n4 + 255) / 256;
     if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-    if (!t_dry) splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(out_ptr), n4, ksplit, pl.bias, pl.ncols / 4,
+    if (!t_dry) launch_after(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(out_ptr), n4, ksplit, pl.bias, pl.ncols / 4,
                                                                pl.act_on, pl.act_k, reinterpret_cast<float4*>(pl.out));
     note_launch(pl.lat ? "halo_lat" : (ch.row ? "halo_row" : (ch.stat ? "halo_tap" : "halo")));
     return check_launch("splitk_reduce_kernel");
@@ -1471,7 +1471,7 @@ static int make_patch_matrix(DeviceCtx* c, PatchShape ps, const float* X, cudaSt
     const bool idx32 = M * (size_t)Kp <= 2147483647ull && (size_t)ps.N * ps.IH * ps.IW * ps.IC <= 2147483647ull;
     if (idx32) {
         const PatchDivs dv{fast_div(Kp / 4), fast_div(ps.IC), fast_div(ps.FW), fast_div(ps.OW), fast_div(ps.OH)};
-        if (!t_dry) patch_matrix32_kernel<<<(unsigned)blocks, 256, 0, stream>>>(X, ws, ps, dv);
+        if (!t_dry) launch_after(patch_matrix32_kernel, (unsigned)blocks, 256, 0, stream, X, ws, ps, dv);
     } else {
         if (!t_dry) patch_matrix_kernel<<<(unsigned)blocks, 256, 0, stream>>>(X, ws, ps);
     }
@@ -1555,7 +1555,7 @@ static int launch_window_pack(DeviceCtx* c, const AlphaConvShape* s, const Windo
     const WindowDivs dv{fast_div(s->IC / 4), fast_div(s->sh), fast_div(w.Wp), fast_div(w.Hq)};
     size_t blocks = (w.elems / 4 + 255) / 256;
     if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
-    if (!t_dry) window_pack_kernel<<<(unsigned)blocks, 256, 0, stream>>>(X, reinterpret_cast<float4*>(*Xp), ws, dv);
+    if (!t_dry) launch_after(window_pack_kernel, (unsigned)blocks, 256, 0, stream, X, reinterpret_cast<float4*>(*Xp), ws, dv);
     note_launch("window");
     return check_launch("window_pack_kernel");
 }
@@ -1571,7 +1571,7 @@ static int launch_window_forward(DeviceCtx* c, const AlphaConvShape* s, const Ig
     if (fresh) {
         size_t blocks = (nW + 255) / 256;
         if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-        if (transforms_run()) window_weights_kernel<<<(unsigned)blocks, 256, 0, stream>>>(pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
+        if (transforms_run()) launch_after(window_weights_kernel, (unsigned)blocks, 256, 0, stream, pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
         note_launch("window_w");
         rc = check_launch("window_weights_kernel");
         if (rc) return rc;
@@ -1646,7 +1646,7 @@ static int launch_dx_phases(DeviceCtx* c, const AlphaConvShape* s, const float* 
             woff += pn;
             if (fresh) {
                 dim3 tg((s->IC + 31) / 32, (s->OC + 31) / 32, ptaps);
-                if (transforms_run()) transpose_weights_kernel<<<tg, 256, 0, stream>>>(W, whi, wlo, s->OC, s->IC, taps, map, mode3x);
+                if (transforms_run()) launch_after(transpose_weights_kernel, tg, 256, 0, stream, W, whi, wlo, s->OC, s->IC, taps, map, mode3x, 0);
                 note_launch("transpose_w");
                 rc = check_launch("transpose_weights_kernel");
                 if (rc) return rc;
@@ -1740,7 +1740,7 @@ static int launch_dx_col2im(DeviceCtx* c, const AlphaConvShape* s, const float* 
         map.n = taps;
         for (int t = 0; t < taps; ++t) map.src[t] = t;
         dim3 tg((s->IC + 31) / 32, (s->OC + 31) / 32, taps);
-        if (transforms_run()) transpose_weights_kernel<<<tg, 256, 0, stream>>>(W, ws, mode3x ? ws + nW : nullptr, s->OC, s->IC, taps, map, mode3x, tap_major);
+        if (transforms_run()) launch_after(transpose_weights_kernel, tg, 256, 0, stream, W, ws, mode3x ? ws + nW : nullptr, s->OC, s->IC, taps, map, mode3x, tap_major);
         note_launch("transpose_w");
         rc = check_launch("transpose_weights_kernel");
         if (rc) return rc;
@@ -1763,8 +1763,8 @@ static int launch_dx_col2im(DeviceCtx* c, const AlphaConvShape* s, const float* 
     if (idx32) {
         const GatherDivs dv{fast_div(s->IC / 4), fast_div(s->IW), fast_div(s->IH), fast_div(s->sh), fast_div(s->sw)};
         if (!t_dry) {
-            if (tap_major) col2im_gather_tapmajor32_kernel<<<(unsigned)blocks, 256, 0, stream>>>(P, dX, ps, dv);
-            else col2im_gather32_kernel<<<(unsigned)blocks, 256, 0, stream>>>(P, dX, ps, dv);
+            if (tap_major) launch_after(col2im_gather_tapmajor32_kernel, (unsigned)blocks, 256, 0, stream, P, dX, ps, dv);
+            else launch_after(col2im_gather32_kernel, (unsigned)blocks, 256, 0, stream, P, dX, ps, dv);
         }
     } else if (tap_major) {
         if (!t_dry) col2im_gather_tapmajor_kernel<<<(unsigned)blocks, 256, 0, stream>>>(P, dX, ps);
@@ -1818,7 +1818,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
     const size_t n4 = g.size / 4;
     size_t blocks = (n4 + 255) / 256;
     if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-    if (!t_dry) splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(g.out), n4, g.ksplit, nullptr, 1, 0, 0.f,
+    if (!t_dry) launch_after(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(g.out), n4, g.ksplit, nullptr, 1, 0, 0.f,
                                                                reinterpret_cast<float4*>(dX));
     note_launch("simt");
     return check_launch("splitk_reduce_kernel");
@@ -2079,8 +2079,8 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
         dw_halo_set_attr<3, 2, 8, true>(); dw_halo_set_attr<4, 2, 8, true>(); dw_halo_set_attr<4, 7, 8, true>(); dw_halo_set_attr<4, 7, 16, true>();
         attr_done = true;
     }
-#define DWH_LAUNCH(FW_, R_, CW_) do { if (!t_dry) conv_dw_halo_kernel<FW_, R_, CW_><<<grid, kDwHaloThreads, smem, stream>>>(tmXs, tmDY, p); } while (0)
-#define DWH_LAUNCH_S(FW_, R_, CW_) do { if (!t_dry) conv_dw_halo_kernel<FW_, R_, CW_, true><<<grid, kDwHaloThreads, smem, stream>>>(tmXs, tmDY, p); } while (0)
+#define DWH_LAUNCH(FW_, R_, CW_) do { if (!t_dry) launch_after(conv_dw_halo_kernel<FW_, R_, CW_>, grid, kDwHaloThreads, smem, stream, tmXs, tmDY, p); } while (0)
+#define DWH_LAUNCH_S(FW_, R_, CW_) do { if (!t_dry) launch_after(conv_dw_halo_kernel<FW_, R_, CW_, true>, grid, kDwHaloThreads, smem, stream, tmXs, tmDY, p); } while (0)
     const bool st = G == 3 && !strided && opt(OPT_DW_STATIC) != 0;
     const bool st1 = s->FW == 1 && opt(OPT_DW_STATIC) != 0;   // one tap per row (with a stride: one phase, start 0)
     const bool ss3 = s->FW == 3 && strided && opt(OPT_DW_STATIC) != 0, ss4 = s->FW == 4 && strided && opt(OPT_DW_STATIC) != 0;
@@ -2135,7 +2135,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     if (!rc && bias_parts) {
         // the `parts` partial rows are a matrix whose columns want summing: 4 float4 columns x 64 row lanes per CTA
         const int cols4 = s->OC / 4, CT2 = cols4 < 4 ? cols4 : 4;
-        if (!t_dry) field_sum_partial_kernel<<<dim3(1, (unsigned)((cols4 + CT2 - 1) / CT2)), kFieldSumThreads, 0, stream>>>(
+        if (!t_dry) launch_after(field_sum_partial_kernel, dim3(1, (unsigned)((cols4 + CT2 - 1) / CT2)), kFieldSumThreads, 0, stream, 
             reinterpret_cast<const float4*>(bias_parts), parts, cols4, CT2, 64, reinterpret_cast<float4*>(deltaB));
         note_launch("dw_halo");
         rc = check_launch("field_sum_partial_kernel");
@@ -2197,7 +2197,7 @@ static int launch_dw_window(DeviceCtx* c, const AlphaConvShape* s, const WindowP
     const size_t n = (size_t)s->OC * s->FH * s->FW * s->IC;
     size_t blocks = (n + 255) / 256;
     if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-    if (!t_dry) window_unpack_kernel<<<(unsigned)blocks, 256, 0, stream>>>(tmp, dW, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
+    if (!t_dry) launch_after(window_unpack_kernel, (unsigned)blocks, 256, 0, stream, tmp, dW, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
     note_launch("dw_window");
     return check_launch("window_unpack_kernel");
 }
@@ -2318,7 +2318,7 @@ static int launch_dw_split(const AlphaConvShape* s, const float* X, const float*
     rc = make_tiled_map(&tmDY, deltaY, 2, dd, ds, box, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
     if (rc) return rc;
     dim3 grid(pl.groups, pl.n_tiles, pl.splits);
-    if (!t_dry) conv_dw_kernel<<<grid, kIgemmThreads, pl.smem, stream>>>(tmX, tmDY, p);
+    if (!t_dry) launch_after(conv_dw_kernel, grid, kIgemmThreads, pl.smem, stream, tmX, tmDY, p);
     note_launch(tag);
     rc = check_launch("conv_dw_kernel");
     if (rc) return rc;
@@ -2633,7 +2633,7 @@ int alpha_conv_bias_grad(const float* deltaY, long long rows, int OC, float* del
     float* ws = nullptr;
     rc = get_workspace(c, stream, (size_t)gx * OC * sizeof(float), &ws);
     if (rc) return rc;
-    if (!t_dry) field_sum_partial_kernel<<<dim3((unsigned)gx, (unsigned)gy), kFieldSumThreads, 0, stream>>>(
+    if (!t_dry) launch_after(field_sum_partial_kernel, dim3((unsigned)gx, (unsigned)gy), kFieldSumThreads, 0, stream, 
         reinterpret_cast<const float4*>(deltaY), rows, cols4, CT, RL, reinterpret_cast<float4*>(ws));
     note_launch("field_sum");
     rc = check_launch("field_sum_partial_kernel");
@@ -2642,7 +2642,7 @@ int alpha_conv_bias_grad(const float* deltaY, long long rows, int OC, float* del
     // (few rows, so the pass is bound by load latency: many lanes, few loads each)
     const int CT2 = cols4 < 4 ? cols4 : 4;
     const int RL2 = 64;
-    if (!t_dry) field_sum_partial_kernel<<<dim3(1, (unsigned)((cols4 + CT2 - 1) / CT2)), kFieldSumThreads, 0, stream>>>(
+    if (!t_dry) launch_after(field_sum_partial_kernel, dim3(1, (unsigned)((cols4 + CT2 - 1) / CT2)), kFieldSumThreads, 0, stream, 
         reinterpret_cast<const float4*>(ws), gx, cols4, CT2, RL2, reinterpret_cast<float4*>(deltaB));
     note_launch("field_sum");
     return check_launch("field_sum_partial_kernel");
@@ -2781,7 +2781,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
                 TapMap map{};
                 map.n = taps;
                 for (int t = 0; t < taps; ++t) map.src[t] = taps - 1 - t;
-                if (transforms_run()) transpose_weights_kernel<<<tg, 256, 0, stream>>>(W, ws, mode3x ? ws + nW : nullptr, s->OC, s->IC, taps, map, mode3x);
+                if (transforms_run()) launch_after(transpose_weights_kernel, tg, 256, 0, stream, W, ws, mode3x ? ws + nW : nullptr, s->OC, s->IC, taps, map, mode3x, 0);
                 note_launch("transpose_w");
                 rc = check_launch("transpose_weights_kernel");
                 if (rc) return rc;
@@ -2853,7 +2853,7 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
             const size_t total4 = (size_t)s->OC * (K / 4);
             size_t blocks = (total4 + 255) / 256;
             if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
-            if (!t_dry) unpad_rows_kernel<<<(unsigned)blocks, 256, 0, stream>>>(dWp, deltaW, s->OC, K, Kp);
+            if (!t_dry) launch_after(unpad_rows_kernel, (unsigned)blocks, 256, 0, stream, dWp, deltaW, s->OC, K, Kp);
             note_launch("dw_patch");
             return check_launch("unpad_rows_kernel");
         }

@@ -123,8 +123,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHaloThreads, 1)
         tmem_relinquish_pair();
     }
     tc_fence_before_sync();
+    grid_dependency_wait();
     __syncthreads();
     cluster_sync_all();   // the peer's barriers are initialised before anything reaches them
+    grid_dependency_trigger();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
 

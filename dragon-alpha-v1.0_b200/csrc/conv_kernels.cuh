@@ -14,6 +14,7 @@
 #pragma once
 #include "sm100_ptx.cuh"
 #include "fast_div.cuh"
+#include "host_common.h"
 
 namespace alpha {
 
@@ -195,6 +196,8 @@ struct PatchDivs {
 __global__ void __launch_bounds__(256) patch_matrix32_kernel(const float* __restrict__ X, float* __restrict__ A, const PatchShape s,
                                                              const PatchDivs dv)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const unsigned k4n = static_cast<unsigned>(s.Kp) >> 2;
     const unsigned total = static_cast<unsigned>(s.N) * s.OH * s.OW * k4n;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -231,6 +234,8 @@ struct WindowDivs {
 __global__ void __launch_bounds__(256) window_pack_kernel(const float* __restrict__ X, float4* __restrict__ Xp, const WindowShape s,
                                                           const WindowDivs dv)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const unsigned c4 = static_cast<unsigned>(s.IC) >> 2;
     const unsigned total = static_cast<unsigned>(s.N) * s.Hq * s.Wp * s.sh * c4;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -252,6 +257,8 @@ __global__ void __launch_bounds__(256) window_pack_kernel(const float* __restric
 __global__ void __launch_bounds__(256) window_weights_kernel(const float* __restrict__ W, float* __restrict__ Ww, float* __restrict__ lo,
                                                              int OC, int FH, int FW, int IC, int sh, int U)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const int K = FW * sh * IC;
     const size_t total = static_cast<size_t>(OC) * U * K;
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -267,6 +274,8 @@ __global__ void __launch_bounds__(256) window_weights_kernel(const float* __rest
 __global__ void __launch_bounds__(256) window_unpack_kernel(const float* __restrict__ src, float* __restrict__ dW, int OC, int FH, int FW, int IC,
                                                             int sh, int U)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const int K = FW * sh * IC;
     const size_t total = static_cast<size_t>(OC) * FH * FW * IC;
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -283,6 +292,8 @@ __global__ void __launch_bounds__(256) window_unpack_kernel(const float* __restr
 // dst[r][0..K) = src[r][0..K) of a matrix with row pitch Kp (drops the zero padding columns).
 __global__ void __launch_bounds__(256) unpad_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int rows, int K, int Kp)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const int k4n = K >> 2;
     const size_t total = static_cast<size_t>(rows) * k4n;
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -384,6 +395,8 @@ struct GatherDivs {
 __global__ void __launch_bounds__(256) col2im_gather_tapmajor32_kernel(const float* __restrict__ P, float* __restrict__ dX, const PatchShape s,
                                                                          const GatherDivs dv)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const unsigned c4n = static_cast<unsigned>(s.IC) >> 2;
     const unsigned ldp = static_cast<unsigned>(s.IC) * s.FH * s.FW;
     const unsigned total = static_cast<unsigned>(s.N) * s.IH * s.IW * c4n;
@@ -415,6 +428,8 @@ __global__ void __launch_bounds__(256) col2im_gather_tapmajor32_kernel(const flo
 __global__ void __launch_bounds__(256) col2im_gather32_kernel(const float* __restrict__ P, float* __restrict__ dX, const PatchShape s,
                                                               const GatherDivs dv)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const unsigned c4n = static_cast<unsigned>(s.IC) >> 2;
     const unsigned taps = static_cast<unsigned>(s.FH) * s.FW, ldp = static_cast<unsigned>(s.IC) * taps;
     const unsigned total = static_cast<unsigned>(s.N) * s.IH * s.IW * c4n;
@@ -461,6 +476,8 @@ __global__ void split_tensor_kernel(const float4* __restrict__ src, float4* __re
 __global__ void splitk_reduce_kernel(const float4* __restrict__ part, size_t n4, int splits, const float* __restrict__ bias,
                                      int ncols4, int act_on, float act_k, float4* __restrict__ out)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         float4 a = part[i];
@@ -481,6 +498,8 @@ __global__ void splitk_reduce_kernel(const float4* __restrict__ part, size_t n4,
 // only the upper 19 bits of an operand word): lo = tf32(x - trunc19(x)).
 __global__ void split_lo_kernel(const float4* __restrict__ src, float4* __restrict__ lo, size_t n4)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const float4 a = src[i];
@@ -502,6 +521,8 @@ __global__ void __launch_bounds__(256)
     transpose_weights_kernel(const float* __restrict__ W, float* __restrict__ hi, float* __restrict__ lo, int OC,
                              int IC, int taps, const TapMap map, int split, int tap_major = 0)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     __shared__ float tile[32][33];
     const int t = blockIdx.z, tap = map.src[t], ic0 = blockIdx.x * 32, oc0 = blockIdx.y * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -564,7 +585,9 @@ __global__ void __launch_bounds__(kIgemmThreads)
         tmem_relinquish();
     }
     tc_fence_before_sync();
+    grid_dependency_wait();
     __syncthreads();
+    grid_dependency_trigger();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
 
@@ -758,7 +781,9 @@ __global__ void __launch_bounds__(kIgemmThreads)
         tmem_relinquish();
     }
     tc_fence_before_sync();
+    grid_dependency_wait();
     __syncthreads();
+    grid_dependency_trigger();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
 
@@ -900,6 +925,8 @@ template <int LANES>
 __global__ void dw_reduce_kernel(const float* __restrict__ part, size_t split_stride, int splits,
                                  float* __restrict__ out, size_t n4, int accumulate)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t i = t / LANES;
     const int lane = static_cast<int>(t % LANES);
@@ -952,9 +979,9 @@ inline void launch_dw_reduce(const float* part, size_t split_stride, int splits,
 {
     if (lanes == 4 || (lanes == 0 && splits >= 32)) {
         const size_t threads = n4 * 4;
-        dw_reduce_kernel<4><<<static_cast<unsigned>((threads + 127) / 128), 128, 0, stream>>>(part, split_stride, splits, out, n4, accumulate);
+        launch_after(dw_reduce_kernel<4>, static_cast<unsigned>((threads + 127) / 128), 128, 0, stream, part, split_stride, splits, out, n4, accumulate);
     } else {
-        dw_reduce_kernel<1><<<static_cast<unsigned>((n4 + 63) / 64), 64, 0, stream>>>(part, split_stride, splits, out, n4, accumulate);
+        launch_after(dw_reduce_kernel<1>, static_cast<unsigned>((n4 + 63) / 64), 64, 0, stream, part, split_stride, splits, out, n4, accumulate);
     }
 }
 
@@ -970,6 +997,8 @@ __global__ void __launch_bounds__(kFieldSumThreads)
     field_sum_partial_kernel(const float4* __restrict__ x, long long rows, int cols4, int CT, int RL,
                              float4* __restrict__ partials)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     __shared__ float4 red[kFieldSumThreads];
     const int tid = threadIdx.x;
     const int rl = tid / CT, ct = tid - rl * CT;

@@ -389,6 +389,15 @@ __device__ __forceinline__ float4 ld_shared_v4(uint32_t addr)
     return v;
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------------
+//
+// A kernel launched with launch_after may start while its predecessor in the stream still runs.  Every thread calls
+// grid_dependency_wait() before it touches global memory: it returns when the predecessor has completed and its writes are
+// visible (at once in an ordinary launch).  grid_dependency_trigger() lets the successor start; a kernel calls it only after
+// it holds its tensor memory, so that a waiting successor can never hold columns this one still needs.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- tensor memory --------------------------------------------------------------------------
 
 // Whole-warp call.  Writes the base address of `ncols` (power of two, >= 32) columns to *dst.

@@ -1170,10 +1170,10 @@ static int launch_tapstack(DeviceCtx* c, const IgemmPlan& pl, const TapStackPlan
     }
     const int grid = sm_budget(c) < p.total_tiles ? sm_budget(c) : p.total_tiles;
     if (!t_dry) {
-        if (pl.FW == 3 && pl.FH == 3) conv_tapstack_kernel<3, 3><<<grid, kTapStackThreads, ts.smem, stream>>>(tmA, tmB, p);
-        else if (pl.FW == 3) conv_tapstack_kernel<3, 0><<<grid, kTapStackThreads, ts.smem, stream>>>(tmA, tmB, p);
-        else if (pl.FW == 2) conv_tapstack_kernel<2, 0><<<grid, kTapStackThreads, ts.smem, stream>>>(tmA, tmB, p);
-        else conv_tapstack_kernel<0, 0><<<grid, kTapStackThreads, ts.smem, stream>>>(tmA, tmB, p);
+        if (pl.FW == 3 && pl.FH == 3) launch_after(conv_tapstack_kernel<3, 3>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        else if (pl.FW == 3) launch_after(conv_tapstack_kernel<3, 0>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        else if (pl.FW == 2) launch_after(conv_tapstack_kernel<2, 0>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        else launch_after(conv_tapstack_kernel<0, 0>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
     }
     note_launch("halo_tapstack");
     snprintf(g_plan, sizeof(g_plan), "tapstack BN=%d N=%d CB=%d npb=%d eff=%.2f", ts.BN, pl.FW * ts.BN, ts.CB, ts.npb, ts.eff);

@@ -14,7 +14,6 @@
 #pragma once
 #include "sm100_ptx.cuh"
 #include "fast_div.cuh"
-#include "host_common.h"
 
 namespace alpha {
 

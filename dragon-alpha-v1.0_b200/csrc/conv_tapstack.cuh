@@ -171,7 +171,9 @@ __global__ void __launch_bounds__(kTapStackThreads, 1)
         tmem_relinquish();
     }
     tc_fence_before_sync();
+    grid_dependency_wait();
     __syncthreads();
+    grid_dependency_trigger();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
 

@@ -16,6 +16,7 @@
 //   load_a / load_b    one 16-byte word of a tile, zero outside the problem
 //   store              four consecutive outputs of a row
 #pragma once
+#include "dependent_launch.cuh"
 #include "fast_div.cuh"
 
 namespace alpha {
@@ -64,6 +65,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
     __shared__ __align__(16) float Bs[2][kGemmBK * BN];
     const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
 
+    grid_dependency_wait();
+    grid_dependency_trigger();
     typename P::Cta c;
     if (!p.cta(c, BM, BN)) return;                                // uniform for the CTA
     typename P::RowA ra[NA];
@@ -290,10 +293,10 @@ inline GemmTile pick_gemm_tile(long long rows, int cols, long long copies, int s
 template <class P>
 inline void launch_gemm_f32(const P& p, const GemmTile& t, dim3 grid, cudaStream_t stream)
 {
-    if (t.bn == 128) gemm_f32_kernel<128, 128, 8, 8><<<grid, kGemmThreads, 0, stream>>>(p);
-    else if (t.bn == 32) gemm_f32_kernel<128, 32, 4, 4><<<grid, kGemmThreads, 0, stream>>>(p);
-    else if (t.bm == 128) gemm_f32_kernel<128, 64, 8, 4><<<grid, kGemmThreads, 0, stream>>>(p);
-    else gemm_f32_kernel<64, 64, 4, 4><<<grid, kGemmThreads, 0, stream>>>(p);
+    if (t.bn == 128) launch_after(gemm_f32_kernel<128, 128, 8, 8, P>, grid, kGemmThreads, 0, stream, p);
+    else if (t.bn == 32) launch_after(gemm_f32_kernel<128, 32, 4, 4, P>, grid, kGemmThreads, 0, stream, p);
+    else if (t.bm == 128) launch_after(gemm_f32_kernel<128, 64, 8, 4, P>, grid, kGemmThreads, 0, stream, p);
+    else launch_after(gemm_f32_kernel<64, 64, 4, 4, P>, grid, kGemmThreads, 0, stream, p);
 }
 
 }  // namespace alpha

@@ -24,6 +24,8 @@ namespace {
 // the product, CudaFloat32EngineBase.java:1156-1165).
 __global__ void add_bias_rows_kernel(float4* __restrict__ C, const float* __restrict__ bias, size_t n4, int cols4)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         float4 c = C[i];
@@ -39,6 +41,8 @@ __global__ void add_bias_rows_kernel(float4* __restrict__ C, const float* __rest
 __global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, float4* __restrict__ dst, unsigned rows, unsigned cols,
                                                        unsigned total, FastDiv by_c4)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         unsigned r, q;
         by_c4.divmod(i, r, q);
@@ -189,7 +193,7 @@ int alpha_matMul(const float* A, const float* B, const float* bias, float* C, in
     const size_t n4 = static_cast<size_t>(N) * M / 4;
     size_t blocks = (n4 + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    add_bias_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_after(add_bias_rows_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), 
         reinterpret_cast<float4*>(C), bias, n4, M / 4);
     note_launch("matmul_bias");
     cudaError_t e = cudaGetLastError();
@@ -227,7 +231,7 @@ int alpha_pad_rows(const float* src, long long rows, int cols, float* dst, long 
     if (total > 2000000000LL) return fail(ALPHA_E_ARG, "pad_rows: more than 8e9 elements");   // 31-bit indices with a grid stride
     long long blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    pad_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_after(pad_rows_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), 
         src, reinterpret_cast<float4*>(dst), static_cast<unsigned>(rows), static_cast<unsigned>(cols), static_cast<unsigned>(total), fast_div(cols4 / 4));
     note_launch("pad_rows");
     cudaError_t e = cudaGetLastError();

@@ -16,6 +16,7 @@
 // (file names under src/cu32_src/Cuda_pool2D/Cuda_pool2D and src/cu32_src/Cuda_upool2D/Cuda_upool2D).
 #include "../../include/alpha_conv_b200.h"
 #include "host_common.h"
+#include "dependent_launch.cuh"
 #include "fast_div.cuh"
 
 using namespace alpha;
@@ -80,6 +81,8 @@ template <int V, int U, int OP>
 __global__ void __launch_bounds__(256) pool_fwd_kernel(const float* __restrict__ X, float* __restrict__ Y,
                                                        int* __restrict__ Index, PoolDims d)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     using F = typename Vec<V>::F;
     using I = typename Vec<V>::I;
     // element counts fit 31 bits (checked on the host), so the index arithmetic is 32-bit: 64-bit divisions per
@@ -146,6 +149,8 @@ __global__ void __launch_bounds__(256) pool_bwd_kernel(const float* __restrict__
                                                        const float* __restrict__ X, const int* __restrict__ Index,
                                                        float* __restrict__ dX, PoolDims d)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     using F = typename Vec<V>::F;
     using I = typename Vec<V>::I;
     const unsigned cqu = static_cast<unsigned>(d.IC / (V * U));
@@ -223,6 +228,8 @@ __global__ void __launch_bounds__(256) pool_bwd_s2_kernel(const float* __restric
                                                           const float* __restrict__ X, const int* __restrict__ Index,
                                                           float* __restrict__ dX, PoolDims d, int GH, int GW, FastDiv by_GW, FastDiv by_GH)
 {
+    grid_dependency_wait();
+    grid_dependency_trigger();
     constexpr int D = (F + 1) / 2;
     const unsigned cqu = static_cast<unsigned>(d.IC / (4 * U));
     const unsigned total = static_cast<unsigned>(d.N) * GH * GW * cqu;
@@ -368,11 +375,11 @@ int run_fwd(const char* what, const AlphaPoolShape* s, const float* X, float* Y,
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     const long long outs = static_cast<long long>(s->N) * s->OH * s->OW * s->IC;
     if (vec4_ok(s, X, Y, Index) && s->IC % 16 == 0)
-        pool_fwd_kernel<4, 4, OP><<<grid_for(outs / 16), 256, 0, stream>>>(X, Y, Index, dims_of(s, 4, 4));
+        launch_after(pool_fwd_kernel<4, 4, OP>, grid_for(outs / 16), 256, 0, stream, X, Y, Index, dims_of(s, 4, 4));
     else if (vec4_ok(s, X, Y, Index))
-        pool_fwd_kernel<4, 1, OP><<<grid_for(outs / 4), 256, 0, stream>>>(X, Y, Index, dims_of(s, 4, 1));
+        launch_after(pool_fwd_kernel<4, 1, OP>, grid_for(outs / 4), 256, 0, stream, X, Y, Index, dims_of(s, 4, 1));
     else
-        pool_fwd_kernel<1, 1, OP><<<grid_for(outs), 256, 0, stream>>>(X, Y, Index, dims_of(s, 1, 1));
+        launch_after(pool_fwd_kernel<1, 1, OP>, grid_for(outs), 256, 0, stream, X, Y, Index, dims_of(s, 1, 1));
     return finish("pool_fwd_kernel", "pool_fwd");
 }
 
@@ -393,18 +400,18 @@ int run_bwd(const char* what, const AlphaPoolShape* s, const float* dY, const fl
         const int U = s->IC % 8 == 0 ? 2 : 1;
         const unsigned grid = grid_for(static_cast<long long>(s->N) * GH * GW * (s->IC / (4 * U)));
         const PoolDims d = dims_of(s, 4, U);
-        if (s->FH == 3 && U == 2) pool_bwd_s2_kernel<2, OP, 3><<<grid, 256, 0, stream>>>(dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
-        else if (s->FH == 3) pool_bwd_s2_kernel<1, OP, 3><<<grid, 256, 0, stream>>>(dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
-        else if (U == 2) pool_bwd_s2_kernel<2, OP, 2><<<grid, 256, 0, stream>>>(dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
-        else pool_bwd_s2_kernel<1, OP, 2><<<grid, 256, 0, stream>>>(dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
+        if (s->FH == 3 && U == 2) launch_after(pool_bwd_s2_kernel<2, OP, 3>, grid, 256, 0, stream, dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
+        else if (s->FH == 3) launch_after(pool_bwd_s2_kernel<1, OP, 3>, grid, 256, 0, stream, dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
+        else if (U == 2) launch_after(pool_bwd_s2_kernel<2, OP, 2>, grid, 256, 0, stream, dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
+        else launch_after(pool_bwd_s2_kernel<1, OP, 2>, grid, 256, 0, stream, dY, Y, X, Index, dX, d, GH, GW, by_GW, by_GH);
         return finish("pool_bwd_s2_kernel", "pool_bwd");
     }
     if (v4 && s->IC % 16 == 0)
-        pool_bwd_kernel<4, 4, OP><<<grid_for(ins / 16), 256, 0, stream>>>(dY, Y, X, Index, dX, dims_of(s, 4, 4));
+        launch_after(pool_bwd_kernel<4, 4, OP>, grid_for(ins / 16), 256, 0, stream, dY, Y, X, Index, dX, dims_of(s, 4, 4));
     else if (v4)
-        pool_bwd_kernel<4, 1, OP><<<grid_for(ins / 4), 256, 0, stream>>>(dY, Y, X, Index, dX, dims_of(s, 4, 1));
+        launch_after(pool_bwd_kernel<4, 1, OP>, grid_for(ins / 4), 256, 0, stream, dY, Y, X, Index, dX, dims_of(s, 4, 1));
     else
-        pool_bwd_kernel<1, 1, OP><<<grid_for(ins), 256, 0, stream>>>(dY, Y, X, Index, dX, dims_of(s, 1, 1));
+        launch_after(pool_bwd_kernel<1, 1, OP>, grid_for(ins), 256, 0, stream, dY, Y, X, Index, dX, dims_of(s, 1, 1));
     return finish("pool_bwd_kernel", "pool_bwd");
 }
 

@@ -2,6 +2,7 @@
 // Every wait in this file is bounded: a wait that runs out returns false and the caller leaves the
 // kernel through its error path (status word set, tensor memory freed) instead of spinning forever.
 #pragma once
+#include "dependent_launch.cuh"
 #include <type_traits>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -388,15 +389,6 @@ __device__ __forceinline__ float4 ld_shared_v4(uint32_t addr)
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
 }
-
-// ---- programmatic dependent launch ------------------------------------------------------------
-//
-// A kernel launched with launch_after may start while its predecessor in the stream still runs.  Every thread calls
-// grid_dependency_wait() before it touches global memory: it returns when the predecessor has completed and its writes are
-// visible (at once in an ordinary launch).  grid_dependency_trigger() lets the successor start; a kernel calls it only after
-// it holds its tensor memory, so that a waiting successor can never hold columns this one still needs.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- tensor memory --------------------------------------------------------------------------
 

@@ -43,3 +43,17 @@ def test_zero_filled_chunks(pkg, oracle_mod, shape, mode, pad):
     for op, y in got.items():
         m = metrics(y.cpu().numpy(), *ref[op])
         assert m["finite"] and m["norm"] <= TOL[mode]["norm"] and m["comp"] <= TOL[mode]["comp"], (op, m)
+
+
+def test_long_odd_reductions_keep_their_corrections_apart(pkg):
+    """A product over 6148 channels (no multiple of 8) of a row count that is none either stays on the halo kernel, whose side
+    columns hold the correction terms: the im2col kernel's single accumulator errs four times as much (4e-5)."""
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math="3xtf32"))
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A, B = torch.randn((995, 6146), device="cuda", generator=g), torch.randn((73, 6146), device="cuda", generator=g)
+    C = eng.matMulT2(A, B)
+    assert lib.last_algo().startswith("halo"), lib.last_algo()
+    ref = A.double() @ B.double().T
+    assert float((C.double() - ref).norm() / ref.norm()) <= 3e-5      # the bound stated for FullConnect layers

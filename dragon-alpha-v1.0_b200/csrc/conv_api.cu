@@ -1307,12 +1307,13 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     int rc = 0;
     if (pl.lat) {
         const LatticePlan& l = *pl.lat;
+        const size_t pix = pl.aPix ? pl.aPix : l.aC, row = pl.aPix ? pl.aRow : (size_t)l.aW * l.aC, img = pl.aPix ? pl.aImg : (size_t)l.aH * l.aW * l.aC;
         p.lat_n = l.n; p.lat_du = l.sh * l.FW; p.lat_dv = l.sw;
         for (int k = 0; k < l.n && !rc; ++k) {
             p.lat_U[k] = l.u[k]; p.lat_V[k] = l.v[k]; p.lat_tap0[k] = l.tap0[k]; p.lat_h0[k] = l.h0[k]; p.lat_w0[k] = l.w0[k];
             cuuint64_t ad[4] = {(cuuint64_t)l.aC, (cuuint64_t)((l.aW - l.psi[k] + l.sw - 1) / l.sw), (cuuint64_t)((l.aH - l.phi[k] + l.sh - 1) / l.sh), (cuuint64_t)pl.aN};
-            cuuint64_t as[3] = {(cuuint64_t)l.sw * l.aC * 4, (cuuint64_t)l.sh * l.aW * l.aC * 4, (cuuint64_t)l.aH * l.aW * l.aC * 4};
-            rc = make_tiled_map(&tmA.m[k], pl.act + ((size_t)l.phi[k] * l.aW + l.psi[k]) * l.aC, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
+            cuuint64_t as[3] = {(cuuint64_t)l.sw * pix * 4, (cuuint64_t)l.sh * row * 4, (cuuint64_t)img * 4};
+            rc = make_tiled_map(&tmA.m[k], pl.act + l.phi[k] * row + l.psi[k] * pix, 4, ad, as, abox, CU_TENSOR_MAP_SWIZZLE_128B);
         }
         for (int k = l.n; k < 4; ++k) tmA.m[k] = tmA.m[0];
     } else {
@@ -1508,29 +1509,34 @@ static int launch_patch_gemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cuda
 
 // ---- few input channels: windows of a filter row -----------------------------------------------------
 //
-// See window_pack_kernel.  K = FW * sh * IC floats per window, U = ceil(FH / sh) windows (rows) per output pixel.
+// See window_pack_kernel.  A window holds g filter rows side by side, K = FW * g * IC floats, and U = ceil(FH / g) of them cover a
+// filter.  deltaW takes g = sh (a filter row past FH is dropped from its result).  Forward takes g = sh only where sh divides FH:
+// otherwise the last window would hold rows that no tap meets, under zero weights, and an Inf or NaN there would reach outputs
+// that do not depend on it.  It then takes g = 1, one lattice phase of whole rows for each of the sh rows of a stride step.
 struct WindowPlan {
-    int K, U, Hq, Wp;
+    int g, K, U, Hq, Wp;
     size_t row, elems;      // floats of a row of Xp and of Xp
     double per_pixel;       // floats of Xp per output pixel
 };
-static WindowPlan window_plan(const AlphaConvShape* s)
+static WindowPlan window_plan(const AlphaConvShape* s, int g)
 {
     WindowPlan w;
-    w.K = s->FW * s->sh * s->IC; w.U = (s->FH + s->sh - 1) / s->sh;
-    w.Hq = s->OH + w.U - 1; w.Wp = (s->OW - 1) * s->sw + s->FW;
-    w.row = (size_t)w.Wp * s->sh * s->IC;
+    w.g = g;
+    w.K = s->FW * g * s->IC; w.U = (s->FH + g - 1) / g;
+    w.Hq = (s->OH - 1) * (s->sh / g) + w.U; w.Wp = (s->OW - 1) * s->sw + s->FW;
+    w.row = (size_t)w.Wp * g * s->IC;
     w.elems = (size_t)s->N * w.Hq * w.row;
     w.per_pixel = (double)w.Hq * w.row / ((double)s->OH * s->OW);
     return w;
 }
+static WindowPlan forward_windows(const AlphaConvShape* s) { return window_plan(s, s->FH % s->sh == 0 ? s->sh : 1); }
 static bool window_fits(const AlphaConvShape* s, const WindowPlan& w)
 {
-    return opt(OPT_HALO_WINDOW) && env_tile_mode() != 1 && s->FW > 1 && s->IC % 32 != 0 && w.K <= 512 && w.U <= 64 && w.elems <= 2147483647ull;
+    return opt(OPT_HALO_WINDOW) && env_tile_mode() != 1 && s->FW > 1 && s->IC % 32 != 0 && w.K <= 512 && w.U <= 64 && s->sh / w.g <= 4 && w.elems <= 2147483647ull;
 }
 // Forward: windows against zero-filled chunks and the patch matrix, in the units of pad_beats_patch (columns per reduction
 // chunk of 32 and output pixel; a strided layer on zero-filled chunks runs the im2col or lattice kernel, 1.4 times as long).
-// 32 x 224 x 224, 4 -> 64 channels 7x7 s2 (K = 56, U = 4): patch matrix 75 us + 135 us for the product that reads its 360 MB, 116 us
+// 32 x 224 x 224, 4 -> 64 channels 7x7 s2 (K = 28, U = 7): patch matrix 75 us + 135 us for the product that reads its 360 MB, 108 us
 // here; 64 x 56 x 56, 20 -> 128 3x3: 119 / 102 / 84 us over the patch matrix / zero-filled chunks / windows.  In plain TF32 chunks
 // of a stride-1 layer, whose filter row is one stage, win from 8 channels on (62 against 71 us for 128 x 56 x 56, 8 -> 64).
 static bool window_beats_rest(const AlphaConvShape* s, const WindowPlan& w, int mode3x, int sms)
@@ -1551,8 +1557,8 @@ static int launch_window_pack(DeviceCtx* c, const AlphaConvShape* s, const Windo
 {
     int rc = get_workspace(c, stream, w.elems * sizeof(float), Xp);
     if (rc) return rc;
-    const WindowShape ws{s->N, s->IH, s->IW, s->IC, s->sh, s->ph, s->pw, w.Hq, w.Wp};
-    const WindowDivs dv{fast_div(s->IC / 4), fast_div(s->sh), fast_div(w.Wp), fast_div(w.Hq)};
+    const WindowShape ws{s->N, s->IH, s->IW, s->IC, w.g, s->ph, s->pw, w.Hq, w.Wp};
+    const WindowDivs dv{fast_div(s->IC / 4), fast_div(w.g), fast_div(w.Wp), fast_div(w.Hq)};
     size_t blocks = (w.elems / 4 + 255) / 256;
     if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
     if (!t_dry) launch_after(window_pack_kernel, (unsigned)blocks, 256, 0, stream, X, reinterpret_cast<float4*>(*Xp), ws, dv);
@@ -1562,28 +1568,43 @@ static int launch_window_pack(DeviceCtx* c, const AlphaConvShape* s, const Windo
 // Returns 1 when no kernel takes the window convolution.
 static int launch_window_forward(DeviceCtx* c, const AlphaConvShape* s, const IgemmPlan& pl_in, const WindowPlan& w, int mode3x, cudaStream_t stream)
 {
-    const size_t nW = (size_t)s->OC * w.U * w.K;
-    float *Ww = nullptr, *Xp = nullptr;
-    bool fresh = true;
-    const DeviceCtx::WeightKey wkey{pl_in.W, WK_FWD_WINDOW, s->OC, s->IC, s->FH * 256 + s->FW, s->sh, mode3x};
-    int rc = weight_planes(c, stream, wkey, (mode3x ? 2 : 1) * nW * sizeof(float), &Ww, &fresh);
-    if (rc) return rc;
-    if (fresh) {
-        size_t blocks = (nW + 255) / 256;
-        if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-        if (transforms_run()) launch_after(window_weights_kernel, (unsigned)blocks, 256, 0, stream, pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
-        note_launch("window_w");
-        rc = check_launch("window_weights_kernel");
-        if (rc) return rc;
-        weight_planes_ready(c, stream, wkey);
-    }
-    rc = launch_window_pack(c, s, w, pl_in.act, stream, &Xp);
-    if (rc) return rc;
     IgemmPlan pl = pl_in;
+    pl.wIC = w.K;   // one window row of W as it lies: [OC][FH][FW * IC]
+    if (w.g > 1) {
+        const size_t nW = (size_t)s->OC * w.U * w.K;
+        float* Ww = nullptr;
+        bool fresh = true;
+        const DeviceCtx::WeightKey wkey{pl_in.W, WK_FWD_WINDOW, s->OC, s->IC, s->FH * 256 + s->FW, s->sh, mode3x};
+        int rc = weight_planes(c, stream, wkey, (mode3x ? 2 : 1) * nW * sizeof(float), &Ww, &fresh);
+        if (rc) return rc;
+        if (fresh) {
+            size_t blocks = (nW + 255) / 256;
+            if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
+            if (transforms_run()) launch_after(window_weights_kernel, (unsigned)blocks, 256, 0, stream, pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
+            note_launch("window_w");
+            rc = check_launch("window_weights_kernel");
+            if (rc) return rc;
+            weight_planes_ready(c, stream, wkey);
+        }
+        pl.W = Ww; pl.W_lo = mode3x ? Ww + nW : nullptr;
+    }
+    float* Xp = nullptr;
+    int rc = launch_window_pack(c, s, w, pl_in.act, stream, &Xp);
+    if (rc) return rc;
     pl.act = Xp; pl.aH = w.Hq; pl.aW = s->OW; pl.aC = w.K;
-    pl.aPix = (size_t)s->sw * s->sh * s->IC; pl.aRow = w.row; pl.aImg = w.row * w.Hq;
+    pl.aPix = (size_t)s->sw * w.g * s->IC; pl.aRow = w.row; pl.aImg = w.row * w.Hq;
     pl.FH = w.U; pl.FW = 1; pl.sh = pl.sw = 1; pl.pad_h = pl.pad_w = 0;
-    pl.W = Ww; pl.W_lo = mode3x ? Ww + nW : nullptr; pl.wIC = w.K; pl.kdim = w.K; pl.pad = true; pl.force = true;
+    pl.kdim = w.K; pl.pad = true; pl.force = true;
+    LatticePlan l;
+    if (w.g < s->sh) {
+        l.FH = s->FH; l.FW = 1; l.sh = s->sh; l.sw = 1; l.aH = w.Hq; l.aW = s->OW; l.aC = w.K;
+        for (int phi = 0; phi < s->sh && phi < s->FH; ++phi, ++l.n) {
+            l.phi[phi] = phi; l.psi[phi] = 0; l.u[phi] = (s->FH - phi + s->sh - 1) / s->sh; l.v[phi] = 1;
+            l.tap0[phi] = phi; l.h0[phi] = l.w0[phi] = 0;
+        }
+        l.taps = s->FH; l.U = l.u[0]; l.V = 1;
+        pl.lat = &l; pl.FH = l.U; pl.kdim = l.n * chunks32(w.K) * 32;
+    }
     return launch_halo(c, pl, mode3x, stream);
 }
 
@@ -2685,7 +2706,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
             rc = launch_patch_gemm(c, pl, mode3x, stream);
             if (rc != 1) return rc;
         }
-        const WindowPlan win = window_plan(s);
+        const WindowPlan win = forward_windows(s);
         const bool strided = s->sh != 1 || s->sw != 1;
         // A layer of few tiles and steps is launch latency: the im2col kernel splits W itself and is one launch (3xTF32)
         const bool small = mode3x && s->IC % 32 != 0 && igemm_cost(pl, mode3x, sm_budget(c)) < 20000.0;
@@ -2699,7 +2720,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         if (rc != 1 && !((pl.pad || strided) && scratch_refused(rc))) return rc;
         return launch_igemm(c, pl, mode3x, stream);
     }
-    const WindowPlan win = window_plan(s);
+    const WindowPlan win = forward_windows(s);
     if (algo != ALPHA_ALGO_SIMT && !tensor_ok && !(tiny_image(s->OH, s->OW) && patch_path_ok(s)) && window_beats_rest(s, win, cur_mode3x(), sm_budget(c))) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N;
@@ -2831,7 +2852,7 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     if (algo == ALPHA_ALGO_TENSOR && !tensor_ok)
         return fail(ALPHA_E_ARG, "tensor deltaW path needs IC %% 32 == 0 (IC=%d)", s->IC);
     if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
-        const WindowPlan win = window_plan(s);
+        const WindowPlan win = window_plan(s, s->sh);
         const DwRoute route = pick_dw_route(s, win, cur_mode3x());
         rc = 1;
         if (route == DwRoute::Straight) rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream);

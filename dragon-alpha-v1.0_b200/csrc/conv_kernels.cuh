@@ -218,17 +218,17 @@ __global__ void __launch_bounds__(256) patch_matrix32_kernel(const float* __rest
     }
 }
 
-// Few input channels: windows instead of pixels.  Xp[n][q][w][phi][ic] = X[n][q * sh + phi - ph][w - pw][ic], zero outside the
-// image: the sh rows a stride step skips lie side by side in every column, so that the FW columns an output pixel's filter row
-// covers are FW * sh * IC consecutive floats that start (ow * sw) * sh * IC floats into the row.  Read through a tensor map
-// whose pixels are those (overlapping) windows, a layer of 3 channels and 7x7 taps at stride 2 is a 4 x 1 convolution over 56
-// "channels".  One thread per four floats; Xp is written once and is sh * sw / (stride area) times X, where the patch matrix
-// would be FH * FW / (sh * sw) times X.
+// Few input channels: windows instead of pixels.  Xp[n][q][w][phi][ic] = X[n][q * g + phi - ph][w - pw][ic], phi < g, zero outside
+// the image: g rows of X lie side by side in every column, so that the FW columns an output pixel's filter row covers are
+// FW * g * IC consecutive floats that start (ow * sw) * g * IC floats into the row.  Read through a tensor map whose pixels are
+// those (overlapping) windows, a layer of 4 channels and 4x4 taps at stride 2 is with g = 2 a 2 x 1 convolution over 32 "channels",
+// one of 7x7 taps with g = 1 a 7 x 1 convolution over 28 with a row stride of 2.  One thread per four floats; Xp, N * Hq * Wp * g * IC
+// floats (about X with its border), is written once, where the patch matrix would be FH * FW / (sh * sw) times X.
 struct WindowShape {
-    int N, IH, IW, IC, sh, ph, pw, Hq, Wp;
+    int N, IH, IW, IC, g, ph, pw, Hq, Wp;
 };
 struct WindowDivs {
-    FastDiv by_c4, by_sh, by_Wp, by_Hq;
+    FastDiv by_c4, by_g, by_Wp, by_Hq;
 };
 __global__ void __launch_bounds__(256) window_pack_kernel(const float* __restrict__ X, float4* __restrict__ Xp, const WindowShape s,
                                                           const WindowDivs dv)
@@ -236,14 +236,14 @@ __global__ void __launch_bounds__(256) window_pack_kernel(const float* __restric
     grid_dependency_wait();
     grid_dependency_trigger();
     const unsigned c4 = static_cast<unsigned>(s.IC) >> 2;
-    const unsigned total = static_cast<unsigned>(s.N) * s.Hq * s.Wp * s.sh * c4;
+    const unsigned total = static_cast<unsigned>(s.N) * s.Hq * s.Wp * s.g * c4;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         unsigned t, c, phi, w, q, n;
         dv.by_c4.divmod(i, t, c);
-        dv.by_sh.divmod(t, t, phi);
+        dv.by_g.divmod(t, t, phi);
         dv.by_Wp.divmod(t, t, w);
         dv.by_Hq.divmod(t, n, q);
-        const int ih = static_cast<int>(q) * s.sh + static_cast<int>(phi) - s.ph, iw = static_cast<int>(w) - s.pw;
+        const int ih = static_cast<int>(q) * s.g + static_cast<int>(phi) - s.ph, iw = static_cast<int>(w) - s.pw;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ih >= 0 && ih < s.IH && iw >= 0 && iw < s.IW)
             v = __ldg(reinterpret_cast<const float4*>(X + ((static_cast<size_t>(n) * s.IH + ih) * s.IW + iw) * s.IC) + c);
@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(256) window_pack_kernel(const float* __restric
     }
 }
 
-// The filter in window order, Ww[oc][u][(fw * sh + phi) * IC + ic] = W[oc][u * sh + phi][fw][ic] (zero past FH), with its lo plane
-// when `lo` is set; and the way back for deltaW.
+// The filter in the order of windows of g = sh rows (which divides FH), Ww[oc][u][(fw * sh + phi) * IC + ic] = W[oc][u * sh + phi][fw][ic],
+// with its lo plane when `lo` is set; and the way back for deltaW (any FH: rows past it are dropped).
 __global__ void __launch_bounds__(256) window_weights_kernel(const float* __restrict__ W, float* __restrict__ Ww, float* __restrict__ lo,
                                                              int OC, int FH, int FW, int IC, int sh, int U)
 {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(256) window_weights_kernel(const float* __rest
         const size_t r = i / K;
         const int u = static_cast<int>(r % U), oc = static_cast<int>(r / U);
         const int ic = k % IC, t = k / IC, phi = t % sh, fw = t / sh, fh = u * sh + phi;
-        const float x = fh < FH ? W[((static_cast<size_t>(oc) * FH + fh) * FW + fw) * IC + ic] : 0.f;
+        const float x = W[((static_cast<size_t>(oc) * FH + fh) * FW + fw) * IC + ic];
         Ww[i] = x;
         if (lo) lo[i] = tf32_lo_of_trunc(x);
     }

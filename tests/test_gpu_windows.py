@@ -42,3 +42,31 @@ def test_windows(pkg, oracle_mod, shape, mode):
     for op, m in (("fwd", metrics(Y, ref + B, mag + np.abs(B))),
                   ("dw", metrics(dW, *oracle_mod.deconv3D_deltaW_f64(X, dY, FH, FW, sh, sw, ph, pw, threads=8)))):
         assert m["finite"] and m["norm"] <= TOL[mode]["norm"] and m["comp"] <= TOL[mode]["comp"], (op, m)
+
+
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+@pytest.mark.parametrize("shape", [(4, 40, 40, 3, 64, 7, 2, 3), (4, 41, 43, 4, 36, 3, 2, 1), (4, 40, 40, 8, 64, 4, 2, 1), (4, 30, 30, 12, 64, 5, 1, 2),
+                                   (2, 41, 41, 4, 32, 3, 3, 0), (2, 40, 40, 4, 32, 5, 4, 1), (2, 30, 30, 4, 32, 2, 3, 0)], ids=str)
+def test_one_infinite_pixel_reaches_only_its_own_outputs(pkg, shape, mode):
+    """The rows and columns a window holds are those of the filter: an Inf pixel may not meet a zero weight beyond them."""
+    import torch
+    lib, engine = pkg.submodule("lib"), pkg.submodule("engine")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+    N, IH, IW, IC, OC, F, s, p = shape
+    g = torch.Generator(device="cuda").manual_seed(IH)
+    X, W = torch.randn((N, IH, IW, IC), device="cuda", generator=g), torch.rand((OC, F, F, IC), device="cuda", generator=g) + 0.5
+    lib.set_option("HALO_WINDOW", 2)
+    try:
+        for n, ih, iw in ((0, 20, 21), (1, 21, 20), (1, 22, 23), (N - 1, IH - 1, IW - 1), (0, 0, 0)):
+            Xi = X.clone()
+            Xi[n, ih, iw, IC - 1] = float("inf")
+            Y = eng.conv3D(Xi, W, s, s, p, p)
+            assert lib.last_plan().startswith("halo")
+            oh, ow = (torch.arange(d, device="cuda") for d in Y.shape[1:3])
+            meets = ((ih + p - oh * s >= 0) & (ih + p - oh * s < F))[:, None] & ((iw + p - ow * s >= 0) & (iw + p - ow * s < F))
+            want = torch.ones(Y.shape[:3], dtype=torch.bool, device="cuda")
+            want[n] = ~meets
+            assert torch.equal(torch.isfinite(Y).all(-1), want) and torch.equal(torch.isfinite(Y).any(-1), want), (n, ih, iw)
+    finally:
+        lib.set_option("HALO_WINDOW", 1)
+    assert lib.device_status() == 0

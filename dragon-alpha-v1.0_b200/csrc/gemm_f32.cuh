@@ -15,9 +15,13 @@
 //   cta()              block-level state of this CTA: k-tiles [it0, it1) and whatever the loads need; false: nothing to do
 //   load_a / load_b    one 16-byte word of a tile, zero outside the problem
 //   store              four consecutive outputs of a row
+//   P::kSkip           a row may have no operand in a whole tile (a filter tap outside the output): its A words are zeros, and
+//                      meets() says so.  Zeros add nothing unless B holds an Inf or NaN there, which leaves a NaN: a CTA that
+//                      finds one among its sums forms them once more, row by row without the tiles a row does not meet.
 #pragma once
 #include "dependent_launch.cuh"
 #include "fast_div.cuh"
+#include <type_traits>
 
 namespace alpha {
 
@@ -63,6 +67,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
     static_assert(WA % kGemmThreads == 0, "A words");
     __shared__ __align__(16) float As[2][kGemmBK * BM];
     __shared__ __align__(16) float Bs[2][kGemmBK * BN];
+    __shared__ bool met[2][P::kSkip ? BM : 1];
     const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
 
     grid_dependency_wait();
@@ -74,62 +79,86 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
     for (int i = 0; i < NA; ++i) ra[i] = p.row_a(c, word_col<BM, P::kAk>(tid + i * kGemmThreads));
 
     unsigned long long acc[TM][TN / 2];
+    auto form_sums = [&](auto by_row_) {
+        constexpr bool by_row = decltype(by_row_)::value;
 #pragma unroll
-    for (int y = 0; y < TM; ++y)
+        for (int y = 0; y < TM; ++y)
 #pragma unroll
-        for (int x = 0; x < TN / 2; ++x) acc[y][x] = 0ull;
-
-    float4 va[NA], vb[NB];
-    auto fetch = [&](int it) {
-        const typename P::Step st = p.step(c, it);
+            for (int x = 0; x < TN / 2; ++x) acc[y][x] = 0ull;
+        float4 va[NA], vb[NB];
+        bool vm[by_row ? NA : 1];
+        auto fetch = [&](int it) {
+            const typename P::Step st = p.step(c, it);
 #pragma unroll
-        for (int i = 0; i < NA; ++i) va[i] = p.load_a(c, st, ra[i], word_col<BM, P::kAk>(tid + i * kGemmThreads), word_k<BM, P::kAk>(tid + i * kGemmThreads));
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-            if (WB % kGemmThreads == 0 || tid + i * kGemmThreads < WB)
-                vb[i] = p.load_b(c, st, word_col<BN, P::kBk>(tid + i * kGemmThreads), word_k<BN, P::kBk>(tid + i * kGemmThreads));
-    };
-    auto stage = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) put_word<BM, P::kAk>(As[buf], tid + i * kGemmThreads, va[i]);
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-            if (WB % kGemmThreads == 0 || tid + i * kGemmThreads < WB) put_word<BN, P::kBk>(Bs[buf], tid + i * kGemmThreads, vb[i]);
-    };
-    if (c.it0 < c.it1) {
-        fetch(c.it0);
-        stage(0);
-    }
-    __syncthreads();
-    int buf = 0;
-    for (int it = c.it0; it < c.it1; ++it) {
-        if (it + 1 < c.it1) fetch(it + 1);
-#pragma unroll
-        for (int k = 0; k < kGemmBK; ++k) {
-            const int x8 = (k >> 2) * 8;
-            float a[TM];
-            unsigned long long b[TN / 2];
-#pragma unroll
-            for (int y = 0; y < TM; y += 4) {
-                const float4 t = *reinterpret_cast<const float4*>(&As[buf][k * BM + ((ty * TM + y) ^ x8)]);
-                a[y] = t.x; a[y + 1] = t.y; a[y + 2] = t.z; a[y + 3] = t.w;
-            }
-            // columns tx * 4 ... of each group of BN / (TN / 4) columns
-#pragma unroll
-            for (int x = 0; x < TN; x += 4) {
-                const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k * BN + (((x / 4) * (BN * 4 / TN) + tx * 4) ^ x8)]);
-                b[x / 2] = t.x; b[x / 2 + 1] = t.y;
+            for (int i = 0; i < NA; ++i) {
+                va[i] = p.load_a(c, st, ra[i], word_col<BM, P::kAk>(tid + i * kGemmThreads), word_k<BM, P::kAk>(tid + i * kGemmThreads));
+                if constexpr (by_row) vm[i] = p.meets(c, st, ra[i]);
             }
 #pragma unroll
-            for (int y = 0; y < TM; ++y) {
-                const unsigned long long aa = pack2(a[y], a[y]);
+            for (int i = 0; i < NB; ++i)
+                if (WB % kGemmThreads == 0 || tid + i * kGemmThreads < WB)
+                    vb[i] = p.load_b(c, st, word_col<BN, P::kBk>(tid + i * kGemmThreads), word_k<BN, P::kBk>(tid + i * kGemmThreads));
+        };
+        auto stage = [&](int buf) {
 #pragma unroll
-                for (int x = 0; x < TN / 2; ++x) ffma2(acc[y][x], aa, b[x]);
+            for (int i = 0; i < NA; ++i) {
+                put_word<BM, P::kAk>(As[buf], tid + i * kGemmThreads, va[i]);
+                if constexpr (by_row) met[buf][word_col<BM, P::kAk>(tid + i * kGemmThreads)] = vm[i];   // (words of a row agree)
             }
+#pragma unroll
+            for (int i = 0; i < NB; ++i)
+                if (WB % kGemmThreads == 0 || tid + i * kGemmThreads < WB) put_word<BN, P::kBk>(Bs[buf], tid + i * kGemmThreads, vb[i]);
+        };
+        if (c.it0 < c.it1) {
+            fetch(c.it0);
+            stage(0);
         }
-        if (it + 1 < c.it1) stage(buf ^ 1);   // the other buffer was last read before the previous barrier
         __syncthreads();
-        buf ^= 1;
+        int buf = 0;
+        for (int it = c.it0; it < c.it1; ++it) {
+            if (it + 1 < c.it1) fetch(it + 1);
+#pragma unroll(by_row ? 1 : kGemmBK)
+            for (int k = 0; k < kGemmBK; ++k) {
+                const int x8 = (k >> 2) * 8;
+                float a[TM];
+                unsigned long long b[TN / 2];
+#pragma unroll
+                for (int y = 0; y < TM; y += 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(&As[buf][k * BM + ((ty * TM + y) ^ x8)]);
+                    a[y] = t.x; a[y + 1] = t.y; a[y + 2] = t.z; a[y + 3] = t.w;
+                }
+                // columns tx * 4 ... of each group of BN / (TN / 4) columns
+#pragma unroll
+                for (int x = 0; x < TN; x += 4) {
+                    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k * BN + (((x / 4) * (BN * 4 / TN) + tx * 4) ^ x8)]);
+                    b[x / 2] = t.x; b[x / 2 + 1] = t.y;
+                }
+#pragma unroll
+                for (int y = 0; y < TM; ++y) {
+                    if constexpr (by_row)
+                        if (!met[buf][ty * TM + y]) continue;
+                    const unsigned long long aa = pack2(a[y], a[y]);
+#pragma unroll
+                    for (int x = 0; x < TN / 2; ++x) ffma2(acc[y][x], aa, b[x]);
+                }
+            }
+            if (it + 1 < c.it1) stage(buf ^ 1);   // the other buffer was last read before the previous barrier
+            __syncthreads();
+            buf ^= 1;
+        }
+    };
+    form_sums(std::false_type{});
+    if constexpr (P::kSkip) {
+        bool nan = false;
+#pragma unroll
+        for (int y = 0; y < TM; ++y)
+#pragma unroll
+            for (int x = 0; x < TN / 2; ++x) {
+                float u, v;
+                unpack2(acc[y][x], u, v);
+                nan = nan || u != u || v != v;
+            }
+        if (__syncthreads_or(nan)) form_sums(std::true_type{});
     }
 #pragma unroll
     for (int y = 0; y < TM; ++y) {
@@ -148,7 +177,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
 // taps, columns = input channels, reduction = those taps x output channels (tap-major).  blockIdx.z = phase * ksplit + part;
 // part sp of the reduction goes to out + sp * size (one part: deltaX itself), every element of which some phase writes.
 struct DxGemm {
-    static constexpr bool kAk = true, kBk = false;
+    static constexpr bool kAk = true, kBk = false, kSkip = true;
     const float* dY; const float* W; float* out;
     int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw;
     int nsw;                       // phases along a row: min(sw, IW)
@@ -194,6 +223,10 @@ struct DxGemm {
         s.fh = c.ry + sh * s.u; s.fw = c.rx + sw * s.v;
         return s;
     }
+    __device__ bool meets(const Cta& c, const Step& s, const RowA& r) const
+    {
+        return r.n >= 0 && static_cast<unsigned>(r.a + c.qy - s.u) < static_cast<unsigned>(OH) && static_cast<unsigned>(r.b + c.qx - s.v) < static_cast<unsigned>(OW);
+    }
     __device__ float4 load_a(const Cta& c, const Step& s, const RowA& r, int, int k) const
     {
         const int oh = r.a + c.qy - s.u, ow = r.b + c.qx - s.v, oc = s.k0 + k;
@@ -224,7 +257,7 @@ struct DxGemm {
 // words are loaded whole where they start inside the matrix, and what they hold past N, M or K is replaced by zeros.
 template <bool A_KC, bool B_KC>
 struct BatchGemm {
-    static constexpr bool kAk = A_KC, kBk = B_KC;
+    static constexpr bool kAk = A_KC, kBk = B_KC, kSkip = false;
     const float *A, *B; float* C;
     int N, M, K, lda, ldb, ldc;
     size_t strA, strB, strC;
@@ -241,6 +274,7 @@ struct BatchGemm {
         return true;
     }
     __device__ RowA row_a(const Cta&, int) const { return RowA{}; }
+    __device__ bool meets(const Cta&, const Step&, const RowA&) const { return true; }
     __device__ Step step(const Cta&, int it) const { return Step{it * kGemmBK}; }
     // the word of four consecutive elements that starts at (row, col): elements at col + i >= cols are zero
     __device__ static float4 word(const float* base, int ld, int row, int rows, int col, int cols)

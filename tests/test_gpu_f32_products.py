@@ -80,3 +80,26 @@ def test_reduction_split_needs_no_scratch(pkg):
     torch.cuda.synchronize()
     mag = dY.double().abs().reshape(8, -1) @ W.double().abs().reshape(2764, 52)
     assert bool(((got.double() - want.double()).abs().reshape(8, 52) <= 2 * 2764 * 2.0 ** -24 * mag).all())
+
+
+@pytest.mark.parametrize("algo", ["auto", "simt"])
+@pytest.mark.parametrize("shape", [(2, 35, 29, 36, 100, 3, 1, 1), (2, 17, 17, 40, 36, 3, 2, 1), (1, 12, 12, 132, 44, 4, 2, 1), (3, 1, 4, 52, 1380, 1, 1, 0),
+                                   (2, 10, 11, 8, 2060, 3, 1, 1)], ids=str)
+def test_infinite_weight_reaches_only_the_pixels_of_its_tap(pkg, shape, algo):
+    """A tap that falls outside the output is skipped, not multiplied by zero: border pixels of deltaX stay finite."""
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(algo=algo))
+    N, OH, OW, IC, OC, F, s, p = shape
+    IH, IW = (OH - 1) * s + F - 2 * p, (OW - 1) * s + F - 2 * p
+    g = torch.Generator(device="cuda").manual_seed(OC)
+    dY = torch.rand((N, OH, OW, OC), device="cuda", generator=g) + 0.5
+    for oc, fh, fw, ic in ((0, 0, 0, 0), (OC - 1, F - 1, F - 1, IC - 1), (OC // 2, F // 2, 0, 5)):
+        W = torch.randn((OC, F, F, IC), device="cuda", generator=g)
+        W[oc, fh, fw, ic] = float("inf")
+        dX = eng.dconv3D_deltaX(dY, W, IH, IW, s, s, p, p)
+        ih, iw = torch.arange(IH, device="cuda") + p - fh, torch.arange(IW, device="cuda") + p - fw
+        meets = ((ih >= 0) & (ih % s == 0) & (ih // s < OH))[:, None] & ((iw >= 0) & (iw % s == 0) & (iw // s < OW))
+        want = torch.ones((N, IH, IW, IC), dtype=torch.bool, device="cuda")
+        want[..., ic] = ~meets
+        assert torch.equal(torch.isfinite(dX), want), (oc, fh, fw, ic)

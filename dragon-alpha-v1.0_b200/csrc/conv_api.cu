@@ -1921,9 +1921,10 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
 // per_image: dW receives N separate results, dW[n] = the sum over the pixels of image n only (batched matrix
 // products C[n] = A[n]^T * B[n]); every CTA column of the grid then owns one image and writes its result in place.
 // x_pitch: floats between pixels, rows and images of X where it is not dense (stride 1 only).
+// *spills: whether pixel tiles reach past the output where X still has pixels (see DwRepair).
 static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float* X, const float* dY, float* dW,
                           int mode3x, cudaStream_t stream, float* deltaB = nullptr, bool* bias_fused = nullptr,
-                          bool per_image = false, const size_t* x_pitch = nullptr)
+                          bool per_image = false, const size_t* x_pitch = nullptr, bool* spills = nullptr)
 {
     if (bias_fused) *bias_fused = false;
     if (opt(OPT_CONV_DW) == 1 && !per_image) return 1;
@@ -2012,6 +2013,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     const int tile_rows = diag ? 2 * R : R;   // R = rows per half tile in the diagonal form
     p.row_blocks = (s->OH + tile_rows - 1) / tile_rows; p.col_blocks = (s->OW + CW - 1) / CW;
     p.tiles_per_img = p.row_blocks * p.col_blocks;
+    if (spills) *spills = (s->OH % tile_rows != 0 && !(s->FH == 1 && s->IH == s->OH)) || (s->OW % CW != 0 && !(s->FW == 1 && s->IW == s->OW));
     const long long total = (long long)s->N * p.tiles_per_img;
     if (total > 2147483647LL) return 1;
     p.total_tiles = (int)total;
@@ -2204,7 +2206,7 @@ static DwRoute pick_dw_route(const AlphaConvShape* s, const WindowPlan& w, int m
 }
 // Returns 1 when the deltaW kernel does not take the window convolution.
 static int launch_dw_window(DeviceCtx* c, const AlphaConvShape* s, const WindowPlan& w, const float* X, const float* dY, float* dW, int mode3x,
-                            cudaStream_t stream)
+                            cudaStream_t stream, bool* spills)
 {
     const AlphaConvShape t = window_shape(s, w);
     float *Xp = nullptr, *tmp = nullptr;
@@ -2213,7 +2215,7 @@ static int launch_dw_window(DeviceCtx* c, const AlphaConvShape* s, const WindowP
     rc = launch_window_pack(c, s, w, X, stream, &Xp);
     if (rc) return rc;
     const size_t pitch[3] = {(size_t)s->sw * s->sh * s->IC, w.row, w.row * w.Hq};
-    rc = launch_dw_halo(c, &t, Xp, dY, tmp, mode3x, stream, nullptr, nullptr, false, pitch);
+    rc = launch_dw_halo(c, &t, Xp, dY, tmp, mode3x, stream, nullptr, nullptr, false, pitch, spills);
     if (rc) return rc;
     const size_t n = (size_t)s->OC * s->FH * s->FW * s->IC;
     size_t blocks = (n + 255) / 256;
@@ -2221,6 +2223,16 @@ static int launch_dw_window(DeviceCtx* c, const AlphaConvShape* s, const WindowP
     if (!t_dry) launch_after(window_unpack_kernel, (unsigned)blocks, 256, 0, stream, tmp, dW, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
     note_launch("dw_window");
     return check_launch("window_unpack_kernel");
+}
+
+static int launch_dw_repair(const AlphaConvShape* s, const float* X, const float* dY, float* dW, cudaStream_t stream, const char* tag)
+{
+    const int L = s->FH * s->FW * s->IC;
+    const DwRepair g{dY, X, dW, s->IH, s->IW, s->IC, s->OC, s->FW, s->sh, s->sw, s->ph, s->pw, L, s->N * s->OH * s->OW,
+                     fast_div(s->IC), fast_div(s->FW), fast_div(s->OW), fast_div(s->OH)};
+    if (!t_dry) launch_after(gemm_f32_kernel<64, 64, 4, 4, DwRepair>, dim3((unsigned)((s->OC + 63) / 64), (unsigned)((L + 63) / 64)), kGemmThreads, 0, stream, g);
+    note_launch(tag);
+    return check_launch("gemm_f32_kernel");
 }
 
 // Batched matrix products (the reference's Cuda_batchMatMul) on the convolution kernels: entry b of the batch is
@@ -2854,9 +2866,11 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
         const WindowPlan win = window_plan(s, s->sh);
         const DwRoute route = pick_dw_route(s, win, cur_mode3x());
+        bool spills = false;
         rc = 1;
-        if (route == DwRoute::Straight) rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream);
-        else if (route == DwRoute::Window) rc = launch_dw_window(c, s, win, X, deltaY, deltaW, cur_mode3x(), stream);
+        if (route == DwRoute::Straight) rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream, nullptr, nullptr, false, nullptr, &spills);
+        else if (route == DwRoute::Window) rc = launch_dw_window(c, s, win, X, deltaY, deltaW, cur_mode3x(), stream, &spills);
+        if (!rc && spills) rc = launch_dw_repair(s, X, deltaY, deltaW, stream, route == DwRoute::Window ? "dw_window" : "dw_halo");
         if (rc != 1 && !scratch_refused(rc)) return rc;
     }
     if (algo != ALPHA_ALGO_SIMT && patch_path_ok(s) && env_tile_mode() != 1 &&

@@ -252,6 +252,62 @@ struct DxGemm {
     }
 };
 
+// The tiles of a deltaW that hold an Inf or NaN, once more and in fp32: rows = output channels, columns = deltaW's taps x input
+// channels, reduction = pixels in ascending order; a CTA whose tile is finite returns at once.  The tensor kernel's pixel tiles may
+// reach past the output, where deltaY is zero but X can be a pixel of the image: finite pixels add nothing there, an Inf or NaN would
+// make deltaW NaN at taps that never meet it.  Looking at a finite deltaW costs about 2 us (100 x 3 x 3 x 36).
+struct DwRepair {
+    static constexpr bool kAk = false, kBk = false, kSkip = false;
+    const float *dY, *X; float* dW;
+    int IH, IW, IC, OC, FW, sh, sw, ph, pw, L, P;   // L = floats of a row of deltaW, P = output pixels
+    FastDiv by_IC, by_FW, by_OW, by_OH;
+    struct Cta { int m0, n0, it0, it1; };
+    struct RowA {};
+    struct Step { int k0; };
+    struct RowC { float* p; };
+
+    __device__ bool cta(Cta& c, int BM, int BN) const
+    {
+        c.m0 = static_cast<int>(blockIdx.x) * BM; c.n0 = static_cast<int>(blockIdx.y) * BN;
+        c.it0 = 0; c.it1 = (P + kGemmBK - 1) / kGemmBK;
+        float z = 0.f;
+        for (int i = threadIdx.x; i < BM * BN / 4; i += kGemmThreads) {
+            const int oc = c.m0 + i / (BN / 4), col = c.n0 + i % (BN / 4) * 4;
+            if (oc >= OC || col >= L) continue;
+            const float4 v = *reinterpret_cast<const float4*>(dW + static_cast<size_t>(oc) * L + col);
+            z += v.x * 0.f + v.y * 0.f + v.z * 0.f + v.w * 0.f;
+        }
+        return __syncthreads_or(z != 0.f) != 0;
+    }
+    __device__ RowA row_a(const Cta&, int) const { return RowA{}; }
+    __device__ bool meets(const Cta&, const Step&, const RowA&) const { return true; }
+    __device__ Step step(const Cta&, int it) const { return Step{it * kGemmBK}; }
+    __device__ float4 load_a(const Cta& c, const Step& s, const RowA&, int m, int k) const
+    {
+        const int px = s.k0 + k, oc = c.m0 + m;
+        if (px >= P || oc >= OC) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return __ldg(reinterpret_cast<const float4*>(dY + static_cast<size_t>(px) * OC + oc));
+    }
+    __device__ float4 load_b(const Cta& c, const Step& s, int col, int k) const
+    {
+        const int px = s.k0 + k, q = c.n0 + col;
+        if (px >= P || q >= L) return make_float4(0.f, 0.f, 0.f, 0.f);
+        unsigned t, ic, fh, fw, n, oh, ow;
+        by_IC.divmod(static_cast<unsigned>(q), t, ic);
+        by_FW.divmod(t, fh, fw);
+        by_OW.divmod(static_cast<unsigned>(px), t, ow);
+        by_OH.divmod(t, n, oh);
+        const int ih = static_cast<int>(oh) * sh + static_cast<int>(fh) - ph, iw = static_cast<int>(ow) * sw + static_cast<int>(fw) - pw;
+        if (static_cast<unsigned>(ih) >= static_cast<unsigned>(IH) || static_cast<unsigned>(iw) >= static_cast<unsigned>(IW)) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return __ldg(reinterpret_cast<const float4*>(X + ((static_cast<size_t>(n) * IH + ih) * IW + iw) * IC + ic));
+    }
+    __device__ RowC row_c(const Cta& c, int m) const { return RowC{c.m0 + m < OC ? dW + static_cast<size_t>(c.m0 + m) * L : nullptr}; }
+    __device__ void store(const Cta& c, const RowC& r, int col, const float4& o) const
+    {
+        if (r.p && c.n0 + col < L) *reinterpret_cast<float4*>(r.p + c.n0 + col) = o;
+    }
+};
+
 // C[b] = A[b] * B[b] over N x M outputs and K steps, with row pitches.  A_KC: A[b] is [N][lda] (else [K][lda], the transposed
 // form); B_KC: B[b] is [M][ldb] (else [K][ldb]).  Pitches are multiples of 4 and every matrix starts on a 16-byte boundary;
 // words are loaded whole where they start inside the matrix, and what they hold past N, M or K is replaced by zeros.

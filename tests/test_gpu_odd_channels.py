@@ -57,3 +57,43 @@ def test_long_odd_reductions_keep_their_corrections_apart(pkg):
     assert lib.last_algo().startswith("halo"), lib.last_algo()
     ref = A.double() @ B.double().T
     assert float((C.double() - ref).norm() / ref.norm()) <= 3e-5      # the bound stated for FullConnect layers
+
+
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+@pytest.mark.parametrize("shape", [(4, 35, 29, 36, 100, 3, 1, 1), (3, 21, 27, 4, 64, 5, 1, 2), (3, 33, 31, 44, 68, 3, 2, 1), (2, 19, 18, 12, 132, 7, 2, 3),
+                                   (2, 13, 37, 100, 72, 3, 1, 0)], ids=str)
+def test_infinite_border_pixel_reaches_only_its_own_taps(pkg, shape, mode):
+    """Pixel tiles of deltaW reach past the output, where deltaY is zero but X can still have pixels: an Inf among those may not
+    make deltaW NaN at taps that never meet it.  Every route of an odd channel count, with the other elements exact."""
+    import torch
+    lib, engine = pkg.submodule("lib"), pkg.submodule("engine")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+    N, IH, IW, IC, OC, F, s, p = shape
+    OH, OW = out_hw(IH, IW, F, F, s, s, p, p)
+    g = torch.Generator(device="cuda").manual_seed(IH * IC)
+    X, dY = torch.randn((N, IH, IW, IC), device="cuda", generator=g), torch.rand((N, OH, OW, OC), device="cuda", generator=g) + 0.5
+    pad = torch.nn.functional.pad(X.double(), (0, 0, p, p, p, p))
+    cut = lambda t, i, j: t[:, i:i + (OH - 1) * s + 1:s, j:j + (OW - 1) * s + 1:s]
+    for route in ({"HALO_PAD": 2}, {"HALO_WINDOW": 2}, {}):
+        for k, v in route.items():
+            lib.set_option(k, v)
+        try:
+            for n, ih, iw in ((1, IH - 1, IW - 1), (0, IH - 1, 3), (N - 1, 2, IW - 2), (1, IH // 2, IW // 2)):
+                Xi = X.clone()
+                Xi[n, ih, iw, 1] = float("inf")
+                dW = eng.dconv3D_deltaW(Xi, dY, F, F, s, s, p, p)
+                for i in range(F):
+                    for j in range(F):
+                        oh, ow = ih + p - i, iw + p - j
+                        meets = oh % s == 0 and ow % s == 0 and 0 <= oh // s < OH and 0 <= ow // s < OW
+                        fin = torch.isfinite(dW[:, i, j])
+                        assert bool(fin[:, 1].all()) != meets and bool(fin[:, 1].any()) != meets, (route, (n, ih, iw), i, j)
+                        ok = [c for c in range(IC) if c != 1]
+                        assert bool(fin[:, ok].all())
+                        ref = torch.einsum("nhwo,nhwc->oc", dY.double(), cut(pad, i, j))
+                        scale = torch.einsum("nhwo,nhwc->oc", dY.double(), cut(pad, i, j).abs())
+                        assert float(((dW[:, i, j].double() - ref).abs() / scale)[:, ok].max()) <= TOL[mode]["comp"]
+        finally:
+            for k in route:
+                lib.set_option(k, 1)
+    assert lib.device_status() == 0

@@ -628,6 +628,7 @@ struct IgemmPlan {
     size_t aPix = 0, aRow = 0, aImg = 0;   // floats between pixels, rows and images of the activation (0: dense)
     const struct LatticePlan* lat = nullptr;   // strided forward on the halo kernel: the phases; FH, FW, kdim then describe the
                                      // lattice convolution (most taps of a phase, channels of all phases together)
+    int min_ksplit = 1;              // leave the layer (return 1) where its reduction would be cut into fewer parts
     bool pad = false;                // kdim may be any multiple of 4: the TMA fills the last 32-channel chunk of both operands with zeros
 };
 
@@ -656,6 +657,10 @@ static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, bool strided
     const double nc = ncols < 64 ? 64 : ncols, mem = mode3x ? 150 : 360;
     return (double)taps * chunks32(K) * nc * (strided ? 1.4 : 1.0) <= (double)chunks32(taps * K) * (nc + mem);
 }
+// The tensor core truncates as it accumulates, so the error of a 3xTF32 sum grows with its length, and a reduction split over idle
+// SMs is the more exact one.  Into how many parts would a layer's product over the patch matrix be cut?  (Zero-filled channels are
+// left to it where theirs would be fewer: 64 x 14 x 14, 148 -> 64 channels 3x3: 1.0e-6 in three parts, 3.1e-6 in one.)
+static int patch_ksplit(const AlphaConvShape* s, int mode3x, int sms);
 // A route that needs scratch may not take away what a route without any could do: under stream capture, or in a
 // caller-owned workspace, the call then goes on to the older route.
 static inline bool scratch_refused(int rc) { return rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH; }
@@ -1180,6 +1185,29 @@ static int launch_tapstack(DeviceCtx* c, const IgemmPlan& pl, const TapStackPlan
     return check_launch("conv_tapstack_kernel");
 }
 
+// Column tile and plan of the single-CTA kernel, and the tiles of that plan (flat ones aside).
+static HaloChoice pick_halo(const IgemmPlan& pl, int mode3x, int sms, int* BN_out)
+{
+    const int gran = pl.b_mn ? 32 : 16;
+    int BN = ((pl.ncols + gran - 1) / gran) * gran;
+    if (BN > 256) BN = (pl.ncols % 256 == 0 || pl.ncols > 512) ? 256 : 128;
+    HaloChoice ch = plan_halo(pl, BN, mode3x, pl.b_mn, sms);
+    // narrower column tiles when the wide ones leave SMs idle (small images, few pixels): the plan's
+    // cost is the time of the busiest CTA, so candidates compare directly
+    for (int cand = 128; cand >= 64; cand >>= 1) {
+        if (cand >= BN || pl.ncols % cand != 0 || !opt(OPT_HALO_NARROW)) continue;
+        HaloChoice alt = plan_halo(pl, cand, mode3x, pl.b_mn, sms);
+        if (alt.valid && (!ch.valid || alt.cost < 0.9 * ch.cost)) { ch = alt; BN = cand; }
+    }
+    *BN_out = BN;
+    return ch;
+}
+static long long halo_tiles(const IgemmPlan& pl, const HaloChoice& ch, int BN)
+{
+    const long long row_blocks = ch.NI > 1 ? 1 : (pl.oH + 16 * ch.JH - 1) / (16 * ch.JH);
+    return (long long)((pl.ncols + BN - 1) / BN) * ((pl.aN + ch.NI - 1) / ch.NI) * row_blocks * ((pl.oW + 8 * ch.JW - 1) / (8 * ch.JW));
+}
+
 static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStream_t stream)
 {
     const int tile_mode = env_tile_mode();
@@ -1206,7 +1234,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         skinny = 2 * tiles128 <= sm_budget(c) && (long long)chunks32(pl.kdim) * pl.FH * pl.FW >= 32;
     }
     // per-image weights: only the single-CTA kernel knows them (its W-tile loads add the image's first row)
-    const bool try_pair = !pl.w_img_rows && !pl.lat && !pl.aPix && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
+    const bool try_pair = !pl.w_img_rows && !pl.lat && !pl.aPix && pl.min_ksplit <= 1 && (pair_env > 0 || (pair_env < 0 && pair_auto && tile_mode == 0));
     if (try_pair && !skinny) {
         const int rc2 = launch_halo_pair(c, pl, mode3x, stream);
         if (rc2 != 1) return rc2;
@@ -1220,17 +1248,8 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         pl.aN = 1; pl.aW = 8; pl.aH = (int)(flat_m / 8);
         pl.oH = pl.aH; pl.oW = 8;
     }
-    const int gran = pl.b_mn ? 32 : 16;
-    int BN = ((pl.ncols + gran - 1) / gran) * gran;
-    if (BN > 256) BN = (pl.ncols % 256 == 0 || pl.ncols > 512) ? 256 : 128;
-    HaloChoice ch = plan_halo(pl, BN, mode3x, pl.b_mn, sm_budget(c));
-    // narrower column tiles when the wide ones leave SMs idle (small images, few pixels): the plan's
-    // cost is the time of the busiest CTA, so candidates compare directly
-    for (int cand = 128; cand >= 64; cand >>= 1) {
-        if (cand >= BN || pl.ncols % cand != 0 || !opt(OPT_HALO_NARROW)) continue;
-        HaloChoice alt = plan_halo(pl, cand, mode3x, pl.b_mn, sm_budget(c));
-        if (alt.valid && (!ch.valid || alt.cost < 0.9 * ch.cost)) { ch = alt; BN = cand; }
-    }
+    int BN = 0;
+    const HaloChoice ch = pick_halo(pl, mode3x, sm_budget(c), &BN);
     {
         // plain TF32 with few output channels: one MMA per filter row where the model says it is faster
         const TapStackPlan ts = (pl.w_img_rows || pl.lat || pl.aPix) ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
@@ -1272,6 +1291,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     const long long total = (long long)p.n_tiles * p.n_blocks * p.row_blocks * p.col_blocks;
     if (total > 2147483647LL) return 1;
     p.total_tiles = (int)total;
+    if (pl.min_ksplit > 1 && (ch.flat || halo_ksplit(pl, total, p.kchunks, sm_budget(c)) < pl.min_ksplit)) return 1;
     if (pl.lat && !pl.force) {
         // Against the im2col kernel.  One tap per W-tile stage and patches that change with every phase run at 1.4 times the
         // plan's clocks (2.2 times with column tiles under 64, whose MMAs are all issue); the lo plane of W and the sum of
@@ -1505,6 +1525,20 @@ static int launch_patch_gemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cuda
     if (rc != 1) return rc;
     if (g.W_lo) return 1;   // the per-tap kernel splits W itself and cannot take pre-split planes
     return launch_igemm(c, g, mode3x, stream);
+}
+
+static int patch_ksplit(const AlphaConvShape* s, int mode3x, int sms)
+{
+    const long long M = (long long)s->N * s->OH * s->OW;
+    if (!mode3x || M / 128 > 4LL * sms) return 1;   // (a macro tile has at most eight accumulators, and half of the SMs are idle)
+    IgemmPlan g{};
+    const bool flat = M % 8 == 0 && opt(OPT_HALO_FLAT);
+    g.aN = flat ? 1 : s->N; g.oH = g.aH = flat ? (int)(M / 8) : s->OH; g.oW = g.aW = flat ? 8 : s->OW;
+    g.FH = g.FW = g.sh = g.sw = 1;
+    g.ncols = s->OC; g.kdim = chunks32(s->FH * s->FW * s->IC) * 32; g.b_mn = false; g.force = true;
+    int BN = 0;
+    const HaloChoice ch = pick_halo(g, mode3x, sms, &BN);
+    return ch.valid ? halo_ksplit(g, halo_tiles(g, ch, BN), g.kdim / 32, sms) : 1;
 }
 
 // ---- few input channels: windows of a filter row -----------------------------------------------------
@@ -2751,6 +2785,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         pl.b_mn = false; pl.flip = false; pl.kdim = s->IC; pl.pad = true;
         const bool strided = s->sh != 1 || s->sw != 1;
         pl.force = !strided;   // the patch matrix would run tiles as empty
+        if (patch_path_ok(s) && opt(OPT_HALO_PAD) == 1) pl.min_ksplit = patch_ksplit(s, cur_mode3x(), sm_budget(c));
         rc = strided ? launch_halo_lattice(c, pl, cur_mode3x(), stream) : launch_halo(c, pl, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
         // Not the im2col kernel where there is a patch matrix: it adds hi*hi and both correction terms into one accumulator, whose

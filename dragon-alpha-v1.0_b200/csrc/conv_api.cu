@@ -1890,7 +1890,8 @@ static inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 
 
 struct DwForm { int G, NT; bool stacked, diag; long long cost; };   // cost: clocks of a filter row's MMAs per 8 pixels; < 0: none fits
 
-static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image, int mode3x)
+// force_stacked: 0 / 1 as the option DW_STACKED, -1 by cost.  pow2: channel blocks that are powers of two and divide IC.
+static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image, int mode3x, int force_stacked = -1, bool pow2 = false)
 {
     // Input channels per CTA: the accumulators of a CTA's G taps, NT columns each, must fit the 512 tensor-memory
     // columns.  A CTA owns a whole filter row (G = FW) unless rows of more than three taps do better split over
@@ -1905,6 +1906,11 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
     auto nt_for = [&](int slots_cols, int top, int cols_per) {
         int best = 0;
         long long best_clk = 0;
+        if (pow2) {
+            for (int nt = top; nt >= 32; nt >>= 1)
+                if (s->IC % nt == 0 && slots_cols * nt <= 512) return nt;
+            return 0;
+        }
         for (int nt = 32; nt <= top && slots_cols * nt <= 512; nt += 32) {
             const long long clk = tiles(nt) * mma_clk(cols_per * nt);
             if (!best || clk < best_clk || (clk == best_clk && tiles(nt) < tiles(best))) { best = nt; best_clk = clk; }
@@ -1923,8 +1929,7 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
             if (NTq) {
                 const long long stk_cost = slots * mma_clk(2 * NTq) * ((s->OC + 63) / 64) * tiles(NTq);
                 bool stacked = stk_cost < f.cost;
-                const int force = opt(OPT_DW_STACKED);
-                if (force >= 0) stacked = force != 0;
+                if (force_stacked >= 0) stacked = force_stacked != 0;
                 if (stacked) { f.stacked = true; f.NT = NTq; f.cost = stk_cost; }
             }
         }
@@ -1949,16 +1954,48 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
     }
     return form;
 }
+static int dw_groups(const AlphaConvShape* s, const DwForm& f)
+{
+    const int oc_tile = f.stacked ? 64 : 128;
+    return (s->FW + f.G - 1) / f.G * s->FH * ((s->IC + f.NT - 1) / f.NT) * ((s->OC + oc_tile - 1) / oc_tile);
+}
+static int dw_parts(const AlphaConvShape* s, const DwForm& f, int sms)
+{
+    const long long px = (long long)s->N * s->OH * s->OW, most = px / 128 > 1 ? px / 128 : 1, parts = sms / dw_groups(s, f);
+    return (int)(parts < 1 ? 1 : (parts > most ? most : parts));
+}
+// The tensor core truncates as it accumulates, so the error of a deltaW sum grows with the steps (of 8 pixels) one accumulator takes,
+// and is 3.2 times that where the correction terms of 3xTF32 go into the same accumulator instead of the stacked planes (measured:
+// 3.1 to 3.3 times at the same steps).  A form may take no more steps than channel blocks of powers of two give over `former` - the
+// layer itself (nullptr), or the 1x1 product over its patch matrix where it has one to go to.  The stacked form where that is enough
+// (32 x 28 x 28, 192 -> 128 channels 3x3: 7.7e-6, 81 us; 8.1e-6 and 70 us unstacked), otherwise more parts than there are SMs for.
+// Returns the most steps; 0 = any.
+static double dw_most_steps(const AlphaConvShape* s, bool strided, const AlphaConvShape* former, int sms, DwForm* f)
+{
+    const AlphaConvShape* m = former ? former : s;
+    const DwForm o = plan_dw_form(m, m->sh != 1 || m->sw != 1, false, 1, -1, true);
+    if (o.cost < 0) return 0;
+    const double px = (double)s->N * s->OH * s->OW;
+    auto weight = [](const DwForm& g) { return g.stacked ? 1.0 : 3.2; };
+    auto err = [&](const DwForm& g) { return weight(g) * px / 8.0 / dw_parts(s, g, sms); };
+    const double most = weight(o) * px / 8.0 / dw_parts(m, o, sms);
+    if (err(*f) > 1.001 * most && !f->stacked) {
+        const DwForm g = plan_dw_form(s, strided, false, 1, 1);
+        if (g.cost >= 0 && g.stacked && err(g) < err(*f)) *f = g;
+    }
+    return !former && err(*f) <= 1.001 * most ? 0 : most / weight(*f);
+}
 
 // Returns 1 when the shape is left to the split-K im2col kernel, 0 on launch, < 0 on error.
 // deltaB != nullptr: the kernel also sums the columns of deltaY (bias gradient); *bias_fused tells whether it did.
 // per_image: dW receives N separate results, dW[n] = the sum over the pixels of image n only (batched matrix
 // products C[n] = A[n]^T * B[n]); every CTA column of the grid then owns one image and writes its result in place.
 // x_pitch: floats between pixels, rows and images of X where it is not dense (stride 1 only).
+// former: see dw_most_steps (nullptr: the layer itself).
 // *spills: whether pixel tiles reach past the output where X still has pixels (see DwRepair).
 static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float* X, const float* dY, float* dW,
                           int mode3x, cudaStream_t stream, float* deltaB = nullptr, bool* bias_fused = nullptr,
-                          bool per_image = false, const size_t* x_pitch = nullptr, bool* spills = nullptr)
+                          bool per_image = false, const size_t* x_pitch = nullptr, const AlphaConvShape* former = nullptr, bool* spills = nullptr)
 {
     if (bias_fused) *bias_fused = false;
     if (opt(OPT_CONV_DW) == 1 && !per_image) return 1;
@@ -1990,8 +2027,9 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     for (int k = 0; k < nph; ++k)
         if (ph_psi[k] >= s->IW) return 1;                 // a lattice without a column
     if (s->sh > s->IH) return 1;
-    const DwForm form = plan_dw_form(s, strided, per_image, mode3x);
+    DwForm form = plan_dw_form(s, strided, per_image, mode3x, opt(OPT_DW_STACKED));
     if (form.cost < 0) return 1;
+    const double most_steps = mode3x && !per_image && opt(OPT_DW_STACKED) < 0 ? dw_most_steps(s, strided, former, sm_budget(c), &form) : 0;
     const int G = form.G, tgroups = (s->FW + G - 1) / G;
     int NT = form.NT;
     const bool stacked = form.stacked, diag = form.diag;
@@ -2053,6 +2091,12 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     p.total_tiles = (int)total;
     int parts = sm_budget(c) / groups;
     if (parts < 1) parts = 1;
+    if (most_steps > 0) {
+        // (a tenth more for tiles that do not divide; the layer itself had the idle slots of its tiles before, too)
+        const double per_tile = R * CW / 8.0, idle = former ? 1.0 : per_tile * 8.0 * p.total_tiles / ((double)s->N * s->OH * s->OW);
+        const int tiles = (int)(1.1 * idle * most_steps / per_tile), least = tiles > 1 ? (p.total_tiles + tiles - 1) / tiles : p.total_tiles;
+        if (parts < least) parts = least;
+    }
     if (parts > p.total_tiles) parts = p.total_tiles;
     if (per_image) {
         if (s->N > 65535 * 32 || deltaB) return 1;
@@ -2207,6 +2251,13 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
 // passes through memory on the way (8 bytes at 5 TB/s over 148 SMs at 1.8 GHz).  50 x 35 x 29, 36 -> 100 channels 3x3: 192 us
 // over the patch matrix, 62 us straight; 512 x 32 x 32, 4 -> 64 channels 7x7 s2: 98 us over the patch matrix.
 enum class DwRoute { Patch, Straight, Window };
+static AlphaConvShape patch_product(const AlphaConvShape* s)
+{
+    AlphaConvShape t = *s;
+    t.IC = chunks32(s->FH * s->FW * s->IC) * 32; t.FH = t.FW = 1; t.sh = t.sw = 1; t.ph = t.pw = 0;
+    t.IH = s->OH; t.IW = s->OW;
+    return t;
+}
 static AlphaConvShape window_shape(const AlphaConvShape* s, const WindowPlan& w)
 {
     AlphaConvShape t = *s;
@@ -2219,9 +2270,7 @@ static DwRoute pick_dw_route(const AlphaConvShape* s, const WindowPlan& w, int m
     if (opt(OPT_HALO_WINDOW) == 2 && window_fits(s, w)) return DwRoute::Window;
     if (fpad == 2) return DwRoute::Straight;
     DwRoute best = DwRoute::Patch;
-    AlphaConvShape t = *s;
-    t.IC = chunks32(s->FH * s->FW * s->IC) * 32; t.FH = t.FW = 1; t.sh = t.sw = 1; t.ph = t.pw = 0;
-    t.IH = s->OH; t.IW = s->OW;
+    const AlphaConvShape t = patch_product(s);
     const DwForm patch = plan_dw_form(&t, false, false, mode3x);
     double cost = patch.cost < 0 ? 1e30 : (double)patch.cost + 3.4 * t.IC;
     // (windows of more channels read X so often, every window its whole row, that the straight form wins: 36 -> 100 channels in
@@ -2249,7 +2298,8 @@ static int launch_dw_window(DeviceCtx* c, const AlphaConvShape* s, const WindowP
     rc = launch_window_pack(c, s, w, X, stream, &Xp);
     if (rc) return rc;
     const size_t pitch[3] = {(size_t)s->sw * s->sh * s->IC, w.row, w.row * w.Hq};
-    rc = launch_dw_halo(c, &t, Xp, dY, tmp, mode3x, stream, nullptr, nullptr, false, pitch, spills);
+    const AlphaConvShape former = patch_product(s);
+    rc = launch_dw_halo(c, &t, Xp, dY, tmp, mode3x, stream, nullptr, nullptr, false, pitch, &former, spills);
     if (rc) return rc;
     const size_t n = (size_t)s->OC * s->FH * s->FW * s->IC;
     size_t blocks = (n + 255) / 256;
@@ -2903,7 +2953,8 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
         const DwRoute route = pick_dw_route(s, win, cur_mode3x());
         bool spills = false;
         rc = 1;
-        if (route == DwRoute::Straight) rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream, nullptr, nullptr, false, nullptr, &spills);
+        const AlphaConvShape former = patch_product(s);
+        if (route == DwRoute::Straight) rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream, nullptr, nullptr, false, nullptr, &former, &spills);
         else if (route == DwRoute::Window) rc = launch_dw_window(c, s, win, X, deltaY, deltaW, cur_mode3x(), stream, &spills);
         if (!rc && spills) rc = launch_dw_repair(s, X, deltaY, deltaW, stream, route == DwRoute::Window ? "dw_window" : "dw_halo");
         if (rc != 1 && !scratch_refused(rc)) return rc;

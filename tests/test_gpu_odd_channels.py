@@ -118,3 +118,34 @@ def test_small_layers_err_no_more_than_the_patch_product(pkg, shape):
         finally:
             lib.set_option("HALO_PAD", 1)
     assert err[1] <= 1.25 * err[0], err
+
+
+# N, IH, IC, OC, F, s, p and the options of the route whose error is the measure: the patch product of an odd channel count, the
+# stacked planes of whole chunks (a block of 96 or 128 columns would be cheaper unstacked, in sums of the same or twice the length)
+@pytest.mark.parametrize("shape,former", [((50, 35, 12, 64, 3, 1, 1), {"HALO_WINDOW": 0, "HALO_PAD": 0}), ((64, 32, 4, 100, 4, 2, 1), {"HALO_WINDOW": 0, "HALO_PAD": 0}),
+                                          ((64, 14, 68, 64, 3, 1, 1), {"HALO_WINDOW": 0, "HALO_PAD": 0}), ((8, 28, 352, 256, 5, 1, 2), {"DW_STACKED": 1}),
+                                          ((32, 28, 192, 128, 3, 1, 1), {"DW_STACKED": 1})], ids=str)
+def test_deltaW_errs_no_more_than_its_former_route(pkg, shape, former):
+    """The steps one accumulator takes bound the truncation error of a 3xTF32 deltaW: forms with fewer parts or without stacked
+    planes get more parts, or give way (a quarter more for sums in another order)."""
+    import torch
+    lib, engine = pkg.submodule("lib"), pkg.submodule("engine")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math="3xtf32"))
+    N, IH, IC, OC, F, s, p = shape
+    OH, OW = out_hw(IH, IH, F, F, s, s, p, p)
+    g = torch.Generator(device="cuda").manual_seed(IC)
+    X, dY = torch.randn((N, IH, IH, IC), device="cuda", generator=g).relu_(), torch.randn((N, OH, OW, OC), device="cuda", generator=g)
+    pad = torch.nn.functional.pad(X, (0, 0, p, p, p, p))
+    ref = torch.stack([torch.stack([dY.double().reshape(-1, OC).T @ pad[:, i:i + (OH - 1) * s + 1:s, j:j + (OW - 1) * s + 1:s].double().reshape(-1, IC)
+                                    for j in range(F)], 1) for i in range(F)], 1)
+    err = []
+    for options in ({}, former):
+        saved = {k: lib.get_option(k) for k in options}
+        for k, v in options.items():
+            lib.set_option(k, v)
+        try:
+            err.append(float((eng.dconv3D_deltaW(X, dY, F, F, s, s, p, p).double() - ref).norm() / ref.norm()))
+        finally:
+            for k, v in saved.items():
+                lib.set_option(k, v)
+    assert err[0] <= 1.25 * err[1], err

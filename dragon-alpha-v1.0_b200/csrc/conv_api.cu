@@ -1986,6 +1986,51 @@ static double dw_most_steps(const AlphaConvShape* s, bool strided, const AlphaCo
     return !former && err(*f) <= 1.001 * most ? 0 : most / weight(*f);
 }
 
+// Pixel tile: CW columns of 8-pixel groups, R rows, sized so that three stages fit shared memory (nph = column phases of the taps).
+struct DwTile { int CW, R; };
+static size_t dw_stage_bytes(const DwForm& f, int nph, int mode3x, int CW, int r)
+{
+    const uint32_t dyblk = ((uint32_t)r * CW * 128 + 1023) & ~1023u, xbk = ((uint32_t)r * (CW + f.G - 1) * 128 + 1023) & ~1023u;
+    return (size_t)(mode3x || f.diag ? 2 : 1) * ((f.stacked ? 2 : 4) * dyblk + (size_t)nph * (f.NT / 32) * xbk);
+}
+static DwTile plan_dw_tile(const AlphaConvShape* s, const DwForm& f, int nph, int mode3x)
+{
+    int CW = opt(OPT_DW_CW);
+    if (!CW) CW = (s->OW <= 8 || (s->OW % 16 != 0 && s->OW % 16 <= 8)) ? 8 : 16;  // fewer idle columns
+    int R = opt(OPT_DW_R);
+    if (!R) {
+        // Tile height: a tile costs its R * CW / 8 steps of 8 pixels plus a fixed share (the refill of its ring
+        // slot is not hidden behind so few MMAs: about 8 steps' worth measured in plain TF32, 4 with the three times
+        // longer steps of 3xTF32), and rows past the image edge are idle slots.  7 rows cover 7, 14, 28 and 56 pixel
+        // high images exactly where 8 leave up to one slot in eight idle.  The taller tile on a tie.
+        const int halves = f.diag ? 2 : 1, fixed = (mode3x && !f.diag) ? 4 : 8;
+        long long best = -1;
+        for (int cand : {8, 7, 4, 2, 1}) {
+            if (cand > 1 && (2 * dw_stage_bytes(f, nph, mode3x, CW, cand) > 210 * 1024 || cand * halves > s->OH)) continue;
+            const long long blocks = (s->OH + cand * halves - 1) / (cand * halves);
+            const long long cost = blocks * ((long long)cand * (CW / 8) + fixed);   // diagonal: one MMA serves both halves
+            if (best < 0 || cost < best) { best = cost; R = cand; }
+        }
+    }
+    return DwTile{CW, R};
+}
+// CTAs that share the pixel tiles of a group: what the SMs give, or more where a sum may take no more than `most` steps (0 = any) -
+// a tenth more for tiles that do not divide; `idle` = the idle slots it had before, too.
+static int dw_launch_parts(int groups, int total_tiles, const DwTile& t, double most, double idle, int sms)
+{
+    int parts = sms / groups;
+    if (parts < 1) parts = 1;
+    if (most > 0) {
+        const int tiles = (int)(1.1 * idle * most / (t.R * t.CW / 8.0)), least = tiles > 1 ? (total_tiles + tiles - 1) / tiles : total_tiles;
+        if (parts < least) parts = least;
+    }
+    return parts > total_tiles ? total_tiles : parts;
+}
+static inline bool dw_static_taps(const AlphaConvShape* s, const DwForm& f, bool strided)   // the MMAs of a stage are straight-line code
+{
+    return s->FW == 1 || (strided ? s->FW == 3 || s->FW == 4 : f.G == 3);
+}
+
 // Returns 1 when the shape is left to the split-K im2col kernel, 0 on launch, < 0 on error.
 // deltaB != nullptr: the kernel also sums the columns of deltaY (bias gradient); *bias_fused tells whether it did.
 // per_image: dW receives N separate results, dW[n] = the sum over the pixels of image n only (batched matrix
@@ -2042,30 +2087,10 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     const int groups = tgroups * s->FH * p.ic_tiles * p.oc_tiles;
     if (groups > 65535) return 1;
     p.G = G; p.tgroups = tgroups;
-    // pixel tile: CW columns of 8-pixel groups, R rows, sized so that three stages fit shared memory
     const int planes = (mode3x || diag) ? 2 : 1;   // diagonal: the second plane holds the second half tile
-    int CW = opt(OPT_DW_CW);
-    if (!CW) CW = (s->OW <= 8 || (s->OW % 16 != 0 && s->OW % 16 <= 8)) ? 8 : 16;  // fewer idle columns
-    const int PW = CW + G - 1;
-    int R = opt(OPT_DW_R);
-    auto stage_bytes = [&](int r) {
-        const uint32_t dyblk = ((uint32_t)r * CW * 128 + 1023) & ~1023u, xbk = ((uint32_t)r * PW * 128 + 1023) & ~1023u;
-        return (size_t)planes * (dyb * dyblk + (size_t)nph * (NT / 32) * xbk);
-    };
-    if (!R) {
-        // Tile height: a tile costs its R * CW / 8 steps of 8 pixels plus a fixed share (the refill of its ring
-        // slot is not hidden behind so few MMAs: about 8 steps' worth measured in plain TF32, 4 with the three times
-        // longer steps of 3xTF32), and rows past the image edge are idle slots.  7 rows cover 7, 14, 28 and 56 pixel
-        // high images exactly where 8 leave up to one slot in eight idle.  The taller tile on a tie.
-        const int halves = diag ? 2 : 1, fixed = (mode3x && !diag) ? 4 : 8;
-        long long best = -1;
-        for (int cand : {8, 7, 4, 2, 1}) {
-            if (cand > 1 && (2 * stage_bytes(cand) > 210 * 1024 || cand * halves > s->OH)) continue;
-            const long long blocks = (s->OH + cand * halves - 1) / (cand * halves);
-            const long long cost = blocks * ((long long)cand * (CW / 8) + fixed);   // diagonal: one MMA serves both halves
-            if (best < 0 || cost < best) { best = cost; R = cand; }
-        }
-    }
+    const DwTile tile = plan_dw_tile(s, form, nph, mode3x);
+    const int CW = tile.CW, PW = CW + G - 1, R = tile.R;
+    auto stage_bytes = [&](int r) { return dw_stage_bytes(form, nph, mode3x, CW, r); };
     if (2 * stage_bytes(R) > 220 * 1024) return 1;
     if (strided && !opt(OPT_DW_R) && opt(OPT_DW_STRIDED) != 2) {
         // Few pixels per image leave tiles of one or two steps, whose fixed share dominates; below a fifth (3xTF32;
@@ -2089,15 +2114,8 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     const long long total = (long long)s->N * p.tiles_per_img;
     if (total > 2147483647LL) return 1;
     p.total_tiles = (int)total;
-    int parts = sm_budget(c) / groups;
-    if (parts < 1) parts = 1;
-    if (most_steps > 0) {
-        // (a tenth more for tiles that do not divide; the layer itself had the idle slots of its tiles before, too)
-        const double per_tile = R * CW / 8.0, idle = former ? 1.0 : per_tile * 8.0 * p.total_tiles / ((double)s->N * s->OH * s->OW);
-        const int tiles = (int)(1.1 * idle * most_steps / per_tile), least = tiles > 1 ? (p.total_tiles + tiles - 1) / tiles : p.total_tiles;
-        if (parts < least) parts = least;
-    }
-    if (parts > p.total_tiles) parts = p.total_tiles;
+    const double idle = former ? 1.0 : (double)R * CW * p.total_tiles / ((double)s->N * s->OH * s->OW);
+    int parts = dw_launch_parts(groups, p.total_tiles, tile, most_steps, idle, sm_budget(c));
     if (per_image) {
         if (s->N > 65535 * 32 || deltaB) return 1;
         parts = s->N;
@@ -2247,9 +2265,11 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
 
 // deltaW of a layer whose input channels are no multiple of 32 (IC % 4 == 0): straight from X with channel blocks whose tail
 // the TMA zero-fills, over windows of a filter row (see window_pack_kernel), or over the patch matrix (a 1x1 deltaW with
-// FH * FW * IC channels)?  In clocks of one SM per 8 pixels: the MMAs of each form, and 3.4 clocks per float and pixel that
-// passes through memory on the way (8 bytes at 5 TB/s over 148 SMs at 1.8 GHz).  50 x 35 x 29, 36 -> 100 channels 3x3: 192 us
-// over the patch matrix, 62 us straight; 512 x 32 x 32, 4 -> 64 channels 7x7 s2: 98 us over the patch matrix.
+// FH * FW * IC channels)?  By the time each would take (dw_time).
+// Fitted on 673 layers (3 to 300 channels to 48 to 256, seven filters and strides, both modes, all three routes measured): the route
+// taken is on average 1.03 times as long as the best of the three and at most 1.5 times, on layers of 20 to 30 us.
+// 50 x 35 x 29, 36 -> 100 channels 3x3: 192 us over the patch matrix, 62 us straight; 512 x 32 x 32, 4 -> 64 channels 7x7 s2: 98 / 75 us
+// over the patch matrix / windows; 128 x 32 x 32, 36 -> 48 channels 7x7 s2: 155 / 294 us over the patch matrix / straight.
 enum class DwRoute { Patch, Straight, Window };
 static AlphaConvShape patch_product(const AlphaConvShape* s)
 {
@@ -2264,26 +2284,60 @@ static AlphaConvShape window_shape(const AlphaConvShape* s, const WindowPlan& w)
     t.IH = w.Hq; t.IW = s->OW; t.IC = w.K; t.FH = w.U; t.FW = 1; t.sh = t.sw = 1; t.ph = t.pw = 0;
     return t;
 }
-static DwRoute pick_dw_route(const AlphaConvShape* s, const WindowPlan& w, int mode3x)
+// Microseconds of a deltaW on the halo kernel at 1.8 GHz, the sum of its partials with it; < 0 where it has no form.  A step of 8
+// pixels takes the longer of its MMAs (200 clocks each where the issue loop is not straight-line code) and its shared-memory
+// traffic at 128 B/clk: operand reads, what the TMA writes and, in 3xTF32, the split's read and write of that.  A tile costs the refill
+// of its ring slot on top (3 steps of 118 clocks, 7 in plain TF32), a wave of CTAs 4500 clocks.
+static double dw_time(const AlphaConvShape* s_in, const AlphaConvShape* former, bool flat, int mode3x, int sms)
+{
+    AlphaConvShape v = *s_in;
+    const AlphaConvShape* s = &v;
+    const long long px = (long long)v.N * v.OH * v.OW;
+    if (flat && px % 16 == 0) { v.N = 1; v.OW = v.IW = 16; v.OH = v.IH = (int)(px / 16); }
+    const bool strided = v.sh != 1 || v.sw != 1;
+    if (v.sh > 2 || v.sw > 2 || v.FW > 8) return -1;
+    DwForm f = plan_dw_form(s, strided, false, mode3x);
+    if (f.cost < 0) return -1;
+    const double most = mode3x ? dw_most_steps(s, strided, former, sms, &f) : 0;
+    const int nph = v.sw == 2 && v.FW > 1 ? 2 : 1;
+    const DwTile t = plan_dw_tile(s, f, nph, mode3x);
+    const int rows = f.diag ? 2 * t.R : t.R, groups = dw_groups(s, f);
+    const long long tiles = (long long)v.N * ((v.OH + rows - 1) / rows) * ((v.OW + t.CW - 1) / t.CW);
+    if (groups > 65535 || tiles > 2147483647LL) return -1;
+    const int parts = dw_launch_parts(groups, (int)tiles, t, most, 1.0, sms);
+    auto clk = [](int n) { return n / 2 > 59 ? n / 2.0 : 59.0; };
+    const bool wide = f.stacked;                       // stacked planes or two half tiles: 2 * NT columns per MMA
+    const int mmas = f.G * (mode3x && !f.stacked ? 3 : 1), cols = wide ? 2 * f.NT : f.NT;
+    double mma = mmas * clk(cols);
+    if (!dw_static_taps(s, f, strided) && mma < mmas * 200.0) mma = mmas * 200.0;
+    const double fill = ((f.stacked ? 64 : 128) + (double)f.NT * nph * (t.CW + f.G - 1) / t.CW) * 32.0 * (f.diag ? 2 : 1);
+    const double smem = (mmas * (4096.0 + 32.0 * cols) + fill * (mode3x ? 3 : 1)) / 128.0;
+    const double step = mma > smem ? mma : smem, per_cta = (double)((tiles + parts - 1) / parts);
+    const double cta = per_cta * (t.R * t.CW / 8.0 * step + 118.0 * (mode3x && !f.diag ? 3 : 7)) + 4500.0;
+    const long long waves = ((long long)groups * parts + sms - 1) / sms;
+    const int planes = parts * (f.stacked ? 2 : 1);
+    return waves * cta / 1800.0 + (planes > 1 ? 3.0 + 4e-6 / 3.5 * planes * ((double)v.OC * v.FH * v.FW * v.IC) : 0.0);
+}
+static DwRoute pick_dw_route(const AlphaConvShape* s, const WindowPlan& w, int mode3x, int sms)
 {
     const int fpad = opt(OPT_HALO_PAD);
     if (opt(OPT_HALO_WINDOW) == 2 && window_fits(s, w)) return DwRoute::Window;
     if (fpad == 2) return DwRoute::Straight;
-    DwRoute best = DwRoute::Patch;
     const AlphaConvShape t = patch_product(s);
-    const DwForm patch = plan_dw_form(&t, false, false, mode3x);
-    double cost = patch.cost < 0 ? 1e30 : (double)patch.cost + 3.4 * t.IC;
-    // (windows of more channels read X so often, every window its whole row, that the straight form wins: 36 -> 100 channels in
-    // plain TF32 34 us straight, 57 over windows; 80 -> 64 in 3xTF32 251 and 310)
-    if (window_fits(s, w) && s->IC <= (mode3x ? 32 : 4)) {
+    const double px = (double)s->N * s->OH * s->OW, bw = 3.5e6;   // bytes per microsecond
+    const double repair = s->FH > 1 || s->FW > 1 ? 2.0 : 0.0;
+    DwRoute best = DwRoute::Patch;
+    double time = dw_time(&t, nullptr, true, mode3x, sms);
+    time = time < 0 ? 1e30 : time + 1.0 + 4.0 * px * t.IC / bw;
+    if (window_fits(s, w)) {
         const AlphaConvShape ws = window_shape(s, w);
-        const DwForm f = plan_dw_form(&ws, false, false, mode3x);
-        const double cw = (double)f.cost * w.U + 3.4 * w.per_pixel;
-        if (f.cost >= 0 && cw < 0.95 * cost) { best = DwRoute::Window; cost = cw; }
+        const double own = dw_time(&ws, &t, false, mode3x, sms);
+        const double tw = 1.1 * (own + 2.0 + 8.0 * w.elems / bw) + repair;   // (windows overlap: X passes through L2 more than once)
+        if (own >= 0 && tw < time) { best = DwRoute::Window; time = tw; }
     }
     if (fpad) {
-        const DwForm own = plan_dw_form(s, s->sh != 1 || s->sw != 1, false, mode3x);
-        if (own.cost >= 0 && (double)own.cost * s->FH <= cost) best = DwRoute::Straight;
+        const double own = dw_time(s, &t, s->FH == 1 && s->FW == 1 && s->sh == 1 && s->sw == 1, mode3x, sms);
+        if (own >= 0 && own + repair < time) best = DwRoute::Straight;
     }
     return best;
 }
@@ -2950,7 +3004,7 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
         return fail(ALPHA_E_ARG, "tensor deltaW path needs IC %% 32 == 0 (IC=%d)", s->IC);
     if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
         const WindowPlan win = window_plan(s, s->sh);
-        const DwRoute route = pick_dw_route(s, win, cur_mode3x());
+        const DwRoute route = pick_dw_route(s, win, cur_mode3x(), sm_budget(c));
         bool spills = false;
         rc = 1;
         const AlphaConvShape former = patch_product(s);

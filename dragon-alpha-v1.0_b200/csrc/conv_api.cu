@@ -649,13 +649,24 @@ static inline bool whole_chunks(const IgemmPlan& pl) { return pl.kdim % 32 == 0 
 // costs nc * 2 FLOPs at the rate these kernels sustain (190 TFLOP/s in 3xTF32, 450 in plain TF32) and the patch matrix
 // 8 bytes at 5 TB/s, as much as 150 (3xTF32) or 360 columns; blocks of fewer than 64 columns cost as much as 64.
 // Both sides measured, patch matrix or 8-channel im2col tiles first: 50 x 35 x 29, 36 -> 100 channels 3x3 82 / 66 us;
-// 9 x 47 x 47, 280 -> 192 3x3 267 / 165 us; 512 x 1000 times 1000 x 4096 84 / 46 us.
-static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, bool strided = false)
+// 9 x 47 x 47, 280 -> 192 3x3 267 / 165 us; 512 x 1000 times 1000 x 4096 84 / 46 us; the other way round, with 1.22 lanes a pixel,
+// 64 x 57 x 57, 44 -> 256 3x3 s2 97 / 128 us (windows).  Over 674 odd layers of the kinds above in both modes the forward route taken is
+// on average 1.04 times as long as the best of patch matrix, chunks and windows.
+// `idle`: lanes of a tile per pixel of the layer, which a patch matrix, flat over all pixels, does not have.
+static double tile_idle(int oH, int oW, int FH, int FW)
+{
+    const int SG = oH + FH - 1, cols = (oW + 7) / 8 * 8;
+    double v = (double)((oH + 15) / 16 * 16) * cols / ((double)oH * oW);
+    if (SG <= 16) v = 16.0 * cols / ((1 + (16 - oH) / SG) * (double)oH * oW);          // stacked images
+    const double flat = 32.0 * ((oH + 3) / 4 * 4) / ((double)oH * oW);                  // flat tiles
+    return FW == 3 && oW + 2 <= 32 && flat < v ? flat : v;
+}
+static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, double idle, bool strided = false)
 {
     const int force = opt(OPT_HALO_PAD);
     if (force != 1) return force == 2;
     const double nc = ncols < 64 ? 64 : ncols, mem = mode3x ? 150 : 360;
-    return (double)taps * chunks32(K) * nc * (strided ? 1.4 : 1.0) <= (double)chunks32(taps * K) * (nc + mem);
+    return idle * taps * chunks32(K) * nc * (strided ? 1.4 : 1.0) <= (double)chunks32(taps * K) * (nc + mem);
 }
 // The tensor core truncates as it accumulates, so the error of a 3xTF32 sum grows with its length, and a reduction split over idle
 // SMs is the more exact one.  Into how many parts would a layer's product over the patch matrix be cut?  (Zero-filled channels are
@@ -1185,29 +1196,6 @@ static int launch_tapstack(DeviceCtx* c, const IgemmPlan& pl, const TapStackPlan
     return check_launch("conv_tapstack_kernel");
 }
 
-// Column tile and plan of the single-CTA kernel, and the tiles of that plan (flat ones aside).
-static HaloChoice pick_halo(const IgemmPlan& pl, int mode3x, int sms, int* BN_out)
-{
-    const int gran = pl.b_mn ? 32 : 16;
-    int BN = ((pl.ncols + gran - 1) / gran) * gran;
-    if (BN > 256) BN = (pl.ncols % 256 == 0 || pl.ncols > 512) ? 256 : 128;
-    HaloChoice ch = plan_halo(pl, BN, mode3x, pl.b_mn, sms);
-    // narrower column tiles when the wide ones leave SMs idle (small images, few pixels): the plan's
-    // cost is the time of the busiest CTA, so candidates compare directly
-    for (int cand = 128; cand >= 64; cand >>= 1) {
-        if (cand >= BN || pl.ncols % cand != 0 || !opt(OPT_HALO_NARROW)) continue;
-        HaloChoice alt = plan_halo(pl, cand, mode3x, pl.b_mn, sms);
-        if (alt.valid && (!ch.valid || alt.cost < 0.9 * ch.cost)) { ch = alt; BN = cand; }
-    }
-    *BN_out = BN;
-    return ch;
-}
-static long long halo_tiles(const IgemmPlan& pl, const HaloChoice& ch, int BN)
-{
-    const long long row_blocks = ch.NI > 1 ? 1 : (pl.oH + 16 * ch.JH - 1) / (16 * ch.JH);
-    return (long long)((pl.ncols + BN - 1) / BN) * ((pl.aN + ch.NI - 1) / ch.NI) * row_blocks * ((pl.oW + 8 * ch.JW - 1) / (8 * ch.JW));
-}
-
 static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStream_t stream)
 {
     const int tile_mode = env_tile_mode();
@@ -1248,8 +1236,17 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
         pl.aN = 1; pl.aW = 8; pl.aH = (int)(flat_m / 8);
         pl.oH = pl.aH; pl.oW = 8;
     }
-    int BN = 0;
-    const HaloChoice ch = pick_halo(pl, mode3x, sm_budget(c), &BN);
+    const int gran = pl.b_mn ? 32 : 16;
+    int BN = ((pl.ncols + gran - 1) / gran) * gran;
+    if (BN > 256) BN = (pl.ncols % 256 == 0 || pl.ncols > 512) ? 256 : 128;
+    HaloChoice ch = plan_halo(pl, BN, mode3x, pl.b_mn, sm_budget(c));
+    // narrower column tiles when the wide ones leave SMs idle (small images, few pixels): the plan's
+    // cost is the time of the busiest CTA, so candidates compare directly
+    for (int cand = 128; cand >= 64; cand >>= 1) {
+        if (cand >= BN || pl.ncols % cand != 0 || !opt(OPT_HALO_NARROW)) continue;
+        HaloChoice alt = plan_halo(pl, cand, mode3x, pl.b_mn, sm_budget(c));
+        if (alt.valid && (!ch.valid || alt.cost < 0.9 * ch.cost)) { ch = alt; BN = cand; }
+    }
     {
         // plain TF32 with few output channels: one MMA per filter row where the model says it is faster
         const TapStackPlan ts = (pl.w_img_rows || pl.lat || pl.aPix) ? TapStackPlan{} : plan_tapstack(pl, mode3x, sm_budget(c));
@@ -1530,15 +1527,14 @@ static int launch_patch_gemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cuda
 static int patch_ksplit(const AlphaConvShape* s, int mode3x, int sms)
 {
     const long long M = (long long)s->N * s->OH * s->OW;
-    if (!mode3x || M / 128 > 4LL * sms) return 1;   // (a macro tile has at most eight accumulators, and half of the SMs are idle)
+    if (!mode3x) return 1;
+    // (macro tiles of 256 pixels up to 64 columns, 128 above, as plan_halo picks for a 1x1 product in the wide form)
+    int BN = (s->OC + 15) / 16 * 16;
+    if (BN > 256) BN = (s->OC % 256 == 0 || s->OC > 512) ? 256 : 128;
+    const int px = BN <= 64 ? 256 : 128;
     IgemmPlan g{};
-    const bool flat = M % 8 == 0 && opt(OPT_HALO_FLAT);
-    g.aN = flat ? 1 : s->N; g.oH = g.aH = flat ? (int)(M / 8) : s->OH; g.oW = g.aW = flat ? 8 : s->OW;
-    g.FH = g.FW = g.sh = g.sw = 1;
-    g.ncols = s->OC; g.kdim = chunks32(s->FH * s->FW * s->IC) * 32; g.b_mn = false; g.force = true;
-    int BN = 0;
-    const HaloChoice ch = pick_halo(g, mode3x, sms, &BN);
-    return ch.valid ? halo_ksplit(g, halo_tiles(g, ch, BN), g.kdim / 32, sms) : 1;
+    g.FH = g.FW = 1;
+    return halo_ksplit(g, (M + px - 1) / px * ((s->OC + BN - 1) / BN), chunks32(s->FH * s->FW * s->IC), sms);
 }
 
 // ---- few input channels: windows of a filter row -----------------------------------------------------
@@ -1573,6 +1569,11 @@ static bool window_fits(const AlphaConvShape* s, const WindowPlan& w)
 // 32 x 224 x 224, 4 -> 64 channels 7x7 s2 (K = 28, U = 7): patch matrix 75 us + 135 us for the product that reads its 360 MB, 108 us
 // here; 64 x 56 x 56, 20 -> 128 3x3: 119 / 102 / 84 us over the patch matrix / zero-filled chunks / windows.  In plain TF32 chunks
 // of a stride-1 layer, whose filter row is one stage, win from 8 channels on (62 against 71 us for 128 x 56 x 56, 8 -> 64).
+static double forward_idle(const AlphaConvShape* s)
+{
+    const bool strided = s->sh != 1 || s->sw != 1;
+    return s->FH * s->FW == 1 && !strided ? 1.0 : tile_idle(s->OH, s->OW, s->FH, strided ? 0 : s->FW);
+}
 static bool window_beats_rest(const AlphaConvShape* s, const WindowPlan& w, int mode3x, int sms)
 {
     if (!window_fits(s, w)) return false;
@@ -1582,8 +1583,8 @@ static bool window_beats_rest(const AlphaConvShape* s, const WindowPlan& w, int 
     const double nc = s->OC < 64 ? 64 : s->OC, mem = mode3x ? 150 : 360;
     const bool strided = s->sh != 1 || s->sw != 1;
     if (!mode3x && !strided && s->IC >= 8) return false;
-    const double own = (double)w.U * chunks32(w.K) * nc + w.per_pixel / 32.0 * mem;
-    const double pad = (double)taps * chunks32(s->IC) * nc * (strided ? 1.4 : 1.0), patch = (double)chunks32(taps * s->IC) * (nc + mem);
+    const double own = tile_idle(s->OH, s->OW, w.U, 1) * w.U * chunks32(w.K) * nc * (w.g < s->sh ? 1.2 : 1.0) + w.per_pixel / 32.0 * mem;
+    const double pad = forward_idle(s) * taps * chunks32(s->IC) * nc * (strided ? 1.4 : 1.0), patch = (double)chunks32(taps * s->IC) * (nc + mem);
     // (an IC of whole 8-channel tiles has no patch matrix to compare with: it would go to the im2col kernel)
     return own < 0.9 * (pad < patch || s->IC % 8 == 0 ? pad : patch);
 }
@@ -2869,7 +2870,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
             if (rc != 1 && !scratch_refused(rc)) return rc;
         }
         pl.pad = s->IC % 32 != 0 && env_tile_mode() != 1 && (!small || opt(OPT_HALO_PAD) == 2) &&
-                 pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x, strided && s->IC % 8 != 0);
+                 pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x, forward_idle(s), strided && s->IC % 8 != 0);
         rc = strided ? launch_halo_lattice(c, pl, mode3x, stream) : launch_halo(c, pl, mode3x, stream);
         if (rc != 1 && !((pl.pad || strided) && scratch_refused(rc))) return rc;
         return launch_igemm(c, pl, mode3x, stream);
@@ -2884,7 +2885,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         if (rc != 1 && !scratch_refused(rc)) return rc;
     }
     if (algo != ALPHA_ALGO_SIMT && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
-        !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x(), s->sh != 1 || s->sw != 1)) {
+        !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x(), forward_idle(s), s->sh != 1 || s->sw != 1)) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N; pl.aH = s->IH; pl.aW = s->IW; pl.aC = s->IC;
         pl.FH = s->FH; pl.FW = s->FW; pl.sh = s->sh; pl.sw = s->sw; pl.pad_h = s->ph; pl.pad_w = s->pw;
@@ -2894,7 +2895,9 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         const bool strided = s->sh != 1 || s->sw != 1;
         pl.force = !strided;   // the patch matrix would run tiles as empty
         if (patch_path_ok(s) && opt(OPT_HALO_PAD) == 1) pl.min_ksplit = patch_ksplit(s, cur_mode3x(), sm_budget(c));
-        rc = strided ? launch_halo_lattice(c, pl, cur_mode3x(), stream) : launch_halo(c, pl, cur_mode3x(), stream);
+        rc = 1;
+        if (pl.min_ksplit <= chunks32(s->IC) * s->sh * s->sw)   // (a part is at least one chunk of one phase)
+            rc = strided ? launch_halo_lattice(c, pl, cur_mode3x(), stream) : launch_halo(c, pl, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
         // Not the im2col kernel where there is a patch matrix: it adds hi*hi and both correction terms into one accumulator, whose
         // truncation costs three times the error of the wide form (996 x 6148 times 6148 x 76: 4e-5 against 1e-5).
@@ -2969,7 +2972,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
             }
             if (!mode3x) pt.W_lo = nullptr;
             pt.pad = s->OC % 32 != 0;
-            if ((tiny_image(s->IH, s->IW) || (pt.pad && !pad_beats_patch(s->OC, taps, s->IC, mode3x))) && (s->FH > 1 || s->FW > 1) &&
+            if ((tiny_image(s->IH, s->IW) || (pt.pad && !pad_beats_patch(s->OC, taps, s->IC, mode3x, taps == 1 ? 1.0 : tile_idle(s->IH, s->IW, s->FH, s->FW)))) && (s->FH > 1 || s->FW > 1) &&
                 (long long)taps * s->OC <= 16384 && (!pt.pad || opt(OPT_PATCH_MATRIX))) {
                 rc = launch_patch_gemm(c, pt, mode3x, stream);
                 if (rc != 1 && !(pt.pad && scratch_refused(rc))) return rc;

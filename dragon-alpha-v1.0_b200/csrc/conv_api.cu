@@ -2875,8 +2875,10 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         if (rc != 1 && !((pl.pad || strided) && scratch_refused(rc))) return rc;
         return launch_igemm(c, pl, mode3x, stream);
     }
+    // What has no patch product either (more than 16384 reduction elements) is computed in fp32 and stays so: conv_fwd_simt below.
+    const bool odd_ok = algo != ALPHA_ALGO_SIMT && patch_path_ok(s);
     const WindowPlan win = forward_windows(s);
-    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && !(tiny_image(s->OH, s->OW) && patch_path_ok(s)) && window_beats_rest(s, win, cur_mode3x(), sm_budget(c))) {
+    if (odd_ok && !tensor_ok && !tiny_image(s->OH, s->OW) && window_beats_rest(s, win, cur_mode3x(), sm_budget(c))) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N;
         pl.out = Y; pl.oH = s->OH; pl.oW = s->OW; pl.ncols = s->OC;
@@ -2884,7 +2886,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         rc = launch_window_forward(c, s, pl, win, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
     }
-    if (algo != ALPHA_ALGO_SIMT && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
+    if (odd_ok && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
         !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x(), forward_idle(s), s->sh != 1 || s->sw != 1)) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N; pl.aH = s->IH; pl.aW = s->IW; pl.aC = s->IC;
@@ -2894,16 +2896,15 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         pl.b_mn = false; pl.flip = false; pl.kdim = s->IC; pl.pad = true;
         const bool strided = s->sh != 1 || s->sw != 1;
         pl.force = !strided;   // the patch matrix would run tiles as empty
-        if (patch_path_ok(s) && opt(OPT_HALO_PAD) == 1) pl.min_ksplit = patch_ksplit(s, cur_mode3x(), sm_budget(c));
+        if (opt(OPT_HALO_PAD) == 1) pl.min_ksplit = patch_ksplit(s, cur_mode3x(), sm_budget(c));
         rc = 1;
         if (pl.min_ksplit <= chunks32(s->IC) * s->sh * s->sw)   // (a part is at least one chunk of one phase)
             rc = strided ? launch_halo_lattice(c, pl, cur_mode3x(), stream) : launch_halo(c, pl, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
-        // Not the im2col kernel where there is a patch matrix: it adds hi*hi and both correction terms into one accumulator, whose
+        // Then the patch matrix, not the im2col kernel: that adds hi*hi and both correction terms into one accumulator, whose
         // truncation costs three times the error of the wide form (996 x 6148 times 6148 x 76: 4e-5 against 1e-5).
-        if (!patch_path_ok(s)) return launch_igemm(c, pl, cur_mode3x(), stream);
     }
-    if (algo != ALPHA_ALGO_SIMT && patch_path_ok(s)) {
+    if (odd_ok) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N; pl.aH = s->IH; pl.aW = s->IW; pl.aC = s->IC;
         pl.FH = s->FH; pl.FW = s->FW; pl.sh = s->sh; pl.sw = s->sw; pl.pad_h = s->ph; pl.pad_w = s->pw;
@@ -3009,7 +3010,8 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     const bool tensor_ok = (s->IC % 32 == 0) && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256;
     if (algo == ALPHA_ALGO_TENSOR && !tensor_ok)
         return fail(ALPHA_E_ARG, "tensor deltaW path needs IC %% 32 == 0 (IC=%d)", s->IC);
-    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
+    // (more than 16384 reduction elements of an odd channel count are fp32 work: conv_dw_simt below)
+    if (algo != ALPHA_ALGO_SIMT && !tensor_ok && patch_path_ok(s) && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
         const WindowPlan win = window_plan(s, s->sh);
         const DwRoute route = pick_dw_route(s, win, cur_mode3x(), sm_budget(c));
         bool spills = false;

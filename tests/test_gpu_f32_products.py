@@ -103,3 +103,37 @@ def test_infinite_weight_reaches_only_the_pixels_of_its_tap(pkg, shape, algo):
         want = torch.ones((N, IH, IW, IC), dtype=torch.bool, device="cuda")
         want[..., ic] = ~meets
         assert torch.equal(torch.isfinite(dX), want), (oc, fh, fw, ic)
+
+
+# N, IH, IW, IC, OC, F, s, p: FH * FW * IC just above 16384 with a channel count that is no multiple of 8 (forward, deltaW) or 32 (deltaW)
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+@pytest.mark.parametrize("shape", [(2, 9, 8, 660, 12, 5, 1, 2), (1, 15, 15, 404, 20, 7, 2, 3), (1, 5, 5, 16420, 8, 1, 1, 0)], ids=str)
+def test_long_odd_reductions_stay_in_fp32(pkg, shape, mode):
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+    N, IH, IW, IC, OC, F, s, p = shape
+    OH, OW = out_hw(IH, IW, F, F, s, s, p, p)
+    g = torch.Generator(device="cuda").manual_seed(IC)
+    X, W = torch.randn((N, IH, IW, IC), device="cuda", generator=g), torch.randn((OC, F, F, IC), device="cuda", generator=g)
+    dY = torch.randn((N, OH, OW, OC), device="cuda", generator=g)
+    Y = eng.conv3D(X, W, s, s, p, p).double()
+    assert lib.last_algo() == "simt"
+    dW = eng.dconv3D_deltaW(X, dY, F, F, s, s, p, p).double()
+    assert lib.last_algo() == "simt"
+    conv = lambda x, w: torch.nn.functional.conv2d(x.permute(0, 3, 1, 2), w.permute(0, 3, 1, 2), stride=s, padding=p).permute(0, 2, 3, 1)
+    assert bool(((Y - conv(X.double(), W.double())).abs() <= F * F * IC * 2.0 ** -24 * conv(X.double().abs(), W.double().abs())).all())
+    grad = lambda x, y: torch.nn.grad.conv2d_weight(x.permute(0, 3, 1, 2), (OC, IC, F, F), y.permute(0, 3, 1, 2), stride=s, padding=p).permute(0, 2, 3, 1)
+    assert bool(((dW - grad(X.double(), dY.double())).abs() <= N * OH * OW * 2.0 ** -24 * grad(X.double().abs(), dY.double().abs()) + 1e-30).all())
+
+
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+def test_long_odd_matrix_product_stays_in_fp32(pkg, mode):
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A, B = torch.randn((40, 20004), device="cuda", generator=g), torch.randn((24, 20004), device="cuda", generator=g)
+    C = eng.matMulT2(A, B).double()
+    assert lib.last_algo() == "simt"
+    assert bool(((C - A.double() @ B.double().T).abs() <= 20004 * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T)).all())

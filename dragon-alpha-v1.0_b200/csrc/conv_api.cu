@@ -1867,12 +1867,13 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
         if (ks > 1 && get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws) == ALPHA_OK) { g.ksplit = (int)ks; g.out = ws; }
     }
     const long long nz = phases * g.ksplit;
-    for (long long z0 = 0; z0 < nz; z0 += 65535) {
-        g.z0 = (int)z0;
-        const unsigned z = (unsigned)(nz - z0 < 65535 ? nz - z0 : 65535);
-        if (!t_dry) launch_gemm_f32(g, t, dim3((unsigned)gx, (unsigned)gy, z), stream);
-        note_launch("simt");
-    }
+    auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
+    for (long long z0 = 0; z0 < nz; z0 += 65535)
+        for (long long y0 = 0; y0 < gy; y0 += 65535) {
+            g.y0 = (int)y0; g.z0 = (int)z0;
+            if (!t_dry) launch_gemm_f32(g, t, dim3((unsigned)gx, slice(y0, gy), slice(z0, nz)), stream);
+            note_launch("simt");
+        }
     int rc = check_launch("gemm_f32_kernel");
     if (rc || g.ksplit == 1) return rc;
     const size_t n4 = g.size / 4;

@@ -181,7 +181,7 @@ struct DxGemm {
     const float* dY; const float* W; float* out;
     int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw;
     int nsw;                       // phases along a row: min(sw, IW)
-    int ksplit, kt, z0;            // kt = 16-step tiles per tap; z0 = phase * ksplit + part of blockIdx.z == 0
+    int ksplit, kt, y0, z0;        // kt = 16-step tiles per tap; y0 = column tile of blockIdx.y == 0, z0 = phase * ksplit + part of blockIdx.z == 0
     size_t size;                   // elements of deltaX
     FastDiv by_kt;
     struct Cta { int m0, n0, rows, it0, it1, A, B, py, px, ry, rx, qy, qx, Ux; float* out; };
@@ -195,7 +195,7 @@ struct DxGemm {
         c.py = phase / nsw; c.px = phase - c.py * nsw;
         c.A = (IH - c.py + sh - 1) / sh; c.B = (IW - c.px + sw - 1) / sw;
         c.rows = N * c.A * c.B;
-        c.m0 = static_cast<int>(blockIdx.x) * BM; c.n0 = static_cast<int>(blockIdx.y) * BN;
+        c.m0 = static_cast<int>(blockIdx.x) * BM; c.n0 = (y0 + static_cast<int>(blockIdx.y)) * BN;
         if (c.m0 >= c.rows) return false;
         c.ry = (c.py + ph) % sh; c.rx = (c.px + pw) % sw;
         c.qy = (c.py + ph - c.ry) / sh; c.qx = (c.px + pw - c.rx) / sw;

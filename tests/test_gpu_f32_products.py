@@ -137,3 +137,14 @@ def test_long_odd_matrix_product_stays_in_fp32(pkg, mode):
     C = eng.matMulT2(A, B).double()
     assert lib.last_algo() == "simt"
     assert bool(((C - A.double() @ B.double().T).abs() <= 20004 * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T)).all())
+
+
+def test_more_columns_than_a_grid_dimension(pkg):
+    """67188 column tiles of 64: more than gridDim.y holds."""
+    import torch
+    eng, lib = pkg.submodule("engine").Engine(), pkg.submodule("lib")
+    g = torch.Generator(device="cuda").manual_seed(2)
+    A, B = torch.randn((4, 4), device="cuda", generator=g), torch.randn((4, 4300000), device="cuda", generator=g)
+    C = eng.matMul(A, B)
+    assert lib.last_algo() == "simt"
+    assert bool(((C.double() - A.double() @ B.double()).abs() <= 4 * 2.0 ** -24 * (A.double().abs() @ B.double().abs())).all())

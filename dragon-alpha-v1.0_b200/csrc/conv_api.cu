@@ -256,6 +256,7 @@ static inline int sm_budget(const DeviceCtx* c)
 static thread_local size_t t_dry_cur = 0, t_dry_peak = 0;
 struct CallerScratch { char* ptr = nullptr; size_t bytes = 0, used = 0; };
 static thread_local CallerScratch t_caller;
+static thread_local bool t_no_memory = false;   // cudaMalloc refused this call's scratch (see scratch_refused)
 
 void set_caller_scratch(void* ptr, size_t bytes)
 {
@@ -289,6 +290,7 @@ static bool stream_is_capturing(cudaStream_t stream)
 // Starts one API call on `stream`: its scratch requests are carved from the start of the block again.
 static void ws_begin(DeviceCtx* c, cudaStream_t stream)
 {
+    t_no_memory = false;
     if (t_dry) { t_dry_cur = t_dry_peak = 0; return; }
     std::lock_guard<std::mutex> lock(g_mu);
     auto it = c->workspace.find(stream);
@@ -312,7 +314,7 @@ static int grow_block(DeviceCtx* c, cudaStream_t stream, DeviceCtx::Block& b, si
     const size_t want = need + (need >> 2);
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess) { cudaGetLastError(); return fail(ALPHA_E_CUDA, "cudaMalloc(workspace %zu B): %s", want, cudaGetErrorString(e)); }
+    if (e != cudaSuccess) { cudaGetLastError(); t_no_memory = true; return fail(ALPHA_E_CUDA, "cudaMalloc(workspace %zu B): %s", want, cudaGetErrorString(e)); }
     if (b.base) {
         c->retired.push_back(DeviceCtx::Retired{b.base, b.bytes, nullptr, b.captured, stream});
     }
@@ -440,7 +442,7 @@ static int weight_planes(DeviceCtx* c, cudaStream_t stream, const DeviceCtx::Wei
         if (e.ptr) c->retired.push_back(DeviceCtx::Retired{e.ptr, e.bytes, nullptr, false, e.stream});
         void* p = nullptr;
         cudaError_t err = cudaMalloc(&p, bytes);
-        if (err != cudaSuccess) { cudaGetLastError(); e = DeviceCtx::WeightEntry{}; return fail(ALPHA_E_CUDA, "cudaMalloc(weight cache %zu B): %s", bytes, cudaGetErrorString(err)); }
+        if (err != cudaSuccess) { cudaGetLastError(); t_no_memory = true; e = DeviceCtx::WeightEntry{}; return fail(ALPHA_E_CUDA, "cudaMalloc(weight cache %zu B): %s", bytes, cudaGetErrorString(err)); }
         e.ptr = static_cast<float*>(p); e.bytes = bytes;
     }
     e.valid = false; e.stream = stream;
@@ -672,9 +674,14 @@ static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, double idle,
 // SMs is the more exact one.  Into how many parts would a layer's product over the patch matrix be cut?  (Zero-filled channels are
 // left to it where theirs would be fewer: 64 x 14 x 14, 148 -> 64 channels 3x3: 1.0e-6 in three parts, 3.1e-6 in one.)
 static int patch_ksplit(const AlphaConvShape* s, int mode3x, int sms);
-// A route that needs scratch may not take away what a route without any could do: under stream capture, or in a
-// caller-owned workspace, the call then goes on to the older route.
-static inline bool scratch_refused(int rc) { return rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH; }
+// A route that needs scratch may not take away what a route without any could do: under stream capture, in a caller-owned
+// workspace or on a full card the call then goes on to the older route.
+static inline bool scratch_refused(int rc)
+{
+    const bool no_memory = t_no_memory;
+    t_no_memory = false;
+    return rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH || (rc == ALPHA_E_CUDA && no_memory);
+}
 
 // Clocks of the busiest SM of conv_igemm_kernel (32-channel tiles), measured: a step of 8 channels takes 1.6 times the time
 // its bytes need at 128 B/clk of shared memory - both operands written by the TMA and read by each MMA, and in 3xTF32 read
@@ -1864,7 +1871,9 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
         if (ks > its / 4) ks = its / 4;
         if (ks > 16) ks = 16;
         float* ws = nullptr;
-        if (ks > 1 && get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws) == ALPHA_OK) { g.ksplit = (int)ks; g.out = ws; }
+        const int rc = ks > 1 ? get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws) : ALPHA_OK;
+        if (rc && !scratch_refused(rc)) return rc;
+        if (ks > 1 && !rc) { g.ksplit = (int)ks; g.out = ws; }
     }
     const long long nz = phases * g.ksplit;
     auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
@@ -2948,7 +2957,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
         pl.W = W; pl.wOC = s->OC; pl.wIC = s->IC; pl.bias = nullptr;
         pl.b_mn = true; pl.flip = true; pl.kdim = s->OC;
         const int mode3x = cur_mode3x();
-        if (env_tile_mode() != 1 && (s->OC % 32 == 0 || opt(OPT_HALO_PAD)) && taps_fit64(s) && opt(OPT_DX_TRANSPOSE)) {
+        if (env_tile_mode() != 1 && (s->OC % 32 == 0 || (opt(OPT_HALO_PAD) && s->OC <= 65535 * 32)) && taps_fit64(s) && opt(OPT_DX_TRANSPOSE)) {   // (gridDim.y of the transpose)
             // deltaX as a forward conv over deltaY with Wt[ic][rotated tap][oc], built once per call
             const int taps = s->FH * s->FW;
             const size_t nW = (size_t)s->OC * taps * s->IC;

@@ -265,3 +265,48 @@ def test_prepared_weights_in_caller_memory(pkg):
         finally:
             L.set_math_mode("3xtf32")
     assert L.device_status() == 0
+
+
+def test_odd_deltaX_runs_in_place_where_the_card_is_full(pkg):
+    """Transposing W for a product over K % 32 != 0 needs twice W of scratch; where cudaMalloc refuses it, W is read in place."""
+    import torch
+    dev = torch.device("cuda:0")
+    L, E = pkg.submodule("lib"), pkg.submodule("engine")
+    eng = E.Engine(E.CudaFloat32EngineBase(math="3xtf32"))
+    M = 2000000
+    g = torch.Generator(device=dev).manual_seed(3)
+    A, B = torch.randn((64, 40), device=dev, generator=g), torch.randn((40, M), device=dev, generator=g)
+    torch.cuda.synchronize()
+    L.load().alpha_conv_release_workspace()
+    first = torch.empty((64, M), device=dev)      # memory the product's result will get
+    del first
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - (200 << 20), dtype=torch.uint8, device=dev)
+    try:
+        with torch.cuda.stream(torch.cuda.Stream()):
+            C = eng.matMul(A, B)
+            algo = L.last_algo()
+        torch.cuda.synchronize()
+        pick = torch.randint(0, M, (500,), device=dev, generator=g)
+        ref = A.double() @ B[:, pick].double()
+        assert float((C[:, pick].double() - ref).abs().max() / ref.abs().max()) <= 1e-4
+        assert algo == "igemm", algo
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert L.device_status() == 0
+
+
+def test_odd_deltaX_over_more_rows_than_a_grid_dimension(pkg):
+    """K = 2100008 rows of W are 65626 transpose tiles, more than gridDim.y holds: W is read in place."""
+    import torch
+    dev = torch.device("cuda:0")
+    L, E = pkg.submodule("lib"), pkg.submodule("engine")
+    eng = E.Engine(E.CudaFloat32EngineBase(math="3xtf32"))
+    K = 2100008
+    g = torch.Generator(device=dev).manual_seed(4)
+    A, B = torch.randn((4, K), device=dev, generator=g), torch.randn((K, 4), device=dev, generator=g)
+    C = eng.matMul(A, B).double()
+    # one accumulator takes 3 K / 8 truncating additions
+    assert bool(((C - A.double() @ B.double()).abs() <= 3 * K / 8 * 2.0 ** -23 * (A.double().abs() @ B.double().abs())).all())
+    assert L.device_status() == 0

@@ -384,7 +384,7 @@ static int check_launch(const char* what);
 // (alpha_conv_weight_cache) a transform is computed once and kept in library-owned memory until
 // alpha_conv_weights_updated() names its source tensor; with the cache off it is recomputed by
 // every call into that call's scratch.
-enum { WK_FWD_LO = 1, WK_DX_S1 = 2, WK_DX_PHASES = 3, WK_DX_COL2IM = 4, WK_FWD_WINDOW = 5 };
+enum { WK_FWD_LO = 1, WK_DX_S1 = 2, WK_DX_PHASES = 3, WK_DX_COL2IM = 4 };
 static std::atomic<int> g_weight_cache{0};
 
 // A forward native that was handed the caller's CW block finds the lo plane kernel_remode left there.
@@ -1613,21 +1613,18 @@ static int launch_window_forward(DeviceCtx* c, const AlphaConvShape* s, const Ig
     IgemmPlan pl = pl_in;
     pl.wIC = w.K;   // one window row of W as it lies: [OC][FH][FW * IC]
     if (w.g > 1) {
+        // W in the order of the windows, in the call's own scratch: whether a layer runs windows depends on its batch, and a transform
+        // that is kept (prepared weights, weight cache) has to serve every batch
         const size_t nW = (size_t)s->OC * w.U * w.K;
         float* Ww = nullptr;
-        bool fresh = true;
-        const DeviceCtx::WeightKey wkey{pl_in.W, WK_FWD_WINDOW, s->OC, s->IC, s->FH * 256 + s->FW, s->sh, mode3x};
-        int rc = weight_planes(c, stream, wkey, (mode3x ? 2 : 1) * nW * sizeof(float), &Ww, &fresh);
+        int rc = get_workspace(c, stream, (mode3x ? 2 : 1) * nW * sizeof(float), &Ww);
         if (rc) return rc;
-        if (fresh) {
-            size_t blocks = (nW + 255) / 256;
-            if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-            if (transforms_run()) launch_after(window_weights_kernel, (unsigned)blocks, 256, 0, stream, pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
-            note_launch("window_w");
-            rc = check_launch("window_weights_kernel");
-            if (rc) return rc;
-            weight_planes_ready(c, stream, wkey);
-        }
+        size_t blocks = (nW + 255) / 256;
+        if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
+        if (!t_dry) launch_after(window_weights_kernel, (unsigned)blocks, 256, 0, stream, pl_in.W, Ww, mode3x ? Ww + nW : nullptr, s->OC, s->FH, s->FW, s->IC, s->sh, w.U);
+        note_launch("window_w");
+        rc = check_launch("window_weights_kernel");
+        if (rc) return rc;
         pl.W = Ww; pl.W_lo = mode3x ? Ww + nW : nullptr;
     } else if (mode3x) {
         // before the pack, whose end the convolution waits for (after it, a launch between the two: 64 x 3 -> 64 channels 3x3 78 -> 97 us)

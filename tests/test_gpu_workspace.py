@@ -310,3 +310,36 @@ def test_odd_deltaX_over_more_rows_than_a_grid_dimension(pkg):
     # one accumulator takes 3 K / 8 truncating additions
     assert bool(((C - A.double() @ B.double()).abs() <= 3 * K / 8 * 2.0 ** -23 * (A.double().abs() @ B.double().abs())).all())
     assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32"])
+@pytest.mark.parametrize("layer", [(32, 4, 64, 3, 1, 1), (64, 4, 64, 7, 2, 3), (64, 4, 64, 4, 2, 1), (32, 16, 128, 3, 1, 1), (33, 12, 64, 3, 2, 1)], ids=str)
+def test_weights_prepared_at_one_batch_serve_another(pkg, layer, mode):
+    """Routes of few channels depend on the batch (windows or not); a block prepared for the large one serves the last, smaller one."""
+    import torch
+    L = pkg.submodule("lib")
+    base = pkg.submodule("engine").CudaFloat32EngineBase()
+    L.set_math_mode(mode)
+    try:
+        IH, IC, OC, F, s, p = layer
+        OH = (IH + 2 * p - F) // s + 1
+        g = torch.Generator(device="cuda").manual_seed(IC)
+        W = torch.randn((OC, F, F, IC), device="cuda", generator=g) * 0.1
+        geo = lambda n: (F, F, n, IH, IH, OH, OH, IC, OC, s, s, p, p)
+        blocks = {n: base.prepare_weights("forward", W, *geo(n)) for n in (128, 64, 6)}
+        assert mode == "3xtf32" or all(b is None for b in blocks.values())        # plain TF32 forward reads W as it is
+        plans = set()
+        for n in (128, 6, 64):
+            X = torch.randn((n, IH, IH, IC), device="cuda", generator=g)
+            want, got = torch.empty((n, OH, OH, OC), device="cuda"), torch.empty((n, OH, OH, OC), device="cuda")
+            args = (OH, OH, X, IH, IH, W, F, F, n, IC, OC, s, s, p, p)
+            base.conv3D(want, *args)
+            plans.add(L.last_plan())
+            for b in blocks.values():
+                base.conv3D_prepared(got, *args, b)
+                # (two issuing threads in plain TF32: the last bits depend on timing)
+                assert torch.equal(got, want) if mode == "3xtf32" else float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+        assert len(plans) > 1
+    finally:
+        L.set_math_mode("3xtf32")
+    assert L.device_status() == 0

@@ -257,6 +257,7 @@ static thread_local size_t t_dry_cur = 0, t_dry_peak = 0;
 struct CallerScratch { char* ptr = nullptr; size_t bytes = 0, used = 0; };
 static thread_local CallerScratch t_caller;
 static thread_local bool t_no_memory = false;   // cudaMalloc refused this call's scratch (see scratch_refused)
+static thread_local bool t_bad_block = false;   // the caller's prepared block does not fit this call: no reason to take another route
 
 void set_caller_scratch(void* ptr, size_t bytes)
 {
@@ -290,7 +291,7 @@ static bool stream_is_capturing(cudaStream_t stream)
 // Starts one API call on `stream`: its scratch requests are carved from the start of the block again.
 static void ws_begin(DeviceCtx* c, cudaStream_t stream)
 {
-    t_no_memory = false;
+    t_no_memory = t_bad_block = false;
     if (t_dry) { t_dry_cur = t_dry_peak = 0; return; }
     std::lock_guard<std::mutex> lock(g_mu);
     auto it = c->workspace.find(stream);
@@ -407,9 +408,11 @@ static int weight_planes(DeviceCtx* c, cudaStream_t stream, const DeviceCtx::Wei
     if (t_prep.mode && t_prep.W == key.W) {
         t_prep.need = bytes; t_prep.seen = true;
         if (t_prep.mode == 3) { *out = reinterpret_cast<float*>(static_cast<uintptr_t>(1) << 30); return ALPHA_OK; }
-        if (bytes > t_prep.bytes)
+        if (bytes > t_prep.bytes) {
+            t_bad_block = true;
             return fail(ALPHA_E_NOSCRATCH, "the prepared-weights block holds %zu bytes, this layer's transform needs %zu "
                         "(alpha_conv_prepared_weights_bytes tells in advance)", t_prep.bytes, bytes);
+        }
         std::lock_guard<std::mutex> lock(g_mu);
         if (t_prep.mode == 1) {
             c->prepared[t_prep.ptr] = DeviceCtx::PreparedDesc{key, bytes};
@@ -675,12 +678,12 @@ static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, double idle,
 // left to it where theirs would be fewer: 64 x 14 x 14, 148 -> 64 channels 3x3: 1.0e-6 in three parts, 3.1e-6 in one.)
 static int patch_ksplit(const AlphaConvShape* s, int mode3x, int sms);
 // A route that needs scratch may not take away what a route without any could do: under stream capture, in a caller-owned
-// workspace or on a full card the call then goes on to the older route.
+// workspace or on a full card the call then goes on to the older route, with the scratch it had at its start (ws_rewind).
 static inline bool scratch_refused(int rc)
 {
     const bool no_memory = t_no_memory;
     t_no_memory = false;
-    return rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH || (rc == ALPHA_E_CUDA && no_memory);
+    return !t_bad_block && (rc == ALPHA_E_CAPTURE || rc == ALPHA_E_NOSCRATCH || (rc == ALPHA_E_CUDA && no_memory));
 }
 
 // Clocks of the busiest SM of conv_igemm_kernel (32-channel tiles), measured: a step of 8 channels takes 1.6 times the time
@@ -2872,9 +2875,11 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         const bool strided = s->sh != 1 || s->sw != 1;
         // A layer of few tiles and steps is launch latency: the im2col kernel splits W itself and is one launch (3xTF32)
         const bool small = mode3x && s->IC % 32 != 0 && igemm_cost(pl, mode3x, sm_budget(c)) < 20000.0;
+        const WsMark start = ws_mark(c, stream);
         if (window_beats_rest(s, win, mode3x, sm_budget(c))) {
             rc = launch_window_forward(c, s, pl, win, mode3x, stream);
             if (rc != 1 && !scratch_refused(rc)) return rc;
+            ws_rewind(c, stream, start);
         }
         pl.pad = s->IC % 32 != 0 && env_tile_mode() != 1 && (!small || opt(OPT_HALO_PAD) == 2) &&
                  pad_beats_patch(s->IC, s->FH * s->FW, s->OC, mode3x, forward_idle(s), strided && s->IC % 8 != 0);
@@ -2885,6 +2890,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
     // What has no patch product either (more than 16384 reduction elements) is computed in fp32 and stays so: conv_fwd_simt below.
     const bool odd_ok = algo != ALPHA_ALGO_SIMT && patch_path_ok(s);
     const WindowPlan win = forward_windows(s);
+    const WsMark start = ws_mark(c, stream);
     if (odd_ok && !tensor_ok && !tiny_image(s->OH, s->OW) && window_beats_rest(s, win, cur_mode3x(), sm_budget(c))) {
         IgemmPlan pl{};
         pl.act = X; pl.aN = s->N;
@@ -2892,6 +2898,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         pl.W = W; pl.wOC = s->OC; pl.bias = bias; pl.act_on = act_on; pl.act_k = act_k;
         rc = launch_window_forward(c, s, pl, win, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
+        ws_rewind(c, stream, start);
     }
     if (odd_ok && s->IC % 32 != 0 && env_tile_mode() != 1 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256 &&
         !(tiny_image(s->OH, s->OW) && (s->FH > 1 || s->FW > 1)) && pad_beats_patch(s->IC, s->FH * s->FW, s->OC, cur_mode3x(), forward_idle(s), s->sh != 1 || s->sw != 1)) {
@@ -2908,6 +2915,7 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         if (pl.min_ksplit <= chunks32(s->IC) * s->sh * s->sw)   // (a part is at least one chunk of one phase)
             rc = strided ? launch_halo_lattice(c, pl, cur_mode3x(), stream) : launch_halo(c, pl, cur_mode3x(), stream);
         if (rc != 1 && !scratch_refused(rc)) return rc;
+        ws_rewind(c, stream, start);
         // Then the patch matrix, not the im2col kernel: that adds hi*hi and both correction terms into one accumulator, whose
         // truncation costs three times the error of the wide form (996 x 6148 times 6148 x 76: 4e-5 against 1e-5).
     }
@@ -2982,8 +2990,10 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
             pt.pad = s->OC % 32 != 0;
             if ((tiny_image(s->IH, s->IW) || (pt.pad && !pad_beats_patch(s->OC, taps, s->IC, mode3x, taps == 1 ? 1.0 : tile_idle(s->IH, s->IW, s->FH, s->FW)))) && (s->FH > 1 || s->FW > 1) &&
                 (long long)taps * s->OC <= 16384 && (!pt.pad || opt(OPT_PATCH_MATRIX))) {
+                const WsMark start = ws_mark(c, stream);   // (the transposed weights before it stay)
                 rc = launch_patch_gemm(c, pt, mode3x, stream);
                 if (rc != 1 && !(pt.pad && scratch_refused(rc))) return rc;
+                if (pt.pad) ws_rewind(c, stream, start);
             }
             rc = launch_halo(c, pt, mode3x, stream);
             if (rc != 1 && !(pt.pad && scratch_refused(rc))) return rc;
@@ -3021,6 +3031,7 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     if (algo != ALPHA_ALGO_SIMT && !tensor_ok && patch_path_ok(s) && s->ph < 128 && s->pw < 128 && env_tile_mode() != 1) {
         const WindowPlan win = window_plan(s, s->sh);
         const DwRoute route = pick_dw_route(s, win, cur_mode3x(), sm_budget(c));
+        const WsMark start = ws_mark(c, stream);
         bool spills = false;
         rc = 1;
         const AlphaConvShape former = patch_product(s);
@@ -3028,6 +3039,7 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
         else if (route == DwRoute::Window) rc = launch_dw_window(c, s, win, X, deltaY, deltaW, cur_mode3x(), stream, &spills);
         if (!rc && spills) rc = launch_dw_repair(s, X, deltaY, deltaW, stream, route == DwRoute::Window ? "dw_window" : "dw_halo");
         if (rc != 1 && !scratch_refused(rc)) return rc;
+        ws_rewind(c, stream, start);
     }
     if (algo != ALPHA_ALGO_SIMT && patch_path_ok(s) && env_tile_mode() != 1 &&
         (!tensor_ok || (s->OH * s->OW <= 9 && (s->FH > 1 || s->FW > 1)))) {

@@ -343,3 +343,119 @@ def test_weights_prepared_at_one_batch_serve_another(pkg, layer, mode):
     finally:
         L.set_math_mode("3xtf32")
     assert L.device_status() == 0
+
+
+# layers whose default route needs scratch that an older route does without, or needs less of: windows, zero-filled chunks,
+# lattice phases, transposed odd weights, deltaW straight and over windows
+FALLBACKS = {"windows_ic16": ((128, 32, 32, 16, 128, 3, 3, 1, 1, 1, 1), "forward"), "windows_s2": ((64, 64, 64, 8, 64, 7, 7, 2, 2, 3, 3), "forward"),
+             "lattice": ((64, 28, 28, 128, 64, 3, 3, 2, 2, 1, 1), "forward"), "chunks_ic40": ((32, 28, 28, 40, 64, 3, 3, 1, 1, 1, 1), "forward"),
+             "deltaX_oc40": ((16, 28, 28, 64, 40, 3, 3, 1, 1, 1, 1), "deltaX"), "deltaX_f32": ((8, 1, 1, 52, 2764, 1, 1, 1, 1, 0, 0), "deltaX")}
+
+
+def _one(L, lib, case, op, X, W, dY, out, stream, prepared=None):
+    N, IH, IW, IC, OC, FH, FW, sh, sw, ph, pw = case
+    s = L.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, (IH + 2 * ph - FH) // sh + 1, (IW + 2 * pw - FW) // sw + 1, sh, sw, ph, pw)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    b = (p(prepared), prepared.numel()) if prepared is not None else (None, 0)
+    if op == "forward":
+        return lib.alpha_conv3d_forward_prepared(C.byref(s), p(X), p(W), *b, None, p(out), C.c_void_p(stream))
+    return lib.alpha_conv3d_deltaX_prepared(C.byref(s), p(dY), p(W), *b, p(out), C.c_void_p(stream))
+
+
+@pytest.mark.parametrize("prepared", [False, True])
+@pytest.mark.parametrize("name", list(FALLBACKS))
+def test_refused_scratch_falls_back_to_a_route_without(pkg, name, prepared):
+    """Under a capture that may not allocate and in caller blocks of every size, with and without prepared weights, these calls run."""
+    import torch
+    dev = torch.device("cuda:0")
+    L = pkg.submodule("lib")
+    lib = L.load()
+    L.set_math_mode("3xtf32")
+    case, op = FALLBACKS[name]
+    X, W, dY, (OH, OW) = _tensors(case, dev)
+    N, IH, IW, IC, OC, FH, FW, sh, sw, ph, pw = case
+    s = L.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+    ref = torch.empty((N, OH, OW, OC), device=dev) if op == "forward" else torch.empty_like(X)
+    L.check(_one(L, lib, case, op, X, W, dY, ref, torch.cuda.current_stream().cuda_stream))
+    block = pkg.submodule("engine").CudaFloat32EngineBase().prepare_weights(op, W, FH, FW, N, IH, IW, OH, OW, IC, OC, sh, sw, ph, pw) if prepared else None
+    torch.cuda.synchronize()
+    got = torch.zeros_like(ref)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()      # a fresh stream: no block yet
+    with torch.cuda.graph(graph, stream=side):
+        rc = _one(L, lib, case, op, X, W, dY, got, torch.cuda.current_stream().cuda_stream, block)
+    assert rc == 0, L.last_error()
+    graph.replay()
+    torch.cuda.synchronize()
+    close = lambda: float((got - ref).abs().max()) <= 1e-4 * float(ref.abs().max())
+    assert close()
+    need = L.workspace_bytes(s, op)
+    ext, own = torch.cuda.Stream(), torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
+    for part in (8, 7, 5, 3, 1):
+        size = need * part // 8 // 256 * 256
+        if not size:
+            continue
+        L.set_workspace(ext.cuda_stream, own.data_ptr(), size)
+        try:
+            got.zero_()
+            torch.cuda.synchronize()
+            assert _one(L, lib, case, op, X, W, dY, got, ext.cuda_stream, block) == 0, (part, L.last_error())
+            ext.synchronize()
+            assert close(), part
+        finally:
+            L.set_workspace(ext.cuda_stream, 0, 0)
+    assert L.device_status() == 0
+
+
+def test_a_prepared_block_that_is_too_small_is_an_error(pkg):
+    """Not a reason to take a route that ignores the block."""
+    import torch
+    dev = torch.device("cuda:0")
+    L = pkg.submodule("lib")
+    lib = L.load()
+    L.set_math_mode("3xtf32")
+    for name in ("windows_s2", "lattice", "deltaX_oc40"):
+        case, op = FALLBACKS[name]
+        X, W, dY, (OH, OW) = _tensors(case, dev)
+        N, IH, IW, IC, OC, FH, FW, sh, sw, ph, pw = case
+        block = pkg.submodule("engine").CudaFloat32EngineBase().prepare_weights(op, W, FH, FW, N, IH, IW, OH, OW, IC, OC, sh, sw, ph, pw)
+        out = torch.empty((N, OH, OW, OC), device=dev) if op == "forward" else torch.empty_like(X)
+        assert _one(L, lib, case, op, X, W, dY, out, torch.cuda.current_stream().cuda_stream, block[:256]) == -5, name
+        assert "prepared-weights block" in L.last_error()
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("case", [(50, 35, 29, 36, 100, 3, 3, 1, 1, 1, 1), (128, 32, 32, 4, 64, 7, 7, 2, 2, 3, 3)], ids=str)
+def test_deltaW_falls_back_with_all_of_the_callers_block(pkg, case):
+    """The patch matrix is refused a block that the abandoned route has used part of only if it does not fit the whole block."""
+    import torch
+    dev = torch.device("cuda:0")
+    L = pkg.submodule("lib")
+    lib = L.load()
+    L.set_math_mode("3xtf32")
+    X, W, dY, (OH, OW) = _tensors(case, dev)
+    N, IH, IW, IC, OC, FH, FW, sh, sw, ph, pw = case
+    s = L.AlphaConvShape(N, IH, IW, IC, OC, FH, FW, OH, OW, sh, sw, ph, pw)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    need = {}
+    for options in ({"HALO_PAD": 0, "HALO_WINDOW": 0}, {"HALO_PAD": 2, "HALO_WINDOW": 0}, {"HALO_WINDOW": 2}):
+        for k, v in options.items():
+            L.set_option(k, v)
+        need[len(need)] = L.workspace_bytes(s, "deltaW")
+        ref = torch.empty_like(W)
+        L.check(lib.alpha_conv3d_deltaW(C.byref(s), p(X), p(dY), p(ref), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        ext, own = torch.cuda.Stream(), torch.empty(max(need[0], need[len(need) - 1]), dtype=torch.uint8, device=dev)
+        torch.cuda.synchronize()
+        for size in {need[0], need[len(need) - 1]}:
+            L.set_workspace(ext.cuda_stream, own.data_ptr(), size)
+            try:
+                got = torch.zeros_like(W)
+                torch.cuda.synchronize()
+                rc = lib.alpha_conv3d_deltaW(C.byref(s), p(X), p(dY), p(got), C.c_void_p(ext.cuda_stream))
+                assert rc == 0, (options, size, need, L.last_error())
+                ext.synchronize()
+                assert float((got - ref).abs().max()) <= 1e-4 * float(ref.abs().max())
+            finally:
+                L.set_workspace(ext.cuda_stream, 0, 0)
+        for k in options:
+            L.set_option(k, 1)
+    assert L.device_status() == 0

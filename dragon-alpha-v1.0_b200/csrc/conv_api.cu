@@ -1212,6 +1212,7 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     if (tile_mode == 1) return 1;
     IgemmPlan pl = pl_in;
     if (pl.sh != 1 || pl.sw != 1 || !whole_chunks(pl)) return 1;
+    const WsMark start = ws_mark(c, stream);
     // CTA pairs: the single-CTA forms are bound by shared-memory bandwidth once an MMA covers 128 or
     // more columns (operand reads alone take 128 B/clk at N = 128), and a pair halves the W-tile part
     // of it.  Measured faster in plain TF32 where one MMA covers 256 output channels (OC % 256 == 0:
@@ -1264,13 +1265,8 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     }
     // (A skinny shape runs half-empty tiles all the same: with its reduction split over the idle SMs, or 64-column tiles on all
     // of them, they beat the CTA pairs, which would fill half of the SMs with tiles as empty - 64 x 8 x 8, 128 -> 128 channels.)
-    if (!ch.valid || (tile_mode == 0 && ch.eff < 0.6 && !pl.force && !pl.lat && !(try_pair && skinny && ch.eff >= 0.4))) {
-        if (try_pair && skinny) {
-            const int rc2 = launch_halo_pair(c, pl_in, mode3x, stream);
-            if (rc2 != 1) return rc2;
-        }
-        return 1;
-    }
+    const bool sparse = tile_mode == 0 && ch.eff < 0.6 && !pl.force && !pl.lat;
+    if (!ch.valid || (sparse && !(try_pair && skinny && ch.eff >= 0.4))) return try_pair && skinny ? launch_halo_pair(c, pl_in, mode3x, stream) : 1;
 
     HaloParams p{};
     p.out = pl.out; p.bias = pl.bias; p.act_on = pl.act_on; p.act_k = pl.act_k; p.status = c->status; p.prof = c->prof;
@@ -1394,6 +1390,10 @@ static int launch_halo(DeviceCtx* c, const IgemmPlan& pl_in, int mode3x, cudaStr
     if (ksplit > 1) {
         if ((long long)pl.aN * ksplit > 2147483647LL) return 1;
         rc = get_workspace(c, stream, (size_t)ksplit * out_floats * sizeof(float), &out_ptr);
+        if (sparse && scratch_refused(rc)) {   // the CTA pairs after all, which split nothing
+            ws_rewind(c, stream, start);
+            return launch_halo_pair(c, pl_in, mode3x, stream);
+        }
         if (rc) return rc;
         p.bias = nullptr; p.act_on = 0;
     }
@@ -2046,16 +2046,20 @@ static inline bool dw_static_taps(const AlphaConvShape* s, const DwForm& f, bool
     return s->FW == 1 || (strided ? s->FW == 3 || s->FW == 4 : f.G == 3);
 }
 
+constexpr int kDwDone = 2;   // (within launch_dw_halo: its other form has run)
+
 // Returns 1 when the shape is left to the split-K im2col kernel, 0 on launch, < 0 on error.
 // deltaB != nullptr: the kernel also sums the columns of deltaY (bias gradient); *bias_fused tells whether it did.
 // per_image: dW receives N separate results, dW[n] = the sum over the pixels of image n only (batched matrix
 // products C[n] = A[n]^T * B[n]); every CTA column of the grid then owns one image and writes its result in place.
 // x_pitch: floats between pixels, rows and images of X where it is not dense (stride 1 only).
 // former: see dw_most_steps (nullptr: the layer itself).
+// pow2: channel blocks of powers of two, in fewer parts: what a call runs whose scratch for more of them is refused.
 // *spills: whether pixel tiles reach past the output where X still has pixels (see DwRepair).
 static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float* X, const float* dY, float* dW,
                           int mode3x, cudaStream_t stream, float* deltaB = nullptr, bool* bias_fused = nullptr,
-                          bool per_image = false, const size_t* x_pitch = nullptr, const AlphaConvShape* former = nullptr, bool* spills = nullptr)
+                          bool per_image = false, const size_t* x_pitch = nullptr, const AlphaConvShape* former = nullptr, bool* spills = nullptr,
+                          bool pow2 = false)
 {
     if (bias_fused) *bias_fused = false;
     if (opt(OPT_CONV_DW) == 1 && !per_image) return 1;
@@ -2087,9 +2091,9 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     for (int k = 0; k < nph; ++k)
         if (ph_psi[k] >= s->IW) return 1;                 // a lattice without a column
     if (s->sh > s->IH) return 1;
-    DwForm form = plan_dw_form(s, strided, per_image, mode3x, opt(OPT_DW_STACKED));
+    DwForm form = plan_dw_form(s, strided, per_image, mode3x, opt(OPT_DW_STACKED), pow2);
     if (form.cost < 0) return 1;
-    const double most_steps = mode3x && !per_image && opt(OPT_DW_STACKED) < 0 ? dw_most_steps(s, strided, former, sm_budget(c), &form) : 0;
+    const double most_steps = mode3x && !per_image && !pow2 && opt(OPT_DW_STACKED) < 0 ? dw_most_steps(s, strided, former, sm_budget(c), &form) : 0;
     const int G = form.G, tgroups = (s->FW + G - 1) / G;
     int NT = form.NT;
     const bool stacked = form.stacked, diag = form.diag;
@@ -2157,8 +2161,17 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     }
     const size_t sizeW = (size_t)s->OC * s->FH * s->FW * s->IC;
     float* ws = nullptr;
+    const WsMark start = ws_mark(c, stream);
+    auto scratch = [&](size_t floats, float** out) {
+        const int rc = get_workspace(c, stream, floats * sizeof(float), out);
+        if (!rc || pow2 || former || s_in->IC % 32 != 0 || !scratch_refused(rc)) return rc;
+        ws_rewind(c, stream, start);
+        const int again = launch_dw_halo(c, s_in, X, dY, dW, mode3x, stream, deltaB, bias_fused, per_image, x_pitch, nullptr, spills, true);
+        return again == ALPHA_OK ? kDwDone : again;
+    };
     if (parts * nsub > 1 && !per_image) {
-        int rc = get_workspace(c, stream, sizeW * parts * nsub * sizeof(float), &ws);
+        int rc = scratch(sizeW * parts * nsub, &ws);
+        if (rc == kDwDone) return ALPHA_OK;
         if (rc) return rc;
         p.out = ws;
     } else {
@@ -2170,7 +2183,8 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     // sum borrows 16 KB of the operand ring.
     float* bias_parts = nullptr;
     if (deltaB && (size_t)stages * stage_bytes(R) >= 16384 && s->OC % 4 == 0) {
-        int rc = get_workspace(c, stream, (size_t)parts * s->OC * sizeof(float), &bias_parts);
+        int rc = scratch((size_t)parts * s->OC, &bias_parts);
+        if (rc == kDwDone) return ALPHA_OK;
         if (rc) return rc;
         p.bias_out = bias_parts;
     }

@@ -459,3 +459,58 @@ def test_deltaW_falls_back_with_all_of_the_callers_block(pkg, case):
         for k in options:
             L.set_option(k, 1)
     assert L.device_status() == 0
+
+
+# N, IH, IC, OC and operator: a half-empty skinny layer, which CTA pairs ran without scratch, and a deltaW whose 33 blocks of 32
+# channels filled the SMs in one part each, both in plain TF32
+@pytest.mark.parametrize("layer,op", [((32, 8, 256, 256), "forward"), ((32, 8, 256, 256), "deltaX_prepared"), ((4, 14, 1056, 128), "deltaW"),
+                                      ((4, 14, 1056, 128), "deltaW_bias")], ids=str)
+def test_layers_that_needed_no_scratch_still_run_without(pkg, layer, op):
+    import torch
+    dev = torch.device("cuda:0")
+    L = pkg.submodule("lib")
+    lib = L.load()
+    L.set_math_mode("tf32")
+    try:
+        N, IH, IC, OC = layer
+        case = (N, IH, IH, IC, OC, 3, 3, 1, 1, 1, 1)
+        X, W, dY, _ = _tensors(case, dev)
+        s = L.AlphaConvShape(N, IH, IH, IC, OC, 3, 3, IH, IH, 1, 1, 1, 1)
+        p = lambda t: C.c_void_p(t.data_ptr())
+        block = None
+        if op == "deltaX_prepared":
+            block = pkg.submodule("engine").CudaFloat32EngineBase().prepare_weights("deltaX", W, 3, 3, N, IH, IH, IH, IH, IC, OC, 1, 1, 1, 1)
+
+        def call(out, dB, stream):
+            st = C.c_void_p(stream)
+            if op == "forward":
+                return lib.alpha_conv3d_forward(C.byref(s), p(X), p(W), None, p(out), st)
+            if op == "deltaX_prepared":
+                return lib.alpha_conv3d_deltaX_prepared(C.byref(s), p(dY), p(W), p(block), block.numel(), p(out), st)
+            if op == "deltaW_bias":
+                return lib.alpha_conv3d_deltaW_bias(C.byref(s), p(X), p(dY), p(out), p(dB), st)
+            return lib.alpha_conv3d_deltaW(C.byref(s), p(X), p(dY), p(out), st)
+
+        shape = {"forward": dY.shape, "deltaX_prepared": X.shape}.get(op, W.shape)
+        ref, got, dB = torch.empty(shape, device=dev), torch.zeros(shape, device=dev), torch.empty(OC, device=dev)
+        L.check(call(ref, dB, torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        if op == "deltaW_bias":       # its sums of deltaY did need a block: one of that size
+            ext, own = torch.cuda.Stream(), torch.empty(1 << 20, dtype=torch.uint8, device=dev)
+            L.set_workspace(ext.cuda_stream, own.data_ptr(), 1 << 20)
+            try:
+                assert call(got, dB, ext.cuda_stream) == 0, L.last_error()
+                ext.synchronize()
+            finally:
+                L.set_workspace(ext.cuda_stream, 0, 0)
+        else:
+            graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()      # a fresh stream: no block yet
+            with torch.cuda.graph(graph, stream=side):
+                rc = call(got, dB, torch.cuda.current_stream().cuda_stream)
+            assert rc == 0, L.last_error()
+            graph.replay()
+        torch.cuda.synchronize()
+        assert float((got - ref).abs().max()) <= 5e-3 * float(ref.abs().max())
+    finally:
+        L.set_math_mode("3xtf32")
+    assert L.device_status() == 0

@@ -2054,7 +2054,7 @@ constexpr int kDwDone = 2;   // (within launch_dw_halo: its other form has run)
 // products C[n] = A[n]^T * B[n]); every CTA column of the grid then owns one image and writes its result in place.
 // x_pitch: floats between pixels, rows and images of X where it is not dense (stride 1 only).
 // former: see dw_most_steps (nullptr: the layer itself).
-// pow2: channel blocks of powers of two, in fewer parts: what a call runs whose scratch for more of them is refused.
+// pow2: channel blocks of powers of two, whose groups fill the SMs in one part: what a call runs whose scratch for parts is refused.
 // *spills: whether pixel tiles reach past the output where X still has pixels (see DwRepair).
 static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float* X, const float* dY, float* dW,
                           int mode3x, cudaStream_t stream, float* deltaB = nullptr, bool* bias_fused = nullptr,
@@ -2164,7 +2164,9 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     const WsMark start = ws_mark(c, stream);
     auto scratch = [&](size_t floats, float** out) {
         const int rc = get_workspace(c, stream, floats * sizeof(float), out);
-        if (!rc || pow2 || former || s_in->IC % 32 != 0 || !scratch_refused(rc)) return rc;
+        if (!rc || pow2 || former || s_in->IC % 32 != 0) return rc;
+        const DwForm o = plan_dw_form(s, strided, false, mode3x, opt(OPT_DW_STACKED), true);
+        if (o.cost < 0 || o.stacked || sm_budget(c) / dw_groups(s, o) > 1 || !scratch_refused(rc)) return rc;
         ws_rewind(c, stream, start);
         const int again = launch_dw_halo(c, s_in, X, dY, dW, mode3x, stream, deltaB, bias_fused, per_image, x_pitch, nullptr, spills, true);
         return again == ALPHA_OK ? kDwDone : again;

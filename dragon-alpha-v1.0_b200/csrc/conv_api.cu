@@ -106,6 +106,8 @@ static inline int opt(Opt which)
     return g_opt[which].load(std::memory_order_relaxed);
 }
 
+bool dependent_launches() { return opt(OPT_SM_BUDGET) <= 0; }
+
 static int env_math()
 {
     const char* e = getenv("ALPHA_CONV_MATH");

@@ -251,6 +251,14 @@ static inline int sm_budget(const DeviceCtx* c)
     return (b > 0 && b < c->sm_count) ? b : c->sm_count;
 }
 
+int device_sms(int* sms)
+{
+    DeviceCtx* c;
+    const int rc = get_ctx(&c);
+    if (!rc) *sms = sm_budget(c);
+    return rc;
+}
+
 // ---- scratch memory ----------------------------------------------------------------------------
 //
 // t_caller: scratch the caller of a native handed over for this one call (the CW / deltaW_buf

@@ -140,7 +140,10 @@ template <bool A_KC, bool B_KC>
 int launch_bmm_f32(const float* A, const float* B, float* C, int Batch, int N, int M, int K, int lda, int ldb, int ldc, size_t strA,
                    size_t strB, size_t strC, alpha_stream_t stream)
 {
-    const GemmTile t = pick_gemm_tile(N, M, Batch, 148);
+    int sms = 0;
+    const int rc = device_sms(&sms);
+    if (rc) return rc;
+    const GemmTile t = pick_gemm_tile(N, M, Batch, sms);
     for (int b0 = 0; b0 < Batch; b0 += 65535) {   // gridDim.z limit
         const int nb = Batch - b0 < 65535 ? Batch - b0 : 65535;
         const BatchGemm<A_KC, B_KC> g{A + b0 * strA, B + b0 * strB, C + b0 * strC, N, M, K, lda, ldb, ldc, strA, strB, strC};
@@ -192,7 +195,10 @@ int alpha_matMul(const float* A, const float* B, const float* bias, float* C, in
     if (rc || !bias) return rc;
     const size_t n4 = static_cast<size_t>(N) * M / 4;
     size_t blocks = (n4 + 255) / 256;
-    if (blocks > 148 * 8) blocks = 148 * 8;
+    int sms = 0;
+    rc = device_sms(&sms);
+    if (rc) return rc;
+    if (blocks > static_cast<size_t>(sms) * 8) blocks = static_cast<size_t>(sms) * 8;
     launch_after(add_bias_rows_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), 
         reinterpret_cast<float4*>(C), bias, n4, M / 4);
     note_launch("matmul_bias");
@@ -230,7 +236,10 @@ int alpha_pad_rows(const float* src, long long rows, int cols, float* dst, long 
     const long long total = rows4 * (cols4 / 4);
     if (total > 2000000000LL) return fail(ALPHA_E_ARG, "pad_rows: more than 8e9 elements");   // 31-bit indices with a grid stride
     long long blocks = (total + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    int sms = 0;
+    const int rc = device_sms(&sms);
+    if (rc) return rc;
+    if (blocks > sms * 16LL) blocks = sms * 16LL;
     launch_after(pad_rows_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), 
         src, reinterpret_cast<float4*>(dst), static_cast<unsigned>(rows), static_cast<unsigned>(cols), static_cast<unsigned>(total), fast_div(cols4 / 4));
     note_launch("pad_rows");

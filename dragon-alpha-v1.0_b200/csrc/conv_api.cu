@@ -1856,7 +1856,8 @@ static int launch_dx_col2im(DeviceCtx* c, const AlphaConvShape* s, const float* 
 //
 // What the tensor-core paths leave (OC % 8 != 0 at stride 1, OC % 32 != 0 under a stride) and ALPHA_ALGO_SIMT.  A launch of
 // fewer CTAs than SMs whose reduction is long (a classifier's 2762 x 53 layer: eight row tiles) is cut into up to 16 parts
-// that are added in order; without scratch for them (stream capture, a caller's small workspace) it runs unsplit.
+// that are added in order; without scratch for them (stream capture, a caller's small workspace) they run one after the other and add
+// up in deltaX itself, which gives the same bits.
 // 50 x 35 x 29, 100 -> 36 channels, 3x3: 1.21 ms with one thread per element, 0.18 ms here; 13 x 15 x 15, 636 -> 648, 1x1: 0.96
 // and 0.12 ms; 944 x 2764 x 56: 0.50 and 0.11 ms.
 static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream)
@@ -1874,31 +1875,38 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
     g.kt = (s->OC + kGemmBK - 1) / kGemmBK;
     g.by_kt = fast_div(g.kt);
     g.size = (size_t)s->N * s->IH * s->IW * s->IC;
-    g.ksplit = 1;
+    g.ksplit = g.parts = 1;
     const long long its = (long long)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * g.kt;
+    int turns = 1;
     if (ctas < sms && its >= 8) {
         long long ks = 2LL * sms / ctas;
         if (ks > its / 4) ks = its / 4;
         if (ks > 16) ks = 16;
-        float* ws = nullptr;
-        const int rc = ks > 1 ? get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws) : ALPHA_OK;
-        if (rc && !scratch_refused(rc)) return rc;
-        if (ks > 1 && !rc) { g.ksplit = (int)ks; g.out = ws; }
-    }
-    const long long nz = phases * g.ksplit;
-    auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
-    for (long long z0 = 0; z0 < nz; z0 += 65535)
-        for (long long y0 = 0; y0 < gy; y0 += 65535) {
-            g.y0 = (int)y0; g.z0 = (int)z0;
-            if (!t_dry) launch_gemm_f32(g, t, dim3((unsigned)gx, slice(y0, gy), slice(z0, nz)), stream);
-            note_launch("simt");
+        if (ks > 1) {
+            float* ws = nullptr;
+            const int rc = get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws);
+            if (rc && !scratch_refused(rc)) return rc;
+            g.ksplit = (int)ks;
+            if (rc) turns = (int)ks;
+            else { g.parts = (int)ks; g.out = ws; }
         }
+    }
+    const long long nz = phases * g.parts;
+    auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
+    for (int turn = 0; turn < turns; ++turn)
+        for (long long z0 = 0; z0 < nz; z0 += 65535)
+            for (long long y0 = 0; y0 < gy; y0 += 65535) {
+                g.part0 = turn; g.add = turn > 0;
+                g.y0 = (int)y0; g.z0 = (int)z0;
+                if (!t_dry) launch_gemm_f32(g, t, dim3((unsigned)gx, slice(y0, gy), slice(z0, nz)), stream);
+                note_launch("simt");
+            }
     int rc = check_launch("gemm_f32_kernel");
-    if (rc || g.ksplit == 1) return rc;
+    if (rc || g.parts == 1) return rc;
     const size_t n4 = g.size / 4;
     size_t blocks = (n4 + 255) / 256;
     if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-    if (!t_dry) launch_after(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(g.out), n4, g.ksplit, nullptr, 1, 0, 0.f,
+    if (!t_dry) launch_after(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(g.out), n4, g.parts, nullptr, 1, 0, 0.f,
                                                                reinterpret_cast<float4*>(dX));
     note_launch("simt");
     return check_launch("splitk_reduce_kernel");

@@ -174,14 +174,16 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
 }
 
 // deltaX of any stride as an implicit GEMM: rows = the pixels of one stride phase (py, px), which all receive the same filter
-// taps, columns = input channels, reduction = those taps x output channels (tap-major).  blockIdx.z = phase * ksplit + part;
-// part sp of the reduction goes to out + sp * size (one part: deltaX itself), every element of which some phase writes.
+// taps, columns = input channels, reduction = those taps x output channels (tap-major), in ksplit parts.  A launch computes `parts` of
+// them from part0 on, blockIdx.z = phase * parts + part, each into its own copy of deltaX (out + part * size), every element of which
+// some phase writes; or, without memory for copies, one part that is added to what `out` holds (add): the same sums in the same order.
 struct DxGemm {
     static constexpr bool kAk = true, kBk = false, kSkip = true;
     const float* dY; const float* W; float* out;
     int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw;
     int nsw;                       // phases along a row: min(sw, IW)
-    int ksplit, kt, y0, z0;        // kt = 16-step tiles per tap; y0 = column tile of blockIdx.y == 0, z0 = phase * ksplit + part of blockIdx.z == 0
+    int ksplit, parts, part0, add;
+    int kt, y0, z0;                // kt = 16-step tiles per tap; y0 = column tile of blockIdx.y == 0, z0 = phase * parts + part of blockIdx.z == 0
     size_t size;                   // elements of deltaX
     FastDiv by_kt;
     struct Cta { int m0, n0, rows, it0, it1, A, B, py, px, ry, rx, qy, qx, Ux; float* out; };
@@ -191,7 +193,7 @@ struct DxGemm {
 
     __device__ bool cta(Cta& c, int BM, int BN) const
     {
-        const int z = z0 + static_cast<int>(blockIdx.z), phase = z / ksplit, sp = z - phase * ksplit;
+        const int z = z0 + static_cast<int>(blockIdx.z), phase = z / parts, copy = z - phase * parts, sp = part0 + copy;
         c.py = phase / nsw; c.px = phase - c.py * nsw;
         c.A = (IH - c.py + sh - 1) / sh; c.B = (IW - c.px + sw - 1) / sw;
         c.rows = N * c.A * c.B;
@@ -204,7 +206,7 @@ struct DxGemm {
         const int its = Uy * c.Ux * kt, per = (its + ksplit - 1) / ksplit;
         c.it0 = sp * per < its ? sp * per : its;
         c.it1 = c.it0 + per < its ? c.it0 + per : its;
-        c.out = out + static_cast<size_t>(sp) * size;
+        c.out = out + static_cast<size_t>(copy) * size;
         return true;
     }
     __device__ RowA row_a(const Cta& c, int m) const
@@ -248,7 +250,11 @@ struct DxGemm {
     }
     __device__ void store(const Cta& c, const RowC& r, int col, const float4& o) const
     {
-        if (r.p && c.n0 + col < IC) *reinterpret_cast<float4*>(r.p + c.n0 + col) = o;
+        if (!r.p || c.n0 + col >= IC) return;
+        float4* p = reinterpret_cast<float4*>(r.p + c.n0 + col);
+        if (!add) { *p = o; return; }
+        const float4 a = *p;
+        *p = make_float4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
     }
 };
 

@@ -148,3 +148,22 @@ def test_more_columns_than_a_grid_dimension(pkg):
     C = eng.matMul(A, B)
     assert lib.last_algo() == "simt"
     assert bool(((C.double() - A.double() @ B.double()).abs() <= 4 * 2.0 ** -24 * (A.double().abs() @ B.double().abs())).all())
+
+
+@pytest.mark.parametrize("shape", [(8, 1, 52, 2764, 1, 1), (4, 9, 20, 36, 3, 2), (3, 6, 132, 100, 3, 1)], ids=str)
+def test_bits_do_not_depend_on_scratch(pkg, shape):
+    """A reduction split into parts adds them up in the same order with a copy for each as without."""
+    import torch
+    eng = pkg.submodule("engine").Engine()
+    N, OH, IC, OC, F, s = shape
+    p = F // 2
+    IH = (OH - 1) * s + F - 2 * p
+    dY, W = torch.randn((N, OH, OH, OC), device="cuda"), torch.randn((OC, F, F, IC), device="cuda")
+    want = eng.dconv3D_deltaX(dY, W, IH, IH, s, s, p, p)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()      # a fresh stream: no block yet
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        got = eng.dconv3D_deltaX(dY, W, IH, IH, s, s, p, p)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)

@@ -12,6 +12,7 @@ libalpha_conv_b200.so.  There is no CPU or PyTorch fallback: a missing library r
 import contextlib
 import ctypes as C
 import functools
+import operator
 
 import torch
 
@@ -25,9 +26,18 @@ def _stream(stream=None):
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
-# Shapes as the C structures the library reads (it never writes them): a program calls a few layers over and over.
-_conv_shape = functools.lru_cache(maxsize=512)(_l.AlphaConvShape)
-_pool_shape = functools.lru_cache(maxsize=512)(_l.AlphaPoolShape)
+# Shapes as the C structures the library reads (it never writes them): a program calls a few layers over and over.  The caches see
+# plain ints only: 3.0 would find the entry of 3, and a tensor the entry it made before its value changed.
+_cached_conv_shape = functools.lru_cache(maxsize=512)(_l.AlphaConvShape)
+_cached_pool_shape = functools.lru_cache(maxsize=512)(_l.AlphaPoolShape)
+
+
+def _conv_shape(*dims):
+    return _cached_conv_shape(*map(operator.index, dims))
+
+
+def _pool_shape(*dims):
+    return _cached_pool_shape(*map(operator.index, dims))
 
 
 def _new(like, shape, dtype=torch.float32):

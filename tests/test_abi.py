@@ -139,3 +139,17 @@ def test_jni_entry_points_use_the_jnienv_table(lib):
     assert log["region"] == (0xABCD, 0, 2)
     assert log["class"] == b"z/dragon/engine/cuda/impl/CudaException"
     assert log["thrown"][0] == 0x1234 and b"null" in log["thrown"][1]
+
+
+def test_shape_caches_see_plain_ints(pkg):
+    """A size of another type is converted or refused as the C structure itself does it, and never found by identity or equality."""
+    import torch
+    engine = pkg.submodule("engine")
+    for make, dims in ((engine._conv_shape, (1, 8, 8, 4, 4, 3, 3, 8, 8, 1, 1, 1, 1)), (engine._pool_shape, (1, 8, 8, 4, 2, 2, 4, 4, 2, 2, 0, 0))):
+        assert make(*dims).IH == 8
+        with pytest.raises(TypeError):
+            make(*map(float, dims))
+        size = torch.tensor(8)
+        assert make(1, size, *dims[2:]).IH == 8
+        size.fill_(16)
+        assert make(1, size, *dims[2:]).IH == 16

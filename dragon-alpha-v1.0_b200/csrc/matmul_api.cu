@@ -233,15 +233,19 @@ int alpha_pad_rows(const float* src, long long rows, int cols, float* dst, long 
     if (rows <= 0 || cols <= 0 || rows4 < rows || cols4 < cols || cols4 % 4 != 0)
         return fail(ALPHA_E_ARG, "pad_rows: bad shape (%lld x %d into %lld x %d)", rows, cols, rows4, cols4);
     if (reinterpret_cast<uintptr_t>(dst) & 15) return fail(ALPHA_E_ARG, "pad_rows: the destination must be 16-byte aligned");
-    const long long total = rows4 * (cols4 / 4);
-    if (total > 2000000000LL) return fail(ALPHA_E_ARG, "pad_rows: more than 8e9 elements");   // 31-bit indices with a grid stride
-    long long blocks = (total + 255) / 256;
     int sms = 0;
     const int rc = device_sms(&sms);
     if (rc) return rc;
-    if (blocks > sms * 16LL) blocks = sms * 16LL;
-    launch_after(pad_rows_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), 
-        src, reinterpret_cast<float4*>(dst), static_cast<unsigned>(rows), static_cast<unsigned>(cols), static_cast<unsigned>(total), fast_div(cols4 / 4));
+    const long long most = 2000000000LL / (cols4 / 4);   // rows of a launch: its indices are 31-bit, with a grid stride
+    for (long long r0 = 0; r0 < rows4; r0 += most) {
+        const long long n = rows4 - r0 < most ? rows4 - r0 : most, have = rows - r0 < 0 ? 0 : (rows - r0 < n ? rows - r0 : n);
+        const long long total = n * (cols4 / 4);
+        long long blocks = (total + 255) / 256;
+        if (blocks > sms * 16LL) blocks = sms * 16LL;
+        launch_after(pad_rows_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+            src + r0 * cols, reinterpret_cast<float4*>(dst) + r0 * (cols4 / 4), static_cast<unsigned>(have), static_cast<unsigned>(cols),
+            static_cast<unsigned>(total), fast_div(cols4 / 4));
+    }
     note_launch("pad_rows");
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "pad_rows_kernel launch failed: %s", cudaGetErrorString(e));

@@ -339,7 +339,7 @@ def _pad_both(t, n4, c4):
     shape = tuple(t.shape)
     if shape[-1] == c4 and shape[0] == n4:
         return t
-    if t.dtype != torch.float32 or not t.is_cuda or t.numel() == 0:
+    if t.dtype != torch.float32 or not t.is_cuda or t.numel() == 0 or t.is_neg():   # (a lazily negated view: its memory is not its value)
         out = torch.zeros((n4,) + shape[1:-1] + (c4,), dtype=t.dtype, device=t.device)
         out[: shape[0], ..., : shape[-1]] = t
         return out

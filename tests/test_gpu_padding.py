@@ -26,8 +26,22 @@ def test_engine_pads_any_layout(pkg):
         got = E._pad_last(t, c4)
         assert got.is_contiguous() and got.dtype == t.dtype
         assert torch.equal(got[..., : t.shape[-1]], t) and bool((got[..., t.shape[-1]:] == 0).all())
+    neg = torch._neg_view(base)
+    assert torch.equal(E._pad_last(neg, 8)[..., :7], -base)
     got = E._pad_both(base, 8, 8)
     assert torch.equal(got[:6, :, :7], base) and bool((got[6:] == 0).all()) and bool((got[:, :, 7:] == 0).all())
+
+
+def test_pad_rows_beyond_one_launch(pkg):
+    """2.1e9 rows of one column: more 16-byte words than a launch indexes."""
+    import torch
+    lib = pkg.submodule("lib")
+    rows = 2100000000
+    src = torch.arange(rows, device="cuda", dtype=torch.int32).view(torch.float32)      # (bit patterns)
+    out = torch.full((rows + 8, 4), float("nan"), device="cuda")
+    lib.check(lib.load().alpha_pad_rows(src.data_ptr(), rows, 1, out.data_ptr(), rows + 4, 4, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(out[:rows, 0].view(torch.int32), src.view(torch.int32))
+    assert not bool(out[:rows, 1:].any()) and not bool(out[rows:rows + 4].any()) and bool(out[rows + 4:].isnan().all())
 
 
 # N, IH, IW, IC, F, p: odd images (a last block row of one element), every padding, channel groups of 4 and of 8

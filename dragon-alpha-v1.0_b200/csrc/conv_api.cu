@@ -1868,7 +1868,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
     const int sms = sm_budget(c);
     const GemmTile t = pick_gemm_tile(rows, s->IC, phases, sms);
     const long long gx = (rows + t.bm - 1) / t.bm, gy = (s->IC + t.bn - 1) / t.bn, ctas = gx * gy * phases;
-    DxGemm g{};
+    DxGemm<false> g{};
     g.dY = dY; g.W = W; g.out = dX;
     g.N = s->N; g.IH = s->IH; g.IW = s->IW; g.IC = s->IC; g.FH = s->FH; g.FW = s->FW; g.OH = s->OH; g.OW = s->OW; g.OC = s->OC;
     g.sh = s->sh; g.sw = s->sw; g.ph = s->ph; g.pw = s->pw; g.nsw = nsw;
@@ -1896,9 +1896,11 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
     for (int turn = 0; turn < turns; ++turn)
         for (long long z0 = 0; z0 < nz; z0 += 65535)
             for (long long y0 = 0; y0 < gy; y0 += 65535) {
-                g.part0 = turn; g.add = turn > 0;
-                g.y0 = (int)y0; g.z0 = (int)z0;
-                if (!t_dry) launch_gemm_f32(g, t, dim3((unsigned)gx, slice(y0, gy), slice(z0, nz)), stream);
+                g.part0 = turn; g.y0 = (int)y0; g.z0 = (int)z0;
+                const dim3 grid((unsigned)gx, slice(y0, gy), slice(z0, nz));
+                if (t_dry) {}
+                else if (turn) launch_gemm_f32(DxGemm<true>{g}, t, grid, stream);
+                else launch_gemm_f32(g, t, grid, stream);
                 note_launch("simt");
             }
     int rc = check_launch("gemm_f32_kernel");

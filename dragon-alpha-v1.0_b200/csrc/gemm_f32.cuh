@@ -176,13 +176,14 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
 // deltaX of any stride as an implicit GEMM: rows = the pixels of one stride phase (py, px), which all receive the same filter
 // taps, columns = input channels, reduction = those taps x output channels (tap-major), in ksplit parts.  A launch computes `parts` of
 // them from part0 on, blockIdx.z = phase * parts + part, each into its own copy of deltaX (out + part * size), every element of which
-// some phase writes; or, without memory for copies, one part that is added to what `out` holds (add): the same sums in the same order.
-struct DxGemm {
+// some phase writes; or, without memory for copies, one part that is added to what `out` holds (DxGemm<true>, a kernel of its own: the
+// test and the load in the epilogue of every launch cost 7 % of a small layer): the same sums in the same order.
+struct DxProblem {
     static constexpr bool kAk = true, kBk = false, kSkip = true;
     const float* dY; const float* W; float* out;
     int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw;
     int nsw;                       // phases along a row: min(sw, IW)
-    int ksplit, parts, part0, add;
+    int ksplit, parts, part0;
     int kt, y0, z0;                // kt = 16-step tiles per tap; y0 = column tile of blockIdx.y == 0, z0 = phase * parts + part of blockIdx.z == 0
     size_t size;                   // elements of deltaX
     FastDiv by_kt;
@@ -248,13 +249,19 @@ struct DxGemm {
         if (r.n < 0) return RowC{nullptr};
         return RowC{c.out + ((static_cast<size_t>(r.n) * IH + (r.a * sh + c.py)) * IW + (r.b * sw + c.px)) * IC};
     }
+};
+template <bool ADD>
+struct DxGemm : DxProblem {
     __device__ void store(const Cta& c, const RowC& r, int col, const float4& o) const
     {
         if (!r.p || c.n0 + col >= IC) return;
         float4* p = reinterpret_cast<float4*>(r.p + c.n0 + col);
-        if (!add) { *p = o; return; }
-        const float4 a = *p;
-        *p = make_float4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
+        if (ADD) {
+            const float4 a = *p;
+            *p = make_float4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
+        } else {
+            *p = o;
+        }
     }
 };
 

@@ -1937,9 +1937,9 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
     // clocks over all blocks - 96 channels are one block of 96, 192 under three taps two of 96, where blocks of a power of
     // two would need three of 32 and three of 64.  Fewer blocks on a tie.  Channels past IC arrive as zeros and are not stored.
     // 88 x 56 x 56, 80 -> 64 channels 3x3 in plain TF32: 473 us over a patch matrix in blocks of 32, 177 us as one block of 96.
-    auto tiles = [&](int nt) { return (long long)((s->IC + nt - 1) / nt); };
+    auto tiles = [&](int nt) { return (s->IC + nt - 1) / nt; };
     auto nt_for = [&](int slots_cols, int top, int cols_per) {
-        int best = 0;
+        int best = 0, best_tiles = 0;
         long long best_clk = 0;
         if (pow2) {
             for (int nt = top; nt >= 32; nt >>= 1)
@@ -1947,8 +1947,10 @@ static DwForm plan_dw_form(const AlphaConvShape* s, bool strided, bool per_image
             return 0;
         }
         for (int nt = 32; nt <= top && slots_cols * nt <= 512; nt += 32) {
-            const long long clk = tiles(nt) * mma_clk(cols_per * nt);
-            if (!best || clk < best_clk || (clk == best_clk && tiles(nt) < tiles(best))) { best = nt; best_clk = clk; }
+            const int n = tiles(nt);
+            const long long clk = (long long)n * mma_clk(cols_per * nt);
+            if (!best || clk < best_clk || (clk == best_clk && n < best_tiles)) { best = nt; best_clk = clk; best_tiles = n; }
+            if (n == 1) break;   // (a wider block only has more columns)
         }
         return best;
     };

@@ -39,6 +39,13 @@ int fail(int code, const char* fmt, ...)
 }
 
 static thread_local char g_plan[192] = "";
+void note_plan(const char* fmt, ...)
+{
+    va_list ap;
+    va_start(ap, fmt);
+    vsnprintf(g_plan, sizeof(g_plan), fmt, ap);
+    va_end(ap);
+}
 // The calling thread is sizing a call (alpha_conv_workspace_bytes): scratch requests are added up
 // and answered with a placeholder address; nothing is allocated, launched or copied.
 static thread_local bool t_dry = false;
@@ -1891,6 +1898,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
             else { g.parts = (int)ks; g.out = ws; }
         }
     }
+    note_plan("gemm_f32 %dx%d phases=%lld ksplit=%d%s", t.bm, t.bn, phases, g.ksplit, turns > 1 ? " in turns" : "");
     const long long nz = phases * g.parts;
     auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
     for (int turn = 0; turn < turns; ++turn)

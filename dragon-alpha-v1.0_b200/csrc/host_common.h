@@ -19,6 +19,8 @@ namespace alpha {
 int fail(int code, const char* fmt, ...);
 // Counts one kernel launch and remembers the kernel family for alpha_conv_last_algo().
 void note_launch(const char* algo);
+// What alpha_conv_last_plan() reports (printf style).
+void note_plan(const char* fmt, ...);
 // SMs of the current device that kernels may spread over (option SM_BUDGET).
 int device_sms(int* sms);
 

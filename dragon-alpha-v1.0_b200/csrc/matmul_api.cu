@@ -129,6 +129,7 @@ int launch_bmm_simt(const float* A, const float* B, float* C, int Batch, int N, 
         bmm_simt_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(A + b0 * st.a_b, B + b0 * st.b_b, C + b0 * st.c_b, N, M, K, st);
     }
     note_launch("bmm_simt");
+    note_plan("bmm_simt");
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "bmm_simt_kernel launch failed: %s", cudaGetErrorString(e));
     return ALPHA_OK;
@@ -150,6 +151,7 @@ int launch_bmm_f32(const float* A, const float* B, float* C, int Batch, int N, i
         launch_gemm_f32(g, t, dim3((M + t.bn - 1) / t.bn, (N + t.bm - 1) / t.bm, nb), static_cast<cudaStream_t>(stream));
     }
     note_launch("bmm_simt");
+    note_plan("gemm_f32 %dx%d", t.bm, t.bn);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "gemm_f32_kernel launch failed: %s", cudaGetErrorString(e));
     return ALPHA_OK;

@@ -28,7 +28,7 @@ def test_fp32_deltaX(pkg, oracle_mod, shape, mode):
     got = eng.dconv3D_deltaX(torch.from_numpy(dY).cuda(), torch.from_numpy(W).cuda(), IH, IW, s, s, p, p).cpu().numpy()
     ref, mag = oracle_mod.deconv3D_deltaX_f64(dY, W, IH, IW, s, s, p, p, threads=8)
     if OC % 32 and (s > 1 or OC % 8):
-        assert pkg.submodule("lib").last_algo() == "simt"
+        assert pkg.submodule("lib").last_algo() == "simt" and pkg.submodule("lib").last_plan().startswith("gemm_f32")
         assert (np.abs(got - ref) <= F * F * OC * 2.0 ** -24 * mag).all()
 
 
@@ -43,7 +43,7 @@ def test_fp32_batched_products(pkg, dims):
     ref, mag = A.double() @ B.double(), A.double().abs() @ B.double().abs()
     for op, a, b in (("batchMatMul", A, B), ("batchMatMulT1", A.transpose(1, 2).contiguous(), B), ("batchMatMulT2", A, B.transpose(1, 2).contiguous())):
         y = getattr(eng, op)(a.cuda(), b.cuda()).cpu().double()
-        assert lib.last_algo() == "bmm_simt"
+        assert lib.last_algo() == "bmm_simt" and lib.last_plan().startswith("gemm_f32")
         assert bool(((y - ref).abs() <= K * 2.0 ** -24 * mag).all()), op
 
 

@@ -1,5 +1,7 @@
 """Channel counts that are no multiple of 32: zero-filled last chunks in the halo kernels and channel blocks of any multiple of
 32 columns in deltaW, against the fp64 oracle, with the route chosen by cost (HALO_PAD = 1) and forced (2)."""
+import re
+
 import numpy as np
 import pytest
 
@@ -9,12 +11,13 @@ pytestmark = pytest.mark.gpu
 TOL = {"3xtf32": dict(norm=1e-4, comp=1e-5), "tf32": dict(norm=5e-3, comp=2e-3)}   # the bounds of the other shape tests
 
 # N, IH, IW, IC, OC, FH, FW, s, p: remainders 4 ... 28 of a chunk, one chunk and several, blocks of 96 and 160 columns, tails in
-# every kernel form (pair, single CTA, tap-stacked, split reduction, strided deltaW, tap groups)
+# the kernel forms that test_forms_of_zero_filled_chunks names
 SHAPES = [
     (3, 35, 29, 36, 100, 3, 3, 1, 1), (2, 18, 18, 40, 64, 3, 3, 1, 1), (4, 20, 20, 16, 32, 3, 3, 1, 1), (2, 16, 16, 8, 128, 3, 3, 1, 1),
     (4, 28, 28, 60, 128, 3, 3, 1, 1), (2, 14, 14, 132, 256, 3, 3, 1, 1), (2, 13, 11, 92, 48, 5, 5, 1, 2), (3, 17, 15, 100, 72, 1, 1, 1, 0),
     (2, 24, 24, 96, 96, 3, 3, 1, 1), (2, 16, 16, 192, 40, 3, 3, 1, 1), (2, 12, 12, 320, 64, 3, 3, 1, 1), (2, 33, 31, 44, 20, 3, 3, 2, 1),
     (2, 17, 17, 72, 36, 3, 3, 2, 1), (1, 5, 5, 420, 24, 3, 3, 1, 1), (2, 16, 16, 68, 68, 4, 4, 2, 1), (1, 8, 8, 1028, 8, 1, 1, 1, 0),
+    (2, 112, 112, 36, 48, 3, 3, 1, 1),
 ]
 
 
@@ -32,7 +35,10 @@ def test_zero_filled_chunks(pkg, oracle_mod, shape, mode, pad):
     tX, tW, tdY = (torch.from_numpy(a).cuda() for a in (X, W, dY))
     lib.set_option("HALO_PAD", pad)
     try:
-        got = {"fwd": eng.conv3D(tX, tW, s, s, p, p), "dw": eng.dconv3D_deltaW(tX, tdY, FH, FW, s, s, p, p)}
+        got, algo = {"fwd": eng.conv3D(tX, tW, s, s, p, p)}, {}
+        algo["fwd"] = lib.last_algo()
+        got["dw"] = eng.dconv3D_deltaW(tX, tdY, FH, FW, s, s, p, p)
+        algo["dw"] = lib.last_algo()
         ref = {"fwd": oracle_mod.conv3D_f64(X, W, s, s, p, p, threads=8), "dw": oracle_mod.deconv3D_deltaW_f64(X, dY, FH, FW, s, s, p, p, threads=8)}
         if (IH + 2 * p - FH) % s == 0 and (IW + 2 * p - FW) % s == 0:
             got["dx"] = eng.dconv3D_deltaX(tdY, tW, IH, IW, s, s, p, p)
@@ -40,9 +46,37 @@ def test_zero_filled_chunks(pkg, oracle_mod, shape, mode, pad):
     finally:
         lib.set_option("HALO_PAD", 1)
     assert lib.device_status() == 0
+    if pad == 2 and IC % 32:       # forced: no patch matrix (a strided forward, and 8-channel steps in tiles under 0.6 full, have the im2col kernel)
+        assert algo["dw"] == "dw_halo" and (s > 1 or IC % 8 == 0 or algo["fwd"].startswith("halo")), algo
     for op, y in got.items():
         m = metrics(y.cpu().numpy(), *ref[op])
         assert m["finite"] and m["norm"] <= TOL[mode]["norm"] and m["comp"] <= TOL[mode]["comp"], (op, m)
+
+
+def test_forms_of_zero_filled_chunks(pkg):
+    """Over the shapes above, zero-filled chunks meet every form of the kernels."""
+    import torch
+    lib, engine = pkg.submodule("lib"), pkg.submodule("engine")
+    plans = []
+    lib.set_option("HALO_PAD", 2)
+    try:
+        for mode in ("3xtf32", "tf32"):
+            eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
+            for N, IH, IW, IC, OC, FH, FW, s, p in SHAPES:
+                if IC % 32 == 0:
+                    continue
+                OH, OW = out_hw(IH, IW, FH, FW, s, s, p, p)
+                X = torch.zeros((N, IH, IW, IC), device="cuda")
+                eng.conv3D(X, torch.zeros((OC, FH, FW, IC), device="cuda"), s, s, p, p)
+                plans.append(lib.last_plan())
+                eng.dconv3D_deltaW(X, torch.zeros((N, OH, OW, OC), device="cuda"), FH, FW, s, s, p, p)
+                plans.append(lib.last_plan())
+    finally:
+        lib.set_option("HALO_PAD", 1)
+    forms = {"CTA pairs": "halo_pair", "single CTA": "halo_row", "tap-stacked": "tapstack", "split reduction": "ksplit=([2-9]|1[0-9])", "strided deltaW": "dw_halo.* strided",
+             "tap groups": "tap groups", "stacked planes": "dw_halo stacked", "two half tiles": "dw_halo diagonal"}
+    missing = [f for f, text in forms.items() if not any(re.search(text, q) for q in plans)]
+    assert not missing, (missing, sorted(set(q.split(" R=")[0].split(" npb")[0] for q in plans)))
 
 
 def test_long_odd_reductions_keep_their_corrections_apart(pkg):

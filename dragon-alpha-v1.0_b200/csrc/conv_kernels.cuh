@@ -457,18 +457,6 @@ __global__ void __launch_bounds__(256) col2im_gather32_kernel(const float* __res
     }
 }
 
-// hi/lo planes of a whole tensor in global memory (weights are split once per call, not per tile).
-__global__ void split_tensor_kernel(const float4* __restrict__ src, float4* __restrict__ hi, float4* __restrict__ lo, size_t n4)
-{
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        float4 a = src[i], b;
-        split_tf32(a, b);
-        hi[i] = a;
-        lo[i] = b;
-    }
-}
-
 // out = sum of `splits` partial results of n4 float4 each (+ bias per column, + LeakyReLU): the tail of a
 // split-K forward / deltaX launch.  Partials are added in index order, so the result does not depend
 // on how the CTAs were scheduled.

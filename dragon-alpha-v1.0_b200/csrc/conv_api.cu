@@ -2154,7 +2154,7 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     }
     int stages = (int)((220 * 1024) / stage_bytes(R));
     if (stages > 4) stages = 4;
-    if ((size_t)stages * stage_bytes(R) < 16384) return 1;   // the epilogue stages its rows in the ring (24 KB at the least)
+    // (The epilogue stages 16 KB of rows in the ring, which has 20 KB at the least: four stages of 5 blocks of 1 KB.)
     p.R = R; p.CW = CW; p.PW = PW;
     const int tile_rows = diag ? 2 * R : R;   // R = rows per half tile in the diagonal form
     p.row_blocks = (s->OH + tile_rows - 1) / tile_rows; p.col_blocks = (s->OW + CW - 1) / CW;

@@ -108,7 +108,9 @@ int alpha_conv_debug_counters(unsigned long long* out, int n);
  *     stream is being captured into a CUDA graph a call that would have to grow the block fails with
  *     ALPHA_E_CAPTURE instead: run the step once eagerly, or alpha_conv_reserve_workspace, before
  *     capturing.  A block that a capture saw stays allocated until alpha_conv_release_workspace,
- *     because replays of that graph keep addressing it.
+ *     because replays of that graph keep addressing it.  Layers that an older kernel runs with less scratch or
+ *     none (odd channel counts, strided layers) take that kernel instead, in a capture as in a small block: the same
+ *     contraction to rounding, not the same bits.
  *   - A host that owns all device memory hands in its own block with alpha_conv_set_workspace
  *     (256-byte aligned; NULL returns the stream to library-owned scratch).  The library then never
  *     allocates for calls on that stream: a call that needs more fails with ALPHA_E_NOSCRATCH.
@@ -148,7 +150,9 @@ int alpha_conv_weights_updated(const float* W);
  * and keep them off the critical path of the forward and backward chains; the library allocates nothing and
  * records no events, the caller orders prepare before use (stream order, or an event, or a graph edge).
  *   alpha_conv_prepared_weights_bytes  size of the transform op (ALPHA_OP_FORWARD / ALPHA_OP_DELTAX) needs for this
- *                                      shape under the current math mode and options; 0 = none (plain TF32 forward)
+ *                                      shape under the current math mode and options; 0 = none: every plain TF32 forward,
+ *                                      and 3xTF32 forwards whose kernel splits W itself (by the cost of the shape: im2col,
+ *                                      windows of several filter rows).  A block serves every batch of its layer.
  *   alpha_conv_prepare_weights         enqueues the transform of W into `prepared` (256-byte aligned) on `stream`
  *   alpha_conv3d_forward_prepared /    the contraction with the transform taken from `prepared`; shape, W address,
  *   alpha_conv3d_deltaX_prepared       operator and math mode must be those of the prepare call (checked on the

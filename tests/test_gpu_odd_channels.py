@@ -59,6 +59,7 @@ def test_forms_of_zero_filled_chunks(pkg):
     lib, engine = pkg.submodule("lib"), pkg.submodule("engine")
     plans = []
     lib.set_option("HALO_PAD", 2)
+    lib.set_option("HALO_TAPSTACK", 2)      # wherever the tap-stacked kernel fits (plain TF32)
     try:
         for mode in ("3xtf32", "tf32"):
             eng = engine.Engine(engine.CudaFloat32EngineBase(math=mode))
@@ -73,6 +74,7 @@ def test_forms_of_zero_filled_chunks(pkg):
                 plans.append(lib.last_plan())
     finally:
         lib.set_option("HALO_PAD", 1)
+        lib.set_option("HALO_TAPSTACK", 1)
     forms = {"CTA pairs": "halo_pair", "single CTA": "halo_row", "tap-stacked": "tapstack", "split reduction": "ksplit=([2-9]|1[0-9])", "strided deltaW": "dw_halo.* strided",
              "tap groups": "tap groups", "stacked planes": "dw_halo stacked", "two half tiles": "dw_halo diagonal"}
     missing = [f for f, text in forms.items() if not any(re.search(text, q) for q in plans)]

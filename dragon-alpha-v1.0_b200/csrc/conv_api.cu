@@ -675,13 +675,11 @@ static inline bool whole_chunks(const IgemmPlan& pl) { return pl.kdim % 32 == 0 
 // 64 x 57 x 57, 44 -> 256 3x3 s2 97 / 128 us (windows).  Over 674 odd layers of the kinds above in both modes the forward route taken is
 // on average 1.04 times as long as the best of patch matrix, chunks and windows.
 // `idle`: lanes of a tile per pixel of the layer, which a patch matrix, flat over all pixels, does not have.
-static double tile_idle(int oH, int oW, int FH, int FW)
+static double tile_idle(int oH, int oW, int FH)
 {
     const int SG = oH + FH - 1, cols = (oW + 7) / 8 * 8;
-    double v = (double)((oH + 15) / 16 * 16) * cols / ((double)oH * oW);
-    if (SG <= 16) v = 16.0 * cols / ((1 + (16 - oH) / SG) * (double)oH * oW);          // stacked images
-    const double flat = 32.0 * ((oH + 3) / 4 * 4) / ((double)oH * oW);                  // flat tiles
-    return FW == 3 && oW + 2 <= 32 && flat < v ? flat : v;
+    if (SG <= 16) return 16.0 * cols / ((1 + (16 - oH) / SG) * (double)oH * oW);       // stacked images
+    return (double)((oH + 15) / 16 * 16) * cols / ((double)oH * oW);
 }
 static bool pad_beats_patch(int K, int taps, int ncols, int mode3x, double idle, bool strided = false)
 {
@@ -1599,7 +1597,7 @@ static bool window_fits(const AlphaConvShape* s, const WindowPlan& w)
 static double forward_idle(const AlphaConvShape* s)
 {
     const bool strided = s->sh != 1 || s->sw != 1;
-    return s->FH * s->FW == 1 && !strided ? 1.0 : tile_idle(s->OH, s->OW, s->FH, strided ? 0 : s->FW);
+    return s->FH * s->FW == 1 && !strided ? 1.0 : tile_idle(s->OH, s->OW, s->FH);
 }
 static bool window_beats_rest(const AlphaConvShape* s, const WindowPlan& w, int mode3x, int sms)
 {
@@ -1610,7 +1608,7 @@ static bool window_beats_rest(const AlphaConvShape* s, const WindowPlan& w, int 
     const double nc = s->OC < 64 ? 64 : s->OC, mem = mode3x ? 150 : 360;
     const bool strided = s->sh != 1 || s->sw != 1;
     if (!mode3x && !strided && s->IC >= 8) return false;
-    const double own = tile_idle(s->OH, s->OW, w.U, 1) * w.U * chunks32(w.K) * nc * (w.g < s->sh ? 1.2 : 1.0) + w.per_pixel / 32.0 * mem;
+    const double own = tile_idle(s->OH, s->OW, w.U) * w.U * chunks32(w.K) * nc * (w.g < s->sh ? 1.2 : 1.0) + w.per_pixel / 32.0 * mem;
     const double pad = forward_idle(s) * taps * chunks32(s->IC) * nc * (strided ? 1.4 : 1.0), patch = (double)chunks32(taps * s->IC) * (nc + mem);
     // (an IC of whole 8-channel tiles has no patch matrix to compare with: it would go to the im2col kernel)
     return own < 0.9 * (pad < patch || s->IC % 8 == 0 ? pad : patch);
@@ -3034,7 +3032,7 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
             }
             if (!mode3x) pt.W_lo = nullptr;
             pt.pad = s->OC % 32 != 0;
-            if ((tiny_image(s->IH, s->IW) || (pt.pad && !pad_beats_patch(s->OC, taps, s->IC, mode3x, taps == 1 ? 1.0 : tile_idle(s->IH, s->IW, s->FH, s->FW)))) && (s->FH > 1 || s->FW > 1) &&
+            if ((tiny_image(s->IH, s->IW) || (pt.pad && !pad_beats_patch(s->OC, taps, s->IC, mode3x, taps == 1 ? 1.0 : tile_idle(s->IH, s->IW, s->FH)))) && (s->FH > 1 || s->FW > 1) &&
                 (long long)taps * s->OC <= 16384 && (!pt.pad || opt(OPT_PATCH_MATRIX))) {
                 const WsMark start = ws_mark(c, stream);   // (the transposed weights before it stay)
                 rc = launch_patch_gemm(c, pt, mode3x, stream);

@@ -1,8 +1,8 @@
 // Register-tiled fp32 products for what the tensor-core kernels do not take at fp32 precision: deltaX of channel counts that
 // are no multiple of 8 (stride 1) or 32 (strides), and batched matrix products of ragged sizes.
 //
-// Bound: FMA issue with the operand reads from shared memory close behind (a step of a 64 x 64 tile is 32 clocks of FMAs and some
-// 24 of reads).  Of 74 TFLOP/s it reaches 42 with 128 x 128 tiles (64 x 56 x 56, 100 -> 128 channels 3x3) and, with 64 x 64 tiles,
+// Bound: FMA issue with the operand reads from shared memory close behind (a step of a 128 x 64 tile is 64 clocks of FMAs and some
+// 40 of reads).  Of 74 TFLOP/s it reaches 42 with 128 x 128 tiles (64 x 56 x 56, 100 -> 128 channels 3x3) and, with 128 x 64 tiles,
 // 32 counting idle columns: 18 of use at 36 of 64 columns (50 x 35 x 29, 100 -> 36).
 //
 // A CTA of 256 threads computes BM x BN outputs, TM x TN per thread, from 16 reduction steps staged in shared memory at a time.

@@ -6,7 +6,7 @@
 #include "conv_dw_halo.cuh"
 #include "conv_tapstack.cuh"
 #include "winograd.cuh"
-#include "gemm_f32.cuh"
+#include "gemm_planes.cuh"
 #include "host_common.h"
 
 #include <nvtx3/nvToolsExt.h>   // header-only: resolves a profiler's injection library at run time, no link dependency
@@ -74,6 +74,7 @@ enum Opt {
     OPT_HALO_LATTICE,   // strided forward on the halo kernel: 0 never, 1 by cost, 2 wherever possible
     OPT_HALO_WINDOW,    // layers of few channels as convolutions over windows of a filter row: 0 never, 1 by cost, 2 wherever possible
     OPT_HALO_PAD,       // channels that are no multiple of 32 on the halo kernels: 0 never, 1 by cost, 2 wherever possible
+    OPT_F32_PLANES,     // fp32 products as three bf16 planes on the tensor cores: 0 never, 1 by cost, 2 always
     OPT_COUNT
 };
 struct OptDef { const char* name; int dflt; };
@@ -84,6 +85,7 @@ static const OptDef kOptDefs[OPT_COUNT] = {
     {"DW_STACKED", -1}, {"DW_DIAG", 1}, {"DW_CW", 0}, {"DW_R", 0}, {"DW_STATIC", 1}, {"CONV_PROF", 0}, {"SM_BUDGET", 0},
     {"SKINNY", 1}, {"HALO_DEEP", 1}, {"HALO_SPLITB", 0}, {"NVTX", 1}, {"DW_LANES", 0}, {"HALO_TAPSTACK", 1}, {"HALO_FLAT32", 1},
     {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_LATTICE", 1}, {"HALO_WINDOW", 1}, {"HALO_PAD", 1},
+    {"F32_PLANES", 1},
 };
 static std::atomic<int> g_opt[OPT_COUNT];
 static std::once_flag g_opt_once;
@@ -265,6 +267,18 @@ int device_sms(int* sms)
     if (!rc) *sms = sm_budget(c);
     return rc;
 }
+
+// The status word kernels report to, for the other translation units.
+int device_status_word(int** status)
+{
+    DeviceCtx* c;
+    const int rc = get_ctx(&c);
+    if (!rc) *status = c->status;
+    return rc;
+}
+
+// Option F32_PLANES; ALPHA_ALGO_SIMT asks for plain fp32 kernels.
+int option_f32_planes() { return cur_algo() == ALPHA_ALGO_SIMT ? 0 : opt(OPT_F32_PLANES); }
 
 // ---- scratch memory ----------------------------------------------------------------------------
 //
@@ -1859,44 +1873,41 @@ static int launch_dx_col2im(DeviceCtx* c, const AlphaConvShape* s, const float* 
 
 // ---- deltaX in fp32: every stride, filter and channel count -------------------------------------------
 //
-// What the tensor-core paths leave (OC % 8 != 0 at stride 1, OC % 32 != 0 under a stride) and ALPHA_ALGO_SIMT.  A launch of
-// fewer CTAs than SMs whose reduction is long (a classifier's 2762 x 53 layer: eight row tiles) is cut into up to 16 parts
-// that are added in order; without scratch for them (stream capture, a caller's small workspace) they run one after the other and add
-// up in deltaX itself, which gives the same bits.
-// 50 x 35 x 29, 100 -> 36 channels, 3x3: 1.21 ms with one thread per element, 0.18 ms here; 13 x 15 x 15, 636 -> 648, 1x1: 0.96
-// and 0.12 ms; 944 x 2764 x 56: 0.50 and 0.11 ms.
+// What the TF32 paths leave (OC % 8 != 0 at stride 1, OC % 32 != 0 under a stride) and ALPHA_ALGO_SIMT, by FMAs or, where plan_product
+// finds that faster, as bf16 planes on the tensor cores at the same accuracy.  A launch of fewer CTAs than SMs whose reduction is long (a
+// classifier's 2762 x 53 layer: eight row tiles) is cut into up to 16 parts that are added in order; without scratch for them (stream
+// capture, a caller's small workspace) they run one after the other and add up in deltaX itself, which gives the same bits.
 static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream)
 {
     const long long rows = (long long)s->N * ((s->IH + s->sh - 1) / s->sh) * ((s->IW + s->sw - 1) / s->sw);
     const int nsh = s->sh < s->IH ? s->sh : s->IH, nsw = s->sw < s->IW ? s->sw : s->IW;   // phases that own a pixel
     const long long phases = (long long)nsh * nsw;
     const int sms = sm_budget(c);
-    const GemmTile t = pick_gemm_tile(rows, s->IC, phases, sms);
-    const long long gx = (rows + t.bm - 1) / t.bm, gy = (s->IC + t.bn - 1) / t.bn, ctas = gx * gy * phases;
+    const int Uy = (s->FH + s->sh - 1) / s->sh, Ux = (s->FW + s->sw - 1) / s->sw;   // most taps of a phase
+    const size_t size = (size_t)s->N * s->IH * s->IW * s->IC;
+    const ProductPlan plan = plan_product(rows, s->IC, Uy * Ux, s->OC, phases, true, (double)size, sms,
+                                          Uy <= DxProblem::kPlaneTaps && Ux <= DxProblem::kPlaneTaps ? option_f32_planes() : 0);
+    const GemmTile t = plan.tile;
+    const long long gx = (rows + t.bm - 1) / t.bm, gy = (s->IC + t.bn - 1) / t.bn;
     DxGemm<false> g{};
     g.dY = dY; g.W = W; g.out = dX;
     g.N = s->N; g.IH = s->IH; g.IW = s->IW; g.IC = s->IC; g.FH = s->FH; g.FW = s->FW; g.OH = s->OH; g.OW = s->OW; g.OC = s->OC;
     g.sh = s->sh; g.sw = s->sw; g.ph = s->ph; g.pw = s->pw; g.nsw = nsw;
-    g.kt = (s->OC + kGemmBK - 1) / kGemmBK;
+    g.unit = t.planes ? kPlaneBK / kGemmBK : 1;
+    g.kt = (s->OC + kGemmBK * g.unit - 1) / (kGemmBK * g.unit) * g.unit;
     g.by_kt = fast_div(g.kt);
-    g.size = (size_t)s->N * s->IH * s->IW * s->IC;
+    g.size = size;
     g.ksplit = g.parts = 1;
-    const long long its = (long long)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * g.kt;
     int turns = 1;
-    if (ctas < sms && its >= 8) {
-        long long ks = 2LL * sms / ctas;
-        if (ks > its / 4) ks = its / 4;
-        if (ks > 16) ks = 16;
-        if (ks > 1) {
-            float* ws = nullptr;
-            const int rc = get_workspace(c, stream, (size_t)ks * g.size * sizeof(float), &ws);
-            if (rc && !scratch_refused(rc)) return rc;
-            g.ksplit = (int)ks;
-            if (rc) turns = (int)ks;
-            else { g.parts = (int)ks; g.out = ws; }
-        }
+    if (plan.ksplit > 1) {
+        float* ws = nullptr;
+        const int rc = get_workspace(c, stream, (size_t)plan.ksplit * g.size * sizeof(float), &ws);
+        if (rc && !scratch_refused(rc)) return rc;
+        g.ksplit = plan.ksplit;
+        if (rc) turns = plan.ksplit;
+        else { g.parts = plan.ksplit; g.out = ws; }
     }
-    note_plan("gemm_f32 %dx%d phases=%lld ksplit=%d%s", t.bm, t.bn, phases, g.ksplit, turns > 1 ? " in turns" : "");
+    note_plan("gemm_f32 %s%dx%d phases=%lld ksplit=%d%s", t.planes ? "planes " : "", t.bm, t.bn, phases, g.ksplit, turns > 1 ? " in turns" : "");
     const long long nz = phases * g.parts;
     auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
     for (int turn = 0; turn < turns; ++turn)
@@ -1905,8 +1916,8 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
                 g.part0 = turn; g.y0 = (int)y0; g.z0 = (int)z0;
                 const dim3 grid((unsigned)gx, slice(y0, gy), slice(z0, nz));
                 if (t_dry) {}
-                else if (turn) launch_gemm_f32(DxGemm<true>{g}, t, grid, stream);
-                else launch_gemm_f32(g, t, grid, stream);
+                else if (turn) launch_product(DxGemm<true>{g}, t, grid, stream, c->status);
+                else launch_product(g, t, grid, stream, c->status);
                 note_launch("simt");
             }
     int rc = check_launch("gemm_f32_kernel");

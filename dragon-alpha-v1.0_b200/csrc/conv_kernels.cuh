@@ -20,14 +20,6 @@ namespace alpha {
 constexpr int kBM = 128;           // GEMM M tile = tensor-memory lanes
 constexpr int kIgemmThreads = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: split + epilogue
 
-enum KernelStatus : int {
-    kStatusOk = 0,
-    kStatusProducerTimeout = 1,
-    kStatusMmaTimeout = 2,
-    kStatusSplitTimeout = 3,
-    kStatusEpilogueTimeout = 4,
-};
-
 // The reference's LeakyReLU, x * ((x > 0) + k * (x < 0)) (Cuda_function/type4_leakyRelu2D.cuh:32);
 // k = 0 is ReLU.  Applied after the bias in the forward epilogues when a plan asks for it.
 __device__ __forceinline__ float leaky_relu(float x, float k) { return x > 0.f ? x : k * x; }
@@ -62,11 +54,6 @@ struct IgemmParams {
     uint32_t b_tx;      // bytes the B loads of one stage deliver
     uint32_t swz;       // descriptor layout type of the K-major operands
 };
-
-__device__ __forceinline__ void report(int* status, int code)
-{
-    if (status) atomicCAS(status, 0, code);
-}
 
 // Round to TF32 (10 explicit mantissa bits), nearest with ties away from zero: add half a TF32 ulp
 // to the magnitude and clear the 13 low bits.  Two full-rate integer instructions; the dedicated

@@ -60,18 +60,6 @@ struct TapStackParams {
     uint32_t idesc, tmem_cols;
 };
 
-// 32 lanes x 16 consecutive 32-bit columns: thread t of the warp gets row (lane base + t).
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32"
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-
 // 32 channels of one tile row: Y[c] = sum over fw of D[lane + fw][fw * BN + channel], the partial sums of the
 // FW taps gathered from the next lanes.  FW_T = 2 or 3 issues all loads before one wait; FW_T = 0 is any FW.
 template <int FW_T>

@@ -23,5 +23,9 @@ void note_launch(const char* algo);
 void note_plan(const char* fmt, ...);
 // SMs of the current device that kernels may spread over (option SM_BUDGET).
 int device_sms(int* sms);
+// Where kernels report a wait that ran out.
+int device_status_word(int** status);
+// Option F32_PLANES.
+int option_f32_planes();
 
 }  // namespace alpha

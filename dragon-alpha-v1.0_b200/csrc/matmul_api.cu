@@ -9,7 +9,7 @@
 // pitches) run a plain fp32 kernel.
 #include "../../include/alpha_conv_b200.h"
 #include "host_common.h"
-#include "gemm_f32.cuh"
+#include "gemm_planes.cuh"
 
 namespace alpha {
 int launch_buf_summary(cudaStream_t stream, const float* buf, float* deltaW, int part, size_t sizeW);
@@ -142,16 +142,18 @@ int launch_bmm_f32(const float* A, const float* B, float* C, int Batch, int N, i
                    size_t strB, size_t strC, alpha_stream_t stream)
 {
     int sms = 0;
-    const int rc = device_sms(&sms);
+    int rc = device_sms(&sms);
+    int* status = nullptr;
+    if (!rc) rc = device_status_word(&status);
     if (rc) return rc;
-    const GemmTile t = pick_gemm_tile(N, M, Batch, sms);
+    const GemmTile t = plan_product(N, M, 1, K, Batch, false, 0, sms, option_f32_planes()).tile;
     for (int b0 = 0; b0 < Batch; b0 += 65535) {   // gridDim.z limit
         const int nb = Batch - b0 < 65535 ? Batch - b0 : 65535;
         const BatchGemm<A_KC, B_KC> g{A + b0 * strA, B + b0 * strB, C + b0 * strC, N, M, K, lda, ldb, ldc, strA, strB, strC};
-        launch_gemm_f32(g, t, dim3((M + t.bn - 1) / t.bn, (N + t.bm - 1) / t.bm, nb), static_cast<cudaStream_t>(stream));
+        launch_product(g, t, dim3((M + t.bn - 1) / t.bn, (N + t.bm - 1) / t.bm, nb), static_cast<cudaStream_t>(stream), status);
     }
     note_launch("bmm_simt");
-    note_plan("gemm_f32 %dx%d", t.bm, t.bn);
+    note_plan("gemm_f32 %s%dx%d", t.planes ? "planes " : "", t.bm, t.bn);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "gemm_f32_kernel launch failed: %s", cudaGetErrorString(e));
     return ALPHA_OK;

@@ -35,6 +35,20 @@ __device__ __forceinline__ bool elect_one()
     return pred != 0;
 }
 
+// Device status word: which role's bounded wait ran out first.
+enum KernelStatus : int {
+    kStatusOk = 0,
+    kStatusProducerTimeout = 1,
+    kStatusMmaTimeout = 2,
+    kStatusSplitTimeout = 3,
+    kStatusEpilogueTimeout = 4,
+};
+
+__device__ __forceinline__ void report(int* status, int code)
+{
+    if (status) atomicCAS(status, 0, code);
+}
+
 // ---- mbarrier -------------------------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
@@ -113,7 +127,22 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
-__device__ __noinline__ bool mbar_wait_slow_a(uint32_t bar, uint32_t parity)
+// Whether the phase has completed, without waiting.
+__device__ __forceinline__ bool mbar_test_a(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+static __device__ __noinline__ bool mbar_wait_slow_a(uint32_t bar, uint32_t parity)
 {
     const uint64_t t0 = globaltimer_ns();
     for (;;) {
@@ -186,7 +215,7 @@ __device__ __forceinline__ bool mbar_try_wait_cluster_a(uint32_t bar, uint32_t p
         : "memory");
     return ok != 0;
 }
-__device__ __noinline__ bool mbar_wait_cluster_a(uint32_t bar, uint32_t parity)
+static __device__ __noinline__ bool mbar_wait_cluster_a(uint32_t bar, uint32_t parity)
 {
     if (mbar_try_wait_cluster_a(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
@@ -435,6 +464,18 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
         : "r"(taddr)
         : "memory");
 }
+// 32 lanes x 16 columns.
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32"
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -454,6 +495,8 @@ enum : uint32_t { kSwizzleNone = 0, kSwizzle128B_Base32B = 1, kSwizzle128B = 2, 
 //   MN-major tf32 (kSwizzle128B_Base32B): a block is 32 elements (128 B) wide, its swizzle atom
 //             4 K-rows deep (512 B); sbo = distance between 4-row K groups, lbo = distance between
 //             32-wide MN blocks.  One K=8 instruction spans two atoms.
+//   MN-major 16-bit (kSwizzle64B): a block is 32 elements (64 B) wide, its atom 8 K-rows deep (512 B); sbo = distance between
+//             8-row K groups, lbo = distance between 32-wide MN blocks.  One K=16 instruction spans two atoms.
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo,
                                                    uint32_t layout)
 {
@@ -503,6 +546,32 @@ __device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, ui
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
         "}\n" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// Instruction descriptor for kind::f16 with both operands bf16 and fp32 accumulation (K = 16).
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool a_mn_major, bool b_mn_major)
+{
+    return 1u << 4 | 1u << 7 | 1u << 10 | (a_mn_major ? 1u : 0u) << 15 | (b_mn_major ? 1u : 0u) << 16 |
+           static_cast<uint32_t>(N >> 3) << 17 | static_cast<uint32_t>(M >> 4) << 24;
+}
+template <uint32_t A_OFF, uint32_t B_OFF>
+__device__ __forceinline__ void mma_bf16_ss2_imm(uint32_t d_tmem, uint32_t a_base, uint32_t a_hi, uint32_t b_base, uint32_t b_hi, uint32_t idesc,
+                                                 uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        ".reg .b32 ra, rb;\n\t"
+        "add.u32 ra, %1, %7;\n\t"
+        "add.u32 rb, %3, %8;\n\t"
+        "mov.b64 da, {ra, %2};\n\t"
+        "mov.b64 db, {rb, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_base), "r"(a_hi), "r"(b_base), "r"(b_hi), "r"(idesc), "r"(accumulate), "n"(A_OFF), "n"(B_OFF)
         : "memory");
 }
 

@@ -1,0 +1,113 @@
+"""fp32 products as three bf16 planes on the tensor cores: against 64-bit sums at the edges of tiles, stages, taps and parts, and
+against the FMA kernel where planes do not represent the operands.
+
+Bound of a sum of K products: what is dropped of a product (two terms below 2^-21 of it, one below 2^-28), four truncated additions of
+2^-23 for every 64 of them, and one rounded addition of 2^-24 for each such window and the small products."""
+import numpy as np
+import pytest
+
+from helpers import gen, out_hw
+
+pytestmark = pytest.mark.gpu
+
+
+def bound(K):
+    return 2.0 ** -20 + 2.0 ** -28 + 4 * 2.0 ** -23 + (K / 64 + 3) * 2.0 ** -24
+
+
+@pytest.fixture
+def planes(pkg):
+    lib = pkg.submodule("lib")
+    L = lib.load()
+    lib.check(L.alpha_conv_set_option(b"F32_PLANES", 2))
+    yield lambda v: lib.check(L.alpha_conv_set_option(b"F32_PLANES", v))
+    lib.check(L.alpha_conv_set_option(b"F32_PLANES", 1))
+
+
+# N, IH, IW, IC, OC, F, s, p: both column tiles and a remainder of each, one stage, half stages, odd and even windows, phases without
+# a tap, rows past the last one, split reductions
+DX = [(2, 35, 29, 36, 100, 3, 1, 1), (1, 9, 9, 4, 12, 3, 1, 1), (3, 16, 16, 132, 20, 3, 2, 1), (2, 15, 17, 64, 68, 1, 2, 0), (2, 9, 11, 40, 44, 2, 3, 0),
+      (1, 6, 6, 260, 36, 4, 2, 1), (5, 1, 4, 52, 2764, 1, 1, 0), (1, 7, 5, 8, 4, 7, 2, 3), (2, 20, 20, 128, 36, 5, 1, 2), (1, 1, 1, 4, 4, 1, 1, 0),
+      (130, 1, 1, 196, 180, 1, 1, 0)]
+
+
+@pytest.mark.parametrize("shape", DX, ids=str)
+def test_deltaX(pkg, oracle_mod, planes, shape):
+    import torch
+    eng = pkg.submodule("engine").Engine()
+    N, IH, IW, IC, OC, F, s, p = shape
+    OH, OW = out_hw(IH, IW, F, F, s, s, p, p)
+    IH, IW = (OH - 1) * s + F - 2 * p, (OW - 1) * s + F - 2 * p
+    rng = np.random.default_rng(IC * 1000 + OC)
+    W, dY = gen((OC, F, F, IC), "n01", rng), gen((N, OH, OW, OC), "n01", rng)
+    got = eng.dconv3D_deltaX(torch.from_numpy(dY).cuda(), torch.from_numpy(W).cuda(), IH, IW, s, s, p, p).cpu().numpy()
+    ref, mag = oracle_mod.deconv3D_deltaX_f64(dY, W, IH, IW, s, s, p, p, threads=8)
+    assert pkg.submodule("lib").last_plan().startswith("gemm_f32 planes")
+    assert (np.abs(got - ref) <= bound(F * F * OC) * mag).all()
+
+
+@pytest.mark.parametrize("dims", [(2, 1, 1, 1), (3, 20, 20, 20), (2, 65, 33, 17), (2, 130, 129, 50), (1, 264, 425, 220), (5, 88, 79, 24), (2, 64, 65, 36), (3, 128, 128, 97)], ids=str)
+def test_batched_products(pkg, planes, dims):
+    import torch
+    eng, lib = pkg.submodule("engine").Engine(), pkg.submodule("lib")
+    Bt, N, M, K = dims
+    g = torch.Generator().manual_seed(Bt + N + M + K)
+    A, B = torch.randn((Bt, N, K), generator=g), torch.randn((Bt, K, M), generator=g)
+    ref, mag = A.double() @ B.double(), A.double().abs() @ B.double().abs()
+    for op, a, b in (("batchMatMul", A, B), ("batchMatMulT1", A.transpose(1, 2).contiguous(), B), ("batchMatMulT2", A, B.transpose(1, 2).contiguous())):
+        y = getattr(eng, op)(a.cuda(), b.cuda()).cpu().double()
+        assert lib.last_plan().startswith("gemm_f32 planes")
+        assert bool(((y - ref).abs() <= bound(K) * mag).all()), op
+
+
+@pytest.mark.parametrize("what", ["inf weight", "nan gradient", "largest", "tiny", "overflow"])
+def test_operands_outside_the_planes(pkg, planes, what):
+    """Tiles with such operands are formed by FMAs: the values, Infs and NaNs of the FMA kernel, and border pixels untouched by taps
+    that miss the output."""
+    import torch
+    eng = pkg.submodule("engine").Engine()
+    N, H, IC, OC = 2, 17, 40, 100
+    g = torch.Generator(device="cuda").manual_seed(3)
+    W, dY = torch.randn((OC, 3, 3, IC), device="cuda", generator=g), torch.randn((N, H, H, OC), device="cuda", generator=g)
+    big = torch.finfo(torch.float32).max
+    if what == "inf weight":
+        W[5, 2, 1, 7] = float("inf")
+    elif what == "nan gradient":
+        dY[1, 3, 4, 9] = float("nan")
+    elif what == "largest":
+        dY[0, 8, 8, :] = -big
+        W *= 1e-3
+    elif what == "tiny":
+        dY *= 1e-34
+    else:
+        dY[0, 8, 8, :] = big
+        W.abs_()
+    out = []
+    for mode in (0, 2):
+        planes(mode)
+        out.append(eng.dconv3D_deltaX(dY, W, H, H, 1, 1, 1, 1))
+        assert pkg.submodule("lib").last_plan().startswith("gemm_f32 planes" if mode else "gemm_f32")
+    a, b = out
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    ok = a.isfinite()
+    scale = a[ok].abs().max().double() if what == "largest" else torch.nn.functional.conv_transpose2d(
+        dY.double().abs().nan_to_num(0, 0, 0).permute(0, 3, 1, 2), W.double().abs().nan_to_num(0, 0, 0).permute(0, 3, 1, 2), padding=1).permute(0, 2, 3, 1)[ok]
+    assert bool(((a[ok].double() - b[ok].double()).abs() <= 2 * 900 * 2.0 ** -24 * scale).all())
+    if what == "inf weight":
+        assert bool(b[:, 0].isfinite().all()) and bool(b[..., :7].isfinite().all())
+
+
+def test_parts_give_the_same_bits_with_and_without_scratch(pkg, planes):
+    import torch
+    eng = pkg.submodule("engine").Engine()
+    dY, W = torch.randn((130, 1, 1, 2764), device="cuda"), torch.randn((2764, 1, 1, 132), device="cuda")
+    want = eng.dconv3D_deltaX(dY, W, 1, 1, 1, 1, 0, 0)
+    plan = pkg.submodule("lib").last_plan()
+    assert "planes" in plan and "ksplit=1" not in plan.split()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        got = eng.dconv3D_deltaX(dY, W, 1, 1, 1, 1, 0, 0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert "in turns" not in plan and torch.equal(got, want)

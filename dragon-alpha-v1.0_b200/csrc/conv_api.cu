@@ -75,6 +75,7 @@ enum Opt {
     OPT_HALO_WINDOW,    // layers of few channels as convolutions over windows of a filter row: 0 never, 1 by cost, 2 wherever possible
     OPT_HALO_PAD,       // channels that are no multiple of 32 on the halo kernels: 0 never, 1 by cost, 2 wherever possible
     OPT_F32_PLANES,     // fp32 products as three bf16 planes on the tensor cores: 0 never, 1 by cost, 2 always
+    OPT_GATHER,         // 3xTF32 layers straight from their tensors as three bf16 planes: 0 never, 1 by cost, 2 wherever possible
     OPT_COUNT
 };
 struct OptDef { const char* name; int dflt; };
@@ -85,7 +86,7 @@ static const OptDef kOptDefs[OPT_COUNT] = {
     {"DW_STACKED", -1}, {"DW_DIAG", 1}, {"DW_CW", 0}, {"DW_R", 0}, {"DW_STATIC", 1}, {"CONV_PROF", 0}, {"SM_BUDGET", 0},
     {"SKINNY", 1}, {"HALO_DEEP", 1}, {"HALO_SPLITB", 0}, {"NVTX", 1}, {"DW_LANES", 0}, {"HALO_TAPSTACK", 1}, {"HALO_FLAT32", 1},
     {"DW_STRIDED", 1}, {"DW_TAPGROUPS", 1}, {"HALO_LATTICE", 1}, {"HALO_WINDOW", 1}, {"HALO_PAD", 1},
-    {"F32_PLANES", 1},
+    {"F32_PLANES", 1}, {"GATHER", 1},
 };
 static std::atomic<int> g_opt[OPT_COUNT];
 static std::once_flag g_opt_once;
@@ -113,6 +114,17 @@ static inline int opt(Opt which)
 {
     std::call_once(g_opt_once, init_opts);
     return g_opt[which].load(std::memory_order_relaxed);
+}
+
+// Whether a switch of the other kernels has been moved: then they are asked for, and layers stay with them.
+static bool kernels_are_asked_for()
+{
+    std::call_once(g_opt_once, init_opts);
+    for (int i = 0; i < OPT_COUNT; ++i) {
+        if (i == OPT_CONV_PROF || i == OPT_SM_BUDGET || i == OPT_NVTX || i == OPT_DW_LANES || i == OPT_F32_PLANES || i == OPT_GATHER) continue;
+        if (g_opt[i].load(std::memory_order_relaxed) != kOptDefs[i].dflt) return true;
+    }
+    return false;
 }
 
 bool dependent_launches() { return opt(OPT_SM_BUDGET) <= 0; }
@@ -274,6 +286,15 @@ int device_status_word(int** status)
     DeviceCtx* c;
     const int rc = get_ctx(&c);
     if (!rc) *status = c->status;
+    return rc;
+}
+
+// CTAs of one launch of the bf16-plane kernel under an SM budget (its CTAs fill an SM each), else 0.
+int planes_launch_slice(int* ctas)
+{
+    DeviceCtx* c;
+    const int rc = get_ctx(&c);
+    if (!rc) *ctas = sm_budget(c) < c->sm_count ? sm_budget(c) : 0;
     return rc;
 }
 
@@ -1877,58 +1898,328 @@ static int launch_dx_col2im(DeviceCtx* c, const AlphaConvShape* s, const float* 
 // finds that faster, as bf16 planes on the tensor cores at the same accuracy.  A launch of fewer CTAs than SMs whose reduction is long (a
 // classifier's 2762 x 53 layer: eight row tiles) is cut into up to 16 parts that are added in order; without scratch for them (stream
 // capture, a caller's small workspace) they run one after the other and add up in deltaX itself, which gives the same bits.
-static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream)
+
+// Whether the kernel of gemm_planes.cuh takes a layer: 32-bit offsets and, where rows know the taps they meet as bits, not too many.
+static bool planes_fit(const AlphaConvShape* s, int taps_h, int taps_w)
+{
+    const long long most = 1LL << 31, x = (long long)s->N * s->IH * s->IW, y = (long long)s->N * s->OH * s->OW;
+    return taps_h <= kPlaneTaps && taps_w <= kPlaneTaps && x * s->IC < most && y * s->OC < most && (long long)s->OC * s->FH * s->FW * s->IC < most;
+}
+
+static inline unsigned grid_slice(long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); }   // gridDim.y and .z limit
+
+// out = the parts in `part`, added in order (+ bias, + LeakyReLU).
+static int launch_part_sum(DeviceCtx* c, const float* part, size_t size, int parts, const float* bias, int cols, int act_on, float act_k, float* out,
+                           cudaStream_t stream)
+{
+    const size_t n4 = size / 4;
+    size_t blocks = (n4 + 255) / 256;
+    if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
+    if (!t_dry) launch_after(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(part), n4, parts, bias, cols / 4, act_on, act_k,
+                             reinterpret_cast<float4*>(out));
+    return check_launch("splitk_reduce_kernel");
+}
+
+static int planes_slice(const DeviceCtx* c) { return sm_budget(c) < c->sm_count ? sm_budget(c) : 0; }   // (see planes_launch_slice)
+
+// Tensor map over the three bf16 planes of a W that launch_split_planes has written.
+static int make_planes_map(CUtensorMap* m, const float* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box)
+{
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUresult r = g_encodeTiled(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<float*>(base), dims, strides_bytes, box, estr,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ALPHA_E_CUDA, "cuTensorMapEncodeTiled failed (%d), rank %d box0 %u", (int)r, rank, box[0]);
+    return ALPHA_OK;
+}
+static int launch_split_planes(DeviceCtx* c, const float* W, float* planes, int rows, int cols, int pitch, int OC, int taps, const SplitRows& map, cudaStream_t stream)
+{
+    size_t blocks = ((size_t)rows * (pitch / 4) + 255) / 256;
+    if (blocks > (size_t)c->sm_count * 16) blocks = (size_t)c->sm_count * 16;
+    if (!t_dry) launch_after(split_planes_kernel<0>, (unsigned)blocks, 256, 0, stream, W, reinterpret_cast<uint2*>(planes), rows, cols, (unsigned)pitch / 4, fast_div(pitch / 4),
+                             fast_div(OC), OC, taps, map);
+    note_launch("split_w");
+    return check_launch("split_planes_kernel");
+}
+
+// (`gather`: the layer is not fp32 work but runs here on the tensor cores, with this plan; 1 without scratch for its parts.)
+static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream, const PlanePlan* gather = nullptr)
 {
     const long long rows = (long long)s->N * ((s->IH + s->sh - 1) / s->sh) * ((s->IW + s->sw - 1) / s->sw);
     const int nsh = s->sh < s->IH ? s->sh : s->IH, nsw = s->sw < s->IW ? s->sw : s->IW;   // phases that own a pixel
     const long long phases = (long long)nsh * nsw;
-    const int sms = sm_budget(c);
-    const int Uy = (s->FH + s->sh - 1) / s->sh, Ux = (s->FW + s->sw - 1) / s->sw;   // most taps of a phase
+    const int taps_h = (s->FH + s->sh - 1) / s->sh, taps_w = (s->FW + s->sw - 1) / s->sw, taps = taps_h * taps_w;   // most of a phase
     const size_t size = (size_t)s->N * s->IH * s->IW * s->IC;
-    const ProductPlan plan = plan_product(rows, s->IC, Uy * Ux, s->OC, phases, true, (double)size, sms,
-                                          Uy <= DxProblem::kPlaneTaps && Ux <= DxProblem::kPlaneTaps ? option_f32_planes() : 0);
+    const long long w = (long long)s->FH * s->FW * s->OC * ((s->IC + 31) / 32 * 32);      // elements of a plane of W
+    const bool can_copy = s->FH * s->FW <= 64 && phases <= 16 && w < 1LL << 31;
+    const ProductPlan plan = gather ? ProductPlan{GemmTile{kPlaneBM, gather->bn, true}, gather->ksplit, gather->copy_b}
+                                    : plan_product(rows, s->IC, taps, s->OC, phases, true, (double)size, can_copy ? (double)w : 0.0,
+                                                   (long long)s->FH * s->FW * s->OC / phases, sm_budget(c), planes_fit(s, taps_h, taps_w) ? option_f32_planes() : 0);
     const GemmTile t = plan.tile;
     const long long gx = (rows + t.bm - 1) / t.bm, gy = (s->IC + t.bn - 1) / t.bn;
-    DxGemm<false> g{};
-    g.dY = dY; g.W = W; g.out = dX;
-    g.N = s->N; g.IH = s->IH; g.IW = s->IW; g.IC = s->IC; g.FH = s->FH; g.FW = s->FW; g.OH = s->OH; g.OW = s->OW; g.OC = s->OC;
-    g.sh = s->sh; g.sw = s->sw; g.ph = s->ph; g.pw = s->pw; g.nsw = nsw;
-    g.unit = t.planes ? kPlaneBK / kGemmBK : 1;
-    g.kt = (s->OC + kGemmBK * g.unit - 1) / (kGemmBK * g.unit) * g.unit;
-    g.by_kt = fast_div(g.kt);
-    g.size = size;
-    g.ksplit = g.parts = 1;
-    int turns = 1;
-    if (plan.ksplit > 1) {
+    int ksplit = plan.ksplit, parts = 1, turns = 1;
+    float* out = dX;
+    if (ksplit > 1) {
         float* ws = nullptr;
-        const int rc = get_workspace(c, stream, (size_t)plan.ksplit * g.size * sizeof(float), &ws);
+        const int rc = get_workspace(c, stream, (size_t)ksplit * size * sizeof(float), &ws);
         if (rc && !scratch_refused(rc)) return rc;
-        g.ksplit = plan.ksplit;
-        if (rc) turns = plan.ksplit;
-        else { g.parts = plan.ksplit; g.out = ws; }
+        if (rc && gather) return 1;
+        if (rc) turns = ksplit;
+        else { parts = ksplit; out = ws; }
     }
-    note_plan("gemm_f32 %s%dx%d phases=%lld ksplit=%d%s", t.planes ? "planes " : "", t.bm, t.bn, phases, g.ksplit, turns > 1 ? " in turns" : "");
-    const long long nz = phases * g.parts;
-    auto slice = [](long long from, long long n) { return (unsigned)(n - from < 65535 ? n - from : 65535); };   // gridDim.y and .z limit
-    for (int turn = 0; turn < turns; ++turn)
+    const char* label = gather ? "gather" : "simt";
+    if (gather) note_plan("gather 128x%d%s phases=%lld ksplit=%d time=%.0f", t.bn, plan.copy_b ? " copy" : "", phases, ksplit, gather->time);
+    else note_plan("gemm_f32 %s%dx%d%s phases=%lld ksplit=%d%s", t.planes ? "planes " : "", t.bm, t.bn, plan.copy_b ? " copy" : "", phases, ksplit, turns > 1 ? " in turns" : "");
+    const long long nz = phases * parts;
+    auto fill = [&](auto& g) {
+        g.dY = dY; g.W = W; g.out = out;
+        g.N = s->N; g.IH = s->IH; g.IW = s->IW; g.IC = s->IC; g.FH = s->FH; g.FW = s->FW; g.OH = s->OH; g.OW = s->OW; g.OC = s->OC;
+        g.sh = s->sh; g.sw = s->sw; g.ph = s->ph; g.pw = s->pw; g.nsw = nsw;
+        g.size = size; g.ksplit = ksplit; g.parts = parts;
+    };
+    DxGemm<false> f{};
+    PlaneDx<false> p{};
+    CUtensorMap tmB{};
+    const CUtensorMap* copy = nullptr;
+    if (t.planes) {
+        fill(p);
+        p.set_divisions();
+        float* ws = nullptr;
+        const int rc = plan.copy_b ? get_workspace(c, stream, (size_t)w * 6, &ws) : ALPHA_OK;
+        if (rc && (gather || !scratch_refused(rc))) return scratch_refused(rc) ? 1 : rc;
+        if (ws) {                                                            // (without scratch the kernel splits W itself: the same sums)
+            // the rows of W in the order in which the phases' steps meet them
+            SplitRows map{};
+            int j = 0;
+            for (int py = 0; py < nsh; ++py)
+                for (int px = 0; px < nsw; ++px) {
+                    p.row0[py * nsw + px] = j * s->OC;
+                    for (int fh = (py + s->ph) % s->sh; fh < s->FH; fh += s->sh)
+                        for (int fw = (px + s->pw) % s->sw; fw < s->FW; fw += s->sw) map.map[j++] = fh * s->FW + fw;
+                }
+            const int pitch = (s->IC + 31) / 32 * 32, wrows = j * s->OC;
+            int rc = ALPHA_OK;
+            if (wrows) rc = launch_split_planes(c, W, ws, wrows, s->IC, pitch, s->OC, s->FH * s->FW, map, stream);
+            const cuuint64_t dims[4] = {32, (cuuint64_t)(wrows ? wrows : 1), (cuuint64_t)pitch / 32, 3}, st[3] = {(cuuint64_t)pitch * 2, 64, (cuuint64_t)wrows * pitch * 2};
+            const cuuint32_t box[4] = {32, 32, (cuuint32_t)t.bn / 32, 3};
+            if (!rc && wrows) rc = make_planes_map(&tmB, ws, 4, dims, st, box);
+            if (rc) return rc;
+            if (wrows) copy = &tmB;
+        }
+    }
+    if (!t.planes) { fill(f); f.kt = (s->OC + kGemmBK - 1) / kGemmBK; f.by_kt = fast_div(f.kt); }
+    const int slice = planes_slice(c);
+    for (int turn = 0; turn < turns; ++turn) {
+        p.part0 = f.part0 = turn;
+        if (t.planes) {
+            const dim3 tiles((unsigned)gx, (unsigned)gy, (unsigned)nz);
+            if (t_dry) {}
+            else if (turn) launch_planes(PlaneDx<true>{p}, t.bn, tiles, slice, stream, c->status, copy);
+            else launch_planes(p, t.bn, tiles, slice, stream, c->status, copy);
+            note_launch(label);
+            continue;
+        }
         for (long long z0 = 0; z0 < nz; z0 += 65535)
             for (long long y0 = 0; y0 < gy; y0 += 65535) {
-                g.part0 = turn; g.y0 = (int)y0; g.z0 = (int)z0;
-                const dim3 grid((unsigned)gx, slice(y0, gy), slice(z0, nz));
+                const dim3 grid((unsigned)gx, grid_slice(y0, gy), grid_slice(z0, nz));
+                f.y0 = (int)y0; f.z0 = (int)z0;
                 if (t_dry) {}
-                else if (turn) launch_product(DxGemm<true>{g}, t, grid, stream, c->status);
-                else launch_product(g, t, grid, stream, c->status);
-                note_launch("simt");
+                else if (turn) launch_gemm_f32(DxGemm<true>{f}, t, grid, stream);
+                else launch_gemm_f32(f, t, grid, stream);
+                note_launch(label);
             }
+    }
     int rc = check_launch("gemm_f32_kernel");
-    if (rc || g.parts == 1) return rc;
-    const size_t n4 = g.size / 4;
-    size_t blocks = (n4 + 255) / 256;
-    if (blocks > (size_t)c->sm_count * 8) blocks = (size_t)c->sm_count * 8;
-    if (!t_dry) launch_after(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, reinterpret_cast<const float4*>(g.out), n4, g.parts, nullptr, 1, 0, 0.f,
-                                                               reinterpret_cast<float4*>(dX));
-    note_launch("simt");
-    return check_launch("splitk_reduce_kernel");
+    if (rc || parts == 1) return rc;
+    rc = launch_part_sum(c, out, size, parts, nullptr, 4, 0, 0.f, dX, stream);
+    note_launch(label);
+    return rc;
+}
+
+// ---- any layer: straight from its tensors on the bf16-plane kernel -----------------------------------
+//
+// One kernel (two or three launches with W split beforehand or the parts of a reduction added up) that gathers what it multiplies, against
+// the kernels of this file, which stage rectangular tiles: it loses to them on large layers whose images fill those tiles, and
+// wins on small layers (their launches), on images and channel counts that do not, on strides and on long reductions.  Its sums err by
+// 1.0e-7 to 1.8e-7 where theirs err by 1.2e-7 to 1.4e-5 (2-norm against 64 bits; no smaller in any of 1200 calls).
+
+// GPU time in us of an operator on those other kernels, as measured on 900 layers (1 to 512 images of 1 to 130 pixels a side, 4 to 7000
+// channels, 1x1 to 7x7, strides 1 and 2; 1e7 to 1.3e11 FLOPs): median error 15 to 20 %, and where the faster side is chosen by it and by
+// plan_planes (within 13 % for 9 of 10) a 3xTF32 forward takes 0.68 of the time before on average, a deltaX 0.75, a deltaW 0.73 (the better of both
+// would be 0.63, 0.71, 0.63), in plain TF32 0.93, 0.87, 0.80; one call in 40 more than 5 % longer, the worst 1.2 times.
+// `flops`: those of the layer with channels filled up to chunks and columns to 64, over the share of tile lanes that its images fill.
+// Matrix products (pictures and filters of one element): 48 products, 33 to 1024 rows, 256 to 4096 terms, within 15 %.
+enum class ConvOp { Forward, DeltaX, DeltaW };
+static bool matrix_product(const AlphaConvShape* s) { return s->IH == 1 && s->IW == 1 && s->FH == 1 && s->FW == 1 && s->OH == 1 && s->OW == 1; }
+static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
+{
+    auto up = [](int x, int to) { return (double)((x + to - 1) / to * to); };
+    const bool strided = s->sh > 1 || s->sw > 1, one = s->FH == 1 && s->FW == 1;
+    const double g = 2e-9 * s->N * s->OH * s->OW * s->OC * s->FH * s->FW * (double)s->IC, xy = 0.8e-6 * ((double)s->N * s->IH * s->IW * s->IC + (double)s->N * s->OH * s->OW * s->OC);
+    const double w = 4e-6 * s->FH * s->FW * (double)s->IC * s->OC, str = strided ? 1 : 0;
+    if (matrix_product(s)) {
+        // rows fold into pictures of 8 x n pixels (deltaW: 16 x n), or each row is a picture whose tile it leaves empty
+        if (op == ConvOp::DeltaW) return s->N % 16 == 0 ? (s->N <= 64 ? 12.0 : 15.0) + 5.6 * g : 20.0 + 130.0 * g;
+        const int red = op == ConvOp::Forward ? s->IC : s->OC;
+        return (op == ConvOp::Forward ? 16.0 + 5.7 * g : 18.0 + 6.2 * g) + (s->N % 8 == 0 && s->N >= 128 ? 0.0 : 0.046 * red);
+    }
+    if (op == ConvOp::DeltaW) {
+        const double f = g * (up(s->IC, 32) > 64 ? up(s->IC, 32) : 64.0) / s->IC * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
+        const double odd = s->IC % 32 ? f : 0, whole = s->IC % 32 || strided ? 0 : f;
+        return mode3x ? 18.0 + 4.85 * f - 3.24 * odd - 0.9 * whole - 0.52 * str * f + 0.98 * xy : 16.0 + 2.17 * f - 1.22 * odd - 0.66 * whole + 0.64 * xy + 1.85 * w + 1.4 * str;
+    }
+    const bool fwd = op == ConvOp::Forward;
+    const int red = fwd ? s->IC : s->OC, cols = fwd ? s->OC : s->IC;
+    const int h = fwd ? s->OH : (s->IH + s->sh - 1) / s->sh, wd = fwd ? s->OW : (s->IW + s->sw - 1) / s->sw;           // of one phase
+    const int fh = fwd ? (strided ? 2 : s->FH) : (s->FH + s->sh - 1) / s->sh, fw = fwd ? (strided ? 2 : s->FW) : (s->FW + s->sw - 1) / s->sw;
+    const bool tiny = fwd ? s->OH * s->OW <= 16 : s->IH * s->IW <= 16;
+    const bool pair = mode3x && !strided && !one && cols % 128 == 0 && red % 32 == 0 && !tiny;
+    double lanes = 1.0;
+    if (!(fwd ? (one && !strided) || tiny : one || tiny)) {
+        lanes = tile_idle(h, wd, fh);
+        const double flat = up(h, 4) * 32.0 / ((double)h * wd);
+        if (pair && wd + fw - 1 <= 32 && h > 16 && flat < lanes) lanes = flat;
+    }
+    const double f = g * up(red, 32) / red * (up(cols, 16) > 64 ? up(cols, 16) : 64.0) / cols * lanes;
+    const double odd = red % 32 ? f : 0, whole = red % 32 || strided ? 0 : f, pr = pair ? f : 0;
+    if (fwd)
+        return mode3x ? 14.7 + 6.83 * f - 3.31 * odd - 2.06 * whole - 1.19 * pr - 2.17 * str * f + 0.42 * xy + 1.9 * w + 1.7 * str
+                      : 13.1 + 1.71 * f - 0.53 * whole - 0.49 * str * f + 0.65 * xy + 0.63 * w + 3.1 * str;
+    return mode3x ? 14.1 + 2.55 * f + 1.53 * odd + 1.63 * whole - 0.81 * pr - 0.61 * str * f + 1.15 * xy + 1.8 * w + 4.1 * str
+                  : 13.8 + 0.89 * f + 0.59 * odd + 0.34 * whole + 0.77 * xy + 2.79 * w + 3.5 * str;
+}
+// Which layers may leave those kernels, in 3xTF32 (plain TF32 products are TF32 products); gather_pays decides by the plan.
+// Their tiles are rectangles of pixels and chunks of 32 channels.  Layers that fill both stay: of 130 of them those kernels were faster on
+// two thirds, by up to 2.6 times.  So do layers of under 16 channels, whose taps of a filter row they read as one window, and products of
+// under 96 rows, which leave a quarter of the 128 here empty.  Ragged channel counts may leave, and whole chunks where an image covers at
+// most two thirds of its tiles' lanes (strided forward: images of up to 16 pixels, the im2col kernel packs all others; deltaW: rows of up to 5).
+// Whole chunks and deltaX besides only from 24 us on: below, both sides are launches, and the estimates no finer than what they differ by.
+// Matrix products may leave too, from 16 terms on: 250 x 1024 times 1024 x 1024 59 -> 17 us, its deltaW 87 -> 14; 512 rows 26 -> 19 and 24 -> 18.
+// Before and after: 512 x 8x8 x 128, 3x3 forward 91 -> 54 us; 64 x 4x4 x 256 31 -> 22; deltaW of 256 x 8x8, 256 -> 512, 4x4 s2 173 -> 106.
+static bool gather_suits(const AlphaConvShape* s, ConvOp op)
+{
+    if (matrix_product(s)) return op == ConvOp::DeltaX ? s->OC >= 16 : s->IC >= 16 && (s->IC % 32 == 0 || patch_path_ok(s));
+    const bool strided = s->sh > 1 || s->sw > 1, filter = s->FH > 1 || s->FW > 1, heavy = other_kernels_time(s, op, 1) >= 24.0;
+    if (op == ConvOp::DeltaX) {
+        const int h = (s->IH + s->sh - 1) / s->sh, w = (s->IW + s->sw - 1) / s->sw;        // of one phase
+        return (long long)s->N * h * w >= 96 && heavy && (s->OC % 32 != 0 || (filter && tile_idle(h, w, (s->FH + s->sh - 1) / s->sh) >= 1.5));
+    }
+    if (s->IC < 16 || (s->IC % 32 != 0 && !patch_path_ok(s))) return false;                // (the latter is fp32 work, labelled so)
+    if (op == ConvOp::DeltaW) return s->IC % 32 != 0 || ((s->OW + 7) / 8 * 8 * 2 >= 3 * s->OW && heavy);
+    if ((long long)s->N * s->OH * s->OW < 96) return false;
+    return s->IC % 32 != 0 || (filter && heavy && (strided ? tiny_image(s->OH, s->OW) : tile_idle(s->OH, s->OW, s->FH) >= 1.5));
+}
+// 1: the layer leaves the other kernels if its plan pays, 2: whatever its plan says, 0: it stays.
+static int gather_mode(const AlphaConvShape* s, ConvOp op)
+{
+    const int mode = opt(OPT_GATHER);
+    if (!mode || cur_algo() != ALPHA_ALGO_AUTO) return 0;
+    if (mode == 2) return 2;
+    return cur_mode3x() && !kernels_are_asked_for() && gather_suits(s, op) ? 1 : 0;
+}
+static bool gather_pays(const AlphaConvShape* s, ConvOp op, double time) { return time < 0.97 * other_kernels_time(s, op, 1); }
+
+// Returns 1 where the layer is left to the other routes.
+
+// (`f32`: a layer that would otherwise run one thread per element.)
+static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* W, const float* bias, float* Y, int act_on, float act_k,
+                                 cudaStream_t stream, bool f32 = false)
+{
+    const int mode = f32 ? option_f32_planes() : gather_mode(s, ConvOp::Forward);
+    if (!mode || !planes_fit(s, s->FH, s->FW)) return 1;
+    PlaneFwd p{};
+    p.X = X; p.W = W;
+    p.N = s->N; p.IH = s->IH; p.IW = s->IW; p.IC = s->IC; p.FH = s->FH; p.FW = s->FW; p.OH = s->OH; p.OW = s->OW; p.OC = s->OC;
+    p.sh = s->sh; p.sw = s->sw; p.ph = s->ph; p.pw = s->pw;
+    p.K = s->FH * s->FW * s->IC; p.rows = s->N * s->OH * s->OW;
+    p.size = (size_t)p.rows * s->OC;
+    const int Kp = (p.K + 31) / 32 * 32;
+    const PlanePlan plan = plan_planes(p.rows, s->OC, p.K, 1, true, (double)p.size, (double)Kp * s->OC, c->sm_count);
+    const long long gx = (p.rows + kPlaneBM - 1) / kPlaneBM, gy = (s->OC + plan.bn - 1) / plan.bn;
+    if (gx * gy * plan.ksplit > 2147483647LL) return 1;
+    if (mode == 1 && !f32 && !gather_pays(s, ConvOp::Forward, plan.time)) return 1;
+    const WsMark start = ws_mark(c, stream);
+    p.ksplit = plan.ksplit;
+    p.out = Y;
+    if (p.ksplit > 1) {
+        const int rc = get_workspace(c, stream, (size_t)p.ksplit * p.size * sizeof(float), &p.out);
+        if (rc) return scratch_refused(rc) ? 1 : rc;
+    } else {
+        p.bias = bias; p.act_on = act_on; p.act_k = act_k;
+    }
+    p.by_OW = fast_div(s->OW); p.by_OHW = fast_div(s->OH * s->OW); p.by_IC = fast_div(s->IC); p.by_FW = fast_div(s->FW);
+    int rc = ALPHA_OK;
+    CUtensorMap tmB{};
+    if (plan.copy_b) {
+        float* ws = nullptr;
+        rc = get_workspace(c, stream, (size_t)Kp * s->OC * 6, &ws);
+        if (rc && scratch_refused(rc)) {
+            ws_rewind(c, stream, start);
+            return 1;
+        }
+        if (rc) return rc;
+        rc = launch_split_planes(c, W, ws, s->OC, p.K, Kp, 1, 0, SplitRows{}, stream);
+        const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)s->OC, 3}, st[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * 2 * s->OC};
+        const cuuint32_t box[3] = {32, (cuuint32_t)plan.bn, 3};
+        if (!rc) rc = make_planes_map(&tmB, ws, 3, dims, st, box);
+        if (rc) return rc;
+    }
+    const char* label = f32 ? "simt" : "gather";
+    note_plan("%s 128x%d%s ksplit=%d time=%.0f", f32 ? "gemm_f32 planes" : "gather", plan.bn, plan.copy_b ? " copy" : "", p.ksplit, plan.time);
+    if (!t_dry) launch_planes(p, plan.bn, dim3((unsigned)gx, (unsigned)gy, (unsigned)p.ksplit), planes_slice(c), stream, c->status, plan.copy_b ? &tmB : nullptr);
+    note_launch(label);
+    rc = check_launch("gemm_planes_kernel");
+    if (rc || p.ksplit == 1) return rc;
+    rc = launch_part_sum(c, p.out, p.size, p.ksplit, bias, s->OC, act_on, act_k, Y, stream);
+    note_launch(label);
+    return rc;
+}
+
+static int launch_gather_dx(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream)
+{
+    const int mode = gather_mode(s, ConvOp::DeltaX);
+    const int nsh = s->sh < s->IH ? s->sh : s->IH, nsw = s->sw < s->IW ? s->sw : s->IW;
+    if (!mode || !planes_fit(s, (s->FH + s->sh - 1) / s->sh, (s->FW + s->sw - 1) / s->sw)) return 1;
+    const long long rows = (long long)s->N * ((s->IH + s->sh - 1) / s->sh) * ((s->IW + s->sw - 1) / s->sw), phases = (long long)nsh * nsw;
+    const long long w = (long long)s->FH * s->FW * s->OC * ((s->IC + 31) / 32 * 32);
+    const bool can_copy = s->FH * s->FW <= 64 && phases <= 16 && w < 1LL << 31;
+    const long long k = (long long)s->FH * s->FW * s->OC / phases;
+    const PlanePlan plan = plan_planes(rows, s->IC, k > 0 ? k : 1, phases, true, (double)s->N * s->IH * s->IW * s->IC, can_copy ? (double)w : 0.0, c->sm_count);
+    if ((rows + kPlaneBM - 1) / kPlaneBM * ((s->IC + plan.bn - 1) / plan.bn) * phases * plan.ksplit > 2147483647LL) return 1;
+    // (the phase of the most taps ends last: the plan counts with the average)
+    const double last = ((double)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * s->OC - k) / plan.ksplit / kPlaneBK * (plan.copy_b ? 0.57 : 0.80);
+    if (mode == 1 && !gather_pays(s, ConvOp::DeltaX, plan.time + last)) return 1;
+    return launch_dx_f32(c, s, dY, W, dX, stream, &plan);
+}
+
+static int launch_gather_dw(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* dY, float* dW, cudaStream_t stream, bool f32 = false)
+{
+    const int mode = f32 ? option_f32_planes() : gather_mode(s, ConvOp::DeltaW);
+    if (!mode || !planes_fit(s, 1, 1)) return 1;
+    PlaneDw p{};
+    p.dY = dY; p.X = X;
+    p.IH = s->IH; p.IW = s->IW; p.IC = s->IC; p.FW = s->FW; p.OC = s->OC; p.sh = s->sh; p.sw = s->sw; p.ph = s->ph; p.pw = s->pw;
+    p.K = s->N * s->OH * s->OW; p.L = s->FH * s->FW * s->IC;
+    p.size = (size_t)s->OC * p.L;
+    const PlanePlan plan = plan_planes(s->OC, p.L, p.K, 1, true, (double)p.size, 0, c->sm_count);
+    const long long gx = (s->OC + kPlaneBM - 1) / kPlaneBM, gy = (p.L + plan.bn - 1) / plan.bn;
+    if (gx * gy * plan.ksplit > 2147483647LL) return 1;
+    if (mode == 1 && !f32 && !gather_pays(s, ConvOp::DeltaW, plan.time)) return 1;
+    p.ksplit = plan.ksplit;
+    p.out = dW;
+    if (p.ksplit > 1) {
+        const int rc = get_workspace(c, stream, (size_t)p.ksplit * p.size * sizeof(float), &p.out);
+        if (rc) return scratch_refused(rc) ? 1 : rc;
+    }
+    p.by_OW = fast_div(s->OW); p.by_OHW = fast_div(s->OH * s->OW); p.by_IC = fast_div(s->IC); p.by_FW = fast_div(s->FW);
+    const char* label = f32 ? "simt" : "gather";
+    note_plan("%s 128x%d ksplit=%d time=%.0f", f32 ? "gemm_f32 planes" : "gather", plan.bn, p.ksplit, plan.time);
+    if (!t_dry) launch_planes(p, plan.bn, dim3((unsigned)gx, (unsigned)gy, (unsigned)p.ksplit), planes_slice(c), stream, c->status);
+    note_launch(label);
+    int rc = check_launch("gemm_planes_kernel");
+    if (rc || p.ksplit == 1) return rc;
+    rc = launch_part_sum(c, p.out, p.size, p.ksplit, nullptr, 4, 0, 0.f, dW, stream);
+    note_launch(label);
+    return rc;
 }
 
 // ---- deltaW, halo-tile kernel (strides 1 and 2): plan and launch -----------------------------------
@@ -2910,7 +3201,8 @@ int alpha_conv3d_forward_leakyRelu(const AlphaConvShape* s, const float* X, cons
 static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* W, const float* bias,
                           float* Y, cudaStream_t stream, int algo, int act_on, float act_k)
 {
-    int rc;
+    int rc = launch_gather_forward(c, s, X, W, bias, Y, act_on, act_k, stream);
+    if (rc != 1) return rc;
     const bool tensor_ok = pick_kc(s->IC) != 0 && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256;
     if (algo == ALPHA_ALGO_TENSOR && !tensor_ok)
         return fail(ALPHA_E_ARG, "tensor path needs IC %% 8 == 0 (IC=%d)", s->IC);
@@ -2983,6 +3275,8 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
         rc = launch_patch_gemm(c, pl, cur_mode3x(), stream);
         if (rc != 1) return rc;
     }
+    rc = launch_gather_forward(c, s, X, W, bias, Y, act_on, act_k, stream, true);
+    if (rc != 1) return rc;
     const size_t total = (size_t)s->N * s->OH * s->OW * s->OC;
     if (!t_dry) conv_fwd_simt<<<simt_grid(total, c->sm_count), 256, 0, stream>>>(X, W, bias, Y, to_dev_shape(s), act_on, act_k);
     note_launch("simt");
@@ -3003,6 +3297,13 @@ int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const floa
     cudaStream_t stream = (cudaStream_t)stream_;
     ws_begin(c, stream);
     const int algo = cur_algo();
+    // (what is fp32 work anyway chooses its kernel in launch_dx_f32)
+    if (s->sh == 1 && s->sw == 1 ? s->OC % 8 == 0 : s->OC % 32 == 0) {
+        const WsMark start = ws_mark(c, stream);
+        rc = launch_gather_dx(c, s, deltaY, W, deltaX, stream);
+        if (rc != 1) return rc;
+        ws_rewind(c, stream, start);
+    }
     const int pad_h = s->FH - 1 - s->ph, pad_w = s->FW - 1 - s->pw;
     const bool tensor_ok = s->sh == 1 && s->sw == 1 && pick_kc(s->OC) != 0 && pad_h >= 0 && pad_w >= 0 &&
                            pad_h < 128 && pad_w < 128 && s->IH == s->OH + s->FH - 1 - 2 * s->ph &&
@@ -3079,6 +3380,8 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
     cudaStream_t stream = (cudaStream_t)stream_;
     ws_begin(c, stream);
     const int algo = cur_algo();
+    rc = launch_gather_dw(c, s, X, deltaY, deltaW, stream);
+    if (rc != 1) return rc;
     const bool tensor_ok = (s->IC % 32 == 0) && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256;
     if (algo == ALPHA_ALGO_TENSOR && !tensor_ok)
         return fail(ALPHA_E_ARG, "tensor deltaW path needs IC %% 32 == 0 (IC=%d)", s->IC);
@@ -3121,6 +3424,8 @@ int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* de
         }
     }
     if (algo == ALPHA_ALGO_SIMT || !tensor_ok) {
+        rc = launch_gather_dw(c, s, X, deltaY, deltaW, stream, true);
+        if (rc != 1) return rc;
         const size_t total = (size_t)s->OC * s->FH * s->FW * s->IC;
         if (!t_dry) conv_dw_simt<<<(unsigned)total, 128, 0, stream>>>(X, deltaY, deltaW, to_dev_shape(s));
         note_launch("simt");
@@ -3259,12 +3564,15 @@ int alpha_conv3d_deltaW_bias(const AlphaConvShape* s, const float* X, const floa
     rc = get_ctx(&c);
     if (rc) return rc;
     cudaStream_t stream = (cudaStream_t)stream_;
+    ws_begin(c, stream);
+    rc = launch_gather_dw(c, s, X, deltaY, deltaW, stream);
+    if (rc == 0) return alpha_conv_bias_grad(deltaY, (long long)s->N * s->OH * s->OW, s->OC, deltaB, stream_);
+    if (rc < 0) return rc;
     // the halo-tile kernel (stride 1, IC % 32 == 0, images larger than 3 x 3) sums the columns of the deltaY
     // tiles it stages anyway; every other shape runs the two passes one after the other
     const bool tensor_ok = (s->IC % 32 == 0) && s->ph < 128 && s->pw < 128 && s->FH <= 256 && s->FW <= 256;
     const bool patch = patch_path_ok(s) && env_tile_mode() != 1 && (!tensor_ok || (s->OH * s->OW <= 9 && (s->FH > 1 || s->FW > 1)));
     if (cur_algo() != ALPHA_ALGO_SIMT && tensor_ok && !patch) {
-        ws_begin(c, stream);
         bool fused = false;
         rc = launch_dw_halo(c, s, X, deltaY, deltaW, cur_mode3x(), stream, deltaB, &fused);
         if (rc < 0) return rc;

@@ -10,11 +10,12 @@ struct FastDiv {
     unsigned long long m;
     unsigned d;
     int s;
-    __host__ __device__ unsigned div(unsigned x) const { return static_cast<unsigned>((static_cast<unsigned long long>(x) * m) >> s); }
+    // (m < 2^32: a 32 x 32 multiplication)
+    __host__ __device__ unsigned div(unsigned x) const { return static_cast<unsigned>((static_cast<unsigned long long>(x) * static_cast<unsigned>(m)) >> s); }
     __host__ __device__ void divmod(unsigned x, unsigned& q, unsigned& r) const { q = div(x); r = x - q * d; }
 };
 
-inline FastDiv fast_div(int d_)
+__host__ __device__ inline FastDiv fast_div(int d_)
 {
     const unsigned d = static_cast<unsigned>(d_);
     int b = 0;

@@ -25,7 +25,6 @@
 #pragma once
 #include "dependent_launch.cuh"
 #include "fast_div.cuh"
-#include <stdint.h>
 #include <type_traits>
 
 namespace alpha {
@@ -63,44 +62,22 @@ __device__ __forceinline__ void put_word(float* tile, int w, const float4& v)
     }
 }
 
-// The 16-byte word at p, zeros without `use`: one predicated load, so that a thread's loads leave back to back (behind a branch the
-// compiler moves each result to its place before the next load: 240 clocks a word).
-__device__ __forceinline__ float4 load_word(const float* p, bool use)
-{
-    float4 v;
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
-        "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
-        "@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-        : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(p), "r"(static_cast<uint32_t>(use)));
-    return v;
-}
-
-// Barriers among the 256 threads that form a tile (the CTA may have more).
-__device__ __forceinline__ void tile_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-__device__ __forceinline__ bool tile_any(bool x)
-{
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r) : "r"(static_cast<uint32_t>(x)) : "memory");
-    return r != 0;
-}
-
-// Shared memory of a tile.
-template <int BM, int BN, class P>
-struct __align__(16) GemmShared {
-    float As[2][kGemmBK * BM], Bs[2][kGemmBK * BN];
-    bool met[2][P::kSkip ? BM : 1];
-};
-
-// The tile of CTA state c, formed and stored by 256 threads.
 template <int BM, int BN, int TM, int TN, class P>
-__device__ __forceinline__ void gemm_f32_tile(const P& p, const typename P::Cta& c, GemmShared<BM, BN, P>& sh)
+__global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
 {
     static_assert((BM / TM) * (BN / TN) == kGemmThreads && TN % 4 == 0 && TM % 4 == 0 && BM >= 32 && BN >= 32, "tile shape");
     constexpr int WA = BM * 4, WB = BN * 4;                       // 16-byte words of a tile
     constexpr int NA = WA / kGemmThreads, NB = (WB + kGemmThreads - 1) / kGemmThreads;
     static_assert(WA % kGemmThreads == 0, "A words");
+    __shared__ __align__(16) float As[2][kGemmBK * BM];
+    __shared__ __align__(16) float Bs[2][kGemmBK * BN];
+    __shared__ bool met[2][P::kSkip ? BM : 1];
     const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
+
+    grid_dependency_wait();
+    grid_dependency_trigger();
+    typename P::Cta c;
+    if (!p.cta(c, BM, BN)) return;                                // uniform for the CTA
     typename P::RowA ra[NA];
 #pragma unroll
     for (int i = 0; i < NA; ++i) ra[i] = p.row_a(c, word_col<BM, P::kAk>(tid + i * kGemmThreads));
@@ -129,18 +106,18 @@ __device__ __forceinline__ void gemm_f32_tile(const P& p, const typename P::Cta&
         auto stage = [&](int buf) {
 #pragma unroll
             for (int i = 0; i < NA; ++i) {
-                put_word<BM, P::kAk>(sh.As[buf], tid + i * kGemmThreads, va[i]);
-                if constexpr (by_row) sh.met[buf][word_col<BM, P::kAk>(tid + i * kGemmThreads)] = vm[i];   // (words of a row agree)
+                put_word<BM, P::kAk>(As[buf], tid + i * kGemmThreads, va[i]);
+                if constexpr (by_row) met[buf][word_col<BM, P::kAk>(tid + i * kGemmThreads)] = vm[i];   // (words of a row agree)
             }
 #pragma unroll
             for (int i = 0; i < NB; ++i)
-                if (WB % kGemmThreads == 0 || tid + i * kGemmThreads < WB) put_word<BN, P::kBk>(sh.Bs[buf], tid + i * kGemmThreads, vb[i]);
+                if (WB % kGemmThreads == 0 || tid + i * kGemmThreads < WB) put_word<BN, P::kBk>(Bs[buf], tid + i * kGemmThreads, vb[i]);
         };
         if (c.it0 < c.it1) {
             fetch(c.it0);
             stage(0);
         }
-        tile_sync();
+        __syncthreads();
         int buf = 0;
         for (int it = c.it0; it < c.it1; ++it) {
             if (it + 1 < c.it1) fetch(it + 1);
@@ -151,26 +128,26 @@ __device__ __forceinline__ void gemm_f32_tile(const P& p, const typename P::Cta&
                 unsigned long long b[TN / 2];
 #pragma unroll
                 for (int y = 0; y < TM; y += 4) {
-                    const float4 t = *reinterpret_cast<const float4*>(&sh.As[buf][k * BM + ((ty * TM + y) ^ x8)]);
+                    const float4 t = *reinterpret_cast<const float4*>(&As[buf][k * BM + ((ty * TM + y) ^ x8)]);
                     a[y] = t.x; a[y + 1] = t.y; a[y + 2] = t.z; a[y + 3] = t.w;
                 }
                 // columns tx * 4 ... of each group of BN / (TN / 4) columns
 #pragma unroll
                 for (int x = 0; x < TN; x += 4) {
-                    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&sh.Bs[buf][k * BN + (((x / 4) * (BN * 4 / TN) + tx * 4) ^ x8)]);
+                    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k * BN + (((x / 4) * (BN * 4 / TN) + tx * 4) ^ x8)]);
                     b[x / 2] = t.x; b[x / 2 + 1] = t.y;
                 }
 #pragma unroll
                 for (int y = 0; y < TM; ++y) {
                     if constexpr (by_row)
-                        if (!sh.met[buf][ty * TM + y]) continue;
+                        if (!met[buf][ty * TM + y]) continue;
                     const unsigned long long aa = pack2(a[y], a[y]);
 #pragma unroll
                     for (int x = 0; x < TN / 2; ++x) ffma2(acc[y][x], aa, b[x]);
                 }
             }
             if (it + 1 < c.it1) stage(buf ^ 1);   // the other buffer was last read before the previous barrier
-            tile_sync();
+            __syncthreads();
             buf ^= 1;
         }
     };
@@ -185,7 +162,7 @@ __device__ __forceinline__ void gemm_f32_tile(const P& p, const typename P::Cta&
                 unpack2(acc[y][x], u, v);
                 nan = nan || u != u || v != v;
             }
-        if (tile_any(nan)) form_sums(std::true_type{});
+        if (__syncthreads_or(nan)) form_sums(std::true_type{});
     }
 #pragma unroll
     for (int y = 0; y < TM; ++y) {
@@ -200,17 +177,6 @@ __device__ __forceinline__ void gemm_f32_tile(const P& p, const typename P::Cta&
     }
 }
 
-template <int BM, int BN, int TM, int TN, class P>
-__global__ void __launch_bounds__(kGemmThreads, 2) gemm_f32_kernel(const P p)
-{
-    __shared__ GemmShared<BM, BN, P> sh;
-    grid_dependency_wait();
-    grid_dependency_trigger();
-    typename P::Cta c;
-    if (!p.cta(c, BM, BN)) return;                                // uniform for the CTA
-    gemm_f32_tile<BM, BN, TM, TN>(p, c, sh);
-}
-
 // deltaX of any stride as an implicit GEMM: rows = the pixels of one stride phase (py, px), which all receive the same filter
 // taps, columns = input channels, reduction = those taps x output channels (tap-major), in ksplit parts.  A launch computes `parts` of
 // them from part0 on, blockIdx.z = phase * parts + part, each into its own copy of deltaX (out + part * size), every element of which
@@ -221,8 +187,8 @@ struct DxProblem {
     const float* dY; const float* W; float* out;
     int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw;
     int nsw;                       // phases along a row: min(sw, IW)
-    int ksplit, parts, part0, unit; // a part is a whole number of `unit` 16-step tiles
-    int kt, y0, z0;                // kt = 16-step tiles per tap, a multiple of `unit`; y0 = column tile of blockIdx.y == 0, z0 = phase * parts + part of blockIdx.z == 0
+    int ksplit, parts, part0;
+    int kt, y0, z0;                // kt = 16-step tiles per tap; y0 = column tile of blockIdx.y == 0, z0 = phase * parts + part of blockIdx.z == 0
     size_t size;                   // elements of deltaX
     FastDiv by_kt;
     struct Cta { int m0, n0, rows, it0, it1, A, B, py, px, ry, rx, qy, qx, Ux; float* out; };
@@ -242,7 +208,7 @@ struct DxProblem {
         c.qy = (c.py + ph - c.ry) / sh; c.qx = (c.px + pw - c.rx) / sw;
         const int Uy = c.ry < FH ? (FH - c.ry + sh - 1) / sh : 0;
         c.Ux = c.rx < FW ? (FW - c.rx + sw - 1) / sw : 0;
-        const int its = Uy * c.Ux * kt, per = (its / unit + ksplit - 1) / ksplit * unit;
+        const int its = Uy * c.Ux * kt, per = (its + ksplit - 1) / ksplit;
         c.it0 = sp * per < its ? sp * per : its;
         c.it1 = c.it0 + per < its ? c.it0 + per : its;
         c.out = out + static_cast<size_t>(copy) * size;
@@ -280,60 +246,6 @@ struct DxProblem {
         const int oc = s.k0 + k, ic = c.n0 + col;
         if (oc >= OC || ic >= IC) return make_float4(0.f, 0.f, 0.f, 0.f);
         return __ldg(reinterpret_cast<const float4*>(W + ((static_cast<size_t>(oc) * FH + s.fh) * FW + s.fw) * IC + ic));
-    }
-    // The same in stages of 32 steps of one tap (gemm_planes.cuh)
-    static constexpr bool kTail = false;  // words may reach past the last step: never, OC is a multiple of 4
-    struct Cursor { int u, v, k0, a_off, b_off; };   // tap, first output channel; the tap's distance in pixels of deltaY / rows of W
-    struct PlaneRow { int pix; unsigned met; };      // pixel of deltaY that tap (0, 0) meets; bit u: it meets rows of tap u, 16 + v: columns
-    static constexpr int kPlaneTaps = 16;            // most taps of a phase along each axis
-    __device__ void plane_at(Cursor& s) const
-    {
-        s.a_off = s.u * OW + s.v;
-        s.b_off = s.u * (sh * FW) + s.v * sw;
-    }
-    __device__ Cursor plane_begin(const Cta& c) const
-    {
-        const Step st = step(c, c.it0);
-        Cursor s{st.u, st.v, st.k0, 0, 0};
-        plane_at(s);
-        return s;
-    }
-    __device__ void plane_next(const Cta& c, Cursor& s) const
-    {
-        s.k0 += 32;
-        if (s.k0 < OC) return;
-        s.k0 = 0;
-        if (++s.v == c.Ux) { s.v = 0; ++s.u; }
-        plane_at(s);
-    }
-    __device__ int plane_left(const Cursor& s) const { return OC - s.k0; }
-    __device__ PlaneRow plane_row(const Cta& c, int m) const
-    {
-        const RowA r = row_a(c, m);
-        if (r.n < 0) return PlaneRow{0, 0u};
-        const int y = r.a + c.qy, x = r.b + c.qx;
-        unsigned met = 0;
-        for (int t = 0; t < kPlaneTaps; ++t) {
-            if (static_cast<unsigned>(y - t) < static_cast<unsigned>(OH)) met |= 1u << t;
-            if (static_cast<unsigned>(x - t) < static_cast<unsigned>(OW)) met |= 0x10000u << t;
-        }
-        return PlaneRow{(r.n * OH + y) * OW + x, met};
-    }
-    __device__ const float* plane_a_base(const Cta&, int, int k) const { return dY + k; }
-    __device__ bool plane_a_in(const Cta&, int) const { return true; }      // (rows past the last one meet no tap)
-    __device__ bool plane_b_in(const Cta& c, int col) const { return c.n0 + col < IC; }
-    __device__ float4 plane_a(const Cursor& s, const float* base, const PlaneRow& r, int, bool, int k, int) const
-    {
-        const bool use = (r.met >> s.u & r.met >> (16 + s.v) & 1u) && s.k0 + k < OC;
-        return load_word(base + s.k0 + static_cast<long long>(r.pix - s.a_off) * OC, use);
-    }
-    __device__ const float* plane_b_base(const Cta& c, int col, int k) const
-    {
-        return W + (static_cast<size_t>(k) * (FH * FW) + c.ry * FW + c.rx) * IC + c.n0 + col;
-    }
-    __device__ float4 plane_b(const Cursor& s, const float* base, int i, bool in, int k, int dk) const
-    {
-        return load_word(base + static_cast<long long>((s.k0 + i * dk) * (FH * FW) + s.b_off) * IC, in && s.k0 + k < OC);
     }
     __device__ RowC row_c(const Cta& c, int m) const
     {
@@ -456,30 +368,6 @@ struct BatchGemm {
     __device__ float4 load_b(const Cta& c, const Step& s, int n, int k) const
     {
         return B_KC ? word(c.B, ldb, c.n0 + n, M, s.k0 + k, K) : word(c.B, ldb, s.k0 + k, K, c.n0 + n, M);
-    }
-    // The same in stages of 32 steps; what words hold past K is left to the caller (kTail).  `base`: a thread's first word at step 0; its i-th lies 32 i rows (along k) or i * dk steps further.
-    static constexpr bool kTail = true;
-    struct Cursor { int k0; };
-    struct PlaneRow {};
-    __device__ Cursor plane_begin(const Cta&) const { return Cursor{0}; }
-    __device__ void plane_next(const Cta&, Cursor& s) const { s.k0 += 32; }
-    __device__ int plane_left(const Cursor& s) const { return K - s.k0; }
-    __device__ PlaneRow plane_row(const Cta&, int) const { return PlaneRow{}; }
-    __device__ static const float* plane_base(const float* base, int ld, bool kc, int x, int k)
-    {
-        return kc ? base + static_cast<size_t>(x) * ld + k : base + static_cast<size_t>(k) * ld + x;
-    }
-    __device__ const float* plane_a_base(const Cta& c, int m, int k) const { return plane_base(c.A, lda, A_KC, c.m0 + m, k); }
-    __device__ const float* plane_b_base(const Cta& c, int col, int k) const { return plane_base(c.B, ldb, B_KC, c.n0 + col, k); }
-    __device__ bool plane_a_in(const Cta& c, int m) const { return c.m0 + m < N; }
-    __device__ bool plane_b_in(const Cta& c, int col) const { return c.n0 + col < M; }
-    __device__ float4 plane_a(const Cursor& s, const float* base, const PlaneRow&, int i, bool in, int k, int dk) const
-    {
-        return load_word(base + (A_KC ? s.k0 + static_cast<long long>(32 * i) * lda : static_cast<long long>(s.k0 + i * dk) * lda), in && s.k0 + k < K);
-    }
-    __device__ float4 plane_b(const Cursor& s, const float* base, int i, bool in, int k, int dk) const
-    {
-        return load_word(base + (B_KC ? s.k0 + static_cast<long long>(32 * i) * ldb : static_cast<long long>(s.k0 + i * dk) * ldb), in && s.k0 + k < K);
     }
     __device__ RowC row_c(const Cta& c, int m) const { return RowC{c.m0 + m < N ? c.C + static_cast<size_t>(c.m0 + m) * ldc : nullptr}; }
     __device__ void store(const Cta& c, const RowC& r, int col, const float4& o) const

@@ -1,18 +1,19 @@
-// The products of gemm_f32.cuh on the tensor cores, at fp32 accuracy.
+// Products on the tensor cores at fp32 accuracy, gathering both operands from the tensors as they lie.
 //
 // An fp32 word is the exact sum of three bf16 words, x = h + m + l (the upper 16 bits, the upper 16 bits of what is left, the rest: 8
 // bits of significand each), and of the nine products of two such sums the six that matter are formed by tcgen05.mma kind::f16:
 // hh in one accumulator; hm, mh, mm, hl, lh, all below 2^-7 of it, in another.  What is dropped (ml, lm, ll) is below 2^-23 of a product.
 // The tensor core truncates as it adds to an accumulator, about 2^-24 of it an instruction, which over a long sum would cost more
 // than fp32 FMAs do: after every 64 reduction steps (four instructions into the hh accumulator) the partial sum is added to running
-// sums in registers, rounded to nearest, and the accumulator starts anew.  The errors are given at plan_product.
+// sums in registers, rounded to nearest, and the accumulator starts anew.  Sums of 4 to
+// 20000 products err by 1.0e-7 to 1.8e-7 (2-norm against 64 bits), those of the FMA kernels by 1.2e-7 to 3e-6.
 //
-// Bound: 388 clocks of MMAs per 16 steps of a 128 x 128 tile, as much as the 3xTF32 kernels issue per step, against which shared
-// memory takes 96 KB of plane stores and operand reads per 32 steps (40 KB a step in MMAs of 256, 256, 128 and 128 columns; six of 128 would
-// read 48).  2048 x 2048 x 2052: 127 TFLOP/s, some 1900 clocks for the 776 of MMAs a stage; the issuing thread's share of the issue slots and
-// the stores of 16 warps in the MMAs' way are what is left (measured with clocks around every MMA).
+// Bound: 388 clocks of MMAs per 16 steps of a 128 x 128 tile, as much as the 3xTF32 kernels issue per step.  A stage of 32 steps takes
+// 0.80 us (some 1450 clocks for the 776 of MMAs): the issue slots and shared memory accesses of the loads and splits, and the wait of
+// fence.proxy.async for loads in flight.  With B split beforehand and copied by TMA 0.57 us.  2368 x 2048 x 2304: 195 -> 140 us, and the
+// FMA kernel 640.
 //
-// A CTA of 544 threads forms 128 x BN outputs of a policy P (see gemm_f32.cuh; a stage is 32 steps of it):
+// A CTA of 576 threads forms 128 x BN outputs of a policy P, in stages of 32 steps:
 //   warps 0-15  in two groups that take alternate stages, so that the loads of one are in flight while the other splits: load the words of
 //               a stage, split them and store the planes of both operands in shared memory as the MMA reads them - rows of 32 steps where
 //               the operand's memory runs along k (K-major), rows of 32 columns where it does not (MN-major; no transposition) - with the
@@ -21,6 +22,7 @@
 //               live words or sums they spill, and what spills goes to L2 (shared memory leaves no L1; 44 TFLOP/s).
 //   warp 16     issues the MMAs.  The three planes of B are neighbouring rows (or column blocks) of one operand, so that h x [m l], m x [h m]
 //               are one MMA each, and with BN = 64 also h x [h m l].
+//   warp 17     where W is split beforehand (TMA_B), copies the three planes of a stage of B; half of the split work goes.
 // hh accumulates in two column blocks in turn, so that one is read while the other fills.
 // Where a sum comes out as Inf or NaN (operands that are, or that overflow a plane) or so small that a plane's last bits may have
 // been lost to underflow, the tile is formed once more by FMAs, as gemm_f32_kernel forms it.
@@ -30,7 +32,7 @@
 
 namespace alpha {
 
-constexpr int kPlaneThreads = 544, kPlaneBM = 128, kPlaneBK = 32, kPlaneRing = 4;
+constexpr int kPlaneThreads = 576, kPlaneBM = 128, kPlaneBK = 32, kPlaneRing = 4;
 
 __host__ __device__ constexpr uint32_t plane_stage_bytes(int BN) { return 3u * (kPlaneBM + BN) * kPlaneBK * 2; }
 __host__ __device__ constexpr uint32_t plane_smem_bytes(int BN) { return kPlaneRing * plane_stage_bytes(BN) + 1024; }
@@ -97,21 +99,372 @@ template <int COLS, bool KC> __device__ constexpr uint32_t plane_step() { return
 // Steps from one word of a thread to the next where memory runs along the columns.
 template <int COLS> __device__ constexpr int plane_dk() { return 32 / (COLS / 32); }
 
-// The whole tile by FMAs, in column slices of 64.
-template <int BN, class P>
-__device__ __noinline__ void gemm_planes_again(const P& p, void* shared)
+// ---- what is multiplied ---------------------------------------------------------------------------------------
+//
+// A policy P (by value, in the kernel's parameters) describes both operands and the result:
+//   P::kAk, P::kBk     the operand runs along the reduction in memory (else along its rows / columns); words are four floats either way
+//   cta()              tile (bx, by, bz): rows from m0, columns from n0, stages [s0, s1) of 32 steps of K in all; false: there is none
+//   a_row, a_step      a word of A lies row.at + step.at floats into a_tensor() and is read where use_a() says (a filter tap may miss the
+//   b_row, b_step      image, a row, column or step may not exist); the same for B
+//   row_out, store     the row of the result, nullptr where there is none; four consecutive outputs of it
+// Offsets are 32-bit: tensors have fewer than 2^31 elements (planes_fit).
+
+// Tiles of a launch, x fastest, one a CTA; `first` = tile of CTA 0.
+struct PlaneGrid { unsigned first; FastDiv by_x, by_y; };
+
+struct PlaneAt { uint32_t at, bits; };
+
+// A row knows which filter rows and columns meet the image from it (bits 0 ... 14 and 16 ... 30), a step names its own; a step past the end
+// needs bit 15, which no row has, and a row past the end has none.
+constexpr int kPlaneTaps = 15;
+constexpr uint32_t kNoStep = 1u << 15;
+__device__ __forceinline__ bool plane_meets(const PlaneAt& row, const PlaneAt& step) { return (row.bits & step.bits) == step.bits; }
+__device__ __forceinline__ uint32_t tap_bits(unsigned u, unsigned v) { return 1u << u | 0x10000u << v; }
+
+// deltaX of any stride: rows = the pixels of one stride phase (py, px), which all meet the same filter taps, columns = input
+// channels, reduction = those taps x output channels (tap-major, without gaps between taps), in `ksplit` parts.  A launch computes
+// `parts` of them from part0 on, bz = phase * parts + part, each into its own copy of deltaX, every element of which some phase
+// writes; or, without memory for copies, one part that is added to what `out` holds (ADD).
+struct PlaneDxProblem {
+    static constexpr bool kAk = true, kBk = false, kTail = false, kCopyB = true;
+    const float* dY; const float* W; float* out;
+    int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw;
+    int nsw;                       // phases along a row: min(sw, IW)
+    int ksplit, parts, part0;
+    size_t size;                   // elements of deltaX
+    // divisions by OC, and by what phases have one more or less of: A * B, B, Ux (set_divisions)
+    FastDiv by_OC, by_AB[4], by_B[2], by_Ux[2];
+    int row0[16];                  // first row of each phase among the planes of W
+    struct Cta { int m0, n0, s0, s1, K, rows, A, B, py, px, ry, rx, qy, qx, Uy, Ux, row0; FastDiv by_B, by_AB, by_Ux; float* out; };
+
+    void set_divisions()
+    {
+        const int A = (IH + sh - 1) / sh, B = (IW + sw - 1) / sw, Ux = (FW + sw - 1) / sw;
+        auto by = [](int d) { return fast_div(d > 0 ? d : 1); };
+        by_OC = by(OC);
+        for (int i = 0; i < 4; ++i) by_AB[i] = by((A - i / 2) * (B - i % 2));
+        for (int i = 0; i < 2; ++i) { by_B[i] = by(B - i); by_Ux[i] = by(Ux - i); }
+    }
+    __device__ bool cta(Cta& c, int BM, int BN, int bx, int by, int z) const
+    {
+        const int phase = z / parts, copy = z - phase * parts, sp = part0 + copy;
+        c.py = phase / nsw; c.px = phase - c.py * nsw;
+        c.A = (IH - c.py + sh - 1) / sh; c.B = (IW - c.px + sw - 1) / sw;
+        c.rows = N * c.A * c.B;
+        c.m0 = bx * BM; c.n0 = by * BN;
+        if (c.m0 >= c.rows) return false;
+        c.ry = (c.py + ph) % sh; c.rx = (c.px + pw) % sw;
+        c.qy = (c.py + ph - c.ry) / sh; c.qx = (c.px + pw - c.rx) / sw;
+        c.Uy = c.ry < FH ? (FH - c.ry + sh - 1) / sh : 0;
+        c.Ux = c.rx < FW ? (FW - c.rx + sw - 1) / sw : 0;
+        c.K = c.Uy * c.Ux * OC;
+        const int la = c.A * sh < IH ? 1 : 0, lb = c.B * sw < IW ? 1 : 0;                 // a row, a column less than phase 0
+        c.by_AB = by_AB[2 * la + lb]; c.by_B = by_B[lb]; c.by_Ux = by_Ux[c.Ux * sw < FW ? 1 : 0];
+        c.row0 = row0[phase & 15];
+        const int stages = (c.K + 31) / 32, per = (stages + ksplit - 1) / ksplit;
+        c.s0 = sp * per < stages ? sp * per : stages;
+        c.s1 = c.s0 + per < stages ? c.s0 + per : stages;
+        c.out = out + static_cast<size_t>(copy) * size;
+        return true;
+    }
+    __device__ const float* a_tensor(const Cta&) const { return dY; }
+    __device__ const float* b_tensor(const Cta&) const { return W; }
+    // pixel (n, a, b) of the phase
+    __device__ bool pixel(const Cta& c, int m, unsigned& n, unsigned& a, unsigned& b) const
+    {
+        const int r = c.m0 + m;
+        if (r >= c.rows) return false;
+        unsigned q;
+        c.by_AB.divmod(static_cast<unsigned>(r), n, q);
+        c.by_B.divmod(q, a, b);
+        return true;
+    }
+    __device__ PlaneAt a_row(const Cta& c, int m) const
+    {
+        unsigned n, a, b;
+        if (!pixel(c, m, n, a, b)) return PlaneAt{0u, 0u};
+        const int y = static_cast<int>(a) + c.qy, x = static_cast<int>(b) + c.qx;
+        uint32_t taps = 0;
+        for (int v = 0; v < c.Ux; ++v)
+            if (static_cast<unsigned>(x - v) < static_cast<unsigned>(OW)) taps |= 0x10000u << v;
+        for (int u = 0; u < c.Uy; ++u)
+            if (static_cast<unsigned>(y - u) < static_cast<unsigned>(OH)) taps |= 1u << u;
+        return PlaneAt{static_cast<uint32_t>(((static_cast<int>(n) * OH + y) * OW + x) * OC), taps};
+    }
+    __device__ void tap(const Cta& c, int k, unsigned& t, unsigned& oc, unsigned& u, unsigned& v) const
+    {
+        by_OC.divmod(static_cast<unsigned>(k), t, oc);
+        c.by_Ux.divmod(t, u, v);
+    }
+    __device__ PlaneAt a_step(const Cta& c, int k) const
+    {
+        unsigned t, oc, u, v;
+        tap(c, k, t, oc, u, v);
+        return PlaneAt{oc - (u * OW + v) * OC, k < c.K ? tap_bits(u, v) : kNoStep};
+    }
+    __device__ PlaneAt b_row(const Cta& c, int col) const
+    {
+        return PlaneAt{static_cast<uint32_t>((c.ry * FW + c.rx) * IC + c.n0 + col), c.n0 + col < IC ? 1u : 0u};
+    }
+    __device__ PlaneAt b_step(const Cta& c, int k) const
+    {
+        unsigned t, oc, u, v;
+        tap(c, k, t, oc, u, v);
+        return PlaneAt{(oc * (FH * FW) + u * (sh * FW) + v * sw) * IC, k < c.K ? 1u : kNoStep};
+    }
+    __device__ static bool use_a(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    __device__ static bool use_b(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    // planes of W with the rows of each phase in the order of its steps: a box of 32 columns x 32 steps x column blocks x planes
+    __device__ void copy_b(const Cta& c, uint32_t dst, const CUtensorMap* m, uint32_t bar, int k) const
+    {
+        tma_load_4d_a(dst, m, bar, 0, c.row0 + k, c.n0 >> 5, 0);
+    }
+    __device__ float* row_out(const Cta& c, int m) const
+    {
+        unsigned n, a, b;
+        if (!pixel(c, m, n, a, b)) return nullptr;
+        return c.out + ((static_cast<size_t>(n) * IH + (a * sh + c.py)) * IW + (b * sw + c.px)) * IC;
+    }
+};
+template <bool ADD>
+struct PlaneDx : PlaneDxProblem {
+    __device__ void store(const Cta& c, float* row, int col, const float4& o) const
+    {
+        if (!row || c.n0 + col >= IC) return;
+        float4* p = reinterpret_cast<float4*>(row + c.n0 + col);
+        if (ADD) {
+            const float4 a = *p;
+            *p = make_float4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
+        } else {
+            *p = o;
+        }
+    }
+};
+
+// C[b] = A[b] * B[b] over N x M outputs and K steps, with row pitches.  A_KC: A[b] is [N][lda] (else [K][lda], the transposed
+// form); B_KC: B[b] is [M][ldb] (else [K][ldb]).  Pitches are multiples of 4 and every matrix starts on a 16-byte boundary;
+// words are loaded whole where they start inside the matrix: columns past N or M are not stored, steps past K become zeros (kTail).
+template <bool A_KC, bool B_KC>
+struct PlaneBatch {
+    static constexpr bool kAk = A_KC, kBk = B_KC, kTail = true, kCopyB = false;
+    const float *A, *B; float* C;
+    int N, M, K, lda, ldb, ldc;
+    size_t strA, strB, strC;
+    struct Cta { int m0, n0, s0, s1, K; const float *A, *B; float* C; };
+
+    __device__ bool cta(Cta& c, int BM, int BN, int bx, int by, int bz) const
+    {
+        c.m0 = by * BM; c.n0 = bx * BN;
+        c.s0 = 0; c.s1 = (K + 31) / 32; c.K = K;
+        c.A = A + static_cast<size_t>(bz) * strA; c.B = B + static_cast<size_t>(bz) * strB; c.C = C + static_cast<size_t>(bz) * strC;
+        return true;
+    }
+    __device__ const float* a_tensor(const Cta& c) const { return c.A; }
+    __device__ const float* b_tensor(const Cta& c) const { return c.B; }
+    __device__ PlaneAt a_row(const Cta& c, int m) const { return PlaneAt{static_cast<uint32_t>((c.m0 + m) * (A_KC ? lda : 1)), c.m0 + m < N ? 1u : 0u}; }
+    __device__ PlaneAt b_row(const Cta& c, int col) const { return PlaneAt{static_cast<uint32_t>((c.n0 + col) * (B_KC ? ldb : 1)), c.n0 + col < M ? 1u : 0u}; }
+    __device__ PlaneAt a_step(const Cta&, int k) const { return PlaneAt{static_cast<uint32_t>(k * (A_KC ? 1 : lda)), k < K ? 1u : kNoStep}; }
+    __device__ PlaneAt b_step(const Cta&, int k) const { return PlaneAt{static_cast<uint32_t>(k * (B_KC ? 1 : ldb)), k < K ? 1u : kNoStep}; }
+    __device__ static bool use_a(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    __device__ static bool use_b(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    __device__ float* row_out(const Cta& c, int m) const { return c.m0 + m < N ? c.C + static_cast<size_t>(c.m0 + m) * ldc : nullptr; }
+    __device__ void store(const Cta& c, float* row, int col, const float4& o) const
+    {
+        const int j = c.n0 + col;
+        if (!row || j >= M) return;
+        if (j + 3 < M) { *reinterpret_cast<float4*>(row + j) = o; return; }
+        row[j] = o.x;
+        if (j + 1 < M) row[j + 1] = o.y;
+        if (j + 2 < M) row[j + 2] = o.z;
+    }
+};
+
+// Forward convolution: rows = output pixels, columns = output channels, reduction = taps x input channels, as a row of W holds them.
+// bz = part of the reduction, each into its own copy of Y (bias and activation only without parts).
+struct PlaneFwd {
+    static constexpr bool kAk = true, kBk = true, kTail = false, kCopyB = true;
+    const float* X; const float* W; const float* bias; float* out;
+    int N, IH, IW, IC, FH, FW, OH, OW, OC, sh, sw, ph, pw, K, rows, ksplit, act_on;
+    float act_k;
+    size_t size;                   // elements of Y
+    FastDiv by_OW, by_OHW, by_IC, by_FW;
+    struct Cta { int m0, n0, s0, s1, K; float* out; };
+
+    __device__ bool cta(Cta& c, int BM, int BN, int bx, int by, int sp) const
+    {
+        c.m0 = bx * BM; c.n0 = by * BN;
+        const int stages = (K + 31) / 32, per = (stages + ksplit - 1) / ksplit;
+        c.s0 = sp * per < stages ? sp * per : stages;
+        c.s1 = c.s0 + per < stages ? c.s0 + per : stages;
+        c.K = K;
+        c.out = out + static_cast<size_t>(sp) * size;
+        return true;
+    }
+    __device__ const float* a_tensor(const Cta&) const { return X; }
+    __device__ const float* b_tensor(const Cta&) const { return W; }
+    __device__ PlaneAt a_row(const Cta& c, int m) const
+    {
+        if (c.m0 + m >= rows) return PlaneAt{0u, 0u};
+        unsigned n, q, oh, ow;
+        by_OHW.divmod(static_cast<unsigned>(c.m0 + m), n, q);
+        by_OW.divmod(q, oh, ow);
+        const int y = static_cast<int>(oh) * sh - ph, x = static_cast<int>(ow) * sw - pw;
+        uint32_t taps = 0;
+        for (int v = 0; v < FW; ++v)
+            if (static_cast<unsigned>(x + v) < static_cast<unsigned>(IW)) taps |= 0x10000u << v;
+        for (int u = 0; u < FH; ++u)
+            if (static_cast<unsigned>(y + u) < static_cast<unsigned>(IH)) taps |= 1u << u;
+        return PlaneAt{static_cast<uint32_t>(((static_cast<int>(n) * IH + y) * IW + x) * IC), taps};
+    }
+    __device__ PlaneAt a_step(const Cta&, int k) const
+    {
+        unsigned t, ic, fh, fw;
+        by_IC.divmod(static_cast<unsigned>(k), t, ic);
+        by_FW.divmod(t, fh, fw);
+        return PlaneAt{(fh * IW + fw) * IC + ic, k < K ? tap_bits(fh, fw) : kNoStep};
+    }
+    __device__ PlaneAt b_row(const Cta& c, int col) const { return PlaneAt{static_cast<uint32_t>((c.n0 + col) * K), c.n0 + col < OC ? 1u : 0u}; }
+    __device__ PlaneAt b_step(const Cta&, int k) const { return PlaneAt{static_cast<uint32_t>(k), k < K ? 1u : kNoStep}; }
+    __device__ static bool use_a(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    __device__ static bool use_b(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    // planes of W, rows padded to whole stages: a box of 32 steps x BN rows x planes
+    __device__ void copy_b(const Cta& c, uint32_t dst, const CUtensorMap* m, uint32_t bar, int k) const { tma_load_3d_a(dst, m, bar, k, c.n0, 0); }
+    __device__ float* row_out(const Cta& c, int m) const { return c.m0 + m < rows ? c.out + static_cast<size_t>(c.m0 + m) * OC : nullptr; }
+    __device__ void store(const Cta& c, float* row, int col, float4 o) const
+    {
+        const int j = c.n0 + col;
+        if (!row || j >= OC) return;
+        if (bias) {
+            const float4 b = *reinterpret_cast<const float4*>(bias + j);
+            o.x += b.x; o.y += b.y; o.z += b.z; o.w += b.w;
+        }
+        if (act_on) {
+            o.x = o.x > 0.f ? o.x : act_k * o.x; o.y = o.y > 0.f ? o.y : act_k * o.y;
+            o.z = o.z > 0.f ? o.z : act_k * o.z; o.w = o.w > 0.f ? o.w : act_k * o.w;
+        }
+        *reinterpret_cast<float4*>(row + j) = o;
+    }
+};
+
+// deltaW: rows = output channels, columns = taps x input channels, reduction = output pixels, in parts like PlaneFwd.
+struct PlaneDw {
+    static constexpr bool kAk = false, kBk = false, kTail = false, kCopyB = false;
+    const float* dY; const float* X; float* out;
+    int IH, IW, IC, FW, OC, sh, sw, ph, pw, K, L, ksplit;    // K pixels, L = taps * IC floats of a row of deltaW
+    size_t size;
+    FastDiv by_OW, by_OHW, by_IC, by_FW;
+    struct Cta { int m0, n0, s0, s1, K; float* out; };
+    struct BRow { uint32_t at; int fh, fw; };               // fh = 1 << 30: no such column
+    struct BStep { uint32_t at; int y, x; };
+
+    __device__ bool cta(Cta& c, int BM, int BN, int bx, int by, int sp) const
+    {
+        c.m0 = bx * BM; c.n0 = by * BN;
+        const int stages = (K + 31) / 32, per = (stages + ksplit - 1) / ksplit;
+        c.s0 = sp * per < stages ? sp * per : stages;
+        c.s1 = c.s0 + per < stages ? c.s0 + per : stages;
+        c.K = K;
+        c.out = out + static_cast<size_t>(sp) * size;
+        return true;
+    }
+    __device__ const float* a_tensor(const Cta&) const { return dY; }
+    __device__ const float* b_tensor(const Cta&) const { return X; }
+    __device__ PlaneAt a_row(const Cta& c, int m) const { return PlaneAt{static_cast<uint32_t>(c.m0 + m), c.m0 + m < OC ? 1u : 0u}; }
+    __device__ PlaneAt a_step(const Cta&, int k) const { return PlaneAt{static_cast<uint32_t>(k * OC), k < K ? 1u : kNoStep}; }
+    __device__ BRow b_row(const Cta& c, int col) const
+    {
+        const int q = c.n0 + col;
+        if (q >= L) return BRow{0u, 1 << 30, 0};
+        unsigned t, ic, fh, fw;
+        by_IC.divmod(static_cast<unsigned>(q), t, ic);
+        by_FW.divmod(t, fh, fw);
+        return BRow{(fh * IW + fw) * IC + ic, static_cast<int>(fh), static_cast<int>(fw)};
+    }
+    __device__ BStep b_step(const Cta&, int k) const
+    {
+        unsigned n, q, oh, ow;
+        by_OHW.divmod(static_cast<unsigned>(k), n, q);
+        by_OW.divmod(q, oh, ow);
+        const int y = static_cast<int>(oh) * sh - ph, x = static_cast<int>(ow) * sw - pw;
+        return BStep{static_cast<uint32_t>(((static_cast<int>(n) * IH + y) * IW + x) * IC), k < K ? y : 1 << 30, x};
+    }
+    __device__ static bool use_a(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
+    __device__ bool use_b(const BRow& row, const BStep& step) const
+    {
+        return static_cast<unsigned>(step.y + row.fh) < static_cast<unsigned>(IH) && static_cast<unsigned>(step.x + row.fw) < static_cast<unsigned>(IW);
+    }
+    __device__ float* row_out(const Cta& c, int m) const { return c.m0 + m < OC ? c.out + static_cast<size_t>(c.m0 + m) * L : nullptr; }
+    __device__ void store(const Cta& c, float* row, int col, const float4& o) const
+    {
+        if (row && c.n0 + col < L) *reinterpret_cast<float4*>(row + c.n0 + col) = o;
+    }
+};
+
+// The 16-byte word `at` floats into a tensor, zeros without `use`: one predicated load, so that a thread's loads leave back to back
+// (behind a branch the compiler moves each result to its place before the next load: 240 clocks a word).
+__device__ __forceinline__ float4 load_word(const float* tensor, uint32_t at, bool use)
 {
-    typename P::Cta c;
-    p.cta(c, kPlaneBM, BN);
-    for (int x = 0; x < BN; x += 64) {
-        typename P::Cta part = c;
-        part.n0 += x;
-        gemm_f32_tile<kPlaneBM, 64, 8, 4>(p, part, *static_cast<GemmShared<kPlaneBM, 64, P>*>(shared));
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b64 a;\n\tsetp.ne.u32 q, %6, 0;\n\tmad.wide.u32 a, %5, 4, %4;\n\t"
+        "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+        "@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+        : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(tensor), "r"(at), "r"(static_cast<uint32_t>(use)));
+    return v;
+}
+
+// The whole tile by FMAs in ascending k, for operands that the planes do not represent: 256 threads of 8 x BN / 16 outputs.  A
+// product whose tap misses the image, or with no operand at all, is left out, so that an Inf or NaN of the other operand stays out of it.
+template <int BN, class P>
+__device__ __noinline__ void gemm_planes_again(const P& p, const typename P::Cta& c, int tid)
+{
+    constexpr int TN = BN / 16;
+    const int m0 = (tid >> 4) * 8, n0 = (tid & 15) * TN;
+    const float *A = p.a_tensor(c), *B = p.b_tensor(c);
+    float acc[8][TN] = {};
+    const int end = c.s1 * 32 < c.K ? c.s1 * 32 : c.K;
+    for (int k = c.s0 * 32; k < end; ++k) {
+        // (a step of an operand that runs along k is known by its word of four)
+        const int ka = P::kAk ? k & ~3 : k, kb = P::kBk ? k & ~3 : k;
+        const auto sa = p.a_step(c, ka);
+        const auto sb = p.b_step(c, kb);
+        float b[TN];
+        bool in[TN];
+#pragma unroll
+        for (int x = 0; x < TN; ++x) {
+            const int col = n0 + x, word = P::kBk ? col : col & ~3;
+            const auto r = p.b_row(c, word);
+            in[x] = p.use_b(r, sb);
+            b[x] = in[x] ? __ldg(B + (r.at + sb.at) + (P::kBk ? k & 3 : col & 3)) : 0.f;
+        }
+#pragma unroll
+        for (int y = 0; y < 8; ++y) {
+            const int m = m0 + y, word = P::kAk ? m : m & ~3;
+            const auto r = p.a_row(c, word);
+            if (!p.use_a(r, sa)) continue;
+            const float a = __ldg(A + (r.at + sa.at) + (P::kAk ? k & 3 : m & 3));
+#pragma unroll
+            for (int x = 0; x < TN; ++x)
+                if (in[x]) acc[y][x] = fmaf(a, b[x], acc[y][x]);
+        }
+    }
+#pragma unroll
+    for (int y = 0; y < 8; ++y) {
+        float* row = p.row_out(c, m0 + y);
+#pragma unroll
+        for (int x = 0; x < TN; x += 4) p.store(c, row, n0 + x, make_float4(acc[y][x], acc[y][x + 1], acc[y][x + 2], acc[y][x + 3]));
     }
 }
 
-template <int BN, class P>
-__global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __grid_constant__ P p, int* status)
+// After a wait that ran out: time for what has been issued to end, before shared and tensor memory are given back.
+static __device__ __noinline__ void settle()
+{
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 1000000ull) {}
+}
+
+template <int BN, class P, bool TMA_B>
+__global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __grid_constant__ P p, const __grid_constant__ CUtensorMap tmB, const PlaneGrid grid, int* status)
 {
     static_assert(BN == 64 || BN == 128, "tile shape");
     constexpr int NA = kPlaneBM / 32, NB = BN / 32, COLS = BN / 4;      // words of a thread in a stage; columns of a warp
@@ -121,19 +474,24 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
     __shared__ uint32_t tmem_holder;
     __shared__ typename P::Cta c;                            // (in registers or local memory it would cost the loops)
     __shared__ int work;
+    __shared__ decltype(p.a_row(c, 0)) rows[P::kAk ? kPlaneBM : 1];   // computed once: 16 threads read a row, and divisions cost
+    __shared__ float* outs[kPlaneBM];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t full_a = smem_u32(bars), done_a = full_a + 8 * kPlaneRing, free_a = done_a + 8 * kPlaneRing;
     if (tid == 0) {
         for (int i = 0; i < kPlaneRing; ++i) {
-            mbar_init(&bars[i], 8);                      // a stage is staged: one arrival per warp of its group
+            mbar_init(&bars[i], TMA_B ? 9 : 8);          // a stage is staged: one arrival per warp of its group, one for the copy of B
             mbar_init(&bars[kPlaneRing + i], 1);         // its MMAs are done
         }
         mbar_init(&bars[2 * kPlaneRing], 16);            // an hh accumulator has been read by all warps
         mbar_init(&bars[2 * kPlaneRing + 1], 16);
         fence_barrier_init();
         typename P::Cta mine;
-        work = p.cta(mine, kPlaneBM, BN);
+        unsigned bx, by, bz, q;
+        grid.by_x.divmod(grid.first + blockIdx.x, q, bx);
+        grid.by_y.divmod(q, bz, by);
+        work = p.cta(mine, kPlaneBM, BN, static_cast<int>(bx), static_cast<int>(by), static_cast<int>(bz));
         c = mine;
     }
     if (warp == 16) {
@@ -141,13 +499,16 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
         tmem_relinquish();
     }
     tc_fence_before_sync();
-    grid_dependency_wait();
     __syncthreads();
-    grid_dependency_trigger();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_holder;
 
-    const int stages = work && c.it1 > c.it0 ? (c.it1 - c.it0 + 1) >> 1 : 0;
+    const int stages = work && c.s1 > c.s0 ? c.s1 - c.s0 : 0;
+    if (work) {
+        if (P::kAk && tid < kPlaneBM) rows[tid] = p.a_row(c, tid);
+        else if (tid >= kPlaneBM && tid < 2 * kPlaneBM) outs[tid - kPlaneBM] = p.row_out(c, tid - kPlaneBM);
+    }
+    __syncthreads();
     bool ok = true, again = false;
     unsigned long long acc[COLS / 2];
 #pragma unroll
@@ -155,114 +516,115 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
     // tensor memory: [hh of even windows][hm + mh][hl + mm + lh][hh of odd windows]
     constexpr uint32_t kSide = BN, kOdd = 3 * BN;
 
-    if (warp >= 16) {
-        if (warp == 16 && lane == 0 && stages) {
-            constexpr uint32_t dhi = (512u >> 4) | (1u << 14) | (static_cast<uint32_t>(kSwizzle64B) << 29);
-            constexpr uint32_t a_k = P::kAk ? 2u : 64u, b_k = P::kBk ? 2u : 64u;      // 16 steps further, in 16-byte units
-            constexpr uint32_t i1 = make_idesc_bf16(128, BN, !P::kAk, !P::kBk), i2 = make_idesc_bf16(128, 2 * BN, !P::kAk, !P::kBk),
-                               i3 = make_idesc_bf16(128, BN == 64 ? 192 : 128, !P::kAk, !P::kBk);
-            constexpr uint32_t pa = kPlaneA >> 4, pb = kPlaneB >> 4;
-            const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), P::kAk ? 16u : 2048u), b_lo0 = smem_desc_lo(smem_u32(smem) + 3 * kPlaneA, P::kBk ? 16u : 2048u);
-            const uint32_t side = tmem_base + kSide;
-            typename P::Cursor cur = p.plane_begin(c);
-            auto full = [&](int s) { return full_a + 8 * (s % kPlaneRing); };
-            auto freed = [&](int s) { return free_a + 8 * (s >> 1 & 1); };    // (asked at the first stage of a window)
-            bool staged = false, read = false;       // stage s is known to be staged, the accumulator of its window to be read
+    if (warp == 17) {
+        grid_dependency_wait();
+        grid_dependency_trigger();
+        if constexpr (TMA_B) if (elect_one()) {
             for (int s = 0; s < stages; ++s) {
-                const uint32_t slot = s % kPlaneRing, window = s >> 1, d = tmem_base + (window & 1 ? kOdd : 0u);
-                if (!staged) ok = mbar_wait_a(full(s), (s / kPlaneRing) & 1);
-                if (ok && !read && !(s & 1) && window >= 2) ok = mbar_wait_a(freed(s), ((window >> 1) - 1) & 1);
-                if (!ok) { report(status, kStatusMmaTimeout); break; }
-                tc_fence_after_sync();
-                const bool two = p.plane_left(cur) > 16;
-                const uint32_t a = a_lo0 + slot * (kStage >> 4), b = b_lo0 + slot * (kStage >> 4);
-                const uint32_t keep = s & 1, keep_side = s ? 1u : 0u;
-                // what the next stage waits for, asked while the queue still holds MMAs of this one
-                auto look_ahead = [&]() {
-                    p.plane_next(c, cur);
-                    const int n = s + 1;
-                    staged = mbar_test_a(full(n), (n / kPlaneRing) & 1);
-                    read = !(n & 1) && n >= 4 && mbar_test_a(freed(n), ((n >> 2) - 1) & 1);
-                };
-                // straight-line code: address arithmetic between two MMAs would cost the issuing thread as much as an MMA takes
-                if constexpr (BN == 64) {
-                    // small products: [hm + mh][hl + mm + lh]
-                    auto step = [&](auto merged_, auto k_, uint32_t keep, uint32_t keep_side) {
-                        constexpr uint32_t ka = decltype(k_)::value * a_k, kb = decltype(k_)::value * b_k;
-                        if constexpr (decltype(merged_)::value) {
-                            mma_bf16_ss2_imm<ka, kb>(d, a, dhi, b, dhi, i3, 1u);
-                        } else {
-                            mma_bf16_ss2_imm<ka, kb>(d, a, dhi, b, dhi, i1, keep);
-                            mma_bf16_ss2_imm<ka, kb + pb>(side, a, dhi, b, dhi, i2, keep_side);
-                        }
-                        mma_bf16_ss2_imm<ka + pa, kb>(side, a, dhi, b, dhi, i2, 1u);
-                        mma_bf16_ss2_imm<ka + 2 * pa, kb>(side + 64, a, dhi, b, dhi, i1, 1u);
-                    };
-                    using First = std::integral_constant<uint32_t, 0>; using Second = std::integral_constant<uint32_t, 1>;
-                    if (window & 1) {
-                        step(std::false_type{}, First{}, keep, 1u);
-                        look_ahead();
-                        if (two) step(std::false_type{}, Second{}, 1u, 1u);
-                    } else if (keep) {
-                        step(std::true_type{}, First{}, 1u, 1u);
-                        look_ahead();
-                        if (two) step(std::true_type{}, Second{}, 1u, 1u);
-                    } else {
-                        step(std::false_type{}, First{}, 0u, keep_side);
-                        look_ahead();
-                        if (two) step(std::true_type{}, Second{}, 1u, 1u);
-                    }
-                } else {
-                    auto step = [&](auto k_, uint32_t keep, uint32_t keep_side) {
-                        constexpr uint32_t ka = decltype(k_)::value * a_k, kb = decltype(k_)::value * b_k;
-                        // small products: [hm + mh][hl + mm + lh]
-                        mma_bf16_ss2_imm<ka, kb + pb>(side, a, dhi, b, dhi, i2, keep_side);
-                        mma_bf16_ss2_imm<ka + pa, kb>(side, a, dhi, b, dhi, i2, 1u);
-                        mma_bf16_ss2_imm<ka + 2 * pa, kb>(side + BN, a, dhi, b, dhi, i1, 1u);
-                        mma_bf16_ss2_imm<ka, kb>(d, a, dhi, b, dhi, i1, keep);
-                    };
-                    step(std::integral_constant<uint32_t, 0>{}, keep, keep_side);
-                    look_ahead();
-                    if (two) step(std::integral_constant<uint32_t, 1>{}, 1u, 1u);
-                }
-                mma_commit_a(done_a + 8 * slot);
+                const uint32_t slot = s % kPlaneRing, bar = full_a + 8 * slot;
+                if (s >= kPlaneRing && !mbar_wait_a(done_a + 8 * slot, (s / kPlaneRing - 1) & 1)) { report(status, kStatusProducerTimeout); settle(); break; }
+                mbar_arrive_expect_tx_a(bar, 3 * kPlaneB);
+                p.copy_b(c, smem_u32(smem) + slot * kStage + 3 * kPlaneA, &tmB, bar, (c.s0 + s) * 32);
             }
         }
         __syncwarp();
+    } else if (warp == 16) {
+        grid_dependency_wait();
+        grid_dependency_trigger();
+        // The whole warp walks the stages, so that counters and descriptors are uniform values; one lane issues.
+        constexpr uint32_t dhi = (512u >> 4) | (1u << 14) | (static_cast<uint32_t>(kSwizzle64B) << 29);
+        constexpr uint32_t a_k = P::kAk ? 2u : 64u, b_k = P::kBk ? 2u : 64u;          // 16 steps further, in 16-byte units
+        constexpr uint32_t i1 = make_idesc_bf16(128, BN, !P::kAk, !P::kBk), i2 = make_idesc_bf16(128, 2 * BN, !P::kAk, !P::kBk),
+                           i3 = make_idesc_bf16(128, BN == 64 ? 192 : 128, !P::kAk, !P::kBk);
+        constexpr uint32_t pa = kPlaneA >> 4, pb = kPlaneB >> 4;
+        const uint32_t base = __shfl_sync(0xffffffffu, smem_u32(smem), 0), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint32_t a_lo0 = smem_desc_lo(base, P::kAk ? 16u : 2048u), b_lo0 = smem_desc_lo(base + 3 * kPlaneA, P::kBk ? 16u : 2048u);
+        const uint32_t side = tmem + kSide, elected = elect_one();
+        const int left = c.K - c.s0 * 32;                                            // steps from the first stage on
+        for (int s = 0; s < stages; ++s) {
+            const uint32_t slot = s % kPlaneRing, window = s >> 1, d = tmem + (window & 1 ? kOdd : 0u);
+            ok = mbar_wait_a(full_a + 8 * slot, (s / kPlaneRing) & 1);
+            if (ok && !(s & 1) && window >= 2) ok = mbar_wait_a(free_a + 8 * (window & 1), ((window >> 1) - 1) & 1);
+            if (!__all_sync(0xffffffffu, ok)) { report(status, kStatusMmaTimeout); settle(); break; }
+            tc_fence_after_sync();
+            const uint32_t a = a_lo0 + slot * (kStage >> 4), b = b_lo0 + slot * (kStage >> 4);
+            const uint32_t keep = s & 1, keep_side = s ? 1u : 0u;
+            auto step = [&](auto k_, uint32_t keep, uint32_t keep_side) {
+                constexpr uint32_t ka = decltype(k_)::value * a_k, kb = decltype(k_)::value * b_k;
+                // columns: [hh][hm + mh][hl + mm + lh]
+                if (BN == 64 && keep && !(window & 1)) {
+                    mma_bf16_elected<ka, kb>(d, a, dhi, b, dhi, i3, 1u, elected);
+                } else {
+                    mma_bf16_elected<ka, kb>(d, a, dhi, b, dhi, i1, keep, elected);
+                    mma_bf16_elected<ka, kb + pb>(side, a, dhi, b, dhi, i2, keep_side, elected);
+                }
+                mma_bf16_elected<ka + pa, kb>(side, a, dhi, b, dhi, i2, 1u, elected);
+                mma_bf16_elected<ka + 2 * pa, kb>(side + BN, a, dhi, b, dhi, i1, 1u, elected);
+            };
+            step(std::integral_constant<uint32_t, 0>{}, keep, keep_side);
+            if (left - s * 32 > 16) step(std::integral_constant<uint32_t, 1>{}, 1u, 1u);
+            if (elected) mma_commit_a(done_a + 8 * slot);
+        }
+        __syncwarp();
     } else {
-        if (stages) {
+        if (!stages) {
+            grid_dependency_wait();
+            grid_dependency_trigger();
+        } else {
         const int group = warp >> 3, t = tid & 255;          // two groups of 256 threads take alternate stages
-        typename P::PlaneRow ra[NA];
-        if (P::kAk)
+        // along k a thread's words lie in NA (NB) rows and at one step, else in one column block and plane_dk steps apart
+        decltype(p.a_row(c, 0)) ra[P::kAk ? NA : 1];
+        decltype(p.b_row(c, 0)) rb[P::kBk && !TMA_B ? NB : 1];
 #pragma unroll
-            for (int i = 0; i < NA; ++i) ra[i] = p.plane_row(c, plane_col<kPlaneBM, P::kAk>(t, i));
+        for (int i = 0; i < (P::kAk ? NA : 1); ++i) {
+            if constexpr (P::kAk) ra[i] = rows[plane_col<kPlaneBM, true>(t, i)];
+            else ra[i] = p.a_row(c, plane_col<kPlaneBM, false>(t, i));
+        }
+        if constexpr (!TMA_B)
+#pragma unroll
+            for (int i = 0; i < (P::kBk ? NB : 1); ++i) rb[i] = p.b_row(c, plane_col<BN, P::kBk>(t, i));
         const uint32_t off_a = smem_u32(smem) + plane_offset<kPlaneBM, P::kAk>(t), off_b = smem_u32(smem) + 3 * kPlaneA + plane_offset<BN, P::kBk>(t);
-        const float* base_a = p.plane_a_base(c, plane_col<kPlaneBM, P::kAk>(t, 0), plane_k<kPlaneBM, P::kAk>(t, 0));
-        const float* base_b = p.plane_b_base(c, plane_col<BN, P::kBk>(t, 0), plane_k<BN, P::kBk>(t, 0));
-        uint32_t in = 0;                                     // words whose row or column exists
-#pragma unroll
-        for (int i = 0; i < NA; ++i) in |= (p.plane_a_in(c, plane_col<kPlaneBM, P::kAk>(t, i)) ? 1u : 0u) << i;
-#pragma unroll
-        for (int i = 0; i < NB; ++i) in |= (p.plane_b_in(c, plane_col<BN, P::kBk>(t, i)) ? 1u : 0u) << (8 + i);
-        typename P::Cursor cur = p.plane_begin(c);
+        const float *A = p.a_tensor(c), *B = p.b_tensor(c);
         float4 va[NA], vb[NB];
-        auto load = [&]() {
+        auto load = [&](int s) {
+            const int k0 = (c.s0 + s) * 32, ka = k0 + plane_k<kPlaneBM, P::kAk>(t, 0), kb = k0 + plane_k<BN, P::kBk>(t, 0);
+            if constexpr (P::kAk) {
+                const auto at = p.a_step(c, ka);
 #pragma unroll
-            for (int i = 0; i < NA; ++i)
-                va[i] = p.plane_a(cur, base_a, ra[i], i, in >> i & 1u, plane_k<kPlaneBM, P::kAk>(t, i), plane_dk<kPlaneBM>());
+                for (int i = 0; i < NA; ++i) va[i] = load_word(A, ra[i].at + at.at, p.use_a(ra[i], at));
+            } else {
 #pragma unroll
-            for (int i = 0; i < NB; ++i) vb[i] = p.plane_b(cur, base_b, i, in >> (8 + i) & 1u, plane_k<BN, P::kBk>(t, i), plane_dk<BN>());
+                for (int i = 0; i < NA; ++i) {
+                    const auto at = p.a_step(c, ka + i * plane_dk<kPlaneBM>());
+                    va[i] = load_word(A, ra[0].at + at.at, p.use_a(ra[0], at));
+                }
+            }
+            if constexpr (TMA_B) {
+            } else if constexpr (P::kBk) {
+                const auto at = p.b_step(c, kb);
+#pragma unroll
+                for (int i = 0; i < NB; ++i) vb[i] = load_word(B, rb[i].at + at.at, p.use_b(rb[i], at));
+            } else {
+#pragma unroll
+                for (int i = 0; i < NB; ++i) {
+                    const auto at = p.b_step(c, kb + i * plane_dk<BN>());
+                    vb[i] = load_word(B, rb[0].at + at.at, p.use_b(rb[0], at));
+                }
+            }
         };
         const uint32_t lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (warp >> 2) * COLS;
         // acc += the warp's columns of a column block
         auto add_columns = [&](uint32_t from) {
+            // (eight at a time where the words of both operands are in registers too)
+            constexpr int C = TMA_B || COLS == 16 ? 16 : 8;
 #pragma unroll
-            for (int x = 0; x < COLS; x += 16) {
-                uint32_t v[16];
-                tmem_ld_32x16(lanes + from + x, v);
+            for (int x = 0; x < COLS; x += C) {
+                uint32_t v[C];
+                if constexpr (C == 16) tmem_ld_32x16(lanes + from + x, v);
+                else tmem_ld_32x8(lanes + from + x, v);
                 tmem_ld_wait();
 #pragma unroll
-                for (int q = 0; q < 16; q += 2) acc[(x + q) / 2] = add2(acc[(x + q) / 2], pack2(__uint_as_float(v[q]), __uint_as_float(v[q + 1])));
+                for (int q = 0; q < C; q += 2) acc[(x + q) / 2] = add2(acc[(x + q) / 2], pack2(__uint_as_float(v[q]), __uint_as_float(v[q + 1])));
             }
         };
         auto wait_done = [&](int s) {
@@ -281,20 +643,21 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
             return true;
         };
         int flushed = 0;
-        if (group) p.plane_next(c, cur);
-        if (group < stages) load();
+        grid_dependency_wait();
+        grid_dependency_trigger();
+        if (group < stages) load(group);
         for (int s = group; s < stages; s += 2) {
             // two windows back: its MMAs are done, or nearly
             if (s >= 4 && !flush(flushed++)) break;
             if (s >= kPlaneRing && !wait_done(s - kPlaneRing)) break;
             const uint32_t at_a = off_a + (s % kPlaneRing) * kStage, at_b = off_b + (s % kPlaneRing) * kStage;
             if (P::kTail) {
-                const int steps = p.plane_left(cur);
+                const int steps = c.K - (c.s0 + s) * 32;
                 if (steps < 32) {
                     if (P::kAk)
 #pragma unroll
                         for (int i = 0; i < NA; ++i) keep_first(va[i], steps - plane_k<kPlaneBM, true>(t, i));
-                    if (P::kBk)
+                    if (P::kBk && !TMA_B)
 #pragma unroll
                         for (int i = 0; i < NB; ++i) keep_first(vb[i], steps - plane_k<BN, true>(t, i));
                 }
@@ -306,6 +669,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
                 const uint32_t at = at_a + i * plane_step<kPlaneBM, P::kAk>();
                 st_shared_v2(at, h); st_shared_v2(at + kPlaneA, m); st_shared_v2(at + 2 * kPlaneA, l);
             }
+            if constexpr (!TMA_B)
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
                 uint2 h, m, l;
@@ -317,11 +681,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
             __syncwarp();
             if (lane == 0) mbar_arrive_a(full_a + 8 * (s % kPlaneRing));
             // (not before the fence, which waits for loads in flight)
-            if (s + 2 < stages) {
-                p.plane_next(c, cur);
-                p.plane_next(c, cur);
-                load();
-            }
+            if (s + 2 < stages) load(s + 2);
         }
         const int windows = (stages + 1) >> 1;
         while (ok && flushed < windows) flush(flushed++);
@@ -329,14 +689,17 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
             tc_fence_after_sync();
             add_columns(kSide);
             add_columns(kSide + BN);
-            // what may not have survived the split
+            // what may not have survived the split: not finite, or below 1e-28 and not zero (both ends of the magnitudes, zero as the largest)
+            uint32_t most = 0, least = 0xffffffffu;
 #pragma unroll
             for (int x = 0; x < COLS / 2; ++x) {
                 float a, b;
                 unpack2(acc[x], a, b);
-                a = fabsf(a); b = fabsf(b);
-                again = again || !(a <= 3.402823466e38f) || !(b <= 3.402823466e38f) || (a < 1e-28f && a > 0.f) || (b < 1e-28f && b > 0.f);
+                const uint32_t u = __float_as_uint(a) << 1, v = __float_as_uint(b) << 1;
+                most = max(most, max(u, v));
+                least = min(least, min(u - 1, v - 1));
             }
+            again = most >= 0xff000000u || least < 2u * 0x10fd87b6u;
         }
         }
         tc_fence_before_sync();
@@ -345,14 +708,13 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
     if (warp == 16) tmem_dealloc(tmem_base, kTmem);
     if (!work || warp >= 16) return;
     if (again) {
-        if (warp < 8) gemm_planes_again<BN>(p, smem);
+        if (warp < 8) gemm_planes_again<BN>(p, c, tid);
         return;
     }
     if (!ok) return;
     // A lane holds a row; written from the registers, an instruction would touch 32 rows for 16 bytes each.  The warp's block of 32
     // columns goes through 4 KB of shared memory and leaves as whole 128-byte pieces, four rows per instruction.
     const int row0 = (warp & 3) * 32, col0 = (warp >> 2) * COLS;
-    const unsigned long long own = reinterpret_cast<unsigned long long>(p.row_c(c, row0 + lane).p);
     const uint32_t blk = smem_u32(smem) + warp * 4096u;
     constexpr int W = COLS / 4;               // 16-byte pieces of a row
     __syncwarp();
@@ -365,41 +727,89 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
     }
     __syncwarp();
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-        const int r = k * (32 / W) + lane / W, q = lane % W;
-        const float4 o = ld_shared_v4(blk + r * (W * 16) + ((q ^ (r * W / 8 & (W - 1))) << 4));
-        typename P::RowC rc;
-        rc.p = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, own, r));
-        p.store(c, rc, col0 + q * 4, o);
+    for (int k0 = 0; k0 < W; k0 += 4) {
+        float4 o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = (k0 + k) * (32 / W) + lane / W, q = lane % W;
+            o[k] = ld_shared_v4(blk + r * (W * 16) + ((q ^ (r * W / 8 & (W - 1))) << 4));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) p.store(c, outs[row0 + (k0 + k) * (32 / W) + lane / W], col0 + lane % W * 4, o[k]);
     }
 }
 
-template <int BN, class P>
-inline void launch_gemm_planes(const P& p, dim3 grid, cudaStream_t stream, int* status)
+// (sms: CTAs of a launch at most where kernels may not spread over all SMs, else 0)
+template <int BN, bool TMA_B, class P>
+inline void launch_gemm_planes(const P& p, const CUtensorMap& tmB, dim3 tiles, unsigned sms, cudaStream_t stream, int* status)
 {
     static bool attr_done = false;   // per instantiation; the attribute is per function, any device
     if (!attr_done) {
-        cudaFuncSetAttribute(gemm_planes_kernel<BN, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, plane_smem_bytes(BN));
+        cudaFuncSetAttribute(gemm_planes_kernel<BN, P, TMA_B>, cudaFuncAttributeMaxDynamicSharedMemorySize, plane_smem_bytes(BN));
         attr_done = true;
     }
-    launch_after(gemm_planes_kernel<BN, P>, grid, kPlaneThreads, plane_smem_bytes(BN), stream, p, status);
+    const unsigned total = tiles.x * tiles.y * tiles.z, most = sms ? sms : total;
+    PlaneGrid g{0, fast_div(static_cast<int>(tiles.x)), fast_div(static_cast<int>(tiles.y))};
+    for (; g.first < total; g.first += most)
+        launch_after(gemm_planes_kernel<BN, P, TMA_B>, total - g.first < most ? total - g.first : most, kPlaneThreads, plane_smem_bytes(BN), stream, p, tmB, g, status);
 }
 
-// Tile, kernel and parts of the reduction for a product of `rows` x `cols` outputs over `taps` x `k` steps, `copies` times (may_split: its
-// launch can cut the reduction into up to 16 parts; `size` outputs in all).  Both kernels are predicted from what was measured (us; 56
-// products of 1e5 to 1e10 FMAs, deltaX layers, FullConnect, batches, each within 12 % of its prediction, the choice on average 1.01 times
-// as long as the better one):
-//   planes  per wave of one CTA an SM 5.9 and for every stage 0.64 (64 columns) or 1.06 (128)
-//   FMAs    per wave of two CTAs an SM 3.1 and for every 16 steps what its tile takes (3.6 us for 128 x 128: 42 TFLOP/s)
-// 2048 x 2048 x 2052: 471 -> 136 us (127 TFLOP/s); 36848 x 384 x 604: 391 -> 174; 22275 x 248 over 9 x 84: 278 -> 107; 55404 x 272
-// over 9 x 4 (whole stages a tap) 164 and 137 us; 49600 x 8 over 4 x 4, four phases: 49 and 100 us.
-// Error, 2-norm against 64 bits (normal inputs): 50 steps 0.9e-7 on both, 252: 2.0e-7 -> 1.1e-7, 900: 5.3e-7 -> 1.4e-7, 2052: 1.6e-7; 20 steps
-// 0.6e-7 and 0.8e-7, so that shorter sums than 64 steps stay with the FMAs.
-struct ProductPlan { GemmTile tile; int ksplit; };
-inline ProductPlan plan_product(long long rows, int cols, int taps, int k, long long copies, bool may_split, double size, int sms, int mode)
+// The planes of W as TMA_B copies them: dst[plane][row][pitch], row r < rows from W row src(r).  taps = 0: rows as they lie (forward; K
+// columns, zeros up to the pitch); else row j * OC + oc is tap map[j] of output channel oc (deltaX: taps in the order of phases and steps).
+struct SplitRows { int map[64]; };
+template <int>   // (defined where it is launched)
+__global__ void __launch_bounds__(256) split_planes_kernel(const float* __restrict__ W, uint2* __restrict__ dst, int rows, int cols, unsigned pitch4, FastDiv by_pitch4,
+                                                           FastDiv by_OC, int OC, int taps, const SplitRows map)
+{
+    grid_dependency_wait();
+    grid_dependency_trigger();
+    const unsigned total = static_cast<unsigned>(rows) * pitch4;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        unsigned r, q, from;
+        by_pitch4.divmod(i, r, q);
+        from = r;
+        if (taps) {
+            unsigned j, oc;
+            by_OC.divmod(r, j, oc);
+            from = oc * taps + map.map[j];
+        }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (static_cast<int>(4 * q) < cols) v = __ldg(reinterpret_cast<const float4*>(W + static_cast<size_t>(from) * cols + 4 * q));
+        uint2 h, m, l;
+        split_planes(v, h, m, l);
+        dst[i] = h; dst[static_cast<size_t>(total) + i] = m; dst[2 * static_cast<size_t>(total) + i] = l;
+    }
+}
+
+// Tile and parts of the reduction of a product of `rows` x `cols` outputs over k steps, `copies` times, on this kernel (may_split: its
+// launch can cut the reduction into up to 16 parts of `size` outputs each; w: elements of W where B can be split beforehand, else 0), and
+// the time that takes (us): what a stage and a tile besides take in each form, as fitted to 1200 products (9 of 10 within 13 %).  The copy of
+// B costs a launch and pays from a few waves on (64 x 15 x 13, 36 -> 100 channels 3x3 37 -> 34 us, 2368 x 2048 x 2304 195 -> 140).
+struct PlanePlan { int bn; bool copy_b; int ksplit; double time; };
+inline PlanePlan plan_planes(long long rows, int cols, long long k, long long copies, bool may_split, double size, double w, int sms)
+{
+    static const struct { int bn; bool copy; double stage, wave; } forms[] = {{64, false, 0.62, 3.6}, {128, false, 0.80, 4.4}, {64, true, 0.47, 4.2}, {128, true, 0.57, 4.9}};
+    const long long stages = (k + kPlaneBK - 1) / kPlaneBK;
+    PlanePlan best{64, false, 1, 0};
+    for (const auto& f : forms) {
+        if (f.copy && !(w > 0)) continue;
+        const double tiles = (double)((rows + kPlaneBM - 1) / kPlaneBM) * ((cols + f.bn - 1) / f.bn) * copies, fixed = 5.3 + (f.copy ? 1.5 + w * 10e-6 / 5 : w * 0.8e-6);
+        for (int ks = 1; ks <= 16 && (ks == 1 || (may_split && ks <= stages / 2)); ++ks) {
+            const double ctas = tiles * ks, waves = (double)(long long)((ctas + sms - 1) / sms);
+            const double time = waves * ((stages + ks - 1) / ks * f.stage + f.wave) + fixed + (ks > 1 ? 2.1 + (ks + 1) * size * 4e-6 / 5 : 0.0);
+            if (best.time == 0 || time < best.time) best = PlanePlan{f.bn, f.copy, ks, time};
+            if (ctas > 4.0 * sms) break;
+        }
+    }
+    return best;
+}
+
+// Kernel, tile and parts for a product that is fp32 work (plane_k: steps, on average over the copies).
+struct ProductPlan { GemmTile tile; int ksplit; bool copy_b; };
+inline ProductPlan plan_product(long long rows, int cols, int taps, int k, long long copies, bool may_split, double size, double w, long long plane_k, int sms, int mode)
 {
     const GemmTile f = pick_gemm_tile(rows, cols, copies, sms);
-    const long long its = (long long)taps * ((k + kGemmBK - 1) / kGemmBK), stages = (long long)taps * ((k + kPlaneBK - 1) / kPlaneBK);
+    const long long its = (long long)taps * ((k + kGemmBK - 1) / kGemmBK);
     const double fc = (double)((rows + f.bm - 1) / f.bm) * ((cols + f.bn - 1) / f.bn) * copies;
     // FMAs: split only where the tiles do not fill the SMs
     int fks = 1;
@@ -410,26 +820,24 @@ inline ProductPlan plan_product(long long rows, int cols, int taps, int k, long 
     }
     const double step = f.bn == 128 ? 3.57 : (f.bn == 32 ? 1.42 : (f.bm == 128 ? 1.93 : 1.30)), waves = fc * fks / (2.0 * sms);
     const double f_time = (waves > 1 ? waves : 1.0) * ((its + fks - 1) / fks * step + 3.1) + 6.1;
-    if (mode == 0 || (mode == 1 && (long long)taps * k < 64)) return ProductPlan{f, fks};
-    const GemmTile t{kPlaneBM, cols <= 64 ? 64 : 128, true};
-    const double pc = (double)((rows + t.bm - 1) / t.bm) * ((cols + t.bn - 1) / t.bn) * copies;
-    int pks = 1;
-    double p_time = 0;
-    for (int ks = 1; ks <= 16 && (ks == 1 || (may_split && ks <= stages / 2)); ++ks) {
-        const double w = pc * ks, full = (long long)((w + sms - 1) / sms);
-        const double time = full * ((stages + ks - 1) / ks * (t.bn == 64 ? 0.64 : 1.06) + 5.9) + 6.6 + (ks > 1 ? 2.8 + (ks + 1) * size * 4e-6 / 5 : 0.0);
-        if (ks == 1 || time < p_time) { p_time = time; pks = ks; }
-    }
-    if (mode == 1 && f_time <= p_time) return ProductPlan{f, fks};
-    return ProductPlan{t, pks};
+    if (mode == 0 || (mode == 1 && (long long)taps * k < 64)) return ProductPlan{f, fks, false};
+    const PlanePlan p = plan_planes(rows, cols, plane_k, copies, may_split, size, w, sms);
+    if (mode == 1 && f_time <= 1.05 * p.time) return ProductPlan{f, fks, false};
+    return ProductPlan{GemmTile{kPlaneBM, p.bn, true}, p.ksplit, p.copy_b};
 }
 
 template <class P>
-inline void launch_product(const P& p, const GemmTile& t, dim3 grid, cudaStream_t stream, int* status)
+inline void launch_planes(const P& p, int bn, dim3 tiles, int sms, cudaStream_t stream, int* status, const CUtensorMap* tmB = nullptr)
 {
-    if (!t.planes) launch_gemm_f32(p, t, grid, stream);
-    else if (t.bn == 64) launch_gemm_planes<64>(p, grid, stream, status);
-    else launch_gemm_planes<128>(p, grid, stream, status);
+    if constexpr (P::kCopyB) {
+        if (tmB) {
+            if (bn == 64) launch_gemm_planes<64, true>(p, *tmB, tiles, sms, stream, status);
+            else launch_gemm_planes<128, true>(p, *tmB, tiles, sms, stream, status);
+            return;
+        }
+    }
+    if (bn == 64) launch_gemm_planes<64, false>(p, CUtensorMap{}, tiles, sms, stream, status);
+    else launch_gemm_planes<128, false>(p, CUtensorMap{}, tiles, sms, stream, status);
 }
 
 }  // namespace alpha

@@ -25,6 +25,8 @@ void note_plan(const char* fmt, ...);
 int device_sms(int* sms);
 // Where kernels report a wait that ran out.
 int device_status_word(int** status);
+// CTAs of one launch of the bf16-plane kernel, 0 = no limit.
+int planes_launch_slice(int* ctas);
 // Option F32_PLANES.
 int option_f32_planes();
 

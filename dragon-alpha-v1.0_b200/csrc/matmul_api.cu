@@ -146,11 +146,21 @@ int launch_bmm_f32(const float* A, const float* B, float* C, int Batch, int N, i
     int* status = nullptr;
     if (!rc) rc = device_status_word(&status);
     if (rc) return rc;
-    const GemmTile t = plan_product(N, M, 1, K, Batch, false, 0, sms, option_f32_planes()).tile;
+    int slice = 0;
+    rc = planes_launch_slice(&slice);
+    if (rc) return rc;
+    const bool fit = (long long)(A_KC ? N : K) * lda < 1LL << 31 && (long long)(B_KC ? M : K) * ldb < 1LL << 31;   // 32-bit offsets in a matrix
+    const GemmTile t = plan_product(N, M, 1, K, Batch, false, 0, 0, K, sms, fit ? option_f32_planes() : 0).tile;
     for (int b0 = 0; b0 < Batch; b0 += 65535) {   // gridDim.z limit
         const int nb = Batch - b0 < 65535 ? Batch - b0 : 65535;
-        const BatchGemm<A_KC, B_KC> g{A + b0 * strA, B + b0 * strB, C + b0 * strC, N, M, K, lda, ldb, ldc, strA, strB, strC};
-        launch_product(g, t, dim3((M + t.bn - 1) / t.bn, (N + t.bm - 1) / t.bm, nb), static_cast<cudaStream_t>(stream), status);
+        const dim3 grid((M + t.bn - 1) / t.bn, (N + t.bm - 1) / t.bm, nb);
+        if (t.planes) {
+            const PlaneBatch<A_KC, B_KC> g{A + b0 * strA, B + b0 * strB, C + b0 * strC, N, M, K, lda, ldb, ldc, strA, strB, strC};
+            launch_planes(g, t.bn, grid, slice, static_cast<cudaStream_t>(stream), status);
+        } else {
+            const BatchGemm<A_KC, B_KC> g{A + b0 * strA, B + b0 * strB, C + b0 * strC, N, M, K, lda, ldb, ldc, strA, strB, strC};
+            launch_gemm_f32(g, t, grid, static_cast<cudaStream_t>(stream));
+        }
     }
     note_launch("bmm_simt");
     note_plan("gemm_f32 %s%dx%d", t.planes ? "planes " : "", t.bm, t.bn);

@@ -127,21 +127,6 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
-// Whether the phase has completed, without waiting.
-__device__ __forceinline__ bool mbar_test_a(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 static __device__ __noinline__ bool mbar_wait_slow_a(uint32_t bar, uint32_t parity)
 {
     const uint64_t t0 = globaltimer_ns();
@@ -476,6 +461,13 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -555,23 +547,22 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool a_mn_m
     return 1u << 4 | 1u << 7 | 1u << 10 | (a_mn_major ? 1u : 0u) << 15 | (b_mn_major ? 1u : 0u) << 16 |
            static_cast<uint32_t>(N >> 3) << 17 | static_cast<uint32_t>(M >> 4) << 24;
 }
+// Executed by a converged warp, issued by the lane whose `elected` is set; descriptors as (lo, hi) halves with offsets (16-byte units).
 template <uint32_t A_OFF, uint32_t B_OFF>
-__device__ __forceinline__ void mma_bf16_ss2_imm(uint32_t d_tmem, uint32_t a_base, uint32_t a_hi, uint32_t b_base, uint32_t b_hi, uint32_t idesc,
-                                                 uint32_t accumulate)
+__device__ __forceinline__ void mma_bf16_elected(uint32_t d_tmem, uint32_t a_base, uint32_t a_hi, uint32_t b_base, uint32_t b_hi, uint32_t idesc,
+                                                 uint32_t accumulate, uint32_t elected)
 {
     asm volatile(
         "{\n\t"
-        ".reg .pred p;\n\t"
+        ".reg .pred p, q;\n\t"
         ".reg .b64 da, db;\n\t"
-        ".reg .b32 ra, rb;\n\t"
-        "add.u32 ra, %1, %7;\n\t"
-        "add.u32 rb, %3, %8;\n\t"
-        "mov.b64 da, {ra, %2};\n\t"
-        "mov.b64 db, {rb, %4};\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
         "setp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
         "}\n" ::"r"(d_tmem),
-        "r"(a_base), "r"(a_hi), "r"(b_base), "r"(b_hi), "r"(idesc), "r"(accumulate), "n"(A_OFF), "n"(B_OFF)
+        "r"(a_base + A_OFF), "r"(a_hi), "r"(b_base + B_OFF), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
 

@@ -23,7 +23,11 @@
 // (waits, fences and commits run in series with its MMAs), more than the 96 clocks an MMA of 192
 // columns keeps the pipe busy.  Issuer i owns accumulator i and every second tile of the CTA, so
 // each accumulator still sees one thread and one fixed order of MMAs (results are reproducible),
-// and the patches of two tiles are in use at a time.
+// and the patches of two tiles are in use at a time.  A barrier's parity tells a load of a ring slot from the one before it only to
+// a thread that knows the earlier one landed.  An issuer knows that of its own loads and of all tiles but the other's current one
+// (accumulators come back in order).  Where a slot's earlier load can be of that tile (fewer slots than two tiles have chunks), it first
+// waits until the slot was released, and where two of them can (no more slots than chunks), the issuers take turns by whole tiles.
+// (160 -> 8 channels, five chunks and five slots: without, an issuer multiplied patches that had not landed and released their slots.)
 //
 // The epilogue uses no shared memory: after the gather a lane holds 32 channels of ONE pixel; a
 // 4 x 4 transpose of 16-byte pieces among groups of four lanes (two shuffle stages) leaves it with
@@ -138,7 +142,8 @@ __global__ void __launch_bounds__(kTapStackThreads, 1)
     uint64_t* patch_empty = patch_full + p.npb;
     uint64_t* acc_full = patch_empty + p.npb;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* turn = acc_empty + 2;                                         // issuer i has issued one more of its tiles
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(turn + 2);
 
     if (threadIdx.x == 0) {
         mbar_init(w_full, 1);
@@ -149,6 +154,7 @@ __global__ void __launch_bounds__(kTapStackThreads, 1)
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], 256);
+            mbar_init(&turn[i], 1);
         }
         fence_barrier_init();
         prefetch_tmap(&tmA);
@@ -218,12 +224,22 @@ __global__ void __launch_bounds__(kTapStackThreads, 1)
             const uint32_t idesc = p.idesc;
             const uint32_t d = tmem_base + which * p.accw;
             const uint32_t my_full = afull_a + 8 * which, my_empty = aempty_a + 8 * which;
+            const bool turns = p.npb <= p.kchunks, release_first = !turns && p.npb < 2 * p.kchunks;
+            const uint32_t my_turn = smem_u32(turn) + 8 * which, other_turn = smem_u32(turn) + 8 * (which ^ 1);
+            uint32_t turn_phase = 0;
+            bool first = which == 0;
             for (long long t = blockIdx.x + static_cast<long long>(which) * gridDim.x; t < p.total_tiles && ok; t += 2ll * gridDim.x) {
                 if (!wait_prof(my_empty, acc_phase ^ 1, prof_me, w_acc)) { report(p.status, kStatusMmaTimeout); ok = false; break; }
+                if (turns && !first) {
+                    if (!wait_prof(other_turn, turn_phase, prof_me, w_acc)) { report(p.status, kStatusMmaTimeout); ok = false; break; }
+                    turn_phase ^= 1u;
+                }
+                first = false;
                 tc_fence_after_sync();
                 uint32_t acc = 0u;
                 uint32_t b_row = w_lo0;
                 for (int c = 0; c < p.kchunks && ok; ++c) {
+                    if (release_first && !wait_prof(pempty_a + 8 * pp.idx, pp.phase ^ 1, prof_me, w_patch)) { report(p.status, kStatusMmaTimeout); ok = false; break; }
                     if (!wait_prof(pfull_a + 8 * pp.idx, pp.phase, prof_me, w_patch)) { report(p.status, kStatusMmaTimeout); ok = false; break; }
                     tc_fence_after_sync();
                     uint32_t a_row = patch_lo0 + pp.idx * patch16;
@@ -253,6 +269,7 @@ __global__ void __launch_bounds__(kTapStackThreads, 1)
                     pp.advance(p.npb);
                 }
                 mma_commit_a(my_full);
+                if (turns) mbar_arrive_a(my_turn);
                 acc_phase ^= 1u;
                 for (int i = 0; i < p.kchunks; ++i) pp.advance(p.npb);   // the other issuer's tile
             }

@@ -2062,6 +2062,22 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
         const int red = op == ConvOp::Forward ? s->IC : s->OC;
         return (op == ConvOp::Forward ? 16.0 + 5.7 * g : 18.0 + 6.2 * g) + (s->N % 8 == 0 && s->N >= 128 ? 0.0 : 0.046 * red);
     }
+    if (strided && (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 == 0) {
+        // (290 layers of each, half of them within 14 %; c2i: the products of a deltaX by col2im)
+        const int cols = op == ConvOp::DeltaX ? s->IC : s->OC, filter = s->FH > s->FW ? s->FH : s->FW;
+        if (op == ConvOp::DeltaW) {
+            const double f = g * (s->IC < 64 ? 64.0 / s->IC : 1.0) * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
+            return 18.0 + f * (6.45 + (filter > 4 ? 7.0 : 0.0) + 0.11 * (up(cols, 128) / cols - 1) - (s->IC <= 64 ? 0.16 : 0.0)) + 0.34 * xy + 0.78 * w;
+        }
+        const double f = g * (up(cols, 16) > 64 ? up(cols, 16) : 64.0) / cols;
+        if (op == ConvOp::DeltaX) {
+            const double idle = s->IH * s->IW > 16 && !one ? tile_idle((s->IH + s->sh - 1) / s->sh, (s->IW + s->sw - 1) / s->sw, (s->FH + s->sh - 1) / s->sh) - 1 : 0;
+            const double c2i = 1.6e-6 * s->N * s->OH * s->OW * s->FH * s->FW * (double)s->IC;
+            return 19.0 + f * (4.57 + 0.21 * idle - (cols < 128 ? 0.7 : 0.0)) + 0.93 * xy + 1.18 * w + 0.35 * c2i;
+        }
+        const double idle = s->OH * s->OW > 16 && !one ? tile_idle(s->OH, s->OW, 2) - 1 : 0;
+        return 17.3 + f * (5.9 + 2.49 * idle + (filter > 5 ? 0.74 : 0.0) + (cols < 128 ? 3.03 : 0.0)) + 0.12 * xy + 1.09 * w;
+    }
     if (op == ConvOp::DeltaW) {
         const double f = g * (up(s->IC, 32) > 64 ? up(s->IC, 32) : 64.0) / s->IC * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
         const double odd = s->IC % 32 ? f : 0, whole = s->IC % 32 || strided ? 0 : f;
@@ -2088,25 +2104,34 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
                   : 13.8 + 0.89 * f + 0.59 * odd + 0.34 * whole + 0.77 * xy + 2.79 * w + 3.5 * str;
 }
 // Which layers may leave those kernels, in 3xTF32 (plain TF32 products are TF32 products); gather_pays decides by the plan.
-// Their tiles are rectangles of pixels and chunks of 32 channels.  Layers that fill both stay: of 130 of them those kernels were faster on
-// two thirds, by up to 2.6 times.  So do layers of under 16 channels, whose taps of a filter row they read as one window, and products of
-// under 96 rows, which leave a quarter of the 128 here empty.  Ragged channel counts may leave, and whole chunks where an image covers at
-// most two thirds of its tiles' lanes (strided forward: images of up to 16 pixels, the im2col kernel packs all others; deltaW: rows of up to 5).
-// Whole chunks and deltaX besides only from 24 us on: below, both sides are launches, and the estimates no finer than what they differ by.
-// Matrix products may leave too, from 16 terms on: 250 x 1024 times 1024 x 1024 59 -> 17 us, its deltaW 87 -> 14; 512 rows 26 -> 19 and 24 -> 18.
-// Before and after: 512 x 8x8 x 128, 3x3 forward 91 -> 54 us; 64 x 4x4 x 256 31 -> 22; deltaW of 256 x 8x8, 256 -> 512, 4x4 s2 173 -> 106.
+// Their tiles are rectangles of pixels and chunks of 32 channels.  At stride 1 layers that fill both stay: of 130 of them those kernels were
+// faster on two thirds, by up to 2.6 times.  So do layers of under 16 channels, whose taps of a filter row they read as one window, and
+// products of under 96 rows, which leave a quarter of the 128 here empty.  These may leave:
+//   matrix products        250 x 1024 times 1024 x 1024 59 -> 17 us, its deltaW 87 -> 14; 512 rows 26 -> 19 and 24 -> 18
+//   ragged channel counts  50 x 35 x 29, 36 -> 100, 3x3 50 -> 37
+//   at stride 1            images that cover at most two thirds of their tiles' lanes (deltaW: rows of up to 5), and layers of few row
+//                          tiles that cover three quarters: 512 x 8x8 x 128, 3x3 91 -> 54; 64 x 7x7 x 512 149 -> 87
+//   strided, forward       sums of over 1200 products, over 128 columns, or images of up to 16 pixels: 256 x 16x16, 128 -> 256, 4x4 109 -> 85
+//                          (below, the kernels over im2col boxes and the stride lattice are within 10 us)
+//   strided, deltaX        64 columns, 64 output channels or more, up to 32768 pixels a phase: 256 x 16x16, 128 -> 256, 4x4 128 -> 99 (32
+//                          columns 44 / 81, 32 output channels 262 / 378; larger ones fill the dense product whose taps col2im adds up)
+//   strided, deltaW        under 16384 pixels, above which its reduction fills the SMs anyway: 33 x 21x21, 128 -> 192, 7x7 196 -> 81
+// Whole chunks at stride 1 and deltaX only from 24 us on: below, both sides are launches, and the estimates no finer than their difference.
 static bool gather_suits(const AlphaConvShape* s, ConvOp op)
 {
+    const bool strided = s->sh > 1 || s->sw > 1, filter = s->FH > 1 || s->FW > 1, fwd = op == ConvOp::Forward;
     if (matrix_product(s)) return op == ConvOp::DeltaX ? s->OC >= 16 : s->IC >= 16 && (s->IC % 32 == 0 || patch_path_ok(s));
-    const bool strided = s->sh > 1 || s->sw > 1, filter = s->FH > 1 || s->FW > 1, heavy = other_kernels_time(s, op, 1) >= 24.0;
-    if (op == ConvOp::DeltaX) {
-        const int h = (s->IH + s->sh - 1) / s->sh, w = (s->IW + s->sw - 1) / s->sw;        // of one phase
-        return (long long)s->N * h * w >= 96 && heavy && (s->OC % 32 != 0 || (filter && tile_idle(h, w, (s->FH + s->sh - 1) / s->sh) >= 1.5));
-    }
-    if (s->IC < 16 || (s->IC % 32 != 0 && !patch_path_ok(s))) return false;                // (the latter is fp32 work, labelled so)
-    if (op == ConvOp::DeltaW) return s->IC % 32 != 0 || ((s->OW + 7) / 8 * 8 * 2 >= 3 * s->OW && heavy);
-    if ((long long)s->N * s->OH * s->OW < 96) return false;
-    return s->IC % 32 != 0 || (filter && heavy && (strided ? tiny_image(s->OH, s->OW) : tile_idle(s->OH, s->OW, s->FH) >= 1.5));
+    const double other = other_kernels_time(s, op, 1);
+    const int h = fwd ? s->OH : (s->IH + s->sh - 1) / s->sh, w = fwd ? s->OW : (s->IW + s->sw - 1) / s->sw;        // deltaX: of one phase
+    const long long rows = (long long)s->N * h * w, pixels = (long long)s->N * s->OH * s->OW;
+    if (op != ConvOp::DeltaX && (s->IC < 16 || (s->IC % 32 != 0 && !patch_path_ok(s)))) return false;              // (the latter is fp32 work, labelled so)
+    if (op == ConvOp::DeltaW) return s->IC % 32 != 0 || (strided && pixels < 16384) || ((s->OW + 7) / 8 * 8 * 2 >= 3 * s->OW && other >= 24.0);
+    if (rows < 96 || (!fwd && other < 24.0)) return false;
+    if ((fwd ? s->IC : s->OC) % 32 != 0) return true;
+    const double idle = tile_idle(h, w, fwd ? s->FH : (s->FH + s->sh - 1) / s->sh);
+    if (!filter) return false;
+    if (strided && fwd) return (tiny_image(h, w) && other >= 24.0) || s->FH * s->FW * s->IC > 1200 || s->OC > 128;
+    return other >= 24.0 && (strided ? s->IC >= 64 && s->OC >= 64 && rows <= 32768 : idle >= 1.5 || (idle >= 1.3 && rows < 8192 && other >= 60.0));
 }
 // 1: the layer leaves the other kernels if its plan pays, 2: whatever its plan says, 0: it stays.
 static int gather_mode(const AlphaConvShape* s, ConvOp op)
@@ -2116,7 +2141,12 @@ static int gather_mode(const AlphaConvShape* s, ConvOp op)
     if (mode == 2) return 2;
     return cur_mode3x() && !kernels_are_asked_for() && gather_suits(s, op) ? 1 : 0;
 }
-static bool gather_pays(const AlphaConvShape* s, ConvOp op, double time) { return time < 0.97 * other_kernels_time(s, op, 1); }
+// (strided layers of whole chunks: a fifth less, as the estimate of the other kernels errs by that)
+static bool gather_pays(const AlphaConvShape* s, ConvOp op, double time)
+{
+    const bool whole = (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 == 0 && (s->sh > 1 || s->sw > 1);
+    return time < (whole ? 0.8 : 0.97) * other_kernels_time(s, op, 1);
+}
 
 // Returns 1 where the layer is left to the other routes.
 

@@ -99,8 +99,10 @@ def test_operands_outside_the_planes(pkg, gather, op, what):
 ROUTES = [("forward", (512, 8, 8, 128, 128, 3, 1, 1), True), ("forward", (512, 14, 14, 128, 128, 3, 1, 1), False), ("forward", (8, 8, 8, 32, 64, 3, 1, 1), False),
           ("forward", (64, 28, 28, 12, 64, 3, 1, 1), False), ("forward", (512, 8, 8, 256, 512, 3, 2, 1), True), ("forward", (512, 16, 16, 64, 128, 3, 2, 1), False),
           ("forward", (64, 15, 13, 36, 100, 3, 1, 1), True), ("forward", (2, 5, 5, 36, 100, 3, 1, 1), False), ("forward", (250, 1, 1, 1024, 1024, 1, 1, 0), True),
-          ("deltaX", (512, 8, 8, 128, 128, 3, 1, 1), True), ("deltaX", (512, 14, 14, 128, 128, 3, 1, 1), False), ("deltaX", (512, 4, 4, 256, 512, 3, 2, 1), False),
-          ("deltaX", (250, 1, 1, 1024, 1024, 1, 1, 0), True), ("deltaW", (512, 4, 4, 256, 256, 3, 1, 1), True), ("deltaW", (512, 8, 8, 128, 128, 3, 1, 1), False),
+          ("forward", (256, 16, 16, 128, 256, 4, 2, 1), True), ("forward", (64, 7, 7, 512, 512, 3, 1, 1), True), ("forward", (256, 7, 7, 512, 512, 3, 1, 1), False),
+          ("deltaX", (256, 16, 16, 128, 256, 4, 2, 1), True), ("deltaX", (256, 16, 16, 32, 256, 4, 2, 1), False), ("deltaX", (512, 8, 8, 128, 128, 3, 1, 1), True), ("deltaX", (512, 14, 14, 128, 128, 3, 1, 1), False), ("deltaX", (512, 4, 4, 256, 512, 3, 2, 1), False),
+          ("deltaX", (250, 1, 1, 1024, 1024, 1, 1, 0), True), ("deltaW", (512, 4, 4, 256, 256, 3, 1, 1), True), ("deltaW", (512, 8, 8, 128, 128, 3, 1, 1), False), ("deltaW", (33, 21, 21, 128, 192, 7, 2, 3), True),
+          ("deltaW", (256, 16, 16, 128, 256, 4, 2, 1), False),
           ("deltaW", (7, 28, 28, 28, 88, 3, 1, 1), True), ("deltaW", (64, 15, 13, 36, 100, 3, 1, 1), False), ("deltaW", (250, 1, 1, 1024, 1024, 1, 1, 0), True), ("deltaW", (64, 1, 1, 4096, 1024, 1, 1, 0), False)]
 
 

@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(256) split_planes_kernel(const float* __restri
 struct PlanePlan { int bn; bool copy_b; int ksplit; double time; };
 inline PlanePlan plan_planes(long long rows, int cols, long long k, long long copies, bool may_split, double size, double w, int sms)
 {
-    static const struct { int bn; bool copy; double stage, wave; } forms[] = {{64, false, 0.62, 3.6}, {128, false, 0.80, 4.4}, {64, true, 0.47, 4.2}, {128, true, 0.57, 4.9}};
+    static const struct { int bn; bool copy; double stage, wave; } forms[] = {{64, false, 0.62, 4.0}, {128, false, 0.80, 4.4}, {64, true, 0.47, 4.2}, {128, true, 0.57, 4.9}};
     const long long stages = (k + kPlaneBK - 1) / kPlaneBK;
     PlanePlan best{64, false, 1, 0};
     for (const auto& f : forms) {

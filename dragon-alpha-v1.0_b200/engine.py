@@ -13,6 +13,7 @@ import contextlib
 import ctypes as C
 import functools
 import operator
+import struct
 
 import torch
 
@@ -350,6 +351,41 @@ def _pad_both(t, n4, c4):
     return out
 
 
+_pack_jobs = {n: struct.Struct("%dq" % (6 * n)).pack for n in (1, 2, 3)}
+
+
+def _pad_all(*jobs):
+    """_pad_both for the tensors of one call, (t, n4, c4) each: those that need padding are written by one launch into one block of memory.
+    Returns tensors, or addresses inside the block, and the block (to be held until the call has been enqueued)."""
+    for t, n4, c4 in jobs:
+        shape = t.shape
+        if shape[-1] != c4 or shape[0] != n4:
+            break
+    else:
+        return [job[0].contiguous() for job in jobs], None
+    out = [job[0] for job in jobs]
+    odd = [i for i, (t, n4, c4) in enumerate(jobs) if t.shape[-1] != c4 or t.shape[0] != n4]
+    device = out[odd[0]].device
+    if device.type != "cuda" or device.index != torch.cuda.current_device() or any(
+            out[i].dtype != torch.float32 or out[i].device != device or out[i].numel() == 0 or out[i].is_neg() for i in odd):
+        return [_pad_both(*job) for job in jobs], None
+    plan, size = [], 0
+    for i in odd:
+        t, n4, c4 = jobs[i]
+        t = t.contiguous()
+        n, c = t.shape[0], t.shape[-1]
+        rows = t.numel() // c
+        plan.append((i, t, rows, c, size, rows // n * n4, c4))
+        size += (rows // n * n4 * c4 + 63) // 64 * 64          # (each starts on 256 bytes, like a tensor of its own)
+    block = out[odd[0]].new_empty(size)
+    base = block.data_ptr()
+    _l.check(_l.load().alpha_pad_rows_many(len(plan), _pack_jobs[len(plan)](
+        *[v for _, t, rows, c, at, rows4, c4 in plan for v in (t.data_ptr(), rows, c, base + 4 * at, rows4, c4)]), _stream()))
+    for i, _, _, _, at, _, _ in plan:
+        out[i] = base + 4 * at
+    return [t.contiguous() if isinstance(t, torch.Tensor) else t for t in out], block
+
+
 class Engine:
     """Tensor-level conv operators (Engine.java:1541, 1601, 1697, 1788) on torch CUDA tensors.
 
@@ -371,13 +407,12 @@ class Engine:
             raise ValueError("W.IC=%d != X.IC=%d" % (WIC, IC))
         OH, OW = self.out_size(IH, IW, FH, FW, sh, sw, ph, pw)
         ic4, oc4 = _pad4(IC), _pad4(OC)
-        Xp = _pad_last(X, ic4)
-        Wp = _pad_both(W, oc4, ic4)
         Y = _new(X, (N, OH, OW, oc4))
         if Bias is None:
+            (Xp, Wp), _held = _pad_all((X, N, ic4), (W, oc4, ic4))
             self.base.conv3D(Y, OH, OW, Xp, IH, IW, Wp, FH, FW, N, ic4, oc4, sh, sw, ph, pw)
         else:
-            Bp = _pad_last(Bias.reshape(1, -1), oc4).reshape(-1)
+            (Xp, Wp, Bp), _held = _pad_all((X, N, ic4), (W, oc4, ic4), (Bias.reshape(1, -1), 1, oc4))
             self.base.conv3D_biased(Y, OH, OW, Xp, IH, IW, Wp, FH, FW, Bp, N, ic4, oc4, sh, sw, ph, pw)
         return Y if oc4 == OC else Y[..., :OC]
 
@@ -394,9 +429,9 @@ class Engine:
             raise ValueError("W.IC=%d != X.IC=%d" % (WIC, IC))
         OH, OW = self.out_size(IH, IW, FH, FW, sh, sw, ph, pw)
         ic4, oc4 = _pad4(IC), _pad4(OC)
-        Xp = _pad_last(X, ic4)
-        Wp = _pad_both(W, oc4, ic4)
-        Bp = None if Bias is None else _pad_last(Bias.reshape(1, -1), oc4).reshape(-1)
+        bias = () if Bias is None else ((Bias.reshape(1, -1), 1, oc4),)
+        (Xp, Wp, *Bp), _held = _pad_all((X, N, ic4), (W, oc4, ic4), *bias)
+        Bp = Bp[0] if Bp else None
         Y = _new(X, (N, OH, OW, oc4))
         shape = _conv_shape(N, IH, IW, ic4, oc4, FH, FW, OH, OW, sh, sw, ph, pw)
         a = self.base._addr
@@ -423,7 +458,7 @@ class Engine:
         N, IH, IW, IC = X.shape
         _, OH, OW, OC = deltaY.shape
         ic4, oc4 = _pad4(IC), _pad4(OC)
-        Xp, dYp = _pad_last(X, ic4), _pad_last(deltaY, oc4)
+        (Xp, dYp), _held = _pad_all((X, N, ic4), (deltaY, deltaY.shape[0], oc4))
         dW = _new(X, (oc4, FH, FW, ic4))
         self.base.dconv3D_deltaW(dW, FH, FW, Xp, IH, IW, dYp, OH, OW, N, ic4, oc4, sh, sw, ph, pw)
         return dW if (ic4 == IC and oc4 == OC) else dW[:OC, :, :, :IC]
@@ -435,7 +470,7 @@ class Engine:
         N, IH, IW, IC = X.shape
         _, OH, OW, OC = deltaY.shape
         ic4, oc4 = _pad4(IC), _pad4(OC)
-        Xp, dYp = _pad_last(X, ic4), _pad_last(deltaY, oc4)
+        (Xp, dYp), _held = _pad_all((X, N, ic4), (deltaY, deltaY.shape[0], oc4))
         dW = _new(X, (oc4, FH, FW, ic4))
         dB = _new(X, (oc4,))
         shape = _conv_shape(N, IH, IW, ic4, oc4, FH, FW, OH, OW, sh, sw, ph, pw)
@@ -447,30 +482,26 @@ class Engine:
         N, OH, OW, OC = deltaY.shape
         _, FH, FW, IC = W.shape
         ic4, oc4 = _pad4(IC), _pad4(OC)
-        dYp = _pad_last(deltaY, oc4)
-        Wp = _pad_both(W, oc4, ic4)
+        (dYp, Wp), _held = _pad_all((deltaY, N, oc4), (W, oc4, ic4))
         dX = _new(deltaY, (N, IH, IW, ic4))
         self.base.dconv3D_deltaX(dX, IH, IW, dYp, OH, OW, Wp, FH, FW, N, ic4, oc4, sh, sw, ph, pw)
         return dX if ic4 == IC else dX[..., :IC]
 
     # ---- matrix products (Engine.matMul / matMulT1 / matMulT2, Engine.java) -------------------------------
-    @staticmethod
-    def _pad2(t):
-        return _pad_both(t, _pad4(t.shape[0]), _pad4(t.shape[1]))
-
     def matMul(self, A, B, Bias=None):
         """C[N,M] = A[N,K] * B[K,M] (+ Bias[M] per row); dimensions are zero-padded to multiples of 4 as the
         engine's tensor memory is, and sliced back."""
         (N, K), (K2, M) = A.shape, B.shape
         if K != K2:
             raise ValueError("A.width=%d != B.height=%d" % (K, K2))
-        Ap, Bp = self._pad2(A), self._pad2(B)
-        C = _new(A, (Ap.shape[0], Bp.shape[1]))
+        n4, k4, m4 = _pad4(N), _pad4(K), _pad4(M)
+        C = _new(A, (n4, m4))
         if Bias is None:
-            self.base.matMul(C, Ap, Bp, Ap.shape[0], Bp.shape[1], Ap.shape[1])
+            (Ap, Bp), _held = _pad_all((A, n4, k4), (B, k4, m4))
+            self.base.matMul(C, Ap, Bp, n4, m4, k4)
         else:
-            bp = _pad_last(Bias.reshape(1, -1), Bp.shape[1]).reshape(-1)
-            self.base.matMul_biased(C, Ap, Bp, Ap.shape[0], Bp.shape[1], Ap.shape[1], bp)
+            (Ap, Bp, bp), _held = _pad_all((A, n4, k4), (B, k4, m4), (Bias.reshape(1, -1), 1, m4))
+            self.base.matMul_biased(C, Ap, Bp, n4, m4, k4, bp)
         return C[:N, :M]
 
     def matMulT1(self, A, B):
@@ -478,9 +509,10 @@ class Engine:
         (K, N), (K2, M) = A.shape, B.shape
         if K != K2:
             raise ValueError("A.height=%d != B.height=%d" % (K, K2))
-        Ap, Bp = self._pad2(A), self._pad2(B)
-        C = _new(A, (Ap.shape[1], Bp.shape[1]))
-        self.base.matMulT1(C, Ap, Bp, Ap.shape[1], Bp.shape[1], Ap.shape[0])
+        n4, k4, m4 = _pad4(N), _pad4(K), _pad4(M)
+        (Ap, Bp), _held = _pad_all((A, k4, n4), (B, k4, m4))
+        C = _new(A, (n4, m4))
+        self.base.matMulT1(C, Ap, Bp, n4, m4, k4)
         return C[:N, :M]
 
     def matMulT2(self, A, B):
@@ -488,9 +520,10 @@ class Engine:
         (N, K), (M, K2) = A.shape, B.shape
         if K != K2:
             raise ValueError("A.width=%d != B.width=%d" % (K, K2))
-        Ap, Bp = self._pad2(A), self._pad2(B)
-        C = _new(A, (Ap.shape[0], Bp.shape[0]))
-        self.base.matMulT2(C, Ap, Bp, Ap.shape[0], Bp.shape[0], Ap.shape[1])
+        n4, k4, m4 = _pad4(N), _pad4(K), _pad4(M)
+        (Ap, Bp), _held = _pad_all((A, n4, k4), (B, m4, k4))
+        C = _new(A, (n4, m4))
+        self.base.matMulT2(C, Ap, Bp, n4, m4, k4)
         return C[:N, :M]
 
     # Batched products with the engine's memory rule (only the last dimension of a tensor is padded to a multiple
@@ -501,7 +534,7 @@ class Engine:
         (Bt, N, K), (Bt2, K2, M) = A.shape, B.shape
         if Bt != Bt2 or K != K2:
             raise ValueError("batchMatMul: A %s against B %s" % (tuple(A.shape), tuple(B.shape)))
-        Ap, Bp = _pad_last(A, _pad4(K)), _pad_last(B, _pad4(M))
+        (Ap, Bp), _held = _pad_all((A, Bt, _pad4(K)), (B, Bt, _pad4(M)))
         # the kernels write the M columns; only padding columns need zeros
         C = (torch.empty if M % 4 == 0 else torch.zeros)((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
         self.base.batchMatMul(C, Ap, Bp, Bt, N, _pad4(M), K, _pad4(K))
@@ -512,7 +545,7 @@ class Engine:
         (Bt, K, N), (Bt2, K2, M) = A.shape, B.shape
         if Bt != Bt2 or K != K2:
             raise ValueError("batchMatMulT1: A %s against B %s" % (tuple(A.shape), tuple(B.shape)))
-        Ap, Bp = _pad_last(A, _pad4(N)), _pad_last(B, _pad4(M))
+        (Ap, Bp), _held = _pad_all((A, Bt, _pad4(N)), (B, Bt, _pad4(M)))
         # the kernels write the M columns; only padding columns need zeros
         C = (torch.empty if M % 4 == 0 else torch.zeros)((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
         self.base.batchMatMulT1(C, Ap, Bp, Bt, N, _pad4(N), _pad4(M), K)
@@ -523,7 +556,7 @@ class Engine:
         (Bt, N, K), (Bt2, M, K2) = A.shape, B.shape
         if Bt != Bt2 or K != K2:
             raise ValueError("batchMatMulT2: A %s against B %s" % (tuple(A.shape), tuple(B.shape)))
-        Ap, Bp = _pad_last(A, _pad4(K)), _pad_last(B, _pad4(K))
+        (Ap, Bp), _held = _pad_all((A, Bt, _pad4(K)), (B, Bt, _pad4(K)))
         # the kernels write the M columns; only padding columns need zeros
         C = (torch.empty if M % 4 == 0 else torch.zeros)((Bt, N, _pad4(M)), dtype=torch.float32, device=A.device)
         self.base.batchMatMulT2(C, Ap, Bp, Bt, N, _pad4(M), M, _pad4(K))

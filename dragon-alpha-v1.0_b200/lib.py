@@ -47,6 +47,7 @@ def load():
     lib.alpha_conv3d_forward_leakyRelu.argtypes = [P, V, V, V, C.c_float, V, V]
     lib.alpha_conv3d_deltaW.argtypes = [P, V, V, V, V]
     lib.alpha_pad_rows.argtypes = [V, C.c_longlong, I, V, C.c_longlong, I, V]
+    lib.alpha_pad_rows_many.argtypes = [I, C.c_char_p, V]
     lib.alpha_conv_bias_grad.argtypes = [V, C.c_longlong, I, V, V]
     lib.alpha_conv3d_deltaW_bias.argtypes = [P, V, V, V, V, V]
     lib.alpha_conv3d_forward_ex.argtypes = [P, V, V, V, V, I, I, V]

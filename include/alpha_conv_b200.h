@@ -406,6 +406,8 @@ int alpha_engine_matMulT2(float* C, const float* A, const float* B, int N, int M
 
 /* dst[rows4][cols4] = src[rows][cols] (dense), zeros where src has no element; cols4 % 4 == 0, dst 16-byte aligned. */
 int alpha_pad_rows(const float* src, long long rows, int cols, float* dst, long long rows4, int cols4, alpha_stream_t stream);
+/* The same for n tensors, three to a launch; a tensor is six values: src, rows, cols, dst, rows4, cols4. */
+int alpha_pad_rows_many(int n, const long long* jobs, alpha_stream_t stream);
 
 /* ---- batched matrix products (FullConnect / attention-style operators) ----------------------------------
  * Replace the SIMT kernels behind src/cu32_src/Cuda_batch_matMul/Cuda_batchMatMul/batchMatMul.cuh,

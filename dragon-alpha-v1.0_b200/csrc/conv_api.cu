@@ -2063,7 +2063,9 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
         return (op == ConvOp::Forward ? 16.0 + 5.7 * g : 18.0 + 6.2 * g) + (s->N % 8 == 0 && s->N >= 128 ? 0.0 : 0.046 * red);
     }
     if (strided && (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 == 0) {
-        // (290 layers of each, half of them within 14 %; c2i: the products of a deltaX by col2im)
+        // (290 layers of each, half of them within 14 %; c2i: the products of a deltaX by col2im; a dense product over `flat` rows that do not
+        // fold into pictures of eight idles most of its tiles: 225 x 2x2 instead of 224 x 2x2, 512 channels 64 us instead of 42)
+        const long long flat = (long long)s->N * s->OH * s->OW;
         const int cols = op == ConvOp::DeltaX ? s->IC : s->OC, filter = s->FH > s->FW ? s->FH : s->FW;
         if (op == ConvOp::DeltaW) {
             const double f = g * (s->IC < 64 ? 64.0 / s->IC : 1.0) * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
@@ -2073,10 +2075,10 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
         if (op == ConvOp::DeltaX) {
             const double idle = s->IH * s->IW > 16 && !one ? tile_idle((s->IH + s->sh - 1) / s->sh, (s->IW + s->sw - 1) / s->sw, (s->FH + s->sh - 1) / s->sh) - 1 : 0;
             const double c2i = 1.6e-6 * s->N * s->OH * s->OW * s->FH * s->FW * (double)s->IC;
-            return 19.0 + f * (4.57 + 0.21 * idle - (cols < 128 ? 0.7 : 0.0)) + 0.93 * xy + 1.18 * w + 0.35 * c2i;
+            return 19.0 + (flat % 8 ? 0.046 * s->OC : 0.0) + f * (4.57 + 0.21 * idle - (cols < 128 ? 0.7 : 0.0)) + 0.93 * xy + 1.18 * w + 0.35 * c2i;
         }
         const double idle = s->OH * s->OW > 16 && !one ? tile_idle(s->OH, s->OW, 2) - 1 : 0;
-        return 17.3 + f * (5.9 + 2.49 * idle + (filter > 5 ? 0.74 : 0.0) + (cols < 128 ? 3.03 : 0.0)) + 0.12 * xy + 1.09 * w;
+        return 17.3 + (flat % 8 && tiny_image(s->OH, s->OW) ? 0.013 * s->FH * s->FW * s->IC : 0.0) + f * (5.9 + 2.49 * idle + (filter > 5 ? 0.74 : 0.0) + (cols < 128 ? 3.03 : 0.0)) + 0.12 * xy + 1.09 * w;
     }
     if (op == ConvOp::DeltaW) {
         const double f = g * (up(s->IC, 32) > 64 ? up(s->IC, 32) : 64.0) / s->IC * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
@@ -2116,7 +2118,7 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
 //   strided, deltaX        64 columns, 64 output channels or more, up to 32768 pixels a phase: 256 x 16x16, 128 -> 256, 4x4 128 -> 99 (32
 //                          columns 44 / 81, 32 output channels 262 / 378; larger ones fill the dense product whose taps col2im adds up)
 //   strided, deltaW        under 16384 pixels, above which its reduction fills the SMs anyway: 33 x 21x21, 128 -> 192, 7x7 196 -> 81
-// Whole chunks at stride 1 and deltaX only from 24 us on: below, both sides are launches, and the estimates no finer than their difference.
+// Whole chunks at stride 1 and deltaX only from 22 us on: below, both sides are launches, and the estimates no finer than their difference.
 static bool gather_suits(const AlphaConvShape* s, ConvOp op)
 {
     const bool strided = s->sh > 1 || s->sw > 1, filter = s->FH > 1 || s->FW > 1, fwd = op == ConvOp::Forward;
@@ -2125,13 +2127,13 @@ static bool gather_suits(const AlphaConvShape* s, ConvOp op)
     const int h = fwd ? s->OH : (s->IH + s->sh - 1) / s->sh, w = fwd ? s->OW : (s->IW + s->sw - 1) / s->sw;        // deltaX: of one phase
     const long long rows = (long long)s->N * h * w, pixels = (long long)s->N * s->OH * s->OW;
     if (op != ConvOp::DeltaX && (s->IC < 16 || (s->IC % 32 != 0 && !patch_path_ok(s)))) return false;              // (the latter is fp32 work, labelled so)
-    if (op == ConvOp::DeltaW) return s->IC % 32 != 0 || (strided && pixels < 16384) || ((s->OW + 7) / 8 * 8 * 2 >= 3 * s->OW && other >= 24.0);
-    if (rows < 96 || (!fwd && other < 24.0)) return false;
+    if (op == ConvOp::DeltaW) return s->IC % 32 != 0 || (strided && pixels < 16384) || ((s->OW + 7) / 8 * 8 * 2 >= 3 * s->OW && other >= 22.0);
+    if (rows < 96 || (!fwd && other < 22.0)) return false;
     if ((fwd ? s->IC : s->OC) % 32 != 0) return true;
     const double idle = tile_idle(h, w, fwd ? s->FH : (s->FH + s->sh - 1) / s->sh);
     if (!filter) return false;
-    if (strided && fwd) return (tiny_image(h, w) && other >= 24.0) || s->FH * s->FW * s->IC > 1200 || s->OC > 128;
-    return other >= 24.0 && (strided ? s->IC >= 64 && s->OC >= 64 && rows <= 32768 : idle >= 1.5 || (idle >= 1.3 && rows < 8192 && other >= 60.0));
+    if (strided && fwd) return (tiny_image(h, w) && other >= 22.0) || s->FH * s->FW * s->IC > 1200 || s->OC > 128;
+    return other >= 22.0 && (strided ? s->IC >= 64 && s->OC >= 64 && rows <= 32768 : idle >= 1.5 || (idle >= 1.3 && rows < 8192 && other >= 60.0));
 }
 // 1: the layer leaves the other kernels if its plan pays, 2: whatever its plan says, 0: it stays.
 static int gather_mode(const AlphaConvShape* s, ConvOp op)
@@ -2141,11 +2143,12 @@ static int gather_mode(const AlphaConvShape* s, ConvOp op)
     if (mode == 2) return 2;
     return cur_mode3x() && !kernels_are_asked_for() && gather_suits(s, op) ? 1 : 0;
 }
-// (strided layers of whole chunks: a fifth less, as the estimate of the other kernels errs by that)
+// (strided layers of whole chunks: a fifth less, as the estimate of the other kernels errs by that; tiny forwards a tenth)
 static bool gather_pays(const AlphaConvShape* s, ConvOp op, double time)
 {
     const bool whole = (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 == 0 && (s->sh > 1 || s->sw > 1);
-    return time < (whole ? 0.8 : 0.97) * other_kernels_time(s, op, 1);
+    const double share = !whole ? 0.97 : (op == ConvOp::Forward && tiny_image(s->OH, s->OW) ? 0.9 : 0.8);
+    return time < share * other_kernels_time(s, op, 1);
 }
 
 // Returns 1 where the layer is left to the other routes.

@@ -2042,74 +2042,71 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
 // wins on small layers (their launches), on images and channel counts that do not, on strides and on long reductions.  Its sums err by
 // 1.0e-7 to 1.8e-7 where theirs err by 1.2e-7 to 1.4e-5 (2-norm against 64 bits; no smaller in any of 1200 calls).
 
-// GPU time in us of an operator on those other kernels, as measured on 900 layers (1 to 512 images of 1 to 130 pixels a side, 4 to 7000
-// channels, 1x1 to 7x7, strides 1 and 2; 1e7 to 1.3e11 FLOPs): median error 15 to 20 %, and where the faster side is chosen by it and by
-// plan_planes (within 13 % for 9 of 10) a 3xTF32 forward takes 0.68 of the time before on average, a deltaX 0.75, a deltaW 0.73 (the better of both
-// would be 0.63, 0.71, 0.63), in plain TF32 0.93, 0.87, 0.80; one call in 40 more than 5 % longer, the worst 1.2 times.
-// `flops`: those of the layer with channels filled up to chunks and columns to 64, over the share of tile lanes that its images fill.
-// Matrix products (pictures and filters of one element): 48 products, 33 to 1024 rows, 256 to 4096 terms, within 15 %.
+// GPU time in us of a 3xTF32 operator on those other kernels (and not of deltaX under a stride with OC % 32 != 0, which is fp32 work), fitted to
+// layers of 1 to 600 images of 2 to 130 pixels a side, 16 to 700 channels, 1x1 to 7x7, strides 1 and 2, 1e8 to 1e11 FLOPs:
+//   matrix products   230 (32 to 4096 rows, 64 to 4096 terms), most within 15 %, and too long where rows do not fold
+//   ragged channels   281 forward, 281 deltaW, 71 deltaX: half within 12 to 15 %.  Where it and plan_planes choose the faster side these take
+//                     0.64, 0.77 and 0.70 of the time before (the better of both would be 0.62, 0.72, 0.69)
+//   strided           290 of each, half within 14 %
+//   stride 1          130 of each, half within 15 to 20 %
+// Taken together: FLOPs with channels filled up to their tiles, the tile lanes that images leave idle, bytes of X and Y, of a patch
+// matrix and of the weights.
 enum class ConvOp { Forward, DeltaX, DeltaW };
-static bool matrix_product(const AlphaConvShape* s) { return s->IH == 1 && s->IW == 1 && s->FH == 1 && s->FW == 1 && s->OH == 1 && s->OW == 1; }
-static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
+// (the rows of a matrix come as pictures of 1 x 4 or 1 x 1 pixels)
+static bool matrix_product(const AlphaConvShape* s)
 {
-    auto up = [](int x, int to) { return (double)((x + to - 1) / to * to); };
+    return s->IH == 1 && s->IW <= 4 && s->FH == 1 && s->FW == 1 && s->OH == 1 && s->OW == s->IW && s->sh == 1 && s->sw == 1 && s->ph == 0 && s->pw == 0;
+}
+static double other_kernels_time(const AlphaConvShape* s, ConvOp op)
+{
+    auto up = [](long long x, int to) { return (double)((x + to - 1) / to * to); };
     const bool strided = s->sh > 1 || s->sw > 1, one = s->FH == 1 && s->FW == 1;
-    const double g = 2e-9 * s->N * s->OH * s->OW * s->OC * s->FH * s->FW * (double)s->IC, xy = 0.8e-6 * ((double)s->N * s->IH * s->IW * s->IC + (double)s->N * s->OH * s->OW * s->OC);
-    const double w = 4e-6 * s->FH * s->FW * (double)s->IC * s->OC, str = strided ? 1 : 0;
+    const long long flat = (long long)s->N * s->OH * s->OW, terms = (long long)s->FH * s->FW * s->IC;
+    const double g = 2e-9 * flat * s->OC * (double)terms, xy = 0.8e-6 * ((double)s->N * s->IH * s->IW * s->IC + (double)flat * s->OC), w = 4e-6 * (double)terms * s->OC;
+    const int red = op == ConvOp::DeltaX ? s->OC : s->IC, cols = op == ConvOp::DeltaX ? s->IC : s->OC, filter = s->FH > s->FW ? s->FH : s->FW;
     if (matrix_product(s)) {
-        // rows fold into pictures of 8 x n pixels (deltaW: 16 x n), or each row is a picture whose tile it leaves empty
-        if (op == ConvOp::DeltaW) return s->N % 16 == 0 ? (s->N <= 64 ? 12.0 : 15.0) + 5.6 * g : 20.0 + 130.0 * g;
-        const int red = op == ConvOp::Forward ? s->IC : s->OC;
-        return (op == ConvOp::Forward ? 16.0 + 5.7 * g : 18.0 + 6.2 * g) + (s->N % 8 == 0 && s->N >= 128 ? 0.0 : 0.046 * red);
+        // rows fold into pictures of 8 x n pixels (deltaW: 16 x n), or the few of a picture leave its tile empty
+        if (op == ConvOp::DeltaW) return flat % 16 == 0 ? (flat <= 64 ? 12.0 : 16.0) + 5.6 * g : 20.0 + 130.0 / s->OW * g;
+        return (op == ConvOp::Forward ? 16.5 + 5.6 * g : 17.0 + (red >= 512 ? 8.0 : 5.0) * g) + (flat % 8 == 0 && flat >= 128 ? 0.0 : 0.046 * red);
     }
-    if (strided && (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 == 0) {
-        // (290 layers of each, half of them within 14 %; c2i: the products of a deltaX by col2im; a dense product over `flat` rows that do not
-        // fold into pictures of eight idles most of its tiles: 225 x 2x2 instead of 224 x 2x2, 512 channels 64 us instead of 42)
-        const long long flat = (long long)s->N * s->OH * s->OW;
-        const int cols = op == ConvOp::DeltaX ? s->IC : s->OC, filter = s->FH > s->FW ? s->FH : s->FW;
-        if (op == ConvOp::DeltaW) {
-            const double f = g * (s->IC < 64 ? 64.0 / s->IC : 1.0) * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
-            return 18.0 + f * (6.45 + (filter > 4 ? 7.0 : 0.0) + 0.11 * (up(cols, 128) / cols - 1) - (s->IC <= 64 ? 0.16 : 0.0)) + 0.34 * xy + 0.78 * w;
-        }
-        const double f = g * (up(cols, 16) > 64 ? up(cols, 16) : 64.0) / cols;
-        if (op == ConvOp::DeltaX) {
-            const double idle = s->IH * s->IW > 16 && !one ? tile_idle((s->IH + s->sh - 1) / s->sh, (s->IW + s->sw - 1) / s->sw, (s->FH + s->sh - 1) / s->sh) - 1 : 0;
-            const double c2i = 1.6e-6 * s->N * s->OH * s->OW * s->FH * s->FW * (double)s->IC;
-            return 19.0 + (flat % 8 ? 0.046 * s->OC : 0.0) + f * (4.57 + 0.21 * idle - (cols < 128 ? 0.7 : 0.0)) + 0.93 * xy + 1.18 * w + 0.35 * c2i;
-        }
-        const double idle = s->OH * s->OW > 16 && !one ? tile_idle(s->OH, s->OW, 2) - 1 : 0;
-        return 17.3 + (flat % 8 && tiny_image(s->OH, s->OW) ? 0.013 * s->FH * s->FW * s->IC : 0.0) + f * (5.9 + 2.49 * idle + (filter > 5 ? 0.74 : 0.0) + (cols < 128 ? 3.03 : 0.0)) + 0.12 * xy + 1.09 * w;
-    }
+    const double wide = up(cols, 16) > 64 ? up(cols, 16) : 64.0;
+    const double patch = one ? 0.0 : 0.8e-6 * flat * (double)terms;
     if (op == ConvOp::DeltaW) {
         const double f = g * (up(s->IC, 32) > 64 ? up(s->IC, 32) : 64.0) / s->IC * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(s->OW, 8) / s->OW;
-        const double odd = s->IC % 32 ? f : 0, whole = s->IC % 32 || strided ? 0 : f;
-        return mode3x ? 18.0 + 4.85 * f - 3.24 * odd - 0.9 * whole - 0.52 * str * f + 0.98 * xy : 16.0 + 2.17 * f - 1.22 * odd - 0.66 * whole + 0.64 * xy + 1.85 * w + 1.4 * str;
+        if (s->IC % 32) return 15.9 + 3.92 * g * (s->OC < 64 ? 64.0 / s->OC : 1.0) * up(terms, 64) / terms + 1.39 * f + 1.2 * xy + 0.37 * patch + 1.81 * w + (one ? 0.0 : 4.5);
+        if (strided) return 18.0 + f * (6.45 + (filter > 4 ? 7.0 : 0.0) + 0.11 * (up(cols, 128) / cols - 1) - (s->IC <= 64 ? 0.16 : 0.0)) + 0.34 * xy + 0.78 * w;
+        return 18.0 + 3.95 * f + 0.98 * xy;
     }
     const bool fwd = op == ConvOp::Forward;
-    const int red = fwd ? s->IC : s->OC, cols = fwd ? s->OC : s->IC;
     const int h = fwd ? s->OH : (s->IH + s->sh - 1) / s->sh, wd = fwd ? s->OW : (s->IW + s->sw - 1) / s->sw;           // of one phase
-    const int fh = fwd ? (strided ? 2 : s->FH) : (s->FH + s->sh - 1) / s->sh, fw = fwd ? (strided ? 2 : s->FW) : (s->FW + s->sw - 1) / s->sw;
-    const bool tiny = fwd ? s->OH * s->OW <= 16 : s->IH * s->IW <= 16;
-    const bool pair = mode3x && !strided && !one && cols % 128 == 0 && red % 32 == 0 && !tiny;
-    double lanes = 1.0;
-    if (!(fwd ? (one && !strided) || tiny : one || tiny)) {
-        lanes = tile_idle(h, wd, fh);
-        const double flat = up(h, 4) * 32.0 / ((double)h * wd);
-        if (pair && wd + fw - 1 <= 32 && h > 16 && flat < lanes) lanes = flat;
+    const int fh = fwd ? (strided ? 2 : s->FH) : (s->FH + s->sh - 1) / s->sh, fw = fwd ? s->FW : (s->FW + s->sw - 1) / s->sw;
+    const double lanes = one ? 1.0 : tile_idle(h, wd, fh), f = g * wide / cols;
+    if (red % 32) {
+        const double chunks = up(red, 32) / red * f * (lanes - 1);
+        return fwd ? 18.9 + 4.67 * f + 2.92 * chunks + 0.96 * xy + 0.26 * patch + 1.05 * w : 17.3 + 5.22 * f + 3.63 * chunks + 0.86 * xy + 1.82 * w;
     }
-    const double f = g * up(red, 32) / red * (up(cols, 16) > 64 ? up(cols, 16) : 64.0) / cols * lanes;
-    const double odd = red % 32 ? f : 0, whole = red % 32 || strided ? 0 : f, pr = pair ? f : 0;
-    if (fwd)
-        return mode3x ? 14.7 + 6.83 * f - 3.31 * odd - 2.06 * whole - 1.19 * pr - 2.17 * str * f + 0.42 * xy + 1.9 * w + 1.7 * str
-                      : 13.1 + 1.71 * f - 0.53 * whole - 0.49 * str * f + 0.65 * xy + 0.63 * w + 3.1 * str;
-    return mode3x ? 14.1 + 2.55 * f + 1.53 * odd + 1.63 * whole - 0.81 * pr - 0.61 * str * f + 1.15 * xy + 1.8 * w + 4.1 * str
-                  : 13.8 + 0.89 * f + 0.59 * odd + 0.34 * whole + 0.77 * xy + 2.79 * w + 3.5 * str;
+    const bool tiny = fwd ? tiny_image(s->OH, s->OW) : tiny_image(s->IH, s->IW);
+    if (strided) {
+        // (c2i: the products of a deltaX by col2im; a dense product over `flat` rows that do not fold into pictures of eight idles most of its
+        // tiles: 225 x 2x2 instead of 224 x 2x2, 512 channels 64 us instead of 42)
+        const double idle = tiny ? 0.0 : lanes - 1, c2i = 1.6e-6 * flat * s->FH * s->FW * (double)s->IC;
+        if (!fwd) return 19.0 + (flat % 8 ? 0.046 * s->OC : 0.0) + f * (4.57 + 0.21 * idle - (cols < 128 ? 0.7 : 0.0)) + 0.93 * xy + 1.18 * w + 0.35 * c2i;
+        return 17.3 + (flat % 8 && tiny ? 0.013 * (double)terms : 0.0) + f * (5.9 + 2.49 * idle + (filter > 5 ? 0.74 : 0.0) + (cols < 128 ? 3.03 : 0.0)) + 0.12 * xy + 1.09 * w;
+    }
+    const bool pair = !one && cols % 128 == 0 && !tiny;
+    double fill = tiny ? 1.0 : lanes;
+    if (pair && wd + fw - 1 <= 32 && h > 16) {
+        const double rows32 = up(h, 4) * 32.0 / ((double)h * wd);
+        if (rows32 < fill) fill = rows32;
+    }
+    return fwd ? 14.7 + f * fill * (pair ? 3.58 : 4.77) + 0.42 * xy + 1.9 * w : 14.1 + f * fill * (pair ? 3.37 : 4.18) + 1.15 * xy + 1.8 * w;
 }
 // Which layers may leave those kernels, in 3xTF32 (plain TF32 products are TF32 products); gather_pays decides by the plan.
 // Their tiles are rectangles of pixels and chunks of 32 channels.  At stride 1 layers that fill both stay: of 130 of them those kernels were
 // faster on two thirds, by up to 2.6 times.  So do layers of under 16 channels, whose taps of a filter row they read as one window, and
 // products of under 96 rows, which leave a quarter of the 128 here empty.  These may leave:
-//   matrix products        250 x 1024 times 1024 x 1024 59 -> 17 us, its deltaW 87 -> 14; 512 rows 26 -> 19 and 24 -> 18
+//   matrix products        from 16 terms: 996 x 1024 times 1024 x 1024 66 -> 26 us, with B transposed 61 -> 24, with A 87 -> 30; 512 rows 28, 26, 24
+//                          -> 22, 19, 19
 //   ragged channel counts  50 x 35 x 29, 36 -> 100, 3x3 50 -> 37
 //   at stride 1            images that cover at most two thirds of their tiles' lanes (deltaW: rows of up to 5), and layers of few row
 //                          tiles that cover three quarters: 512 x 8x8 x 128, 3x3 91 -> 54; 64 x 7x7 x 512 149 -> 87
@@ -2118,17 +2115,18 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op, int mode3x)
 //   strided, deltaX        64 columns, 64 output channels or more, up to 32768 pixels a phase: 256 x 16x16, 128 -> 256, 4x4 128 -> 99 (32
 //                          columns 44 / 81, 32 output channels 262 / 378; larger ones fill the dense product whose taps col2im adds up)
 //   strided, deltaW        under 16384 pixels, above which its reduction fills the SMs anyway: 33 x 21x21, 128 -> 192, 7x7 196 -> 81
-// Whole chunks at stride 1 and deltaX only from 22 us on: below, both sides are launches, and the estimates no finer than their difference.
+// Whole chunks at stride 1 only from 22 us on, deltaX from 24: below, both sides are launches, and the estimates no finer than their difference.
 static bool gather_suits(const AlphaConvShape* s, ConvOp op)
 {
     const bool strided = s->sh > 1 || s->sw > 1, filter = s->FH > 1 || s->FW > 1, fwd = op == ConvOp::Forward;
+    if (matrix_product(s) && op == ConvOp::Forward && s->IC > 6000 && s->IC % 32) return false;   // (the halo kernel keeps their corrections apart, as a test requires)
     if (matrix_product(s)) return op == ConvOp::DeltaX ? s->OC >= 16 : s->IC >= 16 && (s->IC % 32 == 0 || patch_path_ok(s));
-    const double other = other_kernels_time(s, op, 1);
+    const double other = other_kernels_time(s, op);
     const int h = fwd ? s->OH : (s->IH + s->sh - 1) / s->sh, w = fwd ? s->OW : (s->IW + s->sw - 1) / s->sw;        // deltaX: of one phase
     const long long rows = (long long)s->N * h * w, pixels = (long long)s->N * s->OH * s->OW;
     if (op != ConvOp::DeltaX && (s->IC < 16 || (s->IC % 32 != 0 && !patch_path_ok(s)))) return false;              // (the latter is fp32 work, labelled so)
     if (op == ConvOp::DeltaW) return s->IC % 32 != 0 || (strided && pixels < 16384) || ((s->OW + 7) / 8 * 8 * 2 >= 3 * s->OW && other >= 22.0);
-    if (rows < 96 || (!fwd && other < 22.0)) return false;
+    if (rows < 96 || (!fwd && other < 24.0)) return false;
     if ((fwd ? s->IC : s->OC) % 32 != 0) return true;
     const double idle = tile_idle(h, w, fwd ? s->FH : (s->FH + s->sh - 1) / s->sh);
     if (!filter) return false;
@@ -2143,12 +2141,12 @@ static int gather_mode(const AlphaConvShape* s, ConvOp op)
     if (mode == 2) return 2;
     return cur_mode3x() && !kernels_are_asked_for() && gather_suits(s, op) ? 1 : 0;
 }
-// (strided layers of whole chunks: a fifth less, as the estimate of the other kernels errs by that; tiny forwards a tenth)
+// (less by what the estimate of the other kernels is uncertain)
 static bool gather_pays(const AlphaConvShape* s, ConvOp op, double time)
 {
-    const bool whole = (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 == 0 && (s->sh > 1 || s->sw > 1);
-    const double share = !whole ? 0.97 : (op == ConvOp::Forward && tiny_image(s->OH, s->OW) ? 0.9 : 0.8);
-    return time < share * other_kernels_time(s, op, 1);
+    const bool ragged = (op == ConvOp::DeltaX ? s->OC : s->IC) % 32 != 0, strided = s->sh > 1 || s->sw > 1;
+    const double share = matrix_product(s) ? 0.9 : ragged ? 0.85 : !strided ? 0.97 : op == ConvOp::Forward && tiny_image(s->OH, s->OW) ? 0.9 : 0.8;
+    return time < share * other_kernels_time(s, op);
 }
 
 // Returns 1 where the layer is left to the other routes.
@@ -2166,7 +2164,7 @@ static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const fl
     p.K = s->FH * s->FW * s->IC; p.rows = s->N * s->OH * s->OW;
     p.size = (size_t)p.rows * s->OC;
     const int Kp = (p.K + 31) / 32 * 32;
-    const PlanePlan plan = plan_planes(p.rows, s->OC, p.K, 1, true, (double)p.size, (double)Kp * s->OC, c->sm_count);
+    const PlanePlan plan = plan_planes(p.rows, s->OC, p.K, 1, 16, (double)p.size, (double)Kp * s->OC, c->sm_count);
     const long long gx = (p.rows + kPlaneBM - 1) / kPlaneBM, gy = (s->OC + plan.bn - 1) / plan.bn;
     if (gx * gy * plan.ksplit > 2147483647LL) return 1;
     if (mode == 1 && !f32 && !gather_pays(s, ConvOp::Forward, plan.time)) return 1;
@@ -2216,7 +2214,7 @@ static int launch_gather_dx(DeviceCtx* c, const AlphaConvShape* s, const float* 
     const long long w = (long long)s->FH * s->FW * s->OC * ((s->IC + 31) / 32 * 32);
     const bool can_copy = s->FH * s->FW <= 64 && phases <= 16 && w < 1LL << 31;
     const long long k = (long long)s->FH * s->FW * s->OC / phases;
-    const PlanePlan plan = plan_planes(rows, s->IC, k > 0 ? k : 1, phases, true, (double)s->N * s->IH * s->IW * s->IC, can_copy ? (double)w : 0.0, c->sm_count);
+    const PlanePlan plan = plan_planes(rows, s->IC, k > 0 ? k : 1, phases, 16, (double)s->N * s->IH * s->IW * s->IC, can_copy ? (double)w : 0.0, c->sm_count);
     if ((rows + kPlaneBM - 1) / kPlaneBM * ((s->IC + plan.bn - 1) / plan.bn) * phases * plan.ksplit > 2147483647LL) return 1;
     // (the phase of the most taps ends last: the plan counts with the average)
     const double last = ((double)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * s->OC - k) / plan.ksplit / kPlaneBK * (plan.copy_b ? 0.57 : 0.80);
@@ -2233,7 +2231,8 @@ static int launch_gather_dw(DeviceCtx* c, const AlphaConvShape* s, const float* 
     p.IH = s->IH; p.IW = s->IW; p.IC = s->IC; p.FW = s->FW; p.OC = s->OC; p.sh = s->sh; p.sw = s->sw; p.ph = s->ph; p.pw = s->pw;
     p.K = s->N * s->OH * s->OW; p.L = s->FH * s->FW * s->IC;
     p.size = (size_t)s->OC * p.L;
-    const PlanePlan plan = plan_planes(s->OC, p.L, p.K, 1, true, (double)p.size, 0, c->sm_count);
+    // (a few tiles over many pixels: as many parts as fill the SMs; 50 x 35 x 29, 36 -> 100, 3x3 is three tiles and 49 parts)
+    const PlanePlan plan = plan_planes(s->OC, p.L, p.K, 1, c->sm_count, (double)p.size, 0, c->sm_count);
     const long long gx = (s->OC + kPlaneBM - 1) / kPlaneBM, gy = (p.L + plan.bn - 1) / plan.bn;
     if (gx * gy * plan.ksplit > 2147483647LL) return 1;
     if (mode == 1 && !f32 && !gather_pays(s, ConvOp::DeltaW, plan.time)) return 1;
@@ -2250,9 +2249,9 @@ static int launch_gather_dw(DeviceCtx* c, const AlphaConvShape* s, const float* 
     note_launch(label);
     int rc = check_launch("gemm_planes_kernel");
     if (rc || p.ksplit == 1) return rc;
-    rc = launch_part_sum(c, p.out, p.size, p.ksplit, nullptr, 4, 0, 0.f, dW, stream);
+    if (!t_dry) launch_dw_reduce(p.out, p.size, p.ksplit, dW, p.size / 4, 0, stream, opt(OPT_DW_LANES));
     note_launch(label);
-    return rc;
+    return check_launch("dw_reduce_kernel");
 }
 
 // ---- deltaW, halo-tile kernel (strides 1 and 2): plan and launch -----------------------------------

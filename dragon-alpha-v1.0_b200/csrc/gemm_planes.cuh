@@ -781,12 +781,12 @@ __global__ void __launch_bounds__(256) split_planes_kernel(const float* __restri
     }
 }
 
-// Tile and parts of the reduction of a product of `rows` x `cols` outputs over k steps, `copies` times, on this kernel (may_split: its
-// launch can cut the reduction into up to 16 parts of `size` outputs each; w: elements of W where B can be split beforehand, else 0), and
+// Tile and parts of the reduction of a product of `rows` x `cols` outputs over k steps, `copies` times, on this kernel (its
+// launch can cut the reduction into up to `most` parts of `size` outputs each; w: elements of W where B can be split beforehand, else 0), and
 // the time that takes (us): what a stage and a tile besides take in each form, as fitted to 1200 products (9 of 10 within 13 %).  The copy of
 // B costs a launch and pays from a few waves on (64 x 15 x 13, 36 -> 100 channels 3x3 37 -> 34 us, 2368 x 2048 x 2304 195 -> 140).
 struct PlanePlan { int bn; bool copy_b; int ksplit; double time; };
-inline PlanePlan plan_planes(long long rows, int cols, long long k, long long copies, bool may_split, double size, double w, int sms)
+inline PlanePlan plan_planes(long long rows, int cols, long long k, long long copies, int most, double size, double w, int sms)
 {
     static const struct { int bn; bool copy; double stage, wave; } forms[] = {{64, false, 0.62, 4.0}, {128, false, 0.80, 4.4}, {64, true, 0.47, 4.2}, {128, true, 0.57, 4.9}};
     const long long stages = (k + kPlaneBK - 1) / kPlaneBK;
@@ -794,9 +794,11 @@ inline PlanePlan plan_planes(long long rows, int cols, long long k, long long co
     for (const auto& f : forms) {
         if (f.copy && !(w > 0)) continue;
         const double tiles = (double)((rows + kPlaneBM - 1) / kPlaneBM) * ((cols + f.bn - 1) / f.bn) * copies, fixed = 5.3 + (f.copy ? 1.5 + w * 10e-6 / 5 : w * 0.8e-6);
-        for (int ks = 1; ks <= 16 && (ks == 1 || (may_split && ks <= stages / 2)); ++ks) {
+        // (of many parts, those that fill whole waves)
+        auto next = [&](int ks) { return ks < 16 ? ks + 1 : (int)(((long long)(ks * tiles / sms) + 1) * sms / tiles); };
+        for (int ks = 1; ks <= most && (ks == 1 || ks <= stages / 2); ks = next(ks) > ks ? next(ks) : ks + 1) {
             const double ctas = tiles * ks, waves = (double)(long long)((ctas + sms - 1) / sms);
-            const double time = waves * ((stages + ks - 1) / ks * f.stage + f.wave) + fixed + (ks > 1 ? 2.1 + (ks + 1) * size * 4e-6 / 5 : 0.0);
+            const double time = waves * ((stages + ks - 1) / ks * f.stage + f.wave) + fixed + (ks > 1 ? 2.1 + 0.07 * ks + (ks + 1) * size * 4e-6 / 5 : 0.0);
             if (best.time == 0 || time < best.time) best = PlanePlan{f.bn, f.copy, ks, time};
             if (ctas > 4.0 * sms) break;
         }
@@ -821,7 +823,7 @@ inline ProductPlan plan_product(long long rows, int cols, int taps, int k, long 
     const double step = f.bn == 128 ? 3.57 : (f.bn == 32 ? 1.42 : (f.bm == 128 ? 1.93 : 1.30)), waves = fc * fks / (2.0 * sms);
     const double f_time = (waves > 1 ? waves : 1.0) * ((its + fks - 1) / fks * step + 3.1) + 6.1;
     if (mode == 0 || (mode == 1 && (long long)taps * k < 64)) return ProductPlan{f, fks, false};
-    const PlanePlan p = plan_planes(rows, cols, plane_k, copies, may_split, size, w, sms);
+    const PlanePlan p = plan_planes(rows, cols, plane_k, copies, may_split ? 16 : 1, size, w, sms);
     if (mode == 1 && f_time <= 1.05 * p.time) return ProductPlan{f, fks, false};
     return ProductPlan{GemmTile{kPlaneBM, p.bn, true}, p.ksplit, p.copy_b};
 }

@@ -1,7 +1,7 @@
 """Layers gathered straight from their tensors by the bf16-plane kernel: against 64-bit sums at the edges of tiles, stages, taps and
 parts, which layers take that route, and that it gives the same bits under every option that must not change a result.
 
-Bound of a sum of K products: that of test_gpu_planes, and one rounded addition of 2^-24 for each of up to 16 parts."""
+Bound of a sum of K products: that of test_gpu_planes, and one rounded addition of 2^-24 for each of up to 16 parts (the more parts of a deltaW are added with compensation)."""
 import numpy as np
 import pytest
 
@@ -28,7 +28,7 @@ def gather(pkg):
 # beforehand or in the kernel, taps outside the picture on every side, phases without a tap
 SHAPES = [(1, 1, 1, 4, 4, 1, 1, 0), (1, 9, 9, 4, 12, 3, 1, 1), (2, 35, 29, 36, 100, 3, 1, 1), (3, 16, 16, 132, 20, 3, 2, 1), (2, 15, 17, 64, 68, 1, 2, 0),
           (2, 9, 11, 40, 44, 2, 3, 0), (1, 6, 6, 260, 36, 4, 2, 1), (130, 1, 1, 196, 180, 1, 1, 0), (5, 1, 1, 2764, 52, 1, 1, 0), (1, 7, 5, 8, 4, 7, 2, 3),
-          (16, 8, 8, 128, 128, 3, 1, 1), (64, 4, 4, 64, 256, 3, 2, 1), (2, 20, 20, 128, 36, 5, 1, 2), (300, 28, 28, 24, 72, 3, 1, 1)]
+          (16, 8, 8, 128, 128, 3, 1, 1), (64, 4, 4, 64, 256, 3, 2, 1), (2, 20, 20, 128, 36, 5, 1, 2), (300, 28, 28, 24, 72, 3, 1, 1), (37, 31, 29, 36, 100, 3, 1, 1)]
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=str)
@@ -103,7 +103,7 @@ ROUTES = [("forward", (512, 8, 8, 128, 128, 3, 1, 1), True), ("forward", (512, 1
           ("deltaX", (256, 16, 16, 128, 256, 4, 2, 1), True), ("deltaX", (256, 16, 16, 32, 256, 4, 2, 1), False), ("deltaX", (512, 8, 8, 128, 128, 3, 1, 1), True), ("deltaX", (512, 14, 14, 128, 128, 3, 1, 1), False), ("deltaX", (512, 4, 4, 256, 512, 3, 2, 1), False),
           ("deltaX", (250, 1, 1, 1024, 1024, 1, 1, 0), True), ("deltaW", (512, 4, 4, 256, 256, 3, 1, 1), True), ("deltaW", (512, 8, 8, 128, 128, 3, 1, 1), False), ("deltaW", (33, 21, 21, 128, 192, 7, 2, 3), True),
           ("deltaW", (256, 16, 16, 128, 256, 4, 2, 1), False),
-          ("deltaW", (7, 28, 28, 28, 88, 3, 1, 1), True), ("deltaW", (64, 15, 13, 36, 100, 3, 1, 1), False), ("deltaW", (250, 1, 1, 1024, 1024, 1, 1, 0), True), ("deltaW", (64, 1, 1, 4096, 1024, 1, 1, 0), False)]
+          ("deltaW", (7, 28, 28, 28, 88, 3, 1, 1), True), ("deltaW", (50, 35, 29, 36, 100, 3, 1, 1), True), ("deltaW", (250, 1, 1, 1024, 1024, 1, 1, 0), True), ("deltaW", (64, 1, 1, 4096, 1024, 1, 1, 0), False)]
 
 
 @pytest.mark.parametrize("op,shape,taken", ROUTES, ids=str)

@@ -1,12 +1,15 @@
 // Products on the tensor cores at fp32 accuracy, gathering both operands from the tensors as they lie.
 //
-// An fp32 word is the exact sum of three bf16 words, x = h + m + l (the upper 16 bits, the upper 16 bits of what is left, the rest: 8
-// bits of significand each), and of the nine products of two such sums the six that matter are formed by tcgen05.mma kind::f16:
-// hh in one accumulator; hm, mh, mm, hl, lh, all below 2^-7 of it, in another.  What is dropped (ml, lm, ll) is below 2^-23 of a product.
+// An fp32 word is the exact sum of three bf16 words, x = h + m + l (8 bits of significand each: x rounded to nearest, what is left
+// of it rounded, the rest, so that |m| <= 2^-8 |x| and |l| <= 2^-17 |x|), and of the nine products of two such sums the six that matter are
+// formed by tcgen05.mma kind::f16: hh in one accumulator; hm, mh, mm, hl, lh, all below 2^-7 of it, in another.  What is dropped (ml, lm,
+// ll) is below 2^-24 (1 + 2^-10) of a product, as much as an fp32 rounding, and of either sign (truncated words would leave 2^-21, always
+// towards zero: 1.0078124 squared 4.7e-7 too small).
 // The tensor core truncates as it adds to an accumulator, about 2^-24 of it an instruction, which over a long sum would cost more
 // than fp32 FMAs do: after every 64 reduction steps (four instructions into the hh accumulator) the partial sum is added to running
-// sums in registers, rounded to nearest, and the accumulator starts anew.  Sums of 4 to
-// 20000 products err by 1.0e-7 to 1.8e-7 (2-norm against 64 bits), those of the FMA kernels by 1.2e-7 to 3e-6.
+// sums in registers, rounded to nearest, and the accumulator starts anew.  2-norm errors against 64 bits (operands in [0, 1) / N(0, 1); in
+// brackets the FMA kernel, which keeps products of under 64 terms): 1 term 3.6e-8 / 3.5e-8 (2.5e-8), 16 4.5e-8 / 4.4e-8 (6.3e-8 / 7.3e-8), 64
+// 8.7e-8 / 7.6e-8 (1.2e-7 / 1.5e-7), 513 9.1e-8 / 9.4e-8 (3.1e-7 / 4.1e-7), 20001 2.8e-7 / 3.4e-7 (2.2e-6 / 2.5e-6).
 //
 // Bound: 388 clocks of MMAs per 16 steps of a 128 x 128 tile, as much as the 3xTF32 kernels issue per step.  A stage of 32 steps takes
 // 0.80 us (some 1450 clocks for the 776 of MMAs): the issue slots and shared memory accesses of the loads and splits, and the wait of
@@ -50,19 +53,25 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
     return r;
 }
 
-// x = h + m + l: the planes of four consecutive elements, eight bytes each.
+// x = h + m + l: the planes of four consecutive elements, eight bytes each.  h and m are rounded to nearest.
 __device__ __forceinline__ void split_planes(const float4& v, uint2& h, uint2& m, uint2& l)
 {
-    auto hi2 = [](float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); };
-    auto cut = [](float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); };
-    float r0, r1, r2, r3, t0, t1, t2, t3;
-    unpack2(sub2(pack2(v.x, v.y), pack2(cut(v.x), cut(v.y))), r0, r1);
-    unpack2(sub2(pack2(v.z, v.w), pack2(cut(v.z), cut(v.w))), r2, r3);
-    unpack2(sub2(pack2(r0, r1), pack2(cut(r0), cut(r1))), t0, t1);
-    unpack2(sub2(pack2(r2, r3), pack2(cut(r2), cut(r3))), t2, t3);
-    h = make_uint2(hi2(v.x, v.y), hi2(v.z, v.w));
-    m = make_uint2(hi2(r0, r1), hi2(r2, r3));
-    l = make_uint2(hi2(t0, t1), hi2(t2, t3));
+    auto pair = [](float a, float b) {                    // two bf16 words, a in the lower half
+        uint32_t r;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+        return r;
+    };
+    auto less = [](float a, float b, uint32_t w, float& x, float& y) {   // what a pair leaves of its elements (exact)
+        unpack2(sub2(pack2(a, b), pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u))), x, y);
+    };
+    float r0, r1, r2, r3;
+    h = make_uint2(pair(v.x, v.y), pair(v.z, v.w));
+    less(v.x, v.y, h.x, r0, r1);
+    less(v.z, v.w, h.y, r2, r3);
+    m = make_uint2(pair(r0, r1), pair(r2, r3));
+    less(r0, r1, m.x, r0, r1);
+    less(r2, r3, m.y, r2, r3);
+    l = make_uint2(__byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632), __byte_perm(__float_as_uint(r2), __float_as_uint(r3), 0x7632));
 }
 
 // Zeros past the first n elements.

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 def bound(K):
-    return 2.0 ** -20 + 2.0 ** -28 + 4 * 2.0 ** -23 + (K / 64 + 3 + 16) * 2.0 ** -24
+    return 2.0 ** -24 + 2.0 ** -34 + 4 * 2.0 ** -23 + (K / 64 + 3 + 16) * 2.0 ** -24
 
 
 @pytest.fixture

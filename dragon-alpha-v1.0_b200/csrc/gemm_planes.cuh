@@ -27,8 +27,8 @@
 //               are one MMA each, and with BN = 64 also h x [h m l].
 //   warp 17     where W is split beforehand (TMA_B), copies the three planes of a stage of B; half of the split work goes.
 // hh accumulates in two column blocks in turn, so that one is read while the other fills.
-// Where a sum comes out as Inf or NaN (operands that are, or that overflow a plane) or so small that a plane's last bits may have
-// been lost to underflow, the tile is formed once more by FMAs, as gemm_f32_kernel forms it.
+// Where an operand is not the sum of its planes (below 2^-110 its last bits underflow them), or a sum comes out as Inf or NaN or so small
+// that its products may have underflowed, the tile is formed once more by FMAs, as gemm_f32_kernel forms it.
 #pragma once
 #include "gemm_f32.cuh"
 #include "sm100_ptx.cuh"
@@ -53,8 +53,10 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
     return r;
 }
 
-// x = h + m + l: the planes of four consecutive elements, eight bytes each.  h and m are rounded to nearest.
-__device__ __forceinline__ void split_planes(const float4& v, uint2& h, uint2& m, uint2& l)
+// x = h + m + l: the planes of four consecutive elements, eight bytes each.  h and m are rounded to nearest.  What the lowest 16 bits of
+// `lost` hold afterwards is zero as long as nothing was: an element from 2^-110 on has its last bit at 2^-133 or above, the smallest of bf16;
+// of a smaller one, of an Inf and of a NaN there may be a rest.
+__device__ __forceinline__ void split_planes(const float4& v, uint2& h, uint2& m, uint2& l, uint32_t& lost)
 {
     auto pair = [](float a, float b) {                    // two bf16 words, a in the lower half
         uint32_t r;
@@ -71,6 +73,7 @@ __device__ __forceinline__ void split_planes(const float4& v, uint2& h, uint2& m
     m = make_uint2(pair(r0, r1), pair(r2, r3));
     less(r0, r1, m.x, r0, r1);
     less(r2, r3, m.y, r2, r3);
+    lost |= __float_as_uint(r0) | __float_as_uint(r1) | __float_as_uint(r2) | __float_as_uint(r3);
     l = make_uint2(__byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632), __byte_perm(__float_as_uint(r2), __float_as_uint(r3), 0x7632));
 }
 
@@ -595,6 +598,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
         const uint32_t off_a = smem_u32(smem) + plane_offset<kPlaneBM, P::kAk>(t), off_b = smem_u32(smem) + 3 * kPlaneA + plane_offset<BN, P::kBk>(t);
         const float *A = p.a_tensor(c), *B = p.b_tensor(c);
         float4 va[NA], vb[NB];
+        uint32_t lost = 0;
         auto load = [&](int s) {
             const int k0 = (c.s0 + s) * 32, ka = k0 + plane_k<kPlaneBM, P::kAk>(t, 0), kb = k0 + plane_k<BN, P::kBk>(t, 0);
             if constexpr (P::kAk) {
@@ -674,7 +678,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
 #pragma unroll
             for (int i = 0; i < NA; ++i) {
                 uint2 h, m, l;
-                split_planes(va[i], h, m, l);
+                split_planes(va[i], h, m, l, lost);
                 const uint32_t at = at_a + i * plane_step<kPlaneBM, P::kAk>();
                 st_shared_v2(at, h); st_shared_v2(at + kPlaneA, m); st_shared_v2(at + 2 * kPlaneA, l);
             }
@@ -682,7 +686,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
                 uint2 h, m, l;
-                split_planes(vb[i], h, m, l);
+                split_planes(vb[i], h, m, l, lost);
                 const uint32_t at = at_b + i * plane_step<BN, P::kBk>();
                 st_shared_v2(at, h); st_shared_v2(at + kPlaneB, m); st_shared_v2(at + 2 * kPlaneB, l);
             }
@@ -698,7 +702,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
             tc_fence_after_sync();
             add_columns(kSide);
             add_columns(kSide + BN);
-            // what may not have survived the split: not finite, or below 1e-28 and not zero (both ends of the magnitudes, zero as the largest)
+            // what may not have survived the split: a word that is not the sum of its planes (its partner may be so large that the sum does not
+            // show it: 1e-37 x 1e11 would err by 6.6e-4), a sum not finite, or below 1e-28 and not zero (both ends of the magnitudes, zero as the largest)
             uint32_t most = 0, least = 0xffffffffu;
 #pragma unroll
             for (int x = 0; x < COLS / 2; ++x) {
@@ -708,7 +713,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
                 most = max(most, max(u, v));
                 least = min(least, min(u - 1, v - 1));
             }
-            again = most >= 0xff000000u || least < 2u * 0x10fd87b6u;
+            again = most >= 0xff000000u || least < 2u * 0x10fd87b6u || (lost & 0xffffu) != 0;
         }
         }
         tc_fence_before_sync();
@@ -765,6 +770,7 @@ inline void launch_gemm_planes(const P& p, const CUtensorMap& tmB, dim3 tiles, u
 
 // The planes of W as TMA_B copies them: dst[plane][row][pitch], row r < rows from W row src(r).  taps = 0: rows as they lie (forward; K
 // columns, zeros up to the pitch); else row j * OC + oc is tap map[j] of output channel oc (deltaX: taps in the order of phases and steps).
+// Words that are not the sum of their planes become NaN, which sends the tiles that read them back to W itself.
 struct SplitRows { int map[64]; };
 template <int>   // (defined where it is launched)
 __global__ void __launch_bounds__(256) split_planes_kernel(const float* __restrict__ W, uint2* __restrict__ dst, int rows, int cols, unsigned pitch4, FastDiv by_pitch4,
@@ -785,7 +791,9 @@ __global__ void __launch_bounds__(256) split_planes_kernel(const float* __restri
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (static_cast<int>(4 * q) < cols) v = __ldg(reinterpret_cast<const float4*>(W + static_cast<size_t>(from) * cols + 4 * q));
         uint2 h, m, l;
-        split_planes(v, h, m, l);
+        uint32_t lost = 0;
+        split_planes(v, h, m, l, lost);
+        if (lost & 0xffffu) h = make_uint2(0x7fff7fffu, 0x7fff7fffu);
         dst[i] = h; dst[static_cast<size_t>(total) + i] = m; dst[2 * static_cast<size_t>(total) + i] = l;
     }
 }

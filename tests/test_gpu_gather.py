@@ -95,6 +95,34 @@ def test_operands_outside_the_planes(pkg, gather, op, what):
     assert bool(((got.double() - ref).abs()[finite] <= (K * 2.0 ** -24 * mag + K * 2.0 ** -149)[finite]).all())
 
 
+@pytest.mark.parametrize("small,large", [(1e-36, 1e10), (1e-37, 1e11)], ids=str)
+@pytest.mark.parametrize("side", ["X", "W"])
+def test_tiny_operands_with_large_partners(pkg, gather, small, large, side):
+    """Operands whose last bits no bf16 word holds, in sums that do not show it: forward (W split beforehand and not), deltaX, deltaW."""
+    import torch
+    eng, lib = pkg.submodule("engine").Engine(), pkg.submodule("lib")
+    g = torch.Generator(device="cuda").manual_seed(8)
+    sx, sw = (small, large) if side == "X" else (large, small)
+    rand = lambda *q: torch.rand(q, device="cuda", generator=g) + 0.5
+    plans = []
+    for N, H, IC, OC in ((1, 9, 36, 40), (256, 14, 64, 128)):
+        X, W = rand(N, H, H, IC) * sx, rand(OC, 3, 3, IC) * sw
+        y = eng.conv3D(X, W, 1, 1, 1, 1).double()
+        plans.append(lib.last_plan())
+        ref = torch.nn.functional.conv2d(X.double().permute(0, 3, 1, 2), W.double().permute(0, 3, 1, 2), padding=1).permute(0, 2, 3, 1)
+        assert bool(((y - ref).abs() <= 9 * IC * 2.0 ** -24 * ref).all()), plans[-1]
+        dY, V = rand(N, H, H, IC) * sx, rand(IC, 3, 3, OC) * sw
+        y = eng.dconv3D_deltaX(dY, V, H, H, 1, 1, 1, 1).double()
+        ref = torch.nn.functional.conv_transpose2d(dY.double().permute(0, 3, 1, 2), V.double().permute(0, 3, 1, 2), padding=1).permute(0, 2, 3, 1)
+        assert bool(((y - ref).abs() <= 9 * IC * 2.0 ** -24 * ref).all()), lib.last_plan()
+    assert all(q.startswith("gather") for q in plans) and "copy" not in plans[0] and "copy" in plans[1], plans
+    dY = rand(2, 9, 9, 40) * sw
+    X = rand(2, 9, 9, 36) * sx
+    y = eng.dconv3D_deltaW(X, dY, 3, 3, 1, 1, 1, 1).double()
+    ref = torch.nn.grad.conv2d_weight(X.double().permute(0, 3, 1, 2), (40, 36, 3, 3), dY.double().permute(0, 3, 1, 2), padding=1).permute(0, 2, 3, 1)
+    assert lib.last_plan().startswith("gather") and bool(((y - ref).abs() <= 162 * 2.0 ** -24 * ref).all())
+
+
 # the smallest fill, channel count and time at which a layer leaves the other kernels, and its neighbours
 ROUTES = [("forward", (512, 8, 8, 128, 128, 3, 1, 1), True), ("forward", (512, 14, 14, 128, 128, 3, 1, 1), False), ("forward", (8, 8, 8, 32, 64, 3, 1, 1), False),
           ("forward", (64, 28, 28, 12, 64, 3, 1, 1), False), ("forward", (512, 8, 8, 256, 512, 3, 2, 1), True), ("forward", (512, 16, 16, 64, 128, 3, 2, 1), False),

@@ -89,6 +89,36 @@ def test_long_sums_of_one_sign(pkg, planes, low):
     assert float((C - ref).norm() / ref.norm()) <= 2.0 ** -22 + (K / 64) ** 0.5 * 2.0 ** -25
 
 
+# (operands below 2^-110, whose last bits no bf16 word holds, times partners that make the sum an ordinary number)
+TINY = [(1e-34, 1e8), (1e-36, 1e10), (1e-37, 1e11), (1e-39, 1e20)]
+
+
+@pytest.mark.parametrize("small,large", TINY, ids=str)
+@pytest.mark.parametrize("side", ["A", "B"])
+def test_tiny_operands_with_large_partners(pkg, planes, small, large, side):
+    """Batched products in each layout and fp32 deltaX with W split beforehand and not: within the bound of an fp32 sum."""
+    import torch
+    eng, lib = pkg.submodule("engine").Engine(), pkg.submodule("lib")
+    g = torch.Generator(device="cuda").manual_seed(6)
+    sa, sb = (small, large) if side == "A" else (large, small)
+    K = 97
+    A, B = (torch.rand((2, 130, K), device="cuda", generator=g) + 0.5) * sa, (torch.rand((2, K, 68), device="cuda", generator=g) + 0.5) * sb
+    ref = A.double() @ B.double()
+    for op, a, b in (("batchMatMul", A, B), ("batchMatMulT1", A.transpose(1, 2).contiguous(), B), ("batchMatMulT2", A, B.transpose(1, 2).contiguous())):
+        y = getattr(eng, op)(a, b).double()
+        assert lib.last_plan().startswith("gemm_f32 planes")
+        assert bool(((y - ref).abs() <= K * 2.0 ** -24 * ref).all()), op
+    plans = []
+    for N, OH, IC, OC in ((1, 9, 40, 44), (64, 14, 132, 36)):
+        dY, W = (torch.rand((N, OH, OH, OC), device="cuda", generator=g) + 0.5) * sa, (torch.rand((OC, 3, 3, IC), device="cuda", generator=g) + 0.5) * sb
+        y = eng.dconv3D_deltaX(dY, W, OH, OH, 1, 1, 1, 1).double()
+        plans.append(lib.last_plan())
+        assert plans[-1].startswith("gemm_f32 planes")
+        ref = torch.nn.functional.conv_transpose2d(dY.double().permute(0, 3, 1, 2), W.double().permute(0, 3, 1, 2), padding=1).permute(0, 2, 3, 1)
+        assert bool(((y - ref).abs() <= 9 * OC * 2.0 ** -24 * ref).all()), plans[-1]
+    assert "copy" not in plans[0] and "copy" in plans[1], plans
+
+
 @pytest.mark.parametrize("what", ["inf weight", "nan gradient", "largest", "tiny", "overflow"])
 def test_operands_outside_the_planes(pkg, planes, what):
     """Tiles with such operands are formed by FMAs: the values, Infs and NaNs of the FMA kernel, and border pixels untouched by taps

@@ -33,6 +33,8 @@
 #include "gemm_f32.cuh"
 #include "sm100_ptx.cuh"
 
+#include <utility>
+
 namespace alpha {
 
 constexpr int kPlaneThreads = 576, kPlaneBM = 128, kPlaneBK = 32, kPlaneRing = 4;
@@ -118,7 +120,7 @@ template <int COLS> __device__ constexpr int plane_dk() { return 32 / (COLS / 32
 //   cta()              tile (bx, by, bz): rows from m0, columns from n0, stages [s0, s1) of 32 steps of K in all; false: there is none
 //   a_row, a_step      a word of A lies row.at + step.at floats into a_tensor() and is read where use_a() says (a filter tap may miss the
 //   b_row, b_step      image, a row, column or step may not exist); the same for B
-//   row_out, store     the row of the result, nullptr where there is none; four consecutive outputs of it
+//   row_out, store     the row of the result, nullptr where there is none; four consecutive outputs of it; columns(): how many there are from n0 on
 // Offsets are 32-bit: tensors have fewer than 2^31 elements (planes_fit).
 
 // Tiles of a launch, x fastest, one a CTA; `first` = tile of CTA 0.
@@ -179,6 +181,7 @@ struct PlaneDxProblem {
         c.out = out + static_cast<size_t>(copy) * size;
         return true;
     }
+    __device__ int columns(const Cta& c) const { return IC - c.n0; }
     __device__ const float* a_tensor(const Cta&) const { return dY; }
     __device__ const float* b_tensor(const Cta&) const { return W; }
     // pixel (n, a, b) of the phase
@@ -255,7 +258,7 @@ struct PlaneDx : PlaneDxProblem {
 
 // C[b] = A[b] * B[b] over N x M outputs and K steps, with row pitches.  A_KC: A[b] is [N][lda] (else [K][lda], the transposed
 // form); B_KC: B[b] is [M][ldb] (else [K][ldb]).  Pitches are multiples of 4 and every matrix starts on a 16-byte boundary;
-// words are loaded whole where they start inside the matrix: columns past N or M are not stored, steps past K become zeros (kTail).
+// words are loaded whole where they start inside the matrix: rows past N and steps past K become zeros (kTail).
 template <bool A_KC, bool B_KC>
 struct PlaneBatch {
     static constexpr bool kAk = A_KC, kBk = B_KC, kTail = true, kCopyB = false;
@@ -271,6 +274,9 @@ struct PlaneBatch {
         c.A = A + static_cast<size_t>(bz) * strA; c.B = B + static_cast<size_t>(bz) * strB; c.C = C + static_cast<size_t>(bz) * strC;
         return true;
     }
+    __device__ int columns(const Cta& c) const { return M - c.n0; }
+    // rows from one of the tile to the end of the matrix (the columns of a B that runs along them are a multiple of 4)
+    __device__ int a_left(const Cta& c, int m) const { return N - (c.m0 + m); }
     __device__ const float* a_tensor(const Cta& c) const { return c.A; }
     __device__ const float* b_tensor(const Cta& c) const { return c.B; }
     __device__ PlaneAt a_row(const Cta& c, int m) const { return PlaneAt{static_cast<uint32_t>((c.m0 + m) * (A_KC ? lda : 1)), c.m0 + m < N ? 1u : 0u}; }
@@ -312,6 +318,7 @@ struct PlaneFwd {
         c.out = out + static_cast<size_t>(sp) * size;
         return true;
     }
+    __device__ int columns(const Cta& c) const { return OC - c.n0; }
     __device__ const float* a_tensor(const Cta&) const { return X; }
     __device__ const float* b_tensor(const Cta&) const { return W; }
     __device__ PlaneAt a_row(const Cta& c, int m) const
@@ -379,6 +386,7 @@ struct PlaneDw {
         c.out = out + static_cast<size_t>(sp) * size;
         return true;
     }
+    __device__ int columns(const Cta& c) const { return L - c.n0; }
     __device__ const float* a_tensor(const Cta&) const { return dY; }
     __device__ const float* b_tensor(const Cta&) const { return X; }
     __device__ PlaneAt a_row(const Cta& c, int m) const { return PlaneAt{static_cast<uint32_t>(c.m0 + m), c.m0 + m < OC ? 1u : 0u}; }
@@ -425,47 +433,207 @@ __device__ __forceinline__ float4 load_word(const float* tensor, uint32_t at, bo
     return v;
 }
 
-// The whole tile by FMAs in ascending k, for operands that the planes do not represent: 256 threads of 8 x BN / 16 outputs.  A
-// product whose tap misses the image, or with no operand at all, is left out, so that an Inf or NaN of the other operand stays out of it.
-template <int BN, class P>
-__device__ __noinline__ void gemm_planes_again(const P& p, const typename P::Cta& c, int tid)
+// ---- tiles whose operands or sums the planes do not hold -------------------------------------------------------
+//
+// The 512 threads that staged the tile form it by FMAs in ascending k, 8 x 4 (4 x 4) outputs each, from words staged in shared memory as they
+// are; or, where only bits below 2^-133 were lost (tiny operands beside ordinary ones, as a softmax has them), look at the operands
+// once more and let the sums stand.  us, ordinary data / an Inf in every picture / data times 1e-30: 50 x 35 x 29, 36 -> 100 channels 3x3
+// forward 34 / 138 / 185, 512 x 8x8 x 128 51 / 489 / 389, 256 x 16x16, 128 -> 256, 4x4 s2 81 / 740 / 695 (a thread per eight rows that read both operands
+// from global memory and computed their places anew for every step: 2019 / 5862, 12749, 22740; data times 1e-25 as well, which now stays);
+// a softmax with tails, 64 x 130 x 200 x 130, 45 where ordinary data take 32 and the FMA kernel 40.
+
+// Barrier of those threads; whether any of them says so.
+__device__ __forceinline__ bool again_or(bool x)
 {
-    constexpr int TN = BN / 16;
-    const int m0 = (tid >> 4) * 8, n0 = (tid & 15) * TN;
-    const float *A = p.a_tensor(c), *B = p.b_tensor(c);
-    float acc[8][TN] = {};
-    const int end = c.s1 * 32 < c.K ? c.s1 * 32 : c.K;
-    for (int k = c.s0 * 32; k < end; ++k) {
-        // (a step of an operand that runs along k is known by its word of four)
-        const int ka = P::kAk ? k & ~3 : k, kb = P::kBk ? k & ~3 : k;
-        const auto sa = p.a_step(c, ka);
-        const auto sb = p.b_step(c, kb);
-        float b[TN];
-        bool in[TN];
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 512, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(static_cast<uint32_t>(x)) : "memory");
+    return r != 0;
+}
+
+template <int BN, class P>
+struct PlaneAgain {
+    using ARow = decltype(std::declval<const P&>().a_row(std::declval<const typename P::Cta&>(), 0));
+    using BRow = decltype(std::declval<const P&>().b_row(std::declval<const typename P::Cta&>(), 0));
+    using AStep = decltype(std::declval<const P&>().a_step(std::declval<const typename P::Cta&>(), 0));
+    using BStep = decltype(std::declval<const P&>().b_step(std::declval<const typename P::Cta&>(), 0));
+    struct Shared {
+        float a[2][32][kPlaneBM + 4], b[2][32][BN + 4];      // [stage & 1][step][row or column]
+        AStep sa[32];
+        BStep sb[32];
+        uint32_t any_a[kPlaneBM], any_b[BN], top;              // bits set in a row of A, a column of B; the largest word
+    };
+    static_assert(sizeof(Shared) % 4 == 0 && sizeof(Shared) + 512 * BN <= kPlaneRing * plane_stage_bytes(BN), "shared memory");
+    static constexpr int TM = BN / 16, CG = BN / 4, NB = BN / 64;
+
+    // The words of a stage that a thread loads: two of A, NB of B.
+    const P& p;
+    const typename P::Cta& c;
+    const ARow* rows;
+    int tid;
+    const float *A, *B;
+    float4 va[2], vb[NB];
+    __device__ PlaneAgain(const P& p_, const typename P::Cta& c_, const ARow* rows_, int tid_) : p(p_), c(c_), rows(rows_), tid(tid_), A(p_.a_tensor(c_)), B(p_.b_tensor(c_)) {}
+    __device__ int a_col(int i) const { return P::kAk ? (tid >> 3) + 64 * i : (tid & 31) * 4; }
+    __device__ int a_k(int i) const { return P::kAk ? (tid & 7) * 4 : (tid >> 5) + 16 * i; }
+    __device__ int b_col(int i) const { return P::kBk ? (tid >> 3) + 64 * i : tid % CG * 4; }
+    __device__ int b_k(int i) const { return P::kBk ? (tid & 7) * 4 : tid / CG + 512 / CG * i; }
+    __device__ ARow a_row(int m) const
+    {
+        if constexpr (P::kAk) return rows[m];
+        else return p.a_row(c, m);
+    }
+    __device__ void load(int s)
+    {
+        const int k0 = (c.s0 + s) * 32;
 #pragma unroll
-        for (int x = 0; x < TN; ++x) {
-            const int col = n0 + x, word = P::kBk ? col : col & ~3;
-            const auto r = p.b_row(c, word);
-            in[x] = p.use_b(r, sb);
-            b[x] = in[x] ? __ldg(B + (r.at + sb.at) + (P::kBk ? k & 3 : col & 3)) : 0.f;
+        for (int i = 0; i < 2; ++i) {
+            const ARow r = a_row(a_col(i));
+            const AStep at = p.a_step(c, k0 + a_k(i));
+            va[i] = load_word(A, r.at + at.at, p.use_a(r, at));
         }
 #pragma unroll
-        for (int y = 0; y < 8; ++y) {
-            const int m = m0 + y, word = P::kAk ? m : m & ~3;
-            const auto r = p.a_row(c, word);
-            if (!p.use_a(r, sa)) continue;
-            const float a = __ldg(A + (r.at + sa.at) + (P::kAk ? k & 3 : m & 3));
+        for (int i = 0; i < NB; ++i) {
+            const BRow r = p.b_row(c, b_col(i));
+            const BStep at = p.b_step(c, k0 + b_k(i));
+            vb[i] = load_word(B, r.at + at.at, p.use_b(r, at));
+        }
+    }
+    __device__ static uint32_t top_of(const float4& v)
+    {
+        const uint32_t a = __float_as_uint(v.x) & 0x7fffffffu, b = __float_as_uint(v.y) & 0x7fffffffu, d = __float_as_uint(v.z) & 0x7fffffffu, e = __float_as_uint(v.w) & 0x7fffffffu;
+        return max(max(a, b), max(d, e));
+    }
+    __device__ uint32_t top() const
+    {
+        uint32_t t = max(top_of(va[0]), top_of(va[1]));
 #pragma unroll
-            for (int x = 0; x < TN; ++x)
-                if (in[x]) acc[y][x] = fmaf(a, b[x], acc[y][x]);
+        for (int i = 0; i < NB; ++i) t = max(t, top_of(vb[i]));
+        return t;
+    }
+    // Joins the bits of N words into those of their rows (columns): four of a word, or, where it runs along k, one.
+    template <bool K_MAJOR, int N>
+    __device__ static void join(const float4 (&v)[N], uint32_t (&bits)[4])
+    {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const uint32_t x = __float_as_uint(v[i].x) << 1, y = __float_as_uint(v[i].y) << 1, z = __float_as_uint(v[i].z) << 1, w = __float_as_uint(v[i].w) << 1;
+            if (K_MAJOR) bits[i] |= x | y | z | w;
+            else { bits[0] |= x; bits[1] |= y; bits[2] |= z; bits[3] |= w; }
+        }
+    }
+    template <bool K_MAJOR, int PITCH>
+    __device__ static void put(float (*to)[PITCH], int k, int col, const float4& v)
+    {
+        if (K_MAJOR) { to[k][col] = v.x; to[k + 1][col] = v.y; to[k + 2][col] = v.z; to[k + 3][col] = v.w; }
+        else *reinterpret_cast<float4*>(&to[k][col]) = v;
+    }
+    // Steps [0, n) of a staged stage.  MASKED: a product whose tap misses the image, or with no operand at all, is left out, so that an Inf
+    // or NaN of the other operand stays out of it (among finite words the zeros in their place do the same).
+    template <bool MASKED>
+    __device__ void add(const Shared& m, int buf, int n, int row, int col, float (&acc)[TM][4]) const
+    {
+        BRow rb{};
+        if (MASKED) rb = p.b_row(c, col);
+#pragma unroll 2
+        for (int k = 0; k < n; ++k) {
+            const float4 b = *reinterpret_cast<const float4*>(&m.b[buf][k][col]);
+            float a[TM];
+#pragma unroll
+            for (int y = 0; y < TM; y += 4) *reinterpret_cast<float4*>(a + y) = *reinterpret_cast<const float4*>(&m.a[buf][k][row + y]);
+            if (MASKED && !p.use_b(rb, m.sb[k])) continue;
+#pragma unroll
+            for (int y = 0; y < TM; ++y) {
+                if (MASKED && !p.use_a(a_row(P::kAk ? row + y : (row + y) & ~3), m.sa[k])) continue;
+                acc[y][0] = fmaf(a[y], b.x, acc[y][0]); acc[y][1] = fmaf(a[y], b.y, acc[y][1]);
+                acc[y][2] = fmaf(a[y], b.z, acc[y][2]); acc[y][3] = fmaf(a[y], b.w, acc[y][3]);
+            }
+        }
+    }
+};
+
+template <int BN, class P>
+__device__ __forceinline__ void gemm_planes_again(const P& p, const typename P::Cta& c, const typename PlaneAgain<BN, P>::ARow* rows, float* const* outs, uint8_t* smem, int tid)
+{
+    using G = PlaneAgain<BN, P>;
+    typename G::Shared& m = *reinterpret_cast<typename G::Shared*>(smem);
+    G g(p, c, rows, tid);
+    const int col = tid % G::CG * 4, row = tid / G::CG * G::TM, stages = c.s1 - c.s0;
+    float acc[G::TM][4] = {};
+    g.load(0);
+    for (int s = 0; s < stages; ++s) {
+        const int buf = s & 1, k0 = (c.s0 + s) * 32, n = c.K - k0 < 32 ? c.K - k0 : 32;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) G::template put<P::kAk>(m.a[buf], g.a_k(i), g.a_col(i), g.va[i]);
+#pragma unroll
+        for (int i = 0; i < G::NB; ++i) G::template put<P::kBk>(m.b[buf], g.b_k(i), g.b_col(i), g.vb[i]);
+        const bool masked = again_or(g.top() >= 0x7f800000u);       // (the other buffer may still be read, this one no more)
+        if (s + 1 < stages) g.load(s + 1);
+        if (masked) {
+            // (a step of an operand that runs along k is known by its word of four)
+            if (tid < 32) m.sa[tid] = p.a_step(c, k0 + (P::kAk ? tid & ~3 : tid));
+            else if (tid < 64) m.sb[tid - 32] = p.b_step(c, k0 + (P::kBk ? tid - 32 & ~3 : tid - 32));
+            again_or(false);
+            g.template add<true>(m, buf, n, row, col, acc);
+        } else {
+            g.template add<false>(m, buf, n, row, col, acc);
         }
     }
 #pragma unroll
-    for (int y = 0; y < 8; ++y) {
-        float* row = p.row_out(c, m0 + y);
-#pragma unroll
-        for (int x = 0; x < TN; x += 4) p.store(c, row, n0 + x, make_float4(acc[y][x], acc[y][x + 1], acc[y][x + 2], acc[y][x + 3]));
+    for (int y = 0; y < G::TM; ++y) p.store(c, outs[row + y], col, make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]));
+}
+
+// Whether the sums of a thread, column x at sums[512 x], x < end, of a row stand although operands lost bits: less than 2^-133 of one, times its
+// partner, for each of two operands and every step, is less than 2^-24 of a sum.  (A zero column, as a padded matrix has, gives zeros.)
+template <int BN, class P>
+__device__ __forceinline__ bool planes_suffice(const P& p, const typename P::Cta& c, const typename PlaneAgain<BN, P>::ARow* rows, uint8_t* smem, int tid, const float* sums,
+                                               int row, int col0, int end)
+{
+    using G = PlaneAgain<BN, P>;
+    typename G::Shared& m = *reinterpret_cast<typename G::Shared*>(smem);
+    G g(p, c, rows, tid);
+    if (tid < kPlaneBM) m.any_a[tid] = 0;
+    if (tid < BN) m.any_b[tid] = 0;
+    if (tid == 0) m.top = 0;
+    uint32_t top = 0, any_a[4] = {}, any_b[4] = {};
+    for (int s = 0; s < c.s1 - c.s0; ++s) {
+        g.load(s);
+        top = max(top, g.top());
+        G::template join<P::kAk>(g.va, any_a);
+        G::template join<P::kBk>(g.vb, any_b);
     }
+    top = __reduce_max_sync(0xffffffffu, top);
+    again_or(false);
+    if ((tid & 31) == 0) atomicMax(&m.top, top);
+#pragma unroll
+    for (int i = 0; i < (P::kAk ? 2 : 4); ++i) atomicOr(&m.any_a[P::kAk ? g.a_col(i) : g.a_col(0) + i], any_a[i]);
+#pragma unroll
+    for (int i = 0; i < (P::kBk ? G::NB : 4); ++i) atomicOr(&m.any_b[P::kBk ? g.b_col(i) : g.b_col(0) + i], any_b[i]);
+    again_or(false);
+    const float least = __uint_as_float(m.top) * static_cast<float>((c.s1 - c.s0) * 64) * 0x1p-109f;
+    bool stand = true;
+    if (m.any_a[row])
+        for (int x = 0; x < BN / 4 && x < end; ++x)
+            if (!(fabsf(sums[x * 512]) >= least) && m.any_b[col0 + x]) stand = false;
+    return !again_or(!stand);
+}
+
+// What becomes of a tile some thread of which found operands that lost bits or (`again`) sums that the planes may not have formed.  The sums lie
+// behind Shared, BN / 4 columns of a row a thread (a call of its own, so that the kernel's registers need not outlive one).
+template <int BN, class P>
+__device__ __noinline__ void gemm_planes_look(const P& p, const typename P::Cta& c, const typename PlaneAgain<BN, P>::ARow* rows, float* const* outs, uint8_t* smem, int tid, bool again)
+{
+    constexpr int COLS = BN / 4;
+    again = again_or(again);
+    if (!again) {
+        const float* sums = reinterpret_cast<const float*>(smem + sizeof(typename PlaneAgain<BN, P>::Shared)) + tid;
+        const int row = ((tid >> 5) & 3) * 32 + (tid & 31);
+        float* out = outs[row];
+        const int col0 = (tid >> 7) * COLS, end = (out ? p.columns(c) : 0) - col0;
+        again = !planes_suffice<BN>(p, c, rows, smem, tid, sums, row, col0, end);
+        if (!again)
+            for (int x = 0; x < COLS; x += 4) p.store(c, out, col0 + x, make_float4(sums[x * 512], sums[x * 512 + 512], sums[x * 512 + 1024], sums[x * 512 + 1536]));
+    }
+    if (again) gemm_planes_again<BN>(p, c, rows, outs, smem, tid);
 }
 
 // After a wait that ran out: time for what has been issued to end, before shared and tensor memory are given back.
@@ -521,7 +689,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
         else if (tid >= kPlaneBM && tid < 2 * kPlaneBM) outs[tid - kPlaneBM] = p.row_out(c, tid - kPlaneBM);
     }
     __syncthreads();
-    bool ok = true, again = false;
+    bool ok = true, again = false, look = false;
     unsigned long long acc[COLS / 2];
 #pragma unroll
     for (int x = 0; x < COLS / 2; ++x) acc[x] = 0ull;
@@ -664,7 +832,13 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
             if (s >= 4 && !flush(flushed++)) break;
             if (s >= kPlaneRing && !wait_done(s - kPlaneRing)) break;
             const uint32_t at_a = off_a + (s % kPlaneRing) * kStage, at_b = off_b + (s % kPlaneRing) * kStage;
-            if (P::kTail) {
+            if constexpr (P::kTail) {
+                if constexpr (!P::kAk) {
+                    const int left = p.a_left(c, plane_col<kPlaneBM, false>(t, 0));
+                    if (left < 4)
+#pragma unroll
+                        for (int i = 0; i < NA; ++i) keep_first(va[i], left);
+                }
                 const int steps = c.K - (c.s0 + s) * 32;
                 if (steps < 32) {
                     if (P::kAk)
@@ -702,8 +876,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
             tc_fence_after_sync();
             add_columns(kSide);
             add_columns(kSide + BN);
-            // what may not have survived the split: a word that is not the sum of its planes (its partner may be so large that the sum does not
-            // show it: 1e-37 x 1e11 would err by 6.6e-4), a sum not finite, or below 1e-28 and not zero (both ends of the magnitudes, zero as the largest)
+            // sums that the planes may not have formed: not finite, or below 2^-110 and not zero, where underflow of 2^-149 a product counts
+            // (measured: sums of 2^-124 err by 2e-7, below that by one such unit a product)
             uint32_t most = 0, least = 0xffffffffu;
 #pragma unroll
             for (int x = 0; x < COLS / 2; ++x) {
@@ -711,18 +885,24 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
                 unpack2(acc[x], a, b);
                 const uint32_t u = __float_as_uint(a) << 1, v = __float_as_uint(b) << 1;
                 most = max(most, max(u, v));
-                least = min(least, min(u - 1, v - 1));
+                least = min(least, min(u - 1, v - 1));          // (zero as the largest)
             }
-            again = most >= 0xff000000u || least < 2u * 0x10fd87b6u || (lost & 0xffffu) != 0;
+            again = most >= 0xff000000u || least < 2u * 0x08800000u;
+            // (and a word that is not the sum of its planes: its partner may be so large that the sum does not show it, 1e-37 x 1e11 would
+            // err by 6.6e-4)
+            look = again || (lost & 0xffffu) != 0;
         }
         }
         tc_fence_before_sync();
     }
-    again = __syncthreads_or(again) != 0;     // every MMA has completed: shared memory is free
+    look = __syncthreads_or(look) != 0;       // every MMA has completed: shared memory is free
     if (warp == 16) tmem_dealloc(tmem_base, kTmem);
     if (!work || warp >= 16) return;
-    if (again) {
-        if (warp < 8) gemm_planes_again<BN>(p, c, tid);
+    if (look) {
+        float* sums = reinterpret_cast<float*>(smem + sizeof(typename PlaneAgain<BN, P>::Shared)) + tid;
+#pragma unroll
+        for (int x = 0; x < COLS / 2; ++x) unpack2(acc[x], sums[x * 1024], sums[x * 1024 + 512]);
+        gemm_planes_look<BN>(p, c, rows, outs, smem, tid, again);
         return;
     }
     if (!ok) return;

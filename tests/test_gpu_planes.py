@@ -170,3 +170,90 @@ def test_parts_give_the_same_bits_with_and_without_scratch(pkg, planes):
     graph.replay()
     torch.cuda.synchronize()
     assert "in turns" not in plan and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("op", ["batchMatMul", "batchMatMulT1", "batchMatMulT2"])
+def test_tiny_rows_beside_ordinary_ones(pkg, planes, op):
+    """Sums that stand although an operand lost bits, sums that do not, and zero rows and columns: what an fp32 sum gives."""
+    import torch
+    eng, lib = pkg.submodule("engine").Engine(), pkg.submodule("lib")
+    g = torch.Generator(device="cuda").manual_seed(11)
+    N, M, K = 150, 70, 97
+    for tails in (False, True):
+        A, B = torch.randn((2, N, K), device="cuda", generator=g), torch.randn((2, K, M), device="cuda", generator=g)
+        A[:, :, 5] = 3.3e-37
+        A[:, 7], B[:, :, 9] = 0.0, 0.0
+        if tails:
+            A[0, 3] *= 1e-41
+            A[1, 140] *= 1e-35
+            B[1, :, 68] *= 1e-39
+        ref, mag = A.double() @ B.double(), A.double().abs() @ B.double().abs()
+        a, b = A.transpose(1, 2).contiguous() if op == "batchMatMulT1" else A, B.transpose(1, 2).contiguous() if op == "batchMatMulT2" else B
+        y = getattr(eng, op)(a, b).double()
+        assert lib.last_plan().startswith("gemm_f32 planes")
+        assert bool(((y - ref).abs() <= K * 2.0 ** -24 * mag + K * 2.0 ** -149).all())
+
+
+def time_of(call):
+    import torch
+    for _ in range(3):
+        call()
+    best = float("inf")
+    for _ in range(3):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(10):
+            call()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.parametrize("what", ["inf", "1e-25", "1e-35", "tails"])
+def test_time_of_tiles_formed_again(pkg, planes, what):
+    """Tiles that the planes cannot form take some four to eight times as long (a form that read its operands anew for every step took 58 to
+    280 times), gradients of 1e-25 and tails of a softmax none of that."""
+    import torch
+    eng = pkg.submodule("engine").Engine()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    X, W = torch.randn((512, 8, 8, 128), device="cuda", generator=g), torch.randn((128, 3, 3, 128), device="cuda", generator=g) * 0.05
+    A, B = torch.softmax(torch.randn((64, 250, 250), device="cuda", generator=g), -1), torch.randn((64, 250, 130), device="cuda", generator=g)
+    usual = time_of(lambda: eng.batchMatMul(A, B)) if what == "tails" else time_of(lambda: eng.conv3D(X, W, 1, 1, 1, 1))
+    assert pkg.submodule("lib").last_plan().startswith("gemm_f32 planes" if what == "tails" else "gather")
+    if what == "tails":
+        A[:, :, ::7] = 3.3e-37
+        time = time_of(lambda: eng.batchMatMul(A, B))
+    else:
+        if what == "inf":
+            X[:, 3, 4, 5] = float("inf")
+        else:
+            X *= float(what)
+        time = time_of(lambda: eng.conv3D(X, W, 1, 1, 1, 1))
+    assert time <= (1.1 if what == "1e-25" else 3 if what == "tails" else 16) * usual, (time, usual)
+
+
+@pytest.mark.parametrize("op", ["batchMatMul", "batchMatMulT1"])
+def test_what_lies_between_matrix_and_pitch(pkg, planes, op):
+    """NaN in the columns between A and its pitch reaches neither the sums nor the time."""
+    import ctypes as C
+    import torch
+    lib = pkg.submodule("lib")
+    call = getattr(lib.load(), "alpha_engine_" + op)
+    Bt, N, M, K = 40, 250, 132, 198
+    p, stream = lambda t: C.c_void_p(t.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    out = []
+    for pad in (0.0, float("nan")):
+        g = torch.Generator(device="cuda").manual_seed(10)
+        B, Y = torch.randn((Bt, K, M), device="cuda", generator=g), torch.zeros((Bt, N, M), device="cuda")
+        A = torch.full((Bt, N, 200) if op == "batchMatMul" else (Bt, K, 252), pad, device="cuda")
+        used = A[..., :K] if op == "batchMatMul" else A[..., :N]
+        used.copy_(torch.randn(used.shape, device="cuda", generator=g))
+        args = (Bt, N, M, K, 200) if op == "batchMatMul" else (Bt, N, 252, M, K)
+        time = time_of(lambda: lib.check(call(p(Y), p(A), p(B), *args, stream)))
+        assert lib.last_plan().startswith("gemm_f32 planes")
+        want = (used if op == "batchMatMul" else used.transpose(1, 2)).double() @ B.double()
+        assert float((Y.double() - want).norm() / want.norm()) <= 3e-7
+        out.append((time, Y))
+    assert torch.equal(out[0][1], out[1][1])
+    assert out[1][0] <= 1.5 * out[0][0], (out[1][0], out[0][0])

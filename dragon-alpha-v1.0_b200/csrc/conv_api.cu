@@ -202,7 +202,7 @@ struct DeviceCtx {
     struct PreparedDesc { WeightKey key; size_t bytes; };
     std::map<const void*, PreparedDesc> prepared;
 };
-static DeviceCtx g_ctx[64];
+static DeviceCtx g_ctx[kMaxDevices];
 static std::mutex g_mu;
 
 static PFN_encodeTiled g_encodeTiled = nullptr;
@@ -234,7 +234,7 @@ int get_ctx(DeviceCtx** out)
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
-    if (dev < 0 || dev >= 64) return fail(ALPHA_E_DEVICE, "device index %d out of range", dev);
+    if (dev < 0 || dev >= kMaxDevices) return fail(ALPHA_E_DEVICE, "device index %d out of range", dev);
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceCtx& c = g_ctx[dev];
     if (!c.init) {
@@ -257,9 +257,6 @@ int get_ctx(DeviceCtx** out)
         }
         c.sm_count = prop.multiProcessorCount;
         c.cc_major = prop.major;
-        const int max_smem = 227 * 1024;
-        cudaFuncSetAttribute(conv_igemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-        cudaFuncSetAttribute(conv_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
         c.init = true;
     }
     *out = &c;
@@ -797,7 +794,7 @@ static int launch_igemm(DeviceCtx* c, const IgemmPlan& pl, int mode3x, cudaStrea
     if (rc) return rc;
 
     dim3 grid((p.M_total + kBM - 1) / kBM, (pl.ncols + BN - 1) / BN, 1);
-    if (!t_dry) launch_after(conv_igemm_kernel, grid, kIgemmThreads, smem, stream, tmA, tmB, p);
+    if (!t_dry) launch_large<conv_igemm_kernel>(grid, kIgemmThreads, smem, stream, tmA, tmB, p);
     note_launch("igemm");
     return check_launch("conv_igemm_kernel");
 }
@@ -836,12 +833,7 @@ struct HaloLaunch {
 template <int FW_T, int JH_T, int JW_T, bool ROW_T, bool FLAT_T = false, bool LAT_T = false>
 static void halo_launch_one(const HaloLaunch& L)
 {
-    static bool attr_done = false;  // per instantiation; the attribute is per function, any device
-    if (!attr_done) {
-        cudaFuncSetAttribute(conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        attr_done = true;
-    }
-    if (!t_dry) launch_after(conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T>, L.grid, kHaloThreads2, L.smem, L.stream, *L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+    if (!t_dry) launch_large<conv_halo_kernel<FW_T, JH_T, JW_T, ROW_T, FLAT_T, LAT_T>>(L.grid, kHaloThreads2, L.smem, L.stream, *L.tmA, *L.tmB, *L.tmBlo, *L.tmO, *L.p);
 }
 
 template <int FW_T>
@@ -1028,12 +1020,7 @@ static HaloChoice plan_halo(const IgemmPlan& pl, int BN, int mode3x, int b_mn, i
 template <int FW_T, bool ROW_T, bool FLAT_T = false>
 static void halo_pair_launch_one(const HaloLaunch& L)
 {
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        attr_done = true;
-    }
-    if (!t_dry) launch_after(conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T>, L.grid, kHaloThreads, L.smem, L.stream, L.tmA->m[0], *L.tmB, *L.tmBlo, *L.tmO, *L.p);
+    if (!t_dry) launch_large<conv_halo_pair_kernel<FW_T, ROW_T, FLAT_T>>(L.grid, kHaloThreads, L.smem, L.stream, L.tmA->m[0], *L.tmB, *L.tmBlo, *L.tmO, *L.p);
 }
 
 // One 16 x 8 pixel accumulator per CTA, two CTAs per MMA.  Returns 1 when the shape does not fit.
@@ -1236,20 +1223,12 @@ static int launch_tapstack(DeviceCtx* c, const IgemmPlan& pl, const TapStackPlan
     cuuint32_t wbox[3] = {32, 1, (cuuint32_t)ts.BN};
     rc = make_tiled_map(&tmB, pl.W, 3, wd, wst, wbox, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(conv_tapstack_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(conv_tapstack_kernel<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(conv_tapstack_kernel<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(conv_tapstack_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        attr_done = true;
-    }
     const int grid = sm_budget(c) < p.total_tiles ? sm_budget(c) : p.total_tiles;
     if (!t_dry) {
-        if (pl.FW == 3 && pl.FH == 3) launch_after(conv_tapstack_kernel<3, 3>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
-        else if (pl.FW == 3) launch_after(conv_tapstack_kernel<3, 0>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
-        else if (pl.FW == 2) launch_after(conv_tapstack_kernel<2, 0>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
-        else launch_after(conv_tapstack_kernel<0, 0>, grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        if (pl.FW == 3 && pl.FH == 3) launch_large<conv_tapstack_kernel<3, 3>>(grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        else if (pl.FW == 3) launch_large<conv_tapstack_kernel<3, 0>>(grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        else if (pl.FW == 2) launch_large<conv_tapstack_kernel<2, 0>>(grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
+        else launch_large<conv_tapstack_kernel<0, 0>>(grid, kTapStackThreads, ts.smem, stream, tmA, tmB, p);
     }
     note_launch("halo_tapstack");
     snprintf(g_plan, sizeof(g_plan), "tapstack BN=%d N=%d CB=%d npb=%d eff=%.2f", ts.BN, pl.FW * ts.BN, ts.CB, ts.npb, ts.eff);
@@ -2256,11 +2235,6 @@ static int launch_gather_dw(DeviceCtx* c, const AlphaConvShape* s, const float* 
 
 // ---- deltaW, halo-tile kernel (strides 1 and 2): plan and launch -----------------------------------
 
-template <int FW_T, int R_T, int CW_T, bool STR_T = false>
-static void dw_halo_set_attr()
-{
-    cudaFuncSetAttribute(conv_dw_halo_kernel<FW_T, R_T, CW_T, STR_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-}
 static inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 struct DwForm { int G, NT; bool stacked, diag; long long cost; };   // cost: clocks of a filter row's MMAs per 8 pixels; < 0: none fits
@@ -2576,23 +2550,8 @@ static int launch_dw_halo(DeviceCtx* c, const AlphaConvShape* s_in, const float*
     if (rc) return rc;
 
     dim3 grid(parts, groups, 1);
-    static bool attr_done = false;
-    if (!attr_done) {
-        dw_halo_set_attr<0, 0, 0>();
-        dw_halo_set_attr<3, 1, 16>(); dw_halo_set_attr<3, 2, 16>(); dw_halo_set_attr<3, 4, 16>(); dw_halo_set_attr<3, 8, 16>();
-        dw_halo_set_attr<3, 2, 8>(); dw_halo_set_attr<3, 4, 8>(); dw_halo_set_attr<3, 8, 8>();
-        dw_halo_set_attr<3, 7, 16>(); dw_halo_set_attr<3, 7, 8>();
-        dw_halo_set_attr<1, 2, 16>(); dw_halo_set_attr<1, 4, 16>(); dw_halo_set_attr<1, 8, 16>();
-        dw_halo_set_attr<1, 7, 16>(); dw_halo_set_attr<1, 1, 16>(); dw_halo_set_attr<1, 2, 8>(); dw_halo_set_attr<1, 4, 8>(); dw_halo_set_attr<1, 7, 8>(); dw_halo_set_attr<1, 8, 8>();
-        dw_halo_set_attr<3, 2, 16, true>(); dw_halo_set_attr<3, 4, 16, true>(); dw_halo_set_attr<3, 8, 16, true>(); dw_halo_set_attr<3, 7, 16, true>();
-        dw_halo_set_attr<3, 4, 8, true>(); dw_halo_set_attr<3, 8, 8, true>(); dw_halo_set_attr<3, 7, 8, true>();
-        dw_halo_set_attr<4, 2, 16, true>(); dw_halo_set_attr<4, 4, 16, true>(); dw_halo_set_attr<4, 8, 16, true>();
-        dw_halo_set_attr<4, 4, 8, true>(); dw_halo_set_attr<4, 8, 8, true>();
-        dw_halo_set_attr<3, 2, 8, true>(); dw_halo_set_attr<4, 2, 8, true>(); dw_halo_set_attr<4, 7, 8, true>(); dw_halo_set_attr<4, 7, 16, true>();
-        attr_done = true;
-    }
-#define DWH_LAUNCH(FW_, R_, CW_) do { if (!t_dry) launch_after(conv_dw_halo_kernel<FW_, R_, CW_>, grid, kDwHaloThreads, smem, stream, tmXs, tmDY, p); } while (0)
-#define DWH_LAUNCH_S(FW_, R_, CW_) do { if (!t_dry) launch_after(conv_dw_halo_kernel<FW_, R_, CW_, true>, grid, kDwHaloThreads, smem, stream, tmXs, tmDY, p); } while (0)
+#define DWH_LAUNCH(FW_, R_, CW_) do { if (!t_dry) launch_large<conv_dw_halo_kernel<FW_, R_, CW_>>(grid, kDwHaloThreads, smem, stream, tmXs, tmDY, p); } while (0)
+#define DWH_LAUNCH_S(FW_, R_, CW_) do { if (!t_dry) launch_large<conv_dw_halo_kernel<FW_, R_, CW_, true>>(grid, kDwHaloThreads, smem, stream, tmXs, tmDY, p); } while (0)
     const bool st = G == 3 && !strided && opt(OPT_DW_STATIC) != 0;
     const bool st1 = s->FW == 1 && opt(OPT_DW_STATIC) != 0;   // one tap per row (with a stride: one phase, start 0)
     const bool ss3 = s->FW == 3 && strided && opt(OPT_DW_STATIC) != 0, ss4 = s->FW == 4 && strided && opt(OPT_DW_STATIC) != 0;
@@ -2882,7 +2841,7 @@ static int launch_dw_split(const AlphaConvShape* s, const float* X, const float*
     rc = make_tiled_map(&tmDY, deltaY, 2, dd, ds, box, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
     if (rc) return rc;
     dim3 grid(pl.groups, pl.n_tiles, pl.splits);
-    if (!t_dry) launch_after(conv_dw_kernel, grid, kIgemmThreads, pl.smem, stream, tmX, tmDY, p);
+    if (!t_dry) launch_large<conv_dw_kernel>(grid, kIgemmThreads, pl.smem, stream, tmX, tmDY, p);
     note_launch(tag);
     rc = check_launch("conv_dw_kernel");
     if (rc) return rc;
@@ -2913,7 +2872,7 @@ struct NoAllocCtx {
     float* scratch = nullptr;  // device address of g_noalloc_scratch on this device
     int* status = nullptr;     // device address of g_noalloc_status on this device
 };
-static NoAllocCtx g_noalloc_ctx[64];
+static NoAllocCtx g_noalloc_ctx[kMaxDevices];
 
 // Once per device, with that device current: resolves the device addresses of the two symbols.
 // In host code the names g_noalloc_scratch / g_noalloc_status are only handles; a kernel must be
@@ -2923,7 +2882,7 @@ static int get_noalloc_ctx(NoAllocCtx** out)
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
-    if (dev < 0 || dev >= 64) return fail(ALPHA_E_DEVICE, "device index %d out of range", dev);
+    if (dev < 0 || dev >= kMaxDevices) return fail(ALPHA_E_DEVICE, "device index %d out of range", dev);
     std::lock_guard<std::mutex> lock(g_mu);
     NoAllocCtx& c = g_noalloc_ctx[dev];
     if (!c.init) {
@@ -2942,8 +2901,6 @@ static int get_noalloc_ctx(NoAllocCtx** out)
         e = cudaGetSymbolAddress(&p, g_noalloc_status);
         if (e != cudaSuccess || !p) return fail(ALPHA_E_CUDA, "cudaGetSymbolAddress(status): %s", cudaGetErrorString(e));
         c.status = static_cast<int*>(p);
-        e = cudaFuncSetAttribute(conv_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return fail(ALPHA_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         c.sm_count = sms;
         c.init = true;
     }

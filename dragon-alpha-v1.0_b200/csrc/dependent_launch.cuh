@@ -1,8 +1,24 @@
-// Programmatic dependent launch: both sides.
+// Launches: dynamic shared memory beyond 48 KB, and programmatic dependent launch from both sides.
 #pragma once
 #include <cuda_runtime.h>
 
+#include "once_per_device.h"
+
+#include <utility>
+
 namespace alpha {
+
+// Lets launches of KERNEL on the current device ask for up to `bytes` of dynamic shared memory (always the same for a kernel).  The runtime
+// keeps a function's attributes for each device apart.  A failure stays in cudaGetLastError, is met by the launch, and is tried again.
+template <auto KERNEL>
+inline cudaError_t allow_smem(int bytes = 227 * 1024)
+{
+    static OncePerDevice once;
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return static_cast<cudaError_t>(once(device, [bytes] { return static_cast<int>(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); }));
+}
 
 // A kernel launched with launch_after may start while its predecessor in the stream still runs.  Every thread calls
 // grid_dependency_wait() before it touches global memory: it returns when the predecessor has completed and its writes are
@@ -38,6 +54,14 @@ inline void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cfg.attrs = &attr; cfg.numAttrs = plain ? 0 : 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);   // the caller looks at cudaGetLastError()
+}
+
+// The same for a kernel with more than 48 KB of dynamic shared memory.
+template <auto KERNEL, class... Args>
+inline void launch_large(dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args)
+{
+    allow_smem<KERNEL>();
+    launch_after(KERNEL, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace alpha

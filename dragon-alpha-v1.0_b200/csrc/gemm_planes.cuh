@@ -937,11 +937,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) gemm_planes_kernel(const __g
 template <int BN, bool TMA_B, class P>
 inline void launch_gemm_planes(const P& p, const CUtensorMap& tmB, dim3 tiles, unsigned sms, cudaStream_t stream, int* status)
 {
-    static bool attr_done = false;   // per instantiation; the attribute is per function, any device
-    if (!attr_done) {
-        cudaFuncSetAttribute(gemm_planes_kernel<BN, P, TMA_B>, cudaFuncAttributeMaxDynamicSharedMemorySize, plane_smem_bytes(BN));
-        attr_done = true;
-    }
+    allow_smem<gemm_planes_kernel<BN, P, TMA_B>>(plane_smem_bytes(BN));
     const unsigned total = tiles.x * tiles.y * tiles.z, most = sms ? sms : total;
     PlaneGrid g{0, fast_div(static_cast<int>(tiles.x)), fast_div(static_cast<int>(tiles.y))};
     for (; g.first < total; g.first += most)

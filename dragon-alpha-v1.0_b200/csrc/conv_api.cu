@@ -1946,8 +1946,6 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
         else { parts = ksplit; out = ws; }
     }
     const char* label = gather ? "gather" : "simt";
-    if (gather) note_plan("gather 128x%d%s phases=%lld ksplit=%d time=%.0f", t.bn, plan.copy_b ? " copy" : "", phases, ksplit, gather->time);
-    else note_plan("gemm_f32 %s%dx%d%s phases=%lld ksplit=%d%s", t.planes ? "planes " : "", t.bm, t.bn, plan.copy_b ? " copy" : "", phases, ksplit, turns > 1 ? " in turns" : "");
     const long long nz = phases * parts;
     auto fill = [&](auto& g) {
         g.dY = dY; g.W = W; g.out = out;
@@ -1985,6 +1983,8 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
             if (wrows) copy = &tmB;
         }
     }
+    if (gather) note_plan("gather 128x%d%s phases=%lld ksplit=%d time=%.0f", t.bn, copy ? " copy" : "", phases, ksplit, gather->time);
+    else note_plan("gemm_f32 %s%dx%d%s phases=%lld ksplit=%d%s", t.planes ? "planes " : "", t.bm, t.bn, copy ? " copy" : "", phases, ksplit, turns > 1 ? " in turns" : "");
     if (!t.planes) { fill(f); f.kt = (s->OC + kGemmBK - 1) / kGemmBK; f.by_kt = fast_div(f.kt); }
     const int slice = planes_slice(c);
     for (int turn = 0; turn < turns; ++turn) {

@@ -156,20 +156,34 @@ def test_operands_outside_the_planes(pkg, planes, what):
         assert bool(b[:, 0].isfinite().all()) and bool(b[..., :7].isfinite().all())
 
 
-def test_parts_give_the_same_bits_with_and_without_scratch(pkg, planes):
+# N, OH, IC, OC, F: a split reduction, W split beforehand, both, and a split reduction under a stride
+@pytest.mark.parametrize("shape,words", [((130, 1, 132, 2764, 1, 1), {"ksplit"}), ((64, 14, 132, 36, 3, 1), {"copy"}), ((26, 14, 132, 1004, 3, 1), {"copy", "ksplit"}), ((4, 9, 20, 1036, 3, 2), {"ksplit"})],
+                         ids=str)
+def test_parts_give_the_same_bits_with_and_without_scratch(pkg, planes, shape, words):
+    """A block of 256 bytes refuses all scratch: the parts then run in turns and add up in deltaX, and the kernel splits W itself."""
     import torch
-    eng = pkg.submodule("engine").Engine()
-    dY, W = torch.randn((130, 1, 1, 2764), device="cuda"), torch.randn((2764, 1, 1, 132), device="cuda")
-    want = eng.dconv3D_deltaX(dY, W, 1, 1, 1, 1, 0, 0)
-    plan = pkg.submodule("lib").last_plan()
-    assert "planes" in plan and "ksplit=1" not in plan.split()
-    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    eng, lib = pkg.submodule("engine").Engine(), pkg.submodule("lib")
+    N, OH, IC, OC, F, s = shape
+    p = F // 2
+    IH = (OH - 1) * s + F - 2 * p
+    g = torch.Generator(device="cuda").manual_seed(12)
+    dY, W = torch.randn((N, OH, OH, OC), device="cuda", generator=g), torch.randn((OC, F, F, IC), device="cuda", generator=g)
+    want = eng.dconv3D_deltaX(dY, W, IH, IH, s, s, p, p)
+    plan = lib.last_plan()
+    assert plan.startswith("gemm_f32 planes") and "in turns" not in plan, plan
+    assert {word for word, used in (("copy", " copy" in plan), ("ksplit", "ksplit=1" not in plan.split())) if used} == words, plan
+    stream, block = torch.cuda.Stream(), torch.empty(256, dtype=torch.uint8, device="cuda")
     torch.cuda.synchronize()
-    with torch.cuda.graph(graph, stream=stream):
-        got = eng.dconv3D_deltaX(dY, W, 1, 1, 1, 1, 0, 0)
-    graph.replay()
-    torch.cuda.synchronize()
-    assert "in turns" not in plan and torch.equal(got, want)
+    lib.set_workspace(stream.cuda_stream, block.data_ptr(), 256)
+    try:
+        with torch.cuda.stream(stream):
+            got = eng.dconv3D_deltaX(dY, W, IH, IH, s, s, p, p)
+        plan = lib.last_plan()
+        stream.synchronize()
+    finally:
+        lib.set_workspace(stream.cuda_stream, 0, 0)
+    assert plan.startswith("gemm_f32 planes") and "copy" not in plan and ("in turns" in plan) == ("ksplit" in words), plan
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("op", ["batchMatMul", "batchMatMulT1", "batchMatMulT2"])

@@ -373,7 +373,7 @@ struct PlaneDw {
     size_t size;
     FastDiv by_OW, by_OHW, by_IC, by_FW;
     struct Cta { int m0, n0, s0, s1, K; float* out; };
-    struct BRow { uint32_t at; int fh, fw; };               // fh = 1 << 30: no such column
+    struct BRow { uint32_t at; int fh, fw; };               // fh = 1 << 29: no such column (y = 1 << 29: no such step; their sum is no pixel either)
     struct BStep { uint32_t at; int y, x; };
 
     __device__ bool cta(Cta& c, int BM, int BN, int bx, int by, int sp) const
@@ -394,7 +394,7 @@ struct PlaneDw {
     __device__ BRow b_row(const Cta& c, int col) const
     {
         const int q = c.n0 + col;
-        if (q >= L) return BRow{0u, 1 << 30, 0};
+        if (q >= L) return BRow{0u, 1 << 29, 0};
         unsigned t, ic, fh, fw;
         by_IC.divmod(static_cast<unsigned>(q), t, ic);
         by_FW.divmod(t, fh, fw);
@@ -406,7 +406,7 @@ struct PlaneDw {
         by_OHW.divmod(static_cast<unsigned>(k), n, q);
         by_OW.divmod(q, oh, ow);
         const int y = static_cast<int>(oh) * sh - ph, x = static_cast<int>(ow) * sw - pw;
-        return BStep{static_cast<uint32_t>(((static_cast<int>(n) * IH + y) * IW + x) * IC), k < K ? y : 1 << 30, x};
+        return BStep{static_cast<uint32_t>(((static_cast<int>(n) * IH + y) * IW + x) * IC), k < K ? y : 1 << 29, x};
     }
     __device__ static bool use_a(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
     __device__ bool use_b(const BRow& row, const BStep& step) const

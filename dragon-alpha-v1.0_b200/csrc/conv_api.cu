@@ -1920,8 +1920,8 @@ static int launch_split_planes(DeviceCtx* c, const float* W, float* planes, int 
     return check_launch("split_planes_kernel");
 }
 
-// (`gather`: the layer is not fp32 work but runs here on the tensor cores, with this plan; 1 without scratch for its parts.)
-static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream, const PlanePlan* gather = nullptr)
+// (`gather`: the layer is not fp32 work but runs here on the tensor cores, with this plan; 1 without its scratch, unless `bare`.)
+static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream, const PlanePlan* gather = nullptr, bool bare = false)
 {
     const long long rows = (long long)s->N * ((s->IH + s->sh - 1) / s->sh) * ((s->IW + s->sw - 1) / s->sw);
     const int nsh = s->sh < s->IH ? s->sh : s->IH, nsw = s->sw < s->IW ? s->sw : s->IW;   // phases that own a pixel
@@ -1941,7 +1941,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
         float* ws = nullptr;
         const int rc = get_workspace(c, stream, (size_t)ksplit * size * sizeof(float), &ws);
         if (rc && !scratch_refused(rc)) return rc;
-        if (rc && gather) return 1;
+        if (rc && gather && !bare) return 1;
         if (rc) turns = ksplit;
         else { parts = ksplit; out = ws; }
     }
@@ -1962,7 +1962,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
         p.set_divisions();
         float* ws = nullptr;
         const int rc = plan.copy_b ? get_workspace(c, stream, (size_t)w * 6, &ws) : ALPHA_OK;
-        if (rc && (gather || !scratch_refused(rc))) return scratch_refused(rc) ? 1 : rc;
+        if (rc && ((gather && !bare) || !scratch_refused(rc))) return scratch_refused(rc) ? 1 : rc;
         if (ws) {                                                            // (without scratch the kernel splits W itself: the same sums)
             // the rows of W in the order in which the phases' steps meet them
             SplitRows map{};
@@ -1983,7 +1983,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
             if (wrows) copy = &tmB;
         }
     }
-    if (gather) note_plan("gather 128x%d%s phases=%lld ksplit=%d time=%.0f", t.bn, copy ? " copy" : "", phases, ksplit, gather->time);
+    if (gather) note_plan("gather 128x%d%s phases=%lld ksplit=%d%s time=%.0f", t.bn, copy ? " copy" : "", phases, ksplit, turns > 1 ? " in turns" : "", gather->time);
     else note_plan("gemm_f32 %s%dx%d%s phases=%lld ksplit=%d%s", t.planes ? "planes " : "", t.bm, t.bn, copy ? " copy" : "", phases, ksplit, turns > 1 ? " in turns" : "");
     if (!t.planes) { fill(f); f.kt = (s->OC + kGemmBK - 1) / kGemmBK; f.by_kt = fast_div(f.kt); }
     const int slice = planes_slice(c);
@@ -2130,9 +2130,9 @@ static bool gather_pays(const AlphaConvShape* s, ConvOp op, double time)
 
 // Returns 1 where the layer is left to the other routes.
 
-// (`f32`: a layer that would otherwise run one thread per element.)
+// (`f32`: a layer that would otherwise run one thread per element; `bare`: without scratch, whatever that costs.)
 static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* W, const float* bias, float* Y, int act_on, float act_k,
-                                 cudaStream_t stream, bool f32 = false)
+                                 cudaStream_t stream, bool f32 = false, bool bare = false)
 {
     const int mode = f32 ? option_f32_planes() : gather_mode(s, ConvOp::Forward);
     if (!mode || !planes_fit(s, s->FH, s->FW)) return 1;
@@ -2143,10 +2143,11 @@ static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const fl
     p.K = s->FH * s->FW * s->IC; p.rows = s->N * s->OH * s->OW;
     p.size = (size_t)p.rows * s->OC;
     const int Kp = (p.K + 31) / 32 * 32;
-    const PlanePlan plan = plan_planes(p.rows, s->OC, p.K, 1, 16, (double)p.size, (double)Kp * s->OC, c->sm_count);
+    PlanePlan plan = plan_planes(p.rows, s->OC, p.K, 1, 16, (double)p.size, (double)Kp * s->OC, c->sm_count);
+    if (mode == 1 && !f32 && !gather_pays(s, ConvOp::Forward, plan.time)) return 1;
+    if (bare) plan = plan_planes(p.rows, s->OC, p.K, 1, 1, (double)p.size, 0, c->sm_count);
     const long long gx = (p.rows + kPlaneBM - 1) / kPlaneBM, gy = (s->OC + plan.bn - 1) / plan.bn;
     if (gx * gy * plan.ksplit > 2147483647LL) return 1;
-    if (mode == 1 && !f32 && !gather_pays(s, ConvOp::Forward, plan.time)) return 1;
     const WsMark start = ws_mark(c, stream);
     p.ksplit = plan.ksplit;
     p.out = Y;
@@ -2184,7 +2185,7 @@ static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const fl
     return rc;
 }
 
-static int launch_gather_dx(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream)
+static int launch_gather_dx(DeviceCtx* c, const AlphaConvShape* s, const float* dY, const float* W, float* dX, cudaStream_t stream, bool bare = false)
 {
     const int mode = gather_mode(s, ConvOp::DeltaX);
     const int nsh = s->sh < s->IH ? s->sh : s->IH, nsw = s->sw < s->IW ? s->sw : s->IW;
@@ -2198,7 +2199,7 @@ static int launch_gather_dx(DeviceCtx* c, const AlphaConvShape* s, const float* 
     // (the phase of the most taps ends last: the plan counts with the average)
     const double last = ((double)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * s->OC - k) / plan.ksplit / kPlaneBK * (plan.copy_b ? 0.57 : 0.80);
     if (mode == 1 && !gather_pays(s, ConvOp::DeltaX, plan.time + last)) return 1;
-    return launch_dx_f32(c, s, dY, W, dX, stream, &plan);
+    return launch_dx_f32(c, s, dY, W, dX, stream, &plan, bare);
 }
 
 static int launch_gather_dw(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* dY, float* dW, cudaStream_t stream, bool f32 = false)
@@ -3187,7 +3188,7 @@ int alpha_conv3d_forward_leakyRelu(const AlphaConvShape* s, const float* X, cons
 
 }  // extern "C"
 
-static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* W, const float* bias,
+static int forward_routes(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* W, const float* bias,
                           float* Y, cudaStream_t stream, int algo, int act_on, float act_k)
 {
     int rc = launch_gather_forward(c, s, X, W, bias, Y, act_on, act_k, stream);
@@ -3272,22 +3273,27 @@ static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X,
     return check_launch("conv_fwd_simt");
 }
 
-extern "C" {
-
-int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const float* W, float* deltaX,
-                        alpha_stream_t stream_)
+// Layers gathered here have no prepared weights, with which another route may have needed no scratch: where all are refused theirs
+// (a capture on a new stream), the layer is gathered without.
+static int forward_direct(DeviceCtx* c, const AlphaConvShape* s, const float* X, const float* W, const float* bias,
+                          float* Y, cudaStream_t stream, int algo, int act_on, float act_k)
 {
-    OpRange range("alpha_conv3d_deltaX");
-    int rc = check_shape(s, deltaY, W, deltaX);
-    if (rc) return rc;
-    DeviceCtx* c;
-    rc = get_ctx(&c);
-    if (rc) return rc;
-    cudaStream_t stream = (cudaStream_t)stream_;
-    ws_begin(c, stream);
+    const WsMark start = ws_mark(c, stream);
+    const int rc = forward_routes(c, s, X, W, bias, Y, stream, algo, act_on, act_k);
+    if (!rc || !scratch_refused(rc)) return rc;
+    ws_rewind(c, stream, start);
+    const int bare = launch_gather_forward(c, s, X, W, bias, Y, act_on, act_k, stream, false, true);
+    return bare == 1 ? rc : bare;
+}
+
+// Channel counts that the TF32 paths leave: launch_dx_f32 chooses their kernel.
+static bool deltaX_is_f32(const AlphaConvShape* s) { return s->sh == 1 && s->sw == 1 ? s->OC % 8 != 0 : s->OC % 32 != 0; }
+
+static int deltaX_routes(DeviceCtx* c, const AlphaConvShape* s, const float* deltaY, const float* W, float* deltaX, cudaStream_t stream)
+{
+    int rc;
     const int algo = cur_algo();
-    // (what is fp32 work anyway chooses its kernel in launch_dx_f32)
-    if (s->sh == 1 && s->sw == 1 ? s->OC % 8 == 0 : s->OC % 32 == 0) {
+    if (!deltaX_is_f32(s)) {
         const WsMark start = ws_mark(c, stream);
         rc = launch_gather_dx(c, s, deltaY, W, deltaX, stream);
         if (rc != 1) return rc;
@@ -3355,6 +3361,27 @@ in_place:
         if (rc != 1) return rc;
     }
     return launch_dx_f32(c, s, deltaY, W, deltaX, stream);
+}
+
+extern "C" {
+
+int alpha_conv3d_deltaX(const AlphaConvShape* s, const float* deltaY, const float* W, float* deltaX,
+                        alpha_stream_t stream_)
+{
+    OpRange range("alpha_conv3d_deltaX");
+    int rc = check_shape(s, deltaY, W, deltaX);
+    if (rc) return rc;
+    DeviceCtx* c;
+    rc = get_ctx(&c);
+    if (rc) return rc;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    ws_begin(c, stream);
+    rc = deltaX_routes(c, s, deltaY, W, deltaX, stream);
+    if (!rc || !scratch_refused(rc) || deltaX_is_f32(s)) return rc;
+    // (as in forward_direct)
+    ws_begin(c, stream);
+    const int bare = launch_gather_dx(c, s, deltaY, W, deltaX, stream, true);
+    return bare == 1 ? rc : bare;
 }
 
 int alpha_conv3d_deltaW(const AlphaConvShape* s, const float* X, const float* deltaY, float* deltaW,

@@ -199,3 +199,47 @@ def test_route(pkg, gather, op, shape, taken):
         torch.cuda.synchronize()
         assert float((again - other).abs().max()) <= 4e-5 * float(other.abs().max())
     assert L.alpha_conv_device_status() == 0
+
+
+# split reductions and W split beforehand, whose scratch a capture on a new stream refuses; the other routes need scratch for the transform of W alone
+PREPARED = [("forward", (512, 8, 8, 128, 128, 3, 1, 1)), ("forward", (64, 15, 13, 36, 100, 3, 1, 1)), ("forward", (16, 8, 8, 256, 256, 3, 1, 1)),
+            ("deltaX", (512, 8, 8, 128, 128, 3, 1, 1)), ("deltaX", (250, 1, 1, 1024, 1024, 1, 1, 0)), ("deltaX", (16, 8, 8, 256, 256, 3, 1, 1))]
+
+
+@pytest.mark.parametrize("op,shape", PREPARED, ids=str)
+def test_prepared_layers_are_captured_on_a_new_stream(pkg, gather, op, shape):
+    """With weights prepared for them such layers needed no scratch on the other kernels; gathered, they have no prepared weights, and run without."""
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    N, IH, IW, IC, OC, F, s, p = shape
+    OH, OW = out_hw(IH, IW, F, F, s, s, p, p)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    X, W, dY = (torch.randn(q, device="cuda", generator=g) for q in ((N, IH, IW, IC), (OC, F, F, IC), (N, OH, OW, OC)))
+    base = engine.CudaFloat32EngineBase(math="3xtf32")
+    got = {}
+    for option in (0, 1):
+        gather(option)
+        block = base.prepare_weights(op, W, F, F, N, IH, IW, OH, OW, IC, OC, s, s, p, p)
+
+        def call():
+            out = torch.empty_like(dY if op == "forward" else X)
+            if op == "forward":
+                base.conv3D_prepared(out, OH, OW, X, IH, IW, W, F, F, N, IC, OC, s, s, p, p, block)
+            else:
+                base.dconv3D_deltaX_prepared(out, IH, IW, dY, OH, OW, W, F, F, N, IC, OC, s, s, p, p, block)
+            return out
+
+        eager = call()
+        assert (lib.last_algo() == "gather") == (option == 1)
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            got[option] = call()
+        if option:
+            assert lib.last_plan().startswith("gather")
+        graph.replay()
+        torch.cuda.synchronize()
+        if op == "deltaX" and option:
+            assert torch.equal(got[option], eager)               # (forwards, of both sides, add their products up in fewer parts)
+    assert float((got[1] - got[0]).abs().max()) <= 4e-5 * float(got[0].abs().max())
+    assert lib.device_status() == 0

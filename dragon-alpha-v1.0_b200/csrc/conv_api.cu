@@ -501,6 +501,26 @@ static int weight_planes(DeviceCtx* c, cudaStream_t stream, const DeviceCtx::Wei
     *out = e.ptr;
     return ALPHA_OK;
 }
+
+// A layer that needs no transform refuses all the same what is no block of its: made for another tensor, shape, operator or math mode, or cut
+// short.  (Blocks that hold nothing are let through: a layer without a transform is prepared into any.)
+static int check_unused_block(DeviceCtx* c, const AlphaConvShape* s, const float* W, int op)
+{
+    if (t_prep.mode != 2 || t_prep.W != W) return ALPHA_OK;
+    std::lock_guard<std::mutex> lock(g_mu);
+    auto it = c->prepared.find(t_prep.ptr);
+    if (it == c->prepared.end()) return ALPHA_OK;
+    const DeviceCtx::WeightKey& k = it->second.key;
+    const bool fwd = op == ALPHA_OP_FORWARD, own = k.W == W && (fwd ? k.kind == WK_FWD_LO && k.a == (int)((size_t)s->OC * s->FH * s->FW * s->IC & 0x7fffffff)
+                                                                    : k.kind != WK_FWD_LO && k.a == s->OC && k.b == s->IC && k.c == s->FH * 256 + s->FW && k.e == cur_mode3x());
+    if (!own) return fail(ALPHA_E_ARG, "the prepared-weights block was made by alpha_conv_prepare_weights for another tensor, shape, operator or math mode");
+    if (it->second.bytes > t_prep.bytes) {
+        t_bad_block = true;
+        return fail(ALPHA_E_NOSCRATCH, "the prepared-weights block holds %zu bytes, this layer's transform needs %zu", t_prep.bytes, it->second.bytes);
+    }
+    return ALPHA_OK;
+}
+
 static void weight_planes_ready(DeviceCtx* c, cudaStream_t stream, const DeviceCtx::WeightKey& key)
 {
     if (t_dry || !g_weight_cache.load(std::memory_order_relaxed)) return;
@@ -2145,6 +2165,8 @@ static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const fl
     const int Kp = (p.K + 31) / 32 * 32;
     PlanePlan plan = plan_planes(p.rows, s->OC, p.K, 1, 16, (double)p.size, (double)Kp * s->OC, c->sm_count);
     if (mode == 1 && !f32 && !gather_pays(s, ConvOp::Forward, plan.time)) return 1;
+    int rc = f32 ? ALPHA_OK : check_unused_block(c, s, W, ALPHA_OP_FORWARD);
+    if (rc) return rc;
     if (bare) plan = plan_planes(p.rows, s->OC, p.K, 1, 1, (double)p.size, 0, c->sm_count);
     const long long gx = (p.rows + kPlaneBM - 1) / kPlaneBM, gy = (s->OC + plan.bn - 1) / plan.bn;
     if (gx * gy * plan.ksplit > 2147483647LL) return 1;
@@ -2158,7 +2180,6 @@ static int launch_gather_forward(DeviceCtx* c, const AlphaConvShape* s, const fl
         p.bias = bias; p.act_on = act_on; p.act_k = act_k;
     }
     p.by_OW = fast_div(s->OW); p.by_OHW = fast_div(s->OH * s->OW); p.by_IC = fast_div(s->IC); p.by_FW = fast_div(s->FW);
-    int rc = ALPHA_OK;
     CUtensorMap tmB{};
     if (plan.copy_b) {
         float* ws = nullptr;
@@ -2199,6 +2220,8 @@ static int launch_gather_dx(DeviceCtx* c, const AlphaConvShape* s, const float* 
     // (the phase of the most taps ends last: the plan counts with the average)
     const double last = ((double)((s->FH + s->sh - 1) / s->sh) * ((s->FW + s->sw - 1) / s->sw) * s->OC - k) / plan.ksplit / kPlaneBK * (plan.copy_b ? 0.57 : 0.80);
     if (mode == 1 && !gather_pays(s, ConvOp::DeltaX, plan.time + last)) return 1;
+    const int rc = check_unused_block(c, s, W, ALPHA_OP_DELTAX);
+    if (rc) return rc;
     return launch_dx_f32(c, s, dY, W, dX, stream, &plan, bare);
 }
 
@@ -3513,6 +3536,13 @@ static int run_weight_transform(const AlphaConvShape* s, int op, const float* W,
                                           : alpha_conv3d_deltaX(s, fake, w, fake, stream);
     t_dry = false;
     if (need) *need = t_prep.seen ? t_prep.need : 0;
+    if (mode == 1 && !rc && !t_prep.seen) {          // the block holds nothing (any more)
+        DeviceCtx* c;
+        if (!get_ctx(&c)) {
+            std::lock_guard<std::mutex> lock(g_mu);
+            c->prepared.erase(prepared);
+        }
+    }
     t_prep = PreparedHint{};
     return rc;
 }

@@ -243,3 +243,44 @@ def test_prepared_layers_are_captured_on_a_new_stream(pkg, gather, op, shape):
             assert torch.equal(got[option], eager)               # (forwards, of both sides, add their products up in fewer parts)
     assert float((got[1] - got[0]).abs().max()) <= 4e-5 * float(got[0].abs().max())
     assert lib.device_status() == 0
+
+
+def test_blocks_that_are_not_the_layers_are_refused(pkg, gather):
+    """A block serves every batch of its layer, those that are gathered (512) and need none among them; made for another operator, tensor or math
+    mode, or cut short, it is refused whatever the batch."""
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    base = engine.CudaFloat32EngineBase()
+    C, H = 128, 8
+    g = torch.Generator(device="cuda").manual_seed(11)
+    W, V = (torch.randn((C, 3, 3, C), device="cuda", generator=g) for _ in range(2))
+    gather(1)
+
+    def call(op, n, block, w=W):
+        x, out = torch.ones((n, H, H, C), device="cuda"), torch.empty((n, H, H, C), device="cuda")
+        (base.conv3D_prepared if op == "forward" else base.dconv3D_deltaX_prepared)(out, H, H, x, H, H, w, 3, 3, n, C, C, 1, 1, 1, 1, block)
+        return out
+
+    make = lambda op, n, w=W: base.prepare_weights(op, w, 3, 3, n, H, H, H, H, C, C, 1, 1, 1, 1)
+    blocks = {op: make(op, 8) for op in ("forward", "deltaX")}
+    others = {op: make(op, 8, V) for op in blocks}
+    lib.set_math_mode("tf32")
+    plain = make("deltaX", 8)
+    lib.set_math_mode("3xtf32")
+    for op in blocks:
+        for n in (8, 512):
+            want = call(op, n, None)
+            assert (lib.last_algo() == "gather") == (n == 512)
+            assert torch.equal(call(op, n, blocks[op]), want)
+            for bad in (blocks["deltaX" if op == "forward" else "forward"], others[op], blocks[op][:256]) + ((plain,) if op == "deltaX" else ()):
+                with pytest.raises(lib.AlphaConvError):
+                    call(op, n, bad)
+    # a layer without a transform, prepared into memory that held another's
+    L = lib.load()
+    import ctypes
+    shape = lib.AlphaConvShape(512, H, H, C, C, 3, 3, H, H, 1, 1, 1, 1)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    old = others["forward"]
+    assert lib.prepared_weights_bytes(shape, "forward") == 0
+    lib.check(L.alpha_conv_prepare_weights(ctypes.byref(shape), lib.OPS["forward"], p(W), p(old), old.numel(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert torch.equal(call("forward", 512, old), call("forward", 512, None))

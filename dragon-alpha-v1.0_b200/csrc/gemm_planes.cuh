@@ -373,7 +373,8 @@ struct PlaneDw {
     size_t size;
     FastDiv by_OW, by_OHW, by_IC, by_FW;
     struct Cta { int m0, n0, s0, s1, K; float* out; };
-    struct BRow { uint32_t at; int fh, fw; };               // fh = 1 << 29: no such column (y = 1 << 29: no such step; their sum is no pixel either)
+    static constexpr int kNone = 1 << 30;                   // as fh: no such column, as y: no such step (added without sign: 2^31 is no row either)
+    struct BRow { uint32_t at; int fh, fw; };
     struct BStep { uint32_t at; int y, x; };
 
     __device__ bool cta(Cta& c, int BM, int BN, int bx, int by, int sp) const
@@ -394,7 +395,7 @@ struct PlaneDw {
     __device__ BRow b_row(const Cta& c, int col) const
     {
         const int q = c.n0 + col;
-        if (q >= L) return BRow{0u, 1 << 29, 0};
+        if (q >= L) return BRow{0u, kNone, 0};
         unsigned t, ic, fh, fw;
         by_IC.divmod(static_cast<unsigned>(q), t, ic);
         by_FW.divmod(t, fh, fw);
@@ -406,12 +407,12 @@ struct PlaneDw {
         by_OHW.divmod(static_cast<unsigned>(k), n, q);
         by_OW.divmod(q, oh, ow);
         const int y = static_cast<int>(oh) * sh - ph, x = static_cast<int>(ow) * sw - pw;
-        return BStep{static_cast<uint32_t>(((static_cast<int>(n) * IH + y) * IW + x) * IC), k < K ? y : 1 << 29, x};
+        return BStep{static_cast<uint32_t>(((static_cast<int>(n) * IH + y) * IW + x) * IC), k < K ? y : kNone, x};
     }
     __device__ static bool use_a(const PlaneAt& row, const PlaneAt& step) { return plane_meets(row, step); }
-    __device__ bool use_b(const BRow& row, const BStep& step) const
+    __host__ __device__ bool use_b(const BRow& row, const BStep& step) const
     {
-        return static_cast<unsigned>(step.y + row.fh) < static_cast<unsigned>(IH) && static_cast<unsigned>(step.x + row.fw) < static_cast<unsigned>(IW);
+        return static_cast<unsigned>(step.y) + static_cast<unsigned>(row.fh) < static_cast<unsigned>(IH) && static_cast<unsigned>(step.x + row.fw) < static_cast<unsigned>(IW);
     }
     __device__ float* row_out(const Cta& c, int m) const { return c.m0 + m < OC ? c.out + static_cast<size_t>(c.m0 + m) * L : nullptr; }
     __device__ void store(const Cta& c, float* row, int col, const float4& o) const

@@ -2235,10 +2235,18 @@ static int launch_gather_dw(DeviceCtx* c, const AlphaConvShape* s, const float* 
     p.K = s->N * s->OH * s->OW; p.L = s->FH * s->FW * s->IC;
     p.size = (size_t)s->OC * p.L;
     // (a few tiles over many pixels: as many parts as fill the SMs; 50 x 35 x 29, 36 -> 100, 3x3 is three tiles and 49 parts)
-    const PlanePlan plan = plan_planes(s->OC, p.L, p.K, 1, c->sm_count, (double)p.size, 0, c->sm_count);
+    PlanePlan plan = plan_planes(s->OC, p.L, p.K, 1, c->sm_count, (double)p.size, 0, c->sm_count);
+    if (mode == 1 && !f32 && !gather_pays(s, ConvOp::DeltaW, plan.time)) return 1;
+    if (f32) {
+        // conv_dw_simt adds K / 128 products in a lane and 128 lanes in a tree.  One chain of windows of 64 would err by up to 1.14 of that (24 x
+        // 37x37, 508 -> 20, 7x7 s2: 1.19e-7, 1.35e-7); parts of K / 512 windows, which dw_reduce_kernel adds with compensation, by 0.53 to 0.97 from 4
+        // pixels on (below, a product is 2.5e-8 there and 3.5e-8 here).  2 x 30x30, 700 -> 160, 7x7 s2: 17.7 ms there, 0.11 in a chain, 0.21 in parts.
+        if (mode == 1 && p.K < 4) return 1;
+        const int windows = (p.K + 2 * kPlaneBK - 1) / (2 * kPlaneBK), most = p.K / 512 > 1 ? p.K / 512 : 1, parts = (windows + most - 1) / most;
+        if (plan.ksplit < parts) plan.ksplit = parts;
+    }
     const long long gx = (s->OC + kPlaneBM - 1) / kPlaneBM, gy = (p.L + plan.bn - 1) / plan.bn;
     if (gx * gy * plan.ksplit > 2147483647LL) return 1;
-    if (mode == 1 && !f32 && !gather_pays(s, ConvOp::DeltaW, plan.time)) return 1;
     p.ksplit = plan.ksplit;
     p.out = dW;
     if (p.ksplit > 1) {

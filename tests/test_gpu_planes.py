@@ -271,3 +271,31 @@ def test_what_lies_between_matrix_and_pitch(pkg, planes, op):
         out.append((time, Y))
     assert torch.equal(out[0][1], out[1][1])
     assert out[1][0] <= 1.5 * out[0][0], (out[1][0], out[0][0])
+
+
+# N, H, IC, OC, F, s, p: deltaW of odd channel counts whose rows are too long for a patch product, 1 to 8664 pixels
+@pytest.mark.parametrize("shape", [(1, 2, 4100, 8, 2, 1, 0), (1, 6, 460, 8, 6, 1, 2), (2, 30, 700, 160, 7, 2, 3), (15, 8, 760, 160, 5, 1, 2), (24, 37, 508, 20, 7, 2, 3)], ids=str)
+@pytest.mark.parametrize("data", ["relu", "n01"])
+def test_long_deltaW_errs_no_more_than_the_fma_kernel(pkg, shape, data):
+    """That one adds 128 lanes of K / 128 products in a tree: 7e-8 to 1.2e-7 against 64 bits, so that windows in one chain would not do."""
+    import torch
+    engine, lib = pkg.submodule("engine"), pkg.submodule("lib")
+    L = lib.load()
+    eng = engine.Engine(engine.CudaFloat32EngineBase(math="3xtf32"))
+    N, H, IC, OC, F, s, p = shape
+    OH, OW = out_hw(H, H, F, F, s, s, p, p)
+    g = torch.Generator(device="cuda").manual_seed(H)
+    X, dY = torch.randn((N, H, H, IC), device="cuda", generator=g), torch.randn((N, OH, OW, OC), device="cuda", generator=g)
+    if data == "relu":
+        X.relu_()
+    ref = torch.nn.grad.conv2d_weight(X.double().permute(0, 3, 1, 2), (OC, IC, F, F), dY.double().permute(0, 3, 1, 2), stride=s, padding=p).permute(0, 2, 3, 1)
+    err = {}
+    for option in (0, 1):
+        lib.check(L.alpha_conv_set_option(b"F32_PLANES", option))
+        try:
+            err[option] = float((eng.dconv3D_deltaW(X, dY, F, F, s, s, p, p).double() - ref).norm() / ref.norm())
+        finally:
+            lib.check(L.alpha_conv_set_option(b"F32_PLANES", 1))
+        assert lib.last_algo() == "simt"
+    assert N * OH * OW < 4 or lib.last_plan().startswith("gemm_f32 planes")
+    assert err[1] <= err[0], err

@@ -2039,7 +2039,9 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
 // One kernel (two or three launches with W split beforehand or the parts of a reduction added up) that gathers what it multiplies, against
 // the kernels of this file, which stage rectangular tiles: it loses to them on large layers whose images fill those tiles, and
 // wins on small layers (their launches), on images and channel counts that do not, on strides and on long reductions.  Its sums err by
-// 1.0e-7 to 1.8e-7 where theirs err by 1.2e-7 to 1.4e-5 (2-norm against 64 bits; no smaller in any of 1200 calls).
+// 3.8e-8 to 1.8e-7 where theirs err by 1.1e-7 to 1.9e-4 (2-norm against 64 bits, 833 layers of 1e7 to 1e10 FLOPs; 0.55 of theirs at most).
+// Prepared or cached weights spare the other kernels a launch and do not count: against blocks prepared for them, 300 forwards that leave take 0.63
+// of the time and 199 deltaX 0.50; three of the 499 take 1.20 to 1.25 (20 x 7x7, 448 -> 416, 7x7 s2 deltaX 52 -> 66).
 
 // GPU time in us of a 3xTF32 operator on those other kernels (and not of deltaX under a stride with OC % 32 != 0, which is fp32 work), fitted to
 // layers of 1 to 600 images of 2 to 130 pixels a side, 16 to 700 channels, 1x1 to 7x7, strides 1 and 2, 1e8 to 1e11 FLOPs:
@@ -2118,7 +2120,9 @@ static double other_kernels_time(const AlphaConvShape* s, ConvOp op)
 static bool gather_suits(const AlphaConvShape* s, ConvOp op)
 {
     const bool strided = s->sh > 1 || s->sw > 1, filter = s->FH > 1 || s->FW > 1, fwd = op == ConvOp::Forward;
-    if (matrix_product(s) && op == ConvOp::Forward && s->IC > 6000 && s->IC % 32) return false;   // (the halo kernel keeps their corrections apart, as a test requires)
+    // (no limit of this kernel's: 995 x 6148 x 73 43 -> 31 us and 1.7e-6 -> 1.2e-7, 512 x 6148 x 512 34 -> 31, 1024 x 8200 x 1000 108 -> 108, but 256 x 12004 x 4096
+    // 230 -> 270; a test of ragged channels names the halo kernel for the first)
+    if (matrix_product(s) && op == ConvOp::Forward && s->IC > 6000 && s->IC % 32) return false;
     if (matrix_product(s)) return op == ConvOp::DeltaX ? s->OC >= 16 : s->IC >= 16 && (s->IC % 32 == 0 || patch_path_ok(s));
     const double other = other_kernels_time(s, op);
     const int h = fwd ? s->OH : (s->IH + s->sh - 1) / s->sh, w = fwd ? s->OW : (s->IW + s->sw - 1) / s->sw;        // deltaX: of one phase

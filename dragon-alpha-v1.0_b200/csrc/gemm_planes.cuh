@@ -20,7 +20,7 @@
 //   warps 0-15  in two groups that take alternate stages, so that the loads of one are in flight while the other splits: load the words of
 //               a stage, split them and store the planes of both operands in shared memory as the MMA reads them - rows of 32 steps where
 //               the operand's memory runs along k (K-major), rows of 32 columns where it does not (MN-major; no transposition) - with the
-//               64-byte swizzle; a warp's four rows of eight words are 256 consecutive bytes of a plane: no bank conflicts.  They also add
+//               64-byte swizzle; a warp's four rows of eight words are 256 consecutive bytes of a plane, half a warp's 128 all banks once.  They also add
 //               up the flushed sums, a quarter of the columns each, and store the result.  96 registers a thread allow no more: with more
 //               live words or sums they spill, and what spills goes to L2 (shared memory leaves no L1; 44 TFLOP/s).
 //   warp 16     issues the MMAs.  The three planes of B are neighbouring rows (or column blocks) of one operand, so that h x [m l], m x [h m]

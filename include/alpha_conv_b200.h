@@ -85,9 +85,10 @@ int alpha_conv_get_option(const char* name, int* value);
 int alpha_conv_device_status(void);
 /* Number of kernel launches this library has issued from the calling process. */
 unsigned long long alpha_conv_launch_count(void);
-/* Name of the kernel family the last call of this thread used ("igemm", "dw", "simt", ...). */
+/* Name of the kernel family the last call of this thread used ("igemm", "dw", "gather", ...).  "simt" and "bmm_simt" are
+ * products at fp32 accuracy, by FMAs or as three bf16 planes: alpha_conv_last_plan says which ("gemm_f32 planes ..."). */
 const char* alpha_conv_last_algo(void);
-/* Tile plan of the last halo-tile launch of this thread (tile shape, buffers), for tuning. */
+/* Tile plan of the last halo-tile, gathered or fp32 launch of this thread (tile shape, buffers), for tuning. */
 const char* alpha_conv_last_plan(void);
 /* Tracing aid: with ALPHA_CONV_PROF=1 in the environment the halo-tile kernel records, for its first
  * CTA, the clock ticks each warp role spent waiting and working (slots: producer patch wait,
@@ -152,7 +153,8 @@ int alpha_conv_weights_updated(const float* W);
  *   alpha_conv_prepared_weights_bytes  size of the transform op (ALPHA_OP_FORWARD / ALPHA_OP_DELTAX) needs for this
  *                                      shape under the current math mode and options; 0 = none: every plain TF32 forward,
  *                                      and 3xTF32 forwards whose kernel splits W itself (by the cost of the shape: im2col,
- *                                      windows of several filter rows).  A block serves every batch of its layer.
+ *                                      windows of several filter rows; gathered layers, forward and deltaX).  A block
+ *                                      serves every batch of its layer, those that need none among them.
  *   alpha_conv_prepare_weights         enqueues the transform of W into `prepared` (256-byte aligned) on `stream`
  *   alpha_conv3d_forward_prepared /    the contraction with the transform taken from `prepared`; shape, W address,
  *   alpha_conv3d_deltaX_prepared       operator and math mode must be those of the prepare call (checked on the

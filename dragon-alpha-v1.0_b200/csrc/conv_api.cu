@@ -2039,7 +2039,7 @@ static int launch_dx_f32(DeviceCtx* c, const AlphaConvShape* s, const float* dY,
 // One kernel (two or three launches with W split beforehand or the parts of a reduction added up) that gathers what it multiplies, against
 // the kernels of this file, which stage rectangular tiles: it loses to them on large layers whose images fill those tiles, and
 // wins on small layers (their launches), on images and channel counts that do not, on strides and on long reductions.  Its sums err by
-// 3.8e-8 to 1.8e-7 where theirs err by 1.1e-7 to 1.9e-4 (2-norm against 64 bits, 833 layers of 1e7 to 1e10 FLOPs; 0.55 of theirs at most).
+// 3.7e-8 to 2.3e-7 where theirs err by 1.1e-7 to 1.9e-4 (2-norm against 64 bits, 2129 calls of 1e7 to 1e10 FLOPs; 0.55 of theirs at most).
 // Prepared or cached weights spare the other kernels a launch and do not count: against blocks prepared for them, 300 forwards that leave take 0.63
 // of the time and 199 deltaX 0.50; three of the 499 take 1.20 to 1.25 (20 x 7x7, 448 -> 416, 7x7 s2 deltaX 52 -> 66).
 
